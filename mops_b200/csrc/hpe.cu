@@ -25,6 +25,7 @@
 
 #include "checks.hpp"
 #include "device.cuh"
+#include "hpe_tmem.hpp"
 
 namespace mops_b200 {
 namespace {
@@ -730,6 +731,7 @@ const char* const kIndexNames[] = {"indices_A"};
 template <typename T>
 void run_forward(const Call& call, T* O, const T* A, const T* C, const int32_t* P, int64_t I,
                  int N, int64_t J, int K) {
+    if (J > 0 && hpe_forward_tmem<T>(call, O, A, C, P, I, N, J, K)) return;
     const size_t smem = fwd_smem<T, kMaxOrder>(N); // the largest any order needs
     if (smem <= static_cast<size_t>(max_optin_smem(call.device)) && N <= kMaxTileColumns) {
 #define CALL(KK) launch_fwd<T, KK>(call, O, A, C, P, I, N, J)
@@ -746,6 +748,7 @@ void run_forward(const Call& call, T* O, const T* A, const T* C, const int32_t* 
 template <typename T>
 void run_backward(const Call& call, T* gA, const T* gO, const T* A, const T* C, const int32_t* P,
                   int64_t I, int N, int64_t J, int K) {
+    if (J > 0 && hpe_backward_tmem<T>(call, gA, gO, A, C, P, I, N, J, K)) return;
     const size_t smem = vjp_smem<T, kMaxOrder>(N);
     if (smem <= static_cast<size_t>(max_optin_smem(call.device)) && N <= kMaxTileColumns) {
 #define CALL(KK) launch_vjp<T, KK>(call, gA, gO, A, C, P, I, N, J)

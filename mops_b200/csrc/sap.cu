@@ -27,6 +27,7 @@
 
 #include "checks.hpp"
 #include "device.cuh"
+#include "sap_tmem.hpp"
 
 namespace mops_b200 {
 namespace {
@@ -930,6 +931,12 @@ void mops::cuda::sparse_accumulation_of_products(Tensor<scalar_t, 2> output, Ten
         end_call(call, op.c_str(), kIndexNames, 3);
         return;
     }
+    const SapProblem<scalar_t> problem{A.data, B.data, C.data, indices_A.data, indices_B.data,
+                                       indices_output.data, I, K, nA, nB, nO};
+    if (sap_forward_tmem<scalar_t>(call, problem, output.data)) {
+        end_call(call, op.c_str(), kIndexNames, 3);
+        return;
+    }
     if (forward_small<scalar_t>(call, output.data, A.data, B.data, C.data, indices_A.data,
                                 indices_B.data, indices_output.data, I, K, nA, nB, nO)) {
         end_call(call, op.c_str(), kIndexNames, 3);
@@ -982,6 +989,12 @@ void mops::cuda::sparse_accumulation_of_products_vjp(
             MOPS_CUDA_OK(cudaMemsetAsync(grad_A.data, 0, I * nA * sizeof(scalar_t), call.stream));
         if (grad_B.data != nullptr && nB > 0)
             MOPS_CUDA_OK(cudaMemsetAsync(grad_B.data, 0, I * nB * sizeof(scalar_t), call.stream));
+        end_call(call, op.c_str(), kIndexNames, 3);
+        return;
+    }
+    const SapProblem<scalar_t> problem{A.data, B.data, C.data, indices_A.data, indices_B.data,
+                                       indices_output.data, I, K, nA, nB, nO};
+    if (sap_backward_tmem<scalar_t>(call, problem, grad_A.data, grad_B.data, grad_output.data)) {
         end_call(call, op.c_str(), kIndexNames, 3);
         return;
     }
@@ -1047,6 +1060,13 @@ void mops::cuda::sparse_accumulation_of_products_vjp_vjp(
             MOPS_CUDA_OK(cudaMemsetAsync(grad_A_2.data, 0, I * nA * sizeof(scalar_t), call.stream));
         if (grad_B_2.data != nullptr && nB > 0)
             MOPS_CUDA_OK(cudaMemsetAsync(grad_B_2.data, 0, I * nB * sizeof(scalar_t), call.stream));
+        end_call(call, op.c_str(), kIndexNames, 3);
+        return;
+    }
+    const SapProblem<scalar_t> problem{A.data, B.data, C.data, indices_A.data, indices_B.data,
+                                       indices_output.data, I, K, nA, nB, nO};
+    if (sap_second_tmem<scalar_t>(call, problem, grad_grad_output.data, grad_A_2.data, grad_B_2.data,
+                                  grad_grad_A.data, grad_grad_B.data, grad_output.data)) {
         end_call(call, op.c_str(), kIndexNames, 3);
         return;
     }

@@ -1,0 +1,39 @@
+"""The tensor-memory kernels of HPE and SAP at the edges of their tiles (128 rows per slot), of their
+dispatch (rows per lane, blocks per tile, widths that still fit) and of their record tables (columns
+without records, one column, many), against the CPU oracle at the parity tolerances."""
+import numpy as np
+import pytest
+
+from mops_b200 import workloads
+from test_parity_gpu import compare
+
+pytestmark = pytest.mark.gpu
+DTYPES = [np.float64, np.float32]
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("kw", [
+    dict(I=1, N=1, J=1, K=1), dict(I=127, N=3, J=1, K=2), dict(I=129, N=16, J=513, K=4),
+    dict(I=1000, N=101, J=700, K=3),       # odd width: rows end inside a sector
+    dict(I=300, N=127, J=300, K=4), dict(I=300, N=128, J=300, K=2), dict(I=257, N=203, J=300, K=5),
+    dict(I=148 * 128 + 77, N=7, J=90, K=4), dict(I=40000, N=33, J=200, K=3),
+    dict(I=515, N=60, J=150, K=10),
+])
+def test_hpe(oracle, kw, dtype):
+    compare("hpe", workloads.hpe(**kw), dtype, oracle, what=f"hpe {kw}")
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("kw", [
+    dict(I=1, nA=1, nB=1, nO=1, K=3), dict(I=129, nA=20, nB=6, nO=50, K=900),
+    dict(I=1000, nA=5, nB=16, nO=33, K=60),   # most cells and several columns receive nothing
+    dict(I=148 * 256 + 31, nA=20, nB=6, nO=50, K=1000), dict(I=148 * 128 + 129, nA=3, nB=9, nO=7, K=300),
+    dict(I=20000, nA=32, nB=16, nO=99, K=2000), dict(I=19001, nA=16, nB=17, nO=15, K=700),
+])
+def test_sap(oracle, kw, dtype):
+    d = workloads.sap(**kw)
+    r = np.random.default_rng(5)
+    d["indices_output"] = r.permutation(d["indices_output"])
+    d["grad_grad_A"] = r.standard_normal(d["A"].shape)
+    d["grad_grad_B"] = r.standard_normal(d["B"].shape)
+    compare("sap", d, dtype, oracle, second_order=True, what=f"sap {kw}")
