@@ -32,41 +32,13 @@
 #include "bulk.cuh"
 #include "checks.hpp"
 #include "device.cuh"
+#include "unsorted.cuh"
 
 namespace mops_b200 {
 namespace {
 
 constexpr int kFwdWarps = 8;
 constexpr int kMaxTK = 8;
-
-template <typename T, int N> struct VecOf;
-template <> struct VecOf<float, 1> { using type = float; };
-template <> struct VecOf<float, 2> { using type = float2; };
-template <> struct VecOf<float, 4> { using type = float4; };
-template <> struct VecOf<double, 1> { using type = double; };
-template <> struct VecOf<double, 2> { using type = double2; };
-
-template <typename T, int N> __device__ __forceinline__ void load_vec(const T* p, T (&out)[N]) {
-    using V = typename VecOf<T, N>::type;
-    union {
-        V v;
-        T s[N];
-    } u;
-    u.v = *reinterpret_cast<const V*>(p);
-#pragma unroll
-    for (int i = 0; i < N; i++) out[i] = u.s[i];
-}
-
-template <typename T, int N> __device__ __forceinline__ void store_vec(T* p, const T (&in)[N]) {
-    using V = typename VecOf<T, N>::type;
-    union {
-        V v;
-        T s[N];
-    } u;
-#pragma unroll
-    for (int i = 0; i < N; i++) u.s[i] = in[i];
-    *reinterpret_cast<V*>(p) = u.v;
-}
 
 #include "opsa_pipe.cuh"
 
@@ -799,7 +771,9 @@ void forward(const Call& call, T* O, const T* A, const T* B, const T* W, const i
             wait_stream(call);
             need_fallback = host_saw_unsorted(call);
         }
-        if (need_fallback) {
+        if (need_fallback && J <= INT32_MAX) {
+            launch_fwd_unsorted<T, WEIGHTED>(call, O, A, B, W, PW, P, J, K, L, nO);
+        } else if (need_fallback) {
             zero_if_unsorted<T><<<grid_generic, 256, 0, call.stream>>>(O, nO * KL, call.status);
             opsa_fwd_atomic<T, WEIGHTED><<<grid_generic, 256, 0, call.stream>>>(
                 O, A, B, W, PW, P, J, K, L, nO, false, call.status);
@@ -820,6 +794,7 @@ struct VjpPlan {
     int threads;
     size_t smem;
     bool only_if_unsorted; // run only when the segmented kernel of the same call stood down
+    const int32_t* perm;   // order to take the entries in (nullptr: as they are)
 };
 
 template <typename T, int KP, int VL, bool WEIGHTED>
@@ -838,9 +813,19 @@ opsa_vjp_entries(T* __restrict__ gA, T* __restrict__ gB, T* __restrict__ gW,
     T* Ws = Bs + static_cast<size_t>(EPB) * Lp;          // [EPB][Lp]  W rows, then gW terms
     T* Ss = WEIGHTED ? Ws + static_cast<size_t>(EPB) * Lp : Ws; // [EPB][Lp] S, only if nkc > 1
 
-    const int64_t base = static_cast<int64_t>(blockIdx.x) * EPB;
-    const int n = static_cast<int>(J - base < EPB ? J - base : EPB);
     int32_t* pws = reinterpret_cast<int32_t*>(Ss + (nkc > 1 ? static_cast<size_t>(EPB) * Lp : 0));
+    int32_t* order = pws + EPB; // [EPB] the tile's entries, where they come from a permutation
+
+    for (int64_t base = static_cast<int64_t>(blockIdx.x) * EPB; base < J;
+         base += static_cast<int64_t>(gridDim.x) * EPB) {
+    const int n = static_cast<int>(J - base < EPB ? J - base : EPB);
+    if (plan.perm != nullptr) {
+        if (tid < n) order[tid] = plan.perm[base + tid];
+        __syncthreads();
+    }
+    auto entry = [&](int jj) {
+        return plan.perm != nullptr ? static_cast<int64_t>(order[jj]) : base + jj;
+    };
 
     // Stage the entries' rows: element idx of the contiguous slice -> (entry, column), tracked
     // incrementally (no division per element), copied asynchronously so that all of a
@@ -848,9 +833,8 @@ opsa_vjp_entries(T* __restrict__ gA, T* __restrict__ gB, T* __restrict__ gW,
     {
         const int dj = EPB / K, dk = EPB - dj * K;
         int jj = tid / K, k = tid - jj * K;
-        const T* src = A + base * K;
         for (int idx = tid; idx < n * K; idx += EPB) {
-            cp_async<sizeof(T)>(As + jj * Kp + k, src + idx);
+            cp_async<sizeof(T)>(As + jj * Kp + k, A + entry(jj) * K + k);
             jj += dj;
             k += dk;
             if (k >= K) {
@@ -862,9 +846,8 @@ opsa_vjp_entries(T* __restrict__ gA, T* __restrict__ gB, T* __restrict__ gW,
     {
         const int dj = EPB / L, dl = EPB - dj * L;
         int jj = tid / L, l = tid - jj * L;
-        const T* src = B + base * L;
         for (int idx = tid; idx < n * L; idx += EPB) {
-            cp_async<sizeof(T)>(Bs + jj * Lp + l, src + idx);
+            cp_async<sizeof(T)>(Bs + jj * Lp + l, B + entry(jj) * L + l);
             jj += dj;
             l += dl;
             if (l >= L) {
@@ -875,7 +858,7 @@ opsa_vjp_entries(T* __restrict__ gA, T* __restrict__ gB, T* __restrict__ gW,
     }
     if (WEIGHTED) {
         if (tid < n) {
-            int32_t pw = __ldg(PW + base + tid);
+            int32_t pw = __ldg(PW + entry(tid));
             if (clamp_index(pw, static_cast<int32_t>(nO))) report_bad_index(st, 1);
             pws[tid] = pw;
         }
@@ -897,7 +880,7 @@ opsa_vjp_entries(T* __restrict__ gA, T* __restrict__ gB, T* __restrict__ gW,
     __syncthreads();
 
     if (tid < n) {
-        int32_t row = __ldg(P + base + tid);
+        int32_t row = __ldg(P + entry(tid));
         if (clamp_index(row, static_cast<int32_t>(nO))) report_bad_index(st, 0);
         const T* g = gO + static_cast<int64_t>(row) * K * L;
         T* a_row = As + tid * Kp;
@@ -984,9 +967,8 @@ opsa_vjp_entries(T* __restrict__ gA, T* __restrict__ gB, T* __restrict__ gW,
     if (gA != nullptr) {
         const int dj = EPB / K, dk = EPB - dj * K;
         int jj = tid / K, k = tid - jj * K;
-        T* dst = gA + base * K;
         for (int idx = tid; idx < n * K; idx += EPB) {
-            dst[idx] = As[jj * Kp + k];
+            gA[entry(jj) * K + k] = As[jj * Kp + k];
             jj += dj;
             k += dk;
             if (k >= K) {
@@ -999,7 +981,7 @@ opsa_vjp_entries(T* __restrict__ gA, T* __restrict__ gB, T* __restrict__ gW,
         const int dj = EPB / L, dl = EPB - dj * L;
         int jj = tid / L, l = tid - jj * L;
         for (int idx = tid; idx < n * L; idx += EPB) {
-            if (gB != nullptr) gB[base * L + idx] = Bs[jj * Lp + l];
+            if (gB != nullptr) gB[entry(jj) * L + l] = Bs[jj * Lp + l];
             if (WEIGHTED && gW != nullptr)
                 red_add(gW + static_cast<int64_t>(pws[jj]) * L + l, Ws[jj * Lp + l]);
             jj += dj;
@@ -1009,6 +991,8 @@ opsa_vjp_entries(T* __restrict__ gA, T* __restrict__ gB, T* __restrict__ gW,
                 jj++;
             }
         }
+    }
+    __syncthreads(); // the next tile overwrites the rows
     }
 }
 
@@ -1258,7 +1242,10 @@ void launch_vjp_tile(const Call& call, const VjpPlan& plan, int64_t J, Args... a
         MOPS_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           static_cast<int>(plan.smem)));
     }
-    const int64_t blocks = ceil_div(J, plan.threads);
+    // Behind the sorted kernels it mostly has nothing to do: no more blocks than the SMs hold (one
+    // block per 128 entries took 136 us to find out, at 2^24 entries).
+    int64_t blocks = ceil_div(J, plan.threads);
+    if (plan.only_if_unsorted) blocks = std::min<int64_t>(blocks, static_cast<int64_t>(sm_count(call.device)) * 4);
     kernel<<<static_cast<unsigned>(blocks), plan.threads, plan.smem, call.stream>>>(args..., plan,
                                                                                    call.status);
 }
@@ -1336,6 +1323,16 @@ void backward(const Call& call, T* gA, T* gB, T* gW, const T* gO, const T* A, co
             plan.only_if_unsorted = true; // asynchronous calls cannot look: always enqueue
         }
     }
+    // An index that is not sorted: take the entries in the order of their rows.
+    plan.perm = nullptr;
+    void* scratch = nullptr;
+    if (plan.only_if_unsorted && J <= INT32_MAX) {
+        const int blocks = sort_blocks(call, J);
+        scratch = scratch_alloc(call, entry_sort_bytes(J, nO, blocks));
+        const EntrySort sort = entry_sort_at(scratch, nO, blocks);
+        launch_sorting(call, blocks, sort_if_unsorted_grid, sort_if_unsorted_block, sort, P, J, nO, call.status);
+        plan.perm = sort.perm;
+    }
     const int KP = vjp_tile_k(K);
     plan.nkc = static_cast<int>(ceil_div(K, KP));
     plan.Kp = K | 1;
@@ -1344,7 +1341,7 @@ void backward(const Call& call, T* gA, T* gB, T* gW, const T* gO, const T* A, co
     const size_t per_entry = (plan.Kp + static_cast<size_t>(tiles_l) * plan.Lp) * sizeof(T);
     plan.threads = 128;
     while (plan.threads > 32 && plan.threads * per_entry > 96 * 1024) plan.threads /= 2;
-    plan.smem = plan.threads * (per_entry + sizeof(int32_t));
+    plan.smem = plan.threads * (per_entry + 2 * sizeof(int32_t));
 
     const int widest = 16 / static_cast<int>(sizeof(T));
     int VL = 1;
@@ -1379,6 +1376,7 @@ void backward(const Call& call, T* gA, T* gB, T* gW, const T* gO, const T* A, co
             gA, gB, gW, gO, A, B, W, PW, P, J, K, L, nO, plan.only_if_unsorted, call.status);
     }
     MOPS_CUDA_OK(cudaGetLastError());
+    scratch_free(call, scratch);
 }
 
 const char* const kOpsaIndexNames[] = {"indices_output"};

@@ -1,0 +1,23 @@
+"""Scatter operations on unsorted indices: one-block and whole-GPU sorts (the line lies at 512
+entries), widths on both sides of a 32-lane row and an 8-row part, rows without entries, one row that
+receives everything, against the CPU oracle at the parity tolerances."""
+import numpy as np
+import pytest
+
+from mops_b200 import workloads
+from test_parity_gpu import compare
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("E,n,K,L", [(2, 2, 1, 1), (511, 7, 4, 33), (513, 900, 5, 31), (4097, 1, 9, 32),
+                                     (20011, 157, 16, 32), (70001, 40000, 17, 20)])
+def test_outer_products(oracle, E, n, K, L, dtype):
+    r = np.random.default_rng(E)
+    for op, d in (("opsa", workloads.opsa(J=E, K=K, L=L, nO=n)), ("opsaw", workloads.opsaw(E=E, K=K, L=L, n=n))):
+        po = r.permutation(d["indices_output"])
+        if E > 1000:
+            po[::3] = n // 2
+        d["indices_output"] = po.astype(np.int32)
+        compare(op, d, dtype, oracle, what=f"{op} unsorted {E} {n} {K}x{L}")
