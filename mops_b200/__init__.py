@@ -80,6 +80,24 @@ def _check_scalar(value, operation, name):
         raise TypeError(f"`{name}` must be a scalar in {operation}, got {type(value)}")
 
 
+# ------------------------------------------------------------------- calls on CUDA tensors
+# Operations as csrc/python_calls.cpp numbers them.
+_HPE, _HPE_VJP, _SAP, _SAP_VJP, _OPSA, _OPSA_VJP, _OPSAW, _OPSAW_VJP, _SASAW, _SASAW_VJP = range(10)
+
+
+def _native(operation, *args):
+    """The result of an operation on plain CUDA tensors, or NotImplemented (other arrays, arguments
+    that the general path has to convert or to refuse). Replaced by the native function once a
+    call has a torch tensor on a GPU."""
+    global _native
+    import sys
+    torch = sys.modules.get("torch")
+    if torch is None or not isinstance(args[0], torch.Tensor) or not args[0].is_cuda:
+        return NotImplemented
+    _native = _lib.native_calls(MopsError)
+    return _native(operation, *args)
+
+
 def sort_indices(indices, n_rows):
     """Stable sort of a scatter index on the GPU: returns ``(sorted, permutation)`` with
     ``sorted == indices[permutation]`` ascending and equal values in input order, as int32
@@ -359,6 +377,9 @@ def _opt(arena, x, ndim):
 
 # ------------------------------------------------------------------------------------- HPE
 def homogeneous_polynomial_evaluation(A, C, indices_A):
+    result = _native(_HPE, A, C, indices_A)
+    if result is not NotImplemented:
+        return result
     op = "homogeneous_polynomial_evaluation"
     _check(A, 2, "f", op, "A"); _check(C, 1, "f", op, "C"); _check(indices_A, 2, "i", op, "indices_A")
     m = _Arena(A)
@@ -369,6 +390,9 @@ def homogeneous_polynomial_evaluation(A, C, indices_A):
 
 
 def homogeneous_polynomial_evaluation_vjp(grad_output, A, C, indices_A, compute_grad_A=True):
+    result = _native(_HPE_VJP, grad_output, A, C, indices_A, compute_grad_A)
+    if result is not NotImplemented:
+        return result
     op = "homogeneous_polynomial_evaluation_vjp"
     _check(grad_output, 1, "f", op, "grad_output")
     _check(A, 2, "f", op, "A"); _check(C, 1, "f", op, "C"); _check(indices_A, 2, "i", op, "indices_A")
@@ -403,6 +427,9 @@ def _sap_common(op, A, B, C, indices_A, indices_B, indices_output):
 
 
 def sparse_accumulation_of_products(A, B, C, indices_A, indices_B, indices_output, output_size):
+    result = _native(_SAP, A, B, C, indices_A, indices_B, indices_output, output_size)
+    if result is not NotImplemented:
+        return result
     op = "sparse_accumulation_of_products"
     _sap_common(op, A, B, C, indices_A, indices_B, indices_output)
     _check_scalar(output_size, op, "output_size")
@@ -415,6 +442,10 @@ def sparse_accumulation_of_products(A, B, C, indices_A, indices_B, indices_outpu
 
 def sparse_accumulation_of_products_vjp(grad_output, A, B, C, indices_A, indices_B,
                                         indices_output, compute_grad_A=True, compute_grad_B=True):
+    result = _native(_SAP_VJP, grad_output, A, B, C, indices_A, indices_B, indices_output,
+                     compute_grad_A, compute_grad_B)
+    if result is not NotImplemented:
+        return result
     op = "sparse_accumulation_of_products_vjp"
     _check(grad_output, 2, "f", op, "grad_output")
     _sap_common(op, A, B, C, indices_A, indices_B, indices_output)
@@ -448,6 +479,9 @@ def sparse_accumulation_of_products_vjp_vjp(grad_grad_A, grad_grad_B, grad_outpu
 
 # ------------------------------------------------------------------------------------ OPSA
 def outer_product_scatter_add(A, B, indices_output, output_size):
+    result = _native(_OPSA, A, B, indices_output, output_size)
+    if result is not NotImplemented:
+        return result
     op = "outer_product_scatter_add"
     _check(A, 2, "f", op, "A"); _check(B, 2, "f", op, "B")
     _check(indices_output, 1, "i", op, "indices_output")
@@ -461,6 +495,9 @@ def outer_product_scatter_add(A, B, indices_output, output_size):
 
 def outer_product_scatter_add_vjp(grad_output, A, B, indices_output, compute_grad_A=True,
                                   compute_grad_B=True):
+    result = _native(_OPSA_VJP, grad_output, A, B, indices_output, compute_grad_A, compute_grad_B)
+    if result is not NotImplemented:
+        return result
     op = "outer_product_scatter_add_vjp"
     _check(grad_output, 3, "f", op, "grad_output")
     _check(A, 2, "f", op, "A"); _check(B, 2, "f", op, "B")
@@ -494,6 +531,9 @@ def outer_product_scatter_add_vjp_vjp(grad_grad_A, grad_grad_B, grad_output, A, 
 
 # ----------------------------------------------------------------------------------- OPSAW
 def outer_product_scatter_add_with_weights(A, B, W, indices_W, indices_output):
+    result = _native(_OPSAW, A, B, W, indices_W, indices_output)
+    if result is not NotImplemented:
+        return result
     op = "outer_product_scatter_add_with_weights"
     _check(A, 2, "f", op, "A"); _check(B, 2, "f", op, "B"); _check(W, 2, "f", op, "W")
     _check(indices_W, 1, "i", op, "indices_W"); _check(indices_output, 1, "i", op, "indices_output")
@@ -507,6 +547,10 @@ def outer_product_scatter_add_with_weights(A, B, W, indices_W, indices_output):
 def outer_product_scatter_add_with_weights_vjp(grad_output, A, B, W, indices_W, indices_output,
                                                compute_grad_A=True, compute_grad_B=True,
                                                compute_grad_W=True):
+    result = _native(_OPSAW_VJP, grad_output, A, B, W, indices_W, indices_output,
+                     compute_grad_A, compute_grad_B, compute_grad_W)
+    if result is not NotImplemented:
+        return result
     op = "outer_product_scatter_add_with_weights_vjp"
     _check(grad_output, 3, "f", op, "grad_output")
     _check(A, 2, "f", op, "A"); _check(B, 2, "f", op, "B"); _check(W, 2, "f", op, "W")
@@ -548,6 +592,10 @@ def _sasaw_common(op, A, B, C, W, indices_A, indices_W_1, indices_W_2, indices_o
 
 def sparse_accumulation_scatter_add_with_weights(A, B, C, W, indices_A, indices_W_1, indices_W_2,
                                                  indices_output_1, indices_output_2, output_size):
+    result = _native(_SASAW, A, B, C, W, indices_A, indices_W_1, indices_W_2,
+                     indices_output_1, indices_output_2, output_size)
+    if result is not NotImplemented:
+        return result
     op = "sparse_accumulation_scatter_add_with_weights"
     _sasaw_common(op, A, B, C, W, indices_A, indices_W_1, indices_W_2, indices_output_1,
                   indices_output_2)
@@ -564,6 +612,11 @@ def sparse_accumulation_scatter_add_with_weights_vjp(grad_output, A, B, C, W, in
                                                      indices_W_1, indices_W_2, indices_output_1,
                                                      indices_output_2, compute_grad_A=True,
                                                      compute_grad_B=True, compute_grad_W=True):
+    result = _native(_SASAW_VJP, grad_output, A, B, C, W, indices_A, indices_W_1,
+                     indices_W_2, indices_output_1, indices_output_2,
+                     compute_grad_A, compute_grad_B, compute_grad_W)
+    if result is not NotImplemented:
+        return result
     op = "sparse_accumulation_scatter_add_with_weights_vjp"
     _check(grad_output, 3, "f", op, "grad_output")
     _sasaw_common(op, A, B, C, W, indices_A, indices_W_1, indices_W_2, indices_output_1,

@@ -73,6 +73,21 @@ def library():
     return _LIB
 
 
+def native_calls(error):
+    """The function ``call`` of ``_calls.so``, which raises ``error`` for a failed call."""
+    import importlib.machinery
+    import importlib.util
+    library()  # the same library, already loaded
+    path = os.path.join(_HERE, "lib", "_calls.so")
+    if not os.path.isfile(path):
+        raise ImportError(f"{path} not found: build it with `python -m mops_b200.build`")
+    loader = importlib.machinery.ExtensionFileLoader("mops_b200._calls", path)
+    module = importlib.util.module_from_spec(importlib.util.spec_from_loader(loader.name, loader))
+    loader.exec_module(module)
+    module.setup(error)
+    return module.call
+
+
 def last_kernels():
     """Main kernels (with template arguments) of this thread's last call, as a list."""
     text = library().mops_b200_last_kernels().decode("utf8")

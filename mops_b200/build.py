@@ -2,6 +2,7 @@
 
     mops_b200/lib/libmops.so        the sm_100a kernels + C++ API + C ABI (no torch dependency)
     mops_b200/lib/libmops_torch.so  TORCH_LIBRARY(mops) autograd ops on top of it
+    mops_b200/lib/_calls.so         the Python front end's calls on CUDA tensors
 
     python -m mops_b200.build [--force] [--no-torch]
 
@@ -78,27 +79,33 @@ def build_core(force=False, verbose=False):
 
 
 def build_torch(force=False):
+    """The two libraries that need torch: the operators and the Python module."""
+    import sysconfig
+
     import torch
     from torch.utils import cpp_extension
 
     core = build_core()
-    src = os.path.join(CSRC, "torch_ops.cpp")
-    if not os.path.exists(src):
-        return None
-    lib = os.path.join(LIB, "libmops_torch.so")
-    if not (force or _newer(lib, [src, core] + _headers())):
-        return lib
     inc = []
     for p in cpp_extension.include_paths(device_type="cuda"):
         inc += ["-isystem", p]
+    inc += ["-isystem", sysconfig.get_paths()["include"]]
     torch_lib = os.path.join(os.path.dirname(torch.__file__), "lib")
     abi = int(torch._C._GLIBCXX_USE_CXX11_ABI)
-    cmd = [HOST_CXX, "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={abi}",
-           "-I", CSRC, "-I", INCLUDE] + inc + [src, "-o", lib, "-L", LIB, "-lmops",
-           "-L", torch_lib, "-ltorch", "-ltorch_cpu", "-lc10", "-ltorch_cuda", "-lc10_cuda",
-           "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{torch_lib}"]
-    _run(cmd)
-    return lib
+    jobs, libs = [], []
+    for name, source, more in (("libmops_torch.so", "torch_ops.cpp", []),
+                               ("_calls.so", "python_calls.cpp", ["-ltorch_python"])):
+        src, lib = os.path.join(CSRC, source), os.path.join(LIB, name)
+        libs.append(lib)
+        if force or _newer(lib, [src, core] + _headers()):
+            jobs.append([HOST_CXX, "-O2", "-std=c++17", "-fPIC", "-shared",
+                         f"-D_GLIBCXX_USE_CXX11_ABI={abi}", "-I", CSRC, "-I", INCLUDE] + inc +
+                        [src, "-o", lib, "-L", LIB, "-lmops", "-L", torch_lib, "-ltorch",
+                         "-ltorch_cpu", "-lc10", "-ltorch_cuda", "-lc10_cuda"] + more +
+                        ["-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{torch_lib}"])
+    with cf.ThreadPoolExecutor(max_workers=2) as ex:
+        list(ex.map(_run, jobs))
+    return libs[0]
 
 
 def main():

@@ -621,8 +621,7 @@ template <typename Kernel, typename... Args>
 void launch_gather(const Call& call, Kernel kernel, const GatherShape& s, int cluster, Args... args) {
     // More than half of an SM's shared memory: one block per SM, which owns all of its TMEM.
     const size_t smem = std::max<size_t>(s.smem, 117 * 1024);
-    MOPS_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(smem)));
+    allow_dynamic_smem(kernel, call.device, smem);
     const int64_t at_once = std::max<int64_t>(1, sm_count(call.device) / s.parts);
     cudaLaunchConfig_t config{};
     config.gridDim = dim3(static_cast<unsigned>(std::min(s.tiles, at_once) * s.parts));
@@ -663,8 +662,7 @@ bool run_gather(const Call& call, TableKey key, const Source& source, int64_t M,
     int32_t* n_start = reinterpret_cast<int32_t*>(records + b_rec);
     if (ref.fresh) {
         auto build = gather_table<T, NF, Source>;
-        MOPS_CUDA_OK(cudaFuncSetAttribute(build, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          static_cast<int>(builder)));
+        allow_dynamic_smem(build, call.device, builder);
         build<<<1, kTableThreads, builder, call.stream>>>(records, n_start, source, static_cast<int>(M), N,
                                                           s.w, batch, 1, op.total, call.status);
         MOPS_CUDA_OK(cudaGetLastError());

@@ -640,16 +640,12 @@ void launch_fwd(const Call& call, T* O, const T* A, const T* C, const int32_t* P
     note_kernel_f("hpe_fwd_rows<%s,K=%d,R=%d>", scalar_name<T>(), K, two ? 2 : 1);
     if (two) {
         auto kernel = hpe_fwd_rows<T, K, 2>;
-        if (smem > 48 * 1024)
-            MOPS_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              static_cast<int>(smem)));
+        allow_dynamic_smem(kernel, call.device, smem);
         kernel<<<static_cast<unsigned>(ceil_div(I, 64)), kWarps * 32, smem, call.stream>>>(
             O, A, plan.fwd_rec, I, N, static_cast<int>(J));
     } else {
         auto kernel = hpe_fwd_rows<T, K, 1>;
-        if (smem > 48 * 1024)
-            MOPS_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              static_cast<int>(smem)));
+        allow_dynamic_smem(kernel, call.device, smem);
         kernel<<<static_cast<unsigned>(ceil_div(I, kRows)), kWarps * 32, smem, call.stream>>>(
             O, A, plan.fwd_rec, I, N, static_cast<int>(J));
     }
@@ -692,9 +688,7 @@ void launch_vjp(const Call& call, T* gA, const T* gO, const T* A, const T* C, co
     TableRef scratch{};
     HpePlan plan = make_plan<T>(call, &scratch, C, P, J, K, N, false, true, 32 * rpl + 1);
     auto launch = [&](auto kernel) {
-        if (smem > 48 * 1024)
-            MOPS_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              static_cast<int>(smem)));
+        allow_dynamic_smem(kernel, call.device, smem);
         kernel<<<static_cast<unsigned>(ceil_div(I, 32 * rpl)), kWarps * 32, smem, call.stream>>>(
             gA, gO, A, plan, I, N);
     };

@@ -338,10 +338,7 @@ void launch_fwd_tile(const Call& call, const FwdPlan& plan, T* O, const T* A, co
     note_kernel_f("opsa_fwd_rows<%s,TK=%d,NV=%d,VEC=%d,W=%d>", scalar_name<T>(), TK, NV, VEC,
                   WEIGHTED ? 1 : 0);
     const size_t smem = plan.smem_per_warp * kFwdWarps;
-    if (smem > 48 * 1024) {
-        MOPS_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          static_cast<int>(smem)));
-    }
+    allow_dynamic_smem(kernel, call.device, smem);
     const int64_t blocks = ceil_div(nO, kFwdWarps);
     kernel<<<static_cast<unsigned>(blocks), kFwdWarps * 32, smem, call.stream>>>(
         O, A, B, W, PW, offsets, K, L, nO, plan, call.status);
@@ -474,17 +471,9 @@ void launch_fwd_mma_l(int L, unsigned blocks, cudaStream_t stream, Args... args)
 }
 
 // ------------------------------------------------------------- streaming kernels, host side
-// Tuning overrides (development aid): MOPS_B200_PIPE=0 turns the streaming kernels off,
-// MOPS_B200_PIPE_CH / MOPS_B200_PIPE_STAGES change the ring geometry.
-inline int env_int(const char* name, int fallback) {
-    const char* v = std::getenv(name);
-    return v != nullptr && *v != '\0' ? std::atoi(v) : fallback;
-}
-
 template <typename T, bool WEIGHTED>
 bool pipe_usable(const T* A, const T* B, const T* W, const void* extra, int K, int L, bool vjp) {
     auto aligned = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
-    if (env_int("MOPS_B200_PIPE", 1) == 0) return false;
     if (K < 1 || K > 16 || L < 1 || L > 32) return false;
     if (!aligned(A) || !aligned(B) || !aligned(extra)) return false;
     if (WEIGHTED && (!aligned(W) || (L * sizeof(T)) % 16 != 0)) return false;
@@ -505,22 +494,13 @@ template <typename T, bool WEIGHTED> PipeLayout choose_pipe_layout(int K, int L,
     // holds the padded B and W rows (680 bytes per entry), so chunks of 8 keep the warp count
     // up (forward 0.49 ms, VJP 1.00 ms against 0.54 / 1.02 with 16; four stages of 4 or 8:
     // 0.54 / 1.49 and 0.74 / 1.23). The stage count is rounded to a power of two.
-    int ch = env_int("MOPS_B200_PIPE_CH", WEIGHTED ? 8 : sizeof(T) == 4 ? 64 : 32);
-    int stages = env_int("MOPS_B200_PIPE_STAGES", 2);
-    ch = std::max(4, std::min(WEIGHTED ? 32 : 128, ch / 4 * 4)); // weighted: one lane per entry
-    stages = std::max(2, std::min(8, stages));
-    return pipe_layout(sizeof(T), K, L, WEIGHTED, vjp, ch, stages);
+    return pipe_layout(sizeof(T), K, L, WEIGHTED, vjp, WEIGHTED ? 8 : sizeof(T) == 4 ? 64 : 32, 2);
 }
 
 // Grid of a VJP streaming kernel, whose warps split the entries: at most one warp per chunk.
 template <typename Kernel>
 unsigned pipe_grid_entries(const Call& call, Kernel kernel, size_t smem, int64_t J, int ch) {
-    if (smem > 48 * 1024)
-        MOPS_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          static_cast<int>(smem)));
-    int per_sm = 0;
-    MOPS_CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kPipeWarps * 32, smem));
-    per_sm = std::max(1, per_sm);
+    const int per_sm = resident_blocks(kernel, call.device, kPipeWarps * 32, smem);
     return static_cast<unsigned>(std::max<int64_t>(
         1, std::min<int64_t>(ceil_div(J, static_cast<int64_t>(kPipeWarps) * ch),
                              static_cast<int64_t>(sm_count(call.device)) * per_sm)));
@@ -528,12 +508,7 @@ unsigned pipe_grid_entries(const Call& call, Kernel kernel, size_t smem, int64_t
 
 template <typename Kernel>
 unsigned pipe_grid(const Call& call, Kernel kernel, size_t smem, int64_t nO) {
-    if (smem > 48 * 1024)
-        MOPS_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          static_cast<int>(smem)));
-    int per_sm = 0;
-    MOPS_CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kPipeWarps * 32, smem));
-    per_sm = std::max(1, per_sm);
+    const int per_sm = resident_blocks(kernel, call.device, kPipeWarps * 32, smem);
     return static_cast<unsigned>(std::min<int64_t>(
         ceil_div(nO, kPipeWarps), static_cast<int64_t>(sm_count(call.device)) * per_sm));
 }
@@ -566,9 +541,8 @@ bool forward_pipe(const Call& call, T* O, const T* A, const T* B, const T* W, co
     if (static_cast<size_t>(lay.warp_bytes) * kPipeWarps > static_cast<size_t>(max_optin_smem(call.device)))
         return false;
     if constexpr (std::is_same<T, float>::value && !WEIGHTED) {
-        // f32 without weights: the TF32 tensor path (MOPS_B200_TF32=0: development switch back
-        // to the FP64 MMA route)
-        if (env_int("MOPS_B200_TF32", 1) != 0) {
+        // f32 without weights: the TF32 tensor path
+        {
             const size_t smem = static_cast<size_t>(lay.warp_bytes) * kPipeWarps;
             note_kernel_f("opsa_fwd_pipe_tf32<NT=%d> ch=%d stages=%d", (L + 7) / 8, lay.ch,
                           lay.stages);
@@ -591,10 +565,8 @@ bool forward_pipe(const Call& call, T* O, const T* A, const T* B, const T* W, co
         }
     }
     if constexpr (WEIGHTED) {
-        // common shapes with K and L fixed at compile time (MOPS_B200_FIXED=0: development
-        // switch back to the run-time widths)
-        if (fixed_shape(K, L) && lay.ch == kFixedChunk<true> && lay.stages == 2 &&
-            env_int("MOPS_B200_FIXED", 1) != 0) {
+        // common shapes with K and L fixed at compile time
+        if (fixed_shape(K, L) && lay.ch == kFixedChunk<true> && lay.stages == 2) {
             const size_t smem = static_cast<size_t>(lay.warp_bytes) * kPipeWarps;
             note_kernel_f("opsa_fwd_pipe<%s,W=1,K=%d,L=%d> ch=%d stages=2", scalar_name<T>(), K, L, lay.ch);
 #define MOPS_B200_CASE(K_)                                                                         \
@@ -650,7 +622,7 @@ bool backward_pipe(const Call& call, T* gA, T* gB, T* gW, const T* gO, const T* 
     if (static_cast<size_t>(lay.warp_bytes) * kPipeWarps > static_cast<size_t>(max_optin_smem(call.device)))
         return false;
     if constexpr (std::is_same<T, float>::value && !WEIGHTED) {
-        if (env_int("MOPS_B200_TF32", 1) != 0) {
+        {
             const size_t smem = static_cast<size_t>(lay.warp_bytes) * kPipeWarps;
             note_kernel_f("opsa_vjp_pipe_tf32<KS=%d,LS=%d> ch=%d stages=%d", (K + 7) / 8,
                           (L + 7) / 8, lay.ch, lay.stages);
@@ -677,8 +649,7 @@ bool backward_pipe(const Call& call, T* gA, T* gB, T* gW, const T* gO, const T* 
         }
     }
     if constexpr (WEIGHTED) {
-        if (fixed_shape(K, L) && lay.ch == kFixedChunk<true> && lay.stages == 2 &&
-            env_int("MOPS_B200_FIXED", 1) != 0) {
+        if (fixed_shape(K, L) && lay.ch == kFixedChunk<true> && lay.stages == 2) {
             const PipeLayout& lay2 = lay;
             // Rows of 32 entries or more: one grad_output slot per warp instead of two (the
             // copy of the next row then has the whole current row to arrive), which is what
@@ -1238,10 +1209,7 @@ void launch_vjp_tile(const Call& call, const VjpPlan& plan, int64_t J, Args... a
     if (!plan.only_if_unsorted)
         note_kernel_f("opsa_vjp_entries<%s,KP=%d,VL=%d,W=%d>", scalar_name<T>(), KP, VL,
                       WEIGHTED ? 1 : 0);
-    if (plan.smem > 48 * 1024) {
-        MOPS_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          static_cast<int>(plan.smem)));
-    }
+    allow_dynamic_smem(kernel, call.device, plan.smem);
     // Behind the sorted kernels it mostly has nothing to do: no more blocks than the SMs hold (one
     // block per 128 entries took 136 us to find out, at 2^24 entries).
     int64_t blocks = ceil_div(J, plan.threads);

@@ -4,6 +4,7 @@
 #include <vector>
 #include <map>
 #include <mutex>
+#include <tuple>
 #include <unordered_map>
 #include <utility>
 
@@ -19,18 +20,38 @@ namespace mops_b200 {
         ":" + std::to_string(line));
 }
 
+// What a thread keeps for a (device, stream): calls on one stream run in order, so a call's status
+// words and workspace cannot be overwritten before its own kernels are done with them, and calls on
+// different streams (which may overlap) never share them. The status block is a few bytes and lives
+// until the process exits.
+struct StreamState {
+    Status status{};
+    unsigned char* workspace = nullptr;
+    size_t size = 0, used = 0;
+    size_t wanted = 0; // by the previous call
+};
+
 namespace {
+
+constexpr size_t kMostWorkspace = 4 << 20; // bytes per (thread, device, stream)
+constexpr int kMostWorkspaces = 16;        // per thread
 
 struct ThreadState {
     cudaStream_t stream = nullptr;
     bool wait = true;
     uint32_t epoch = 0;
-    // One status block per (device, stream) this thread has used: calls on one stream run in
-    // order, so a call's words cannot be overwritten before its own kernels have read them,
-    // and calls on different streams (which may overlap) never share a block. The blocks are
-    // a few bytes and live until the process exits.
-    std::map<std::pair<int, cudaStream_t>, Status> blocks;
+    // by device and stream id: a handle may come back for another stream, an id does not
+    std::map<std::pair<int, unsigned long long>, StreamState> streams;
+    std::pair<int, unsigned long long> last_key{-1, 0};
+    StreamState* last = nullptr; // of the previous call
+    int workspaces = 0;
     std::string kernels; // main kernels dispatched by the current / last call
+
+    // The thread is gone, so are its calls; cudaFree waits for what may still run.
+    ~ThreadState() {
+        for (auto& s : streams)
+            if (s.second.workspace != nullptr) (void)cudaFree(s.second.workspace);
+    }
 };
 
 thread_local ThreadState g_thread;
@@ -72,24 +93,30 @@ Call begin_call() {
     call.wait = g_thread.wait;
 
     g_thread.kernels.clear();
-    const auto key = std::make_pair(call.device, call.stream);
-    auto it = g_thread.blocks.find(key);
-    if (it == g_thread.blocks.end()) {
-        Status block{};
-        void* host = nullptr;
-        MOPS_CUDA_OK(cudaHostAlloc(&host, kStatusWords * sizeof(uint32_t),
-                                   cudaHostAllocMapped | cudaHostAllocPortable));
-        for (int i = 0; i < kStatusWords; i++) static_cast<volatile uint32_t*>(host)[i] = 0;
-        void* host_dev = nullptr;
-        MOPS_CUDA_OK(cudaHostGetDevicePointer(&host_dev, host, 0));
-        (void)host_dev; // with unified addressing the host pointer is the device-visible one
-        block.host = static_cast<uint32_t*>(host);
-        MOPS_CUDA_OK(cudaMalloc(reinterpret_cast<void**>(&block.dev),
-                                kStatusWords * sizeof(uint32_t)));
-        MOPS_CUDA_OK(cudaMemset(block.dev, 0, kStatusWords * sizeof(uint32_t)));
-        it = g_thread.blocks.emplace(key, block).first;
+    unsigned long long id = 0;
+    MOPS_CUDA_OK(cudaStreamGetId(call.stream, &id));
+    const auto key = std::make_pair(call.device, id);
+    if (g_thread.last == nullptr || key != g_thread.last_key) {
+        StreamState& state = g_thread.streams[key];
+        if (state.status.dev == nullptr) {
+            Status block{};
+            void* host = nullptr;
+            // (with unified addressing the host pointer is the device-visible one)
+            MOPS_CUDA_OK(cudaHostAlloc(&host, kStatusWords * sizeof(uint32_t),
+                                       cudaHostAllocMapped | cudaHostAllocPortable));
+            for (int i = 0; i < kStatusWords; i++) static_cast<volatile uint32_t*>(host)[i] = 0;
+            block.host = static_cast<uint32_t*>(host);
+            MOPS_CUDA_OK(cudaMalloc(reinterpret_cast<void**>(&block.dev),
+                                    kStatusWords * sizeof(uint32_t)));
+            MOPS_CUDA_OK(cudaMemset(block.dev, 0, kStatusWords * sizeof(uint32_t)));
+            state.status = block;
+        }
+        g_thread.last = &state;
+        g_thread.last_key = key;
     }
-    call.status = it->second;
+    call.state = g_thread.last;
+    call.state->used = 0;
+    call.status = call.state->status;
     g_thread.epoch += 1;
     if (g_thread.epoch == 0) g_thread.epoch = 1;
     call.status.epoch = g_thread.epoch;
@@ -281,13 +308,76 @@ void release_table(const Call& call, const TableRef& ref) {
 }
 
 void* scratch_alloc(const Call& call, size_t bytes) {
+    StreamState& w = *call.state;
+    bytes = (bytes + 255) / 256 * 256;
+    if (bytes <= kMostWorkspace) {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(call.stream, &capture) != cudaSuccess) (void)cudaGetLastError();
+        if (capture == cudaStreamCaptureStatusNone) {
+            if (w.used == 0 && w.size < w.wanted) { // grow between calls, in stream order
+                if (w.workspace != nullptr) {
+                    MOPS_CUDA_OK(cudaFreeAsync(w.workspace, call.stream));
+                    w.workspace = nullptr;
+                    w.size = 0;
+                    g_thread.workspaces--;
+                }
+                if (g_thread.workspaces < kMostWorkspaces) {
+                    void* ptr = nullptr;
+                    MOPS_CUDA_OK(cudaMallocFromPoolAsync(&ptr, w.wanted, scratch_pool(call.device), call.stream));
+                    w.workspace = static_cast<unsigned char*>(ptr);
+                    w.size = w.wanted;
+                    g_thread.workspaces++;
+                }
+            }
+            if (w.used + bytes <= w.size) {
+                void* ptr = w.workspace + w.used;
+                w.used += bytes;
+                return ptr;
+            }
+            // not now: remember for the next call
+            size_t want = w.used + bytes;
+            want = want + want / 2 < kMostWorkspace ? want + want / 2 : kMostWorkspace;
+            if (want > w.wanted) w.wanted = want;
+        }
+    }
     void* ptr = nullptr;
     MOPS_CUDA_OK(cudaMallocFromPoolAsync(&ptr, bytes, scratch_pool(call.device), call.stream));
     return ptr;
 }
 
 void scratch_free(const Call& call, void* ptr) {
-    if (ptr != nullptr) MOPS_CUDA_OK(cudaFreeAsync(ptr, call.stream));
+    const unsigned char* p = static_cast<unsigned char*>(ptr);
+    const StreamState& w = *call.state;
+    if (p == nullptr || (w.workspace != nullptr && p >= w.workspace && p < w.workspace + w.size)) return;
+    MOPS_CUDA_OK(cudaFreeAsync(ptr, call.stream));
+}
+
+// ---- launch settings
+namespace {
+std::mutex g_kernel_mutex;
+std::map<std::pair<const void*, int>, size_t> g_kernel_smem;
+std::map<std::tuple<const void*, int, int, size_t>, int> g_kernel_blocks;
+} // namespace
+
+void allow_dynamic_smem(const void* kernel, int device, size_t smem) {
+    if (smem <= 48 * 1024) return; // allowed as it is
+    std::lock_guard<std::mutex> lock(g_kernel_mutex);
+    size_t& allowed = g_kernel_smem[{kernel, device}];
+    if (smem <= allowed) return;
+    MOPS_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      static_cast<int>(smem)));
+    allowed = smem;
+}
+
+int resident_blocks(const void* kernel, int device, int threads, size_t smem) {
+    allow_dynamic_smem(kernel, device, smem);
+    std::lock_guard<std::mutex> lock(g_kernel_mutex);
+    int& blocks = g_kernel_blocks[{kernel, device, threads, smem}];
+    if (blocks == 0) {
+        MOPS_CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kernel, threads, smem));
+        if (blocks < 1) blocks = 1;
+    }
+    return blocks;
 }
 
 } // namespace mops_b200

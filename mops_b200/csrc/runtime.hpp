@@ -36,11 +36,14 @@ struct Status {
     uint32_t epoch; // identifies this call; never 0
 };
 
+struct StreamState; // what a thread keeps for a (device, stream), runtime.cu
+
 struct Call {
     cudaStream_t stream;
     bool wait; // true: results complete when the entry point returns
     Status status;
     int device;
+    StreamState* state;
 };
 
 [[noreturn]] void throw_cuda(cudaError_t err, const char* what, const char* file, int line);
@@ -85,7 +88,10 @@ void* get_stream();
 void set_wait(bool wait); // false: entry points return after enqueueing (used by the torch ops)
 bool get_wait();
 
-// Scratch memory for one call, ordered on the call's stream.
+// Scratch memory for one call, ordered on the call's stream. Small requests are pieces of a workspace
+// that the thread keeps for the stream (calls on one stream run in order, so the next call may use
+// it again); larger ones, and those of a stream that is being captured into a graph, come from a
+// stream-ordered pool. scratch_free of a piece does nothing.
 void* scratch_alloc(const Call& call, size_t bytes);
 void scratch_free(const Call& call, void* ptr);
 
@@ -150,6 +156,20 @@ void release_table(const Call& call, const TableRef& ref);
 
 int sm_count(int device);
 int max_optin_smem(int device);
+
+// Lets `kernel` use `smem` bytes of dynamic shared memory. The driver is asked once per kernel and
+// device (and again only for more); the setting is never lowered, which would break a launch of
+// another thread.
+void allow_dynamic_smem(const void* kernel, int device, size_t smem);
+template <typename R, typename... P> void allow_dynamic_smem(R (*kernel)(P...), int device, size_t smem) {
+    allow_dynamic_smem(reinterpret_cast<const void*>(kernel), device, smem);
+}
+// Blocks of `threads` threads and `smem` bytes that fit an SM, at least 1 (asked once).
+int resident_blocks(const void* kernel, int device, int threads, size_t smem);
+template <typename R, typename... P>
+int resident_blocks(R (*kernel)(P...), int device, int threads, size_t smem) {
+    return resident_blocks(reinterpret_cast<const void*>(kernel), device, threads, smem);
+}
 
 } // namespace mops_b200
 

@@ -478,12 +478,6 @@ int rows_per_block(const Call& call, int cols, int n_tables, int64_t K, size_t* 
     return 0;
 }
 
-template <typename Kernel> void allow_smem(Kernel kernel, size_t smem) {
-    if (smem > 48 * 1024)
-        MOPS_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          static_cast<int>(smem)));
-}
-
 // Allocates the call-scoped plan tables and runs the plan kernel.
 template <typename T>
 Plan<T> make_plan(const Call& call, TableRef* scratch, const T* C, const int32_t* PA,
@@ -839,7 +833,7 @@ bool forward_small(const Call& call, T* O, const T* A, const T* B, const T* C, c
     note_kernel_f("sap_fwd_small<%s,NS=%d> rows/block=%d", scalar_name<T>(), NS, R);
 #define MOPS_B200_LAUNCH(NS_)                                                                      \
     {                                                                                              \
-        allow_smem(sap_fwd_small<T, NS_>, smem);                                                   \
+        allow_dynamic_smem(sap_fwd_small<T, NS_>, call.device, smem);                                                   \
         sap_fwd_small<T, NS_><<<blocks, R, smem, call.stream>>>(O, S, Tm, plan, I, nS, nT, nO,     \
                                                                 static_cast<int>(K));              \
     }
@@ -875,7 +869,7 @@ bool backward_small(const Call& call, T* gA, T* gB, const T* gO, const T* A, con
     note_kernel_f("sap_vjp_small<%s,NS=%d> rows/block=%d", scalar_name<T>(), NS, R);
 #define MOPS_B200_LAUNCH(NS_)                                                                      \
     {                                                                                              \
-        allow_smem(sap_vjp_small<T, NS_>, smem);                                                   \
+        allow_dynamic_smem(sap_vjp_small<T, NS_>, call.device, smem);                                                   \
         sap_vjp_small<T, NS_><<<blocks, R, smem, call.stream>>>(gS, gT, gO, S, Tm, plan, I, nS,    \
                                                                 nT, nO, static_cast<int>(K));      \
     }
@@ -952,7 +946,7 @@ void mops::cuda::sparse_accumulation_of_products(Tensor<scalar_t, 2> output, Ten
                                                   nO, R + 1, true, false);
         auto kernel = in_smem ? sap_fwd_rows<scalar_t, true> : sap_fwd_rows<scalar_t, false>;
         note_kernel_f("sap_fwd_rows<%s,smem=%d>", scalar_name<scalar_t>(), in_smem ? 1 : 0);
-        allow_smem(kernel, smem);
+        allow_dynamic_smem(kernel, call.device, smem);
         kernel<<<static_cast<unsigned>(ceil_div(I, R)), R, smem, call.stream>>>(
             output.data, A.data, B.data, plan, I, nA, nB, nO, static_cast<int>(K));
         MOPS_CUDA_OK(cudaGetLastError());
@@ -1013,7 +1007,7 @@ void mops::cuda::sparse_accumulation_of_products_vjp(
                                                   indices_B.data, indices_output.data, K, nA, nB,
                                                   nO, R + 1, false, true);
         auto kernel = in_smem ? sap_vjp_rows<scalar_t, true> : sap_vjp_rows<scalar_t, false>;
-        allow_smem(kernel, smem);
+        allow_dynamic_smem(kernel, call.device, smem);
         kernel<<<static_cast<unsigned>(ceil_div(I, R)), R, smem, call.stream>>>(
             grad_A.data, grad_B.data, grad_output.data, A.data, B.data, plan, I, nA, nB, nO,
             static_cast<int>(K));
@@ -1080,7 +1074,7 @@ void mops::cuda::sparse_accumulation_of_products_vjp_vjp(
                                                   nO, R + 1, true, true);
         auto kernel =
             in_smem ? sap_vjp_vjp_rows<scalar_t, true> : sap_vjp_vjp_rows<scalar_t, false>;
-        allow_smem(kernel, smem);
+        allow_dynamic_smem(kernel, call.device, smem);
         kernel<<<static_cast<unsigned>(ceil_div(I, R)), R, smem, call.stream>>>(
             grad_grad_output.data, grad_A_2.data, grad_B_2.data, grad_grad_A.data,
             grad_grad_B.data, grad_output.data, A.data, B.data, plan, I, nA, nB, nO,

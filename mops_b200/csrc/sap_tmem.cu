@@ -282,8 +282,7 @@ bool backward_cells(const Call& call, const SapProblem<T>& p, T* gA, T* gB, cons
     int32_t* starts = reinterpret_cast<int32_t*>(records + b_rec);
     if (ref.fresh) {
         auto build = gather_table<T, 1, CellSource<T>>;
-        MOPS_CUDA_OK(cudaFuncSetAttribute(build, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          static_cast<int>(builder)));
+        allow_dynamic_smem(build, call.device, builder);
         const CellSource<T> source{p.C, b_narrow ? p.PA : p.PB, b_narrow ? p.PB : p.PA, p.PO, nT, nS, p.nO,
                                    b_narrow ? 0 : 1, b_narrow ? 1 : 0};
         build<<<1, kTableThreads, builder, call.stream>>>(records, starts, source, static_cast<int>(p.K),

@@ -2119,12 +2119,6 @@ int pick_warps(const Call& call, const Coupling<T>& cp, size_t per_warp_scalars,
     return 0;
 }
 
-template <typename Kernel> void allow_smem(Kernel kernel, size_t smem) {
-    if (smem > 48 * 1024)
-        MOPS_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          static_cast<int>(smem)));
-}
-
 // Shared memory of a fast-kernel block, and the largest warp count (8, 4, 2, 1) that fits.
 template <typename T>
 int pick_warps_fast(const Call& call, int ncc, int ds, size_t per_warp, size_t* smem) {
@@ -2159,7 +2153,7 @@ bool forward_fast(const Call& call, T* O, const Problem<T>& p) {
     if (!build_coupling(call, p, cp, &scratch, TP, ds)) return false;
     SegmentTable seg = segment_table(call, p.Io, p.E, p.nW0);
     const int64_t* offsets = seg.offsets;
-    allow_smem(sasaw_fwd_fast<T, TP, NAP, true>, smem_seg);
+    allow_dynamic_smem(sasaw_fwd_fast<T, TP, NAP, true>, call.device, smem_seg);
     note_kernel_f("sasaw_fwd_fast<%s,TP=%d,NAP=%d>", scalar_name<T>(), TP, NAP);
     sasaw_fwd_fast<T, TP, NAP, true><<<static_cast<unsigned>(ceil_div(p.nW0, warps_seg)),
                                        warps_seg * 32, smem_seg, call.stream>>>(
@@ -2174,7 +2168,7 @@ bool forward_fast(const Call& call, T* O, const Problem<T>& p) {
     }
     if (need_fallback) {
         zero_if_unsorted<T><<<grid_generic, 256, 0, call.stream>>>(O, p.nW0 * rowsize, call.status);
-        allow_smem(sasaw_fwd_fast<T, TP, NAP, false>, smem_edge);
+        allow_dynamic_smem(sasaw_fwd_fast<T, TP, NAP, false>, call.device, smem_edge);
         const int64_t blocks = std::min<int64_t>(ceil_div(p.E, warps_edge), grid_generic);
         sasaw_fwd_fast<T, TP, NAP, false><<<static_cast<unsigned>(blocks), warps_edge * 32,
                                             smem_edge, call.stream>>>(
@@ -2197,7 +2191,7 @@ bool backward_fast(const Call& call, T* gA, T* gB, T* gW, const T* gO, const Pro
     Coupling<T> cp{};
     TableRef scratch{};
     if (!build_coupling(call, p, cp, &scratch, TP, ds)) return false;
-    allow_smem(sasaw_vjp_fast<T, TP, NAP>, smem);
+    allow_dynamic_smem(sasaw_vjp_fast<T, TP, NAP>, call.device, smem);
     note_kernel_f("sasaw_vjp_fast<%s,TP=%d,NAP=%d>", scalar_name<T>(), TP, NAP);
     const int64_t blocks =
         std::min<int64_t>(ceil_div(p.E, warps), static_cast<int64_t>(sm_count(call.device)) * 16);
@@ -2232,7 +2226,7 @@ bool forward_mma_launch(const Call& call, T* O, const Problem<T>& p, bool segmen
         SegmentTable seg = segment_table(call, p.Io, p.E, p.nW0);
         const int64_t* offsets = seg.offsets;
         known_sorted = seg.known_sorted;
-        allow_smem(sasaw_fwd_mma<TP, true>, smem);
+        allow_dynamic_smem(sasaw_fwd_mma<TP, true>, call.device, smem);
         note_kernel_f("sasaw_fwd_mma<TP=%d,SEG=1>", TP);
         const int64_t seg_blocks = std::min<int64_t>(ceil_div(p.nW0, warps), sms * 3);
         sasaw_fwd_mma<TP, true><<<static_cast<unsigned>(seg_blocks), warps * 32, smem,
@@ -2249,7 +2243,7 @@ bool forward_mma_launch(const Call& call, T* O, const Problem<T>& p, bool segmen
     }
     if (need_fallback) {
         zero_if_unsorted<T><<<sms * 8, 256, 0, call.stream>>>(O, p.nW0 * rowsize, call.status);
-        allow_smem(sasaw_fwd_mma<TP, false>, smem);
+        allow_dynamic_smem(sasaw_fwd_mma<TP, false>, call.device, smem);
         const int64_t blocks = std::min<int64_t>(ceil_div(ceil_div(p.E, 8), warps), sms * 3);
         sasaw_fwd_mma<TP, false><<<static_cast<unsigned>(blocks), warps * 32, smem, call.stream>>>(
             O, p.A, p.B, p.W, p.Jw, p.Io, nullptr, cp, p.E, p.nA, p.L, p.nW0, p.nW1, p.nO1,
@@ -2260,11 +2254,6 @@ bool forward_mma_launch(const Call& call, T* O, const Problem<T>& p, bool segmen
     return true;
 }
 
-inline int env_flag(const char* name, int fallback) {
-    const char* v = std::getenv(name);
-    return v != nullptr && *v != '\0' ? std::atoi(v) : fallback;
-}
-
 // Sorted scatter index through the quad kernel. Returns 0 when it does not apply, 1 when it
 // ran and the index was seen to be sorted (nothing left to do), 2 when it was launched but
 // the kernels for unsorted input must still be enqueued (asynchronous call, or the index
@@ -2273,8 +2262,6 @@ template <typename T> int forward_quad(const Call& call, T* O, const Problem<T>&
     if constexpr (!std::is_same<T, double>::value) {
         return 0;
     } else {
-        // (MOPS_B200_SASAW_QUAD=0: development switch back to the batch-of-eight kernels)
-        if (env_flag("MOPS_B200_SASAW_QUAD", 1) == 0) return 0;
         auto aligned = [](const void* ptr) { return reinterpret_cast<uintptr_t>(ptr) % 16 == 0; };
         if (p.L % 2 != 0 || !aligned(p.W) || !aligned(p.B) || !aligned(O)) return 0;
         const QuadLayout q = quad_layout(p.nA, p.nW1, p.nO1);
@@ -2296,7 +2283,7 @@ template <typename T> int forward_quad(const Call& call, T* O, const Problem<T>&
         note_kernel_f("sasaw_fwd_quad<MODE=%d,%s> warps=%d", mode, fixed ? "fixed widths" : "any widths", warps);
 #define MOPS_B200_CASE(MODE_, NA_, NW_, NO_)                                                       \
     {                                                                                              \
-        allow_smem(sasaw_fwd_quad<MODE_, NA_, NW_, NO_>, smem);                                    \
+        allow_dynamic_smem(sasaw_fwd_quad<MODE_, NA_, NW_, NO_>, call.device, smem);                                    \
         sasaw_fwd_quad<MODE_, NA_, NW_, NO_><<<blocks, warps * 32, smem, call.stream>>>(           \
             O, p.A, p.B, p.W, p.Jw, offsets, cp, p.E, p.nA, p.L, p.nW0, p.nW1, p.nO1, call.status); \
     }
@@ -2349,7 +2336,7 @@ bool backward_mma_launch(const Call& call, T* gA, T* gB, T* gW, const T* gO, con
     Coupling<T> cp{};
     TableRef scratch{};
     if (!build_coupling(call, p, cp, &scratch, Lay::TS, Lay::d_stride(p.nA), true)) return false;
-    allow_smem(sasaw_vjp_mma<TP, KS3>, smem);
+    allow_dynamic_smem(sasaw_vjp_mma<TP, KS3>, call.device, smem);
     if (!only_if_unsorted) note_kernel_f("sasaw_vjp_mma<TP=%d,KS3=%d>", TP, KS3);
     const bool wide_copies = p.L % 2 == 0 && reinterpret_cast<uintptr_t>(p.W) % 16 == 0 &&
                              reinterpret_cast<uintptr_t>(p.B) % 16 == 0;
@@ -2371,7 +2358,6 @@ int backward_quad(const Call& call, T* gA, T* gB, T* gW, const T* gO, const Prob
     if constexpr (!std::is_same<T, double>::value) {
         return 0;
     } else {
-        if (env_flag("MOPS_B200_SASAW_QUAD", 1) == 0) return 0;
         if (!(p.nA == 9 && p.nW1 == 9 && p.nO1 == 9)) return 0;
         auto aligned = [](const void* ptr) { return reinterpret_cast<uintptr_t>(ptr) % 16 == 0; };
         if (p.L % 2 != 0 || !aligned(p.W) || !aligned(p.B) || !aligned(gB)) return 0;
@@ -2391,11 +2377,11 @@ int backward_quad(const Call& call, T* gA, T* gB, T* gW, const T* gO, const Prob
         const unsigned blocks = static_cast<unsigned>(std::min<int64_t>(ceil_div(p.nW0, warps), sms));
         note_kernel_f("sasaw_vjp_quad<9,9,9,L=%d> warps=%d", p.L == 32 ? 32 : 0, warps);
         if (p.L == 32) {
-            allow_smem(sasaw_vjp_quad<9, 9, 9, 32>, smem);
+            allow_dynamic_smem(sasaw_vjp_quad<9, 9, 9, 32>, call.device, smem);
             sasaw_vjp_quad<9, 9, 9, 32><<<blocks, warps * 32, smem, call.stream>>>(
                 gA, gB, gW, gO, p.A, p.B, p.W, p.Jw, offsets, cp, p.L, p.nW0, call.status);
         } else {
-            allow_smem(sasaw_vjp_quad<9, 9, 9, 0>, smem);
+            allow_dynamic_smem(sasaw_vjp_quad<9, 9, 9, 0>, call.device, smem);
             sasaw_vjp_quad<9, 9, 9, 0><<<blocks, warps * 32, smem, call.stream>>>(
                 gA, gB, gW, gO, p.A, p.B, p.W, p.Jw, offsets, cp, p.L, p.nW0, call.status);
         }
@@ -2482,7 +2468,7 @@ template <typename T> void forward(const Call& call, T* O, const Problem<T>& p) 
         warps_edge = pick_warps(call, cp, static_cast<size_t>(p.nA) + cp.ncell, false, &smem_edge);
     }
     if (grouped && warps_seg > 0 && warps_edge > 0) {
-        allow_smem(sasaw_fwd<T, true>, smem_seg);
+        allow_dynamic_smem(sasaw_fwd<T, true>, call.device, smem_seg);
         sasaw_fwd<T, true><<<static_cast<unsigned>(ceil_div(p.nW0, warps_seg)), warps_seg * 32,
                              smem_seg, call.stream>>>(O, p.A, p.B, p.W, p.Jw, p.Io, cp, p.E, p.nA,
                                                       p.L, p.nW0, p.nW1, p.nO1, false, call.status);
@@ -2495,7 +2481,7 @@ template <typename T> void forward(const Call& call, T* O, const Problem<T>& p) 
         if (need_fallback) {
             zero_if_unsorted<T><<<grid_generic, 256, 0, call.stream>>>(O, p.nW0 * rowsize,
                                                                        call.status);
-            allow_smem(sasaw_fwd<T, false>, smem_edge);
+            allow_dynamic_smem(sasaw_fwd<T, false>, call.device, smem_edge);
             const int64_t blocks = std::min<int64_t>(ceil_div(p.E, warps_edge), grid_generic);
             sasaw_fwd<T, false><<<static_cast<unsigned>(blocks), warps_edge * 32, smem_edge,
                                   call.stream>>>(O, p.A, p.B, p.W, p.Jw, p.Io, cp, p.E, p.nA, p.L,
@@ -2535,7 +2521,7 @@ void backward(const Call& call, T* gA, T* gB, T* gW, const T* gO, const Problem<
         if (gB != nullptr && p.L > 0)
             MOPS_CUDA_OK(cudaMemsetAsync(gB, 0, p.E * p.L * sizeof(T), call.stream));
     } else if (grouped && warps > 0) {
-        allow_smem(sasaw_vjp<T>, smem);
+        allow_dynamic_smem(sasaw_vjp<T>, call.device, smem);
         const int64_t blocks =
             std::min<int64_t>(ceil_div(p.E, warps), static_cast<int64_t>(sm_count(call.device)) * 16);
         sasaw_vjp<T><<<static_cast<unsigned>(blocks), warps * 32, smem, call.stream>>>(
@@ -2794,7 +2780,7 @@ void forward_noalloc(double* O, const Problem<double>& p) {
                                  "point's shared-memory kernels; use "
                                  "mops_cuda_sparse_accumulation_scatter_add_with_weights_f64");
     }
-    allow_smem(sasaw_fwd<T, true>, smem_seg);
+    allow_dynamic_smem(sasaw_fwd<T, true>, call.device, smem_seg);
     sasaw_fwd<T, true><<<static_cast<unsigned>(ceil_div(p.nW0, warps_seg)), warps_seg * 32,
                          smem_seg, call.stream>>>(O, p.A, p.B, p.W, p.Jw, p.Io, cp, p.E, p.nA, p.L,
                                                   p.nW0, p.nW1, p.nO1, false, call.status);
@@ -2806,7 +2792,7 @@ void forward_noalloc(double* O, const Problem<double>& p) {
     if (words[kUnsortedEpoch] == call.status.epoch) {
         const int grid_generic = sm_count(call.device) * 8;
         zero_if_unsorted<T><<<grid_generic, 256, 0, call.stream>>>(O, p.nW0 * rowsize, call.status);
-        allow_smem(sasaw_fwd<T, false>, smem_edge);
+        allow_dynamic_smem(sasaw_fwd<T, false>, call.device, smem_edge);
         const int64_t blocks = std::min<int64_t>(ceil_div(p.E, warps_edge), grid_generic);
         sasaw_fwd<T, false><<<static_cast<unsigned>(blocks), warps_edge * 32, smem_edge,
                               call.stream>>>(O, p.A, p.B, p.W, p.Jw, p.Io, cp, p.E, p.nA, p.L,

@@ -120,10 +120,16 @@ Tensor requested(const Tensor& t) { return t.defined() && t.numel() == 0 ? Tenso
                     std::string("second derivatives are not supported in CUDA for ") + op);
 }
 
+// The gradients of an operation: through the differentiable Function when this backward pass is itself
+// recorded (create_graph), else straight from the kernels, without a node and saved variables that
+// nobody would use.
+template <typename Backward, typename... Args> tensor_list backward_of(const Args&... args) {
+    return at::GradMode::is_enabled() ? Backward::apply(args...) : Backward::run(args...);
+}
+
 // =============================================================================== HPE
 struct HpeBackward : torch::autograd::Function<HpeBackward> {
-    static tensor_list forward(AutogradContext* ctx, Tensor grad_output, Tensor A, Tensor C,
-                               Tensor indices_A) {
+    static tensor_list run(const Tensor& grad_output, const Tensor& A, const Tensor& C, const Tensor& indices_A) {
         if (C.requires_grad()) {
             C10_THROW_ERROR(ValueError, "gradients with respect to the coefficients C are not "
                                         "supported in homogeneous_polynomial_evaluation");
@@ -136,10 +142,13 @@ struct HpeBackward : torch::autograd::Function<HpeBackward> {
                     view<scalar_t, 1>(C), view<int32_t, 2>(indices_A));
             });
         });
+        return {defined(grad_A, A)};
+    }
+    static tensor_list forward(AutogradContext* ctx, Tensor grad_output, Tensor A, Tensor C, Tensor indices_A) {
         if (grad_output.requires_grad() || A.requires_grad()) {
             ctx->save_for_backward({grad_output, A, C, indices_A});
         }
-        return {defined(grad_A, A)};
+        return run(grad_output, A, C, indices_A);
     }
     static tensor_list backward(AutogradContext* ctx, tensor_list grads) {
         auto saved = ctx->get_saved_variables();
@@ -186,16 +195,14 @@ struct Hpe : torch::autograd::Function<Hpe> {
     }
     static tensor_list backward(AutogradContext* ctx, tensor_list grad_outputs) {
         auto saved = ctx->get_saved_variables();
-        auto results = HpeBackward::apply(grad_outputs[0].contiguous(), saved[0], saved[1], saved[2]);
+        auto results = backward_of<HpeBackward>(grad_outputs[0].contiguous(), saved[0], saved[1], saved[2]);
         return {requested(results[0]), Tensor(), Tensor()};
     }
 };
 
 // =============================================================================== SAP
 struct SapBackward : torch::autograd::Function<SapBackward> {
-    static tensor_list forward(AutogradContext* ctx, Tensor grad_output, Tensor A, Tensor B,
-                               Tensor C, Tensor indices_A, Tensor indices_B,
-                               Tensor indices_output) {
+    static tensor_list run(const Tensor& grad_output, const Tensor& A, const Tensor& B, const Tensor& C, const Tensor& indices_A, const Tensor& indices_B, const Tensor& indices_output) {
         if (C.requires_grad()) {
             C10_THROW_ERROR(ValueError, "gradients with respect to the coefficients C are not "
                                         "supported in sparse_accumulation_of_products");
@@ -210,10 +217,13 @@ struct SapBackward : torch::autograd::Function<SapBackward> {
                     view<int32_t, 1>(indices_output));
             });
         });
+        return {defined(grad_A, A), defined(grad_B, A)};
+    }
+    static tensor_list forward(AutogradContext* ctx, Tensor grad_output, Tensor A, Tensor B, Tensor C, Tensor indices_A, Tensor indices_B, Tensor indices_output) {
         if (grad_output.requires_grad() || A.requires_grad() || B.requires_grad()) {
             ctx->save_for_backward({grad_output, A, B, C, indices_A, indices_B, indices_output});
         }
-        return {defined(grad_A, A), defined(grad_B, A)};
+        return run(grad_output, A, B, C, indices_A, indices_B, indices_output);
     }
     static tensor_list backward(AutogradContext* ctx, tensor_list grads) {
         auto saved = ctx->get_saved_variables();
@@ -276,15 +286,14 @@ struct Sap : torch::autograd::Function<Sap> {
     }
     static tensor_list backward(AutogradContext* ctx, tensor_list grad_outputs) {
         auto s = ctx->get_saved_variables();
-        auto r = SapBackward::apply(grad_outputs[0].contiguous(), s[0], s[1], s[2], s[3], s[4], s[5]);
+        auto r = backward_of<SapBackward>(grad_outputs[0].contiguous(), s[0], s[1], s[2], s[3], s[4], s[5]);
         return {requested(r[0]), requested(r[1]), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
     }
 };
 
 // =============================================================================== OPSA
 struct OpsaBackward : torch::autograd::Function<OpsaBackward> {
-    static tensor_list forward(AutogradContext* ctx, Tensor grad_output, Tensor A, Tensor B,
-                               Tensor indices_output) {
+    static tensor_list run(const Tensor& grad_output, const Tensor& A, const Tensor& B, const Tensor& indices_output) {
         Tensor grad_A = maybe_empty_like(A), grad_B = maybe_empty_like(B);
         on_stream_of(A, [&] {
             AT_DISPATCH_FLOATING_TYPES(A.scalar_type(), "outer_product_scatter_add_vjp", [&] {
@@ -294,10 +303,13 @@ struct OpsaBackward : torch::autograd::Function<OpsaBackward> {
                     view<int32_t, 1>(indices_output));
             });
         });
+        return {defined(grad_A, A), defined(grad_B, A)};
+    }
+    static tensor_list forward(AutogradContext* ctx, Tensor grad_output, Tensor A, Tensor B, Tensor indices_output) {
         if (grad_output.requires_grad() || A.requires_grad() || B.requires_grad()) {
             ctx->save_for_backward({grad_output, A, B, indices_output});
         }
-        return {defined(grad_A, A), defined(grad_B, A)};
+        return run(grad_output, A, B, indices_output);
     }
     static tensor_list backward(AutogradContext* ctx, tensor_list grads) {
         auto saved = ctx->get_saved_variables();
@@ -349,15 +361,14 @@ struct Opsa : torch::autograd::Function<Opsa> {
     }
     static tensor_list backward(AutogradContext* ctx, tensor_list grad_outputs) {
         auto s = ctx->get_saved_variables();
-        auto r = OpsaBackward::apply(grad_outputs[0].contiguous(), s[0], s[1], s[2]);
+        auto r = backward_of<OpsaBackward>(grad_outputs[0].contiguous(), s[0], s[1], s[2]);
         return {requested(r[0]), requested(r[1]), Tensor(), Tensor()};
     }
 };
 
 // =============================================================================== OPSAW
 struct OpsawBackward : torch::autograd::Function<OpsawBackward> {
-    static tensor_list forward(AutogradContext*, Tensor grad_output, Tensor A, Tensor B, Tensor W,
-                               Tensor indices_W, Tensor indices_output) {
+    static tensor_list run(const Tensor& grad_output, const Tensor& A, const Tensor& B, const Tensor& W, const Tensor& indices_W, const Tensor& indices_output) {
         Tensor grad_A = maybe_empty_like(A), grad_B = maybe_empty_like(B),
                grad_W = maybe_empty_like(W);
         on_stream_of(A, [&] {
@@ -370,6 +381,9 @@ struct OpsawBackward : torch::autograd::Function<OpsawBackward> {
             });
         });
         return {defined(grad_A, A), defined(grad_B, A), defined(grad_W, A)};
+    }
+    static tensor_list forward(AutogradContext*, Tensor grad_output, Tensor A, Tensor B, Tensor W, Tensor indices_W, Tensor indices_output) {
+        return run(grad_output, A, B, W, indices_W, indices_output);
     }
     static tensor_list backward(AutogradContext*, tensor_list) {
         no_second_derivative("outer_product_scatter_add_with_weights");
@@ -410,16 +424,14 @@ struct Opsaw : torch::autograd::Function<Opsaw> {
     }
     static tensor_list backward(AutogradContext* ctx, tensor_list grad_outputs) {
         auto s = ctx->get_saved_variables();
-        auto r = OpsawBackward::apply(grad_outputs[0].contiguous(), s[0], s[1], s[2], s[3], s[4]);
+        auto r = backward_of<OpsawBackward>(grad_outputs[0].contiguous(), s[0], s[1], s[2], s[3], s[4]);
         return {requested(r[0]), requested(r[1]), requested(r[2]), Tensor(), Tensor()};
     }
 };
 
 // =============================================================================== SASAW
 struct SasawBackward : torch::autograd::Function<SasawBackward> {
-    static tensor_list forward(AutogradContext*, Tensor grad_output, Tensor A, Tensor B, Tensor C,
-                               Tensor W, Tensor indices_A, Tensor indices_W_1, Tensor indices_W_2,
-                               Tensor indices_output_1, Tensor indices_output_2) {
+    static tensor_list run(const Tensor& grad_output, const Tensor& A, const Tensor& B, const Tensor& C, const Tensor& W, const Tensor& indices_A, const Tensor& indices_W_1, const Tensor& indices_W_2, const Tensor& indices_output_1, const Tensor& indices_output_2) {
         if (C.requires_grad()) {
             C10_THROW_ERROR(ValueError,
                             "gradients with respect to the coefficients C are not supported in "
@@ -440,6 +452,9 @@ struct SasawBackward : torch::autograd::Function<SasawBackward> {
                 });
         });
         return {defined(grad_A, A), defined(grad_B, A), defined(grad_W, A)};
+    }
+    static tensor_list forward(AutogradContext*, Tensor grad_output, Tensor A, Tensor B, Tensor C, Tensor W, Tensor indices_A, Tensor indices_W_1, Tensor indices_W_2, Tensor indices_output_1, Tensor indices_output_2) {
+        return run(grad_output, A, B, C, W, indices_A, indices_W_1, indices_W_2, indices_output_1, indices_output_2);
     }
     static tensor_list backward(AutogradContext*, tensor_list) {
         no_second_derivative("sparse_accumulation_scatter_add_with_weights");
@@ -492,7 +507,7 @@ struct Sasaw : torch::autograd::Function<Sasaw> {
     }
     static tensor_list backward(AutogradContext* ctx, tensor_list grad_outputs) {
         auto s = ctx->get_saved_variables();
-        auto r = SasawBackward::apply(grad_outputs[0].contiguous(), s[0], s[1], s[2], s[3], s[4],
+        auto r = backward_of<SasawBackward>(grad_outputs[0].contiguous(), s[0], s[1], s[2], s[3], s[4],
                                       s[5], s[6], s[7], s[8]);
         return {requested(r[0]), requested(r[1]), Tensor(), requested(r[2]), Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
     }
