@@ -76,7 +76,8 @@ __device__ __forceinline__ int64_t warp_lower_bound(const int32_t* __restrict__ 
 // Number of i in [0, n) with t[i] + row_weight * i <= x, for an ascending table t, found by
 // the whole warp with 32-way probes (as warp_lower_bound). All lanes call it with the same
 // arguments.
-__device__ __forceinline__ int64_t warp_count_weighted_le(const int64_t* __restrict__ t, int64_t n,
+template <typename Off>
+__device__ __forceinline__ int64_t warp_count_weighted_le(const Off* __restrict__ t, int64_t n,
                                                           int64_t row_weight, int64_t x, int lane) {
     int64_t lo = 0, hi = n;
     while (hi > lo) {
@@ -106,7 +107,8 @@ __device__ __forceinline__ int64_t warp_count_weighted_le(const int64_t* __restr
 // first row of worker `part`, who owns rows [split(part), split(part + 1)). All lanes of a
 // warp call it together.
 constexpr int64_t kRowWeight = 4;
-__device__ __forceinline__ int64_t balanced_row_split(const int64_t* __restrict__ offsets,
+template <typename Off>
+__device__ __forceinline__ int64_t balanced_row_split(const Off* __restrict__ offsets,
                                                       int64_t n_rows, int64_t part, int64_t parts,
                                                       int lane) {
     if (part <= 0) return 0;

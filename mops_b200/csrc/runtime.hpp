@@ -110,7 +110,9 @@ enum TableKind : int {
     kSasawCouplingTable = 2,
     kHpeTable = 3,
     kSapTable = 4,
-    kSapSmallTable = 5
+    kSapSmallTable = 5,
+    kSasawDenseTable = 6,
+    kEdgeOrder = 7
 };
 
 struct TableKey {

@@ -34,6 +34,7 @@
 
 #include "checks.hpp"
 #include "device.cuh"
+#include "sasaw_rows.hpp"
 
 namespace mops_b200 {
 namespace {
@@ -2447,14 +2448,42 @@ bool backward_mma(const Call& call, T* gA, T* gB, T* gW, const T* gO, const Prob
         }                                                                                          \
     }()
 
+template <typename T> SasawProblem<T> rows_problem(const Problem<T>& p) {
+    return {p.A, p.B, p.C, p.W, p.M1, p.Jw, p.M2, p.Io, p.M3, p.E, p.N, p.nW0, p.nA, p.nW1, p.nO1, p.L};
+}
+
+// The row kernels (sasaw_rows.cu) or the ones here, from measurements on B200:
+//   forward   f64 with fewer than 24 edges per row: the coupling per row then costs more than the
+//             coupling per edge of the MMA kernels (200 000 edges, 10 per row, 9 x 9 x 9 channels, 32
+//             columns: 190 against 122 us; 61 per row: 110 against 116 us).
+//   gradients f64, where the MMA kernels apply and W and gW stay in L2, these are faster from 100 000
+//             edges on (10^6 edges, 9 x 9 x 9: 1.20 against 1.37 ms; 60 000: 148 against 120 us;
+//             4.2 10^6 with W and gW of 151 MB each: 5.70 against 4.85 ms).
+//             Output channels in several passes (more than 9) and few of W (up to 4): here it pays
+//             to gather W and to add to gW, f32 0.21 against 0.45 ms, f64 0.15 against 0.42 ms.
+constexpr int64_t kShortRows = 24;
+constexpr int64_t kFewEdges = 100000;
+constexpr double kCacheBytes = 100e6; // of the 126 MB of L2
+
+template <typename T> bool rows_first_backward(const Problem<T>& p) {
+    const bool long_rows = p.E >= kShortRows * p.nW0;
+    if (p.nW1 <= 4 && p.nO1 > 9) return false;
+    if (sizeof(T) == 4) return true;
+    const double tables = 2.0 * p.nW0 * p.nW1 * p.L * sizeof(T);
+    return long_rows && (tables > kCacheBytes || (p.E < kFewEdges && p.nW1 == 9 && p.nO1 == 9 && p.nA == 9));
+}
+
 template <typename T> void forward(const Call& call, T* O, const Problem<T>& p) {
+    const bool short_rows = sizeof(T) == 8 && p.E < kShortRows * p.nW0;
     const int64_t rowsize = static_cast<int64_t>(p.nO1) * p.L;
     if (p.nW0 == 0 || rowsize == 0) return;
     if (p.E == 0 || p.N == 0) {
         MOPS_CUDA_OK(cudaMemsetAsync(O, 0, p.nW0 * rowsize * sizeof(T), call.stream));
         return;
     }
+    if (!short_rows && sasaw_forward_rows<T>(call, rows_problem(p), O)) return;
     if (forward_mma(call, O, p)) return;
+    if (short_rows && sasaw_forward_rows<T>(call, rows_problem(p), O)) return;
     if (MOPS_B200_SASAW_FAST(forward_fast, call, O, p)) return;
     const int grid_generic = sm_count(call.device) * 8;
     Coupling<T> cp{};
@@ -2501,11 +2530,14 @@ template <typename T>
 void backward(const Call& call, T* gA, T* gB, T* gW, const T* gO, const Problem<T>& p) {
     if (gA == nullptr && gB == nullptr && gW == nullptr) return;
     const int64_t wsize = p.nW0 * static_cast<int64_t>(p.nW1) * p.L;
+    const bool some = p.E > 0 && p.N > 0 && p.L > 0;
+    if (some && rows_first_backward(p) && sasaw_backward_rows<T>(call, rows_problem(p), gA, gB, gW, gO)) return;
     if (gW != nullptr && wsize > 0)
         MOPS_CUDA_OK(cudaMemsetAsync(gW, 0, wsize * sizeof(T), call.stream));
     if (p.E == 0) return;
     const bool empty = p.N == 0 || p.L == 0 || p.nO1 == 0 || p.nW1 == 0 || p.nA == 0;
     if (!empty && backward_mma(call, gA, gB, gW, gO, p)) return;
+    if (some && !(p.nW1 <= 4 && p.nO1 > 9) && sasaw_backward_rows<T>(call, rows_problem(p), gA, gB, gW, gO)) return;
     if (!empty && MOPS_B200_SASAW_FAST(backward_fast, call, gA, gB, gW, gO, p)) return;
     Coupling<T> cp{};
     TableRef scratch{};

@@ -1,0 +1,819 @@
+// Sparse accumulation scatter-add with weights, row by row with the coupling applied per row and
+// not per edge. With D[m3,m2,m1] the coupling as a dense table and lane = column b:
+//
+//   forward      G_i[m1,m2,b] = sum over the edges e of row i of A[e,m1] B[e,b] W[J_e,m2,b]
+//                O[i,m3,b]    = sum_{m1,m2} D[m3,m2,m1] G_i[m1,m2,b]
+//   gradients, with the edges in the order of J (row j of W):
+//                F_j[m1,m3,b] = sum over the edges e with J_e = j of A[e,m1] B[e,b] gO[I_e,m3,b]
+//                gW[j,m2,b]   = sum_{m1,m3} D[m3,m2,m1] F_j[m1,m3,b]
+//                E_j[m1,m3,b] = sum_m2 D[m3,m2,m1] W[j,m2,b]
+//                Z[m1,b]      = sum_m3 E_j[m1,m3,b] gO[I_e,m3,b]
+//                gB[e,b]      = sum_m1 A[e,m1] Z[m1,b],      gA[e,m1] = sum_b B[e,b] Z[m1,b]
+//
+// G, F and E stay in registers while a warp walks the edges of a row, so that an edge costs
+// nA x nW (forward) or 2 nA x nO (gradients) multiply-adds per column and nothing else: no coupling
+// matrix per edge, no reduction over lanes but the nA sums of gA, no atomics (gW is a sum over a row)
+// and hence no dependence on the order of I. The coupling costs nA x nW x nO per row and column,
+// shared by the row's edges. The gathered rows (of W, of gO) come through a ring of asynchronous
+// copies in shared memory, eight edges deep, into which every lane copies what it will read itself.
+//
+// What bounds them: latency at two warps per scheduler (the sums take 162 registers per lane), the FP64
+// pipe then 39 % (sums) and 25 % (edge gradients) busy, issue slots 44 %; L2 or DRAM where the
+// gathered table is large. Against the kernels of sasaw.cu, sums and gradients, 9 x 9 x 9 channels:
+// f32 250 000 edges, 64 columns 0.44 + 1.13 -> 0.14 + 0.36 ms; f64 60 000 edges, 32 columns 70 + 148
+// -> 45 + 120 us. Half the products per warp and three warps per scheduler were slower (62 -> 111 us):
+// what an edge costs beside its products then counts twice.
+#include <algorithm>
+#include <initializer_list>
+#include <type_traits>
+
+#include "sasaw_rows.hpp"
+#include "unsorted.cuh"
+
+namespace mops_b200 {
+namespace {
+
+enum { kBitI = 0, kBitM1 = 1, kBitJ = 2, kBitM2 = 3, kBitM3 = 4 };
+constexpr int kWidest = 16;
+constexpr int kDepth = 8; // steps in the ring
+constexpr int kRowWarps = 8;
+constexpr int kTableOut = 3; // outputs contracted together
+
+// One 64-bit (or 32-bit) element per lane: a double, two floats, or a float.
+template <typename T, int VEC> struct Pack;
+template <typename T> struct Pack<T, 1> {
+    using V = T;
+    static __device__ __forceinline__ V dup(T x) { return x; }
+    static __device__ __forceinline__ V fma(V a, V b, V c) { return a * b + c; }
+    static __device__ __forceinline__ V mul(V a, V b) { return a * b; }
+    static __device__ __forceinline__ V add(V a, V b) { return a + b; }
+    static __device__ __forceinline__ T sum(V a) { return a; }
+    static __device__ __forceinline__ V shift(V a, int o) { return __shfl_xor_sync(kFullMask, a, o); }
+};
+template <> struct Pack<float, 2> { // FFMA2: two multiply-adds per instruction
+    using V = unsigned long long;
+    static __device__ __forceinline__ V dup(float x) {
+        V v;
+        asm("mov.b64 %0, {%1, %1};" : "=l"(v) : "f"(x));
+        return v;
+    }
+    static __device__ __forceinline__ V fma(V a, V b, V c) {
+        V d;
+        asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+        return d;
+    }
+    static __device__ __forceinline__ V mul(V a, V b) {
+        V d;
+        asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+        return d;
+    }
+    static __device__ __forceinline__ V add(V a, V b) {
+        V d;
+        asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+        return d;
+    }
+    static __device__ __forceinline__ float sum(V a) {
+        float x, y;
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a));
+        return x + y;
+    }
+    static __device__ __forceinline__ V shift(V a, int o) { return __shfl_xor_sync(kFullMask, a, o); }
+};
+
+// ---- the dense coupling table D[out][a][c], padded with zeros: `out` is m3 (forward) or m2
+// (gradients), c the other one. A warp per entry of the table, lanes over the coupling entries in a
+// fixed order, so the sums are reproducible.
+template <typename T>
+__global__ void __launch_bounds__(256)
+sasaw_dense_table(T* __restrict__ D, const T* __restrict__ C, const int32_t* __restrict__ M1,
+                  const int32_t* __restrict__ M2, const int32_t* __restrict__ M3, int64_t N, int nA, int nW,
+                  int nO, bool out_is_m2, int pad_out, int pad_a, int pad_c, Status st) {
+    const int lane = threadIdx.x & 31;
+    const int slot = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (slot >= pad_out * pad_a * pad_c) return;
+    const int c = slot % pad_c, a = slot / pad_c % pad_a, o = slot / (pad_c * pad_a);
+    T sum = T(0);
+    if (o < (out_is_m2 ? nW : nO) && a < nA && c < (out_is_m2 ? nO : nW)) {
+        const int want2 = out_is_m2 ? o : c, want3 = out_is_m2 ? c : o;
+        for (int64_t n = lane; n < N; n += 32) {
+            int32_t m1 = __ldg(M1 + n), m2 = __ldg(M2 + n), m3 = __ldg(M3 + n);
+            const bool b1 = clamp_index(m1, nA), b2 = clamp_index(m2, nW), b3 = clamp_index(m3, nO);
+            if (slot == 0) {
+                if (b1) report_bad_index(st, kBitM1);
+                if (b2) report_bad_index(st, kBitM2);
+                if (b3) report_bad_index(st, kBitM3);
+            }
+            if (m1 == a && m2 == want2 && m3 == want3) sum += __ldg(C + n);
+        }
+    }
+    sum = warp_sum(sum);
+    if (lane == 0) D[slot] = sum;
+}
+
+// ---- walking the edges of a range of rows
+template <typename T> struct RowsArgs {
+    const T *A, *B, *G;          // [E][nA], [E][L], gathered rows [rows][nC][L]
+    const int32_t* gather;       // [E] row of G
+    const int32_t* perm;         // order of the edges; nullptr: as they are
+    const T* D;                  // table [pad_out][NA][pad_c]
+    int64_t rows;
+    int nA, nC, nOut, L;
+    int pad_out, pad_c;
+    int lanes;                   // lanes per edge (a power of two); 32 / lanes edges side by side
+    int bit;                     // status bit of `gather`
+};
+
+// One slot of a warp's ring: NC rows of 32 lanes, B, the A rows of the edges side by side, their numbers.
+template <typename T, int VEC, int NA, int NC> struct Slot {
+    using V = typename Pack<T, VEC>::V;
+    static constexpr int kB = NC * 32 * sizeof(V);
+    static constexpr int kA = kB + 32 * sizeof(V);
+    static constexpr int kRow = (NA * sizeof(T) + 15) / 16 * 16; // bytes of an A row
+    // (rounded up so that A rows start at a multiple of 128 bytes: kB and kA are multiples, too)
+    static __host__ __device__ constexpr int bytes(int side_by_side) {
+        return (kA + side_by_side * kRow + (side_by_side * 4 + 15) / 16 * 16 + 127) / 128 * 128;
+    }
+};
+
+template <int BYTES, int OFFSET> __device__ __forceinline__ void cp_async_at(unsigned dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0 + %1], [%2], %3;\n" ::"r"(dst), "n"(OFFSET), "l"(src), "n"(BYTES)
+                 : "memory");
+}
+template <int BYTES, int STEP, int C, int N>
+__device__ __forceinline__ void cp_async_rows(unsigned dst, const unsigned char* src, int64_t row_bytes) {
+    if constexpr (C < N) {
+        cp_async_at<BYTES, C * STEP>(dst, src + C * row_bytes);
+        cp_async_rows<BYTES, STEP, C + 1, N>(dst, src, row_bytes);
+    }
+}
+
+// How a warp takes the edges: several side by side (L <= 16 columns and f64 or f32 of one column per lane),
+// one at a time, or one at a time with L = 32 VEC columns (then every offset is a constant).
+enum Mode { kSideBySide = 0, kOneEdge = 1, kExact = 2 };
+
+// Walks rows [row_lo, row_hi) for columns [b0, ...) and c in [c0, c0 + nc): begin(row), step(w[NC] and B
+// of this lane, A row, edge, live), end(row) in order. All lanes together.
+//
+// One edge at a time the copies do not care about rows: they run along the positions, and a step is
+// straight-line code (wait, start the copies of the step seven ahead, read, multiply), which the
+// compiler can interleave: at 9 x 9 channels, f64, 337 -> 210 instructions per edge of the sums,
+// 640 -> 450 us at 10^6 edges.
+template <typename T, int VEC, int NA, int NC, Mode MODE, typename Off, typename Begin, typename Step, typename End>
+__device__ __forceinline__ void walk_rows(const RowsArgs<T>& g, const Off* __restrict__ offsets, int64_t row_lo,
+                                          int64_t row_hi, int b0, int c0, unsigned char* ring, int lane,
+                                          const Status& st, Begin&& begin, Step&& step, End&& end) {
+    using P = Pack<T, VEC>;
+    using V = typename P::V;
+    using Sl = Slot<T, VEC, NA, NC>;
+    constexpr bool kSide = MODE == kSideBySide;
+    const int LP = kSide ? g.lanes : 32, S = kSide ? 32 / LP : 1;
+    const int sub = kSide ? lane / LP : 0, lb = kSide ? lane & (LP - 1) : lane;
+    const int L = MODE == kExact ? 32 * VEC : g.L;
+    const int nc = g.nC - c0 < NC ? g.nC - c0 : NC;
+    const int b = MODE == kExact ? lane * VEC : b0 + lb * VEC;
+    const bool valid = MODE == kExact || b < L;
+    const int bc = valid ? b : L - VEC; // lanes beyond the last column read it again, with B = 0
+    const int slot_bytes = kSide ? Sl::bytes(S) : Sl::bytes(1);
+    const unsigned ring32 = static_cast<unsigned>(__cvta_generic_to_shared(ring));
+    const unsigned lane_off = lane * static_cast<unsigned>(sizeof(V));
+    // what no copy writes: channels beyond nc and nA, B of the lanes beyond the last column
+    for (int x = lane * 4; x < kDepth * slot_bytes; x += 128) *reinterpret_cast<int*>(ring + x) = 0;
+    __syncwarp();
+
+    const int p_lo = static_cast<int>(offsets[row_lo]), p_hi = static_cast<int>(offsets[row_hi]);
+    // Edge numbers and gathered rows, 32 positions per register: the block that the copies have
+    // reached (0), the next (1), and of the one after that the edge numbers only (2).
+    auto load_edge = [&](int base) {
+        int e = min(base + lane, p_hi - 1);
+        if (g.perm != nullptr) e = __ldg(g.perm + e);
+        return e;
+    };
+    auto load_row = [&](int e) {
+        int32_t r = __ldg(g.gather + e);
+        if (clamp_index(r, static_cast<int32_t>(g.rows))) report_bad_index(st, g.bit);
+        return r;
+    };
+    int block = p_lo;
+    int e0 = 0, e1 = 0, e2 = 0, g0 = 0, g1 = 0;
+    if (p_lo < p_hi) {
+        e0 = load_edge(block), e1 = load_edge(block + 32), e2 = load_edge(block + 64);
+        g0 = load_row(e0), g1 = load_row(e1);
+    }
+    auto next_block = [&] {
+        block += 32;
+        e0 = e1, g0 = g1, e1 = e2;
+        g1 = load_row(e1);
+        e2 = load_edge(block + 64);
+    };
+    constexpr int64_t kScalar = sizeof(T);
+    const unsigned char* g_base = reinterpret_cast<const unsigned char*>(g.G + static_cast<int64_t>(c0) * L + bc);
+    const int64_t g_row = g.nC * (L * kScalar);
+    const unsigned char* b_base = reinterpret_cast<const unsigned char*>(g.B + bc);
+    const unsigned char* a_base = reinterpret_cast<const unsigned char*>(g.A + lb);
+    constexpr int kStep = 32 * sizeof(V);
+    auto copy_edge = [&](int slot, int e, int r) { // W (or gO) row and B
+        const unsigned dst = ring32 + slot + lane_off;
+        const unsigned char* src = g_base + r * g_row;
+        if (nc == NC) {
+            cp_async_rows<sizeof(V), kStep, 0, NC>(dst, src, L * kScalar);
+        } else {
+            for (int c = 0; c < nc; c++) cp_async_at<sizeof(V), 0>(dst + c * kStep, src + c * (L * kScalar));
+        }
+        if (valid) cp_async_at<sizeof(V), Sl::kB>(dst, b_base + e * (L * kScalar));
+    };
+
+    // the copies: the next step to start
+    int64_t f_row = row_lo;
+    int f_p = p_lo, f_end = row_lo < row_hi ? static_cast<int>(offsets[row_lo + 1]) : p_lo;
+    auto start = [&](int slot) { // slot: byte offset in the ring
+        if constexpr (!kSide) { // (behind the last edge it is copied again: nobody reads it)
+            const int at = f_p - block;
+            const int e = __shfl_sync(kFullMask, e0, at), r = __shfl_sync(kFullMask, g0, at);
+            copy_edge(slot, e, r);
+            if (lb < g.nA)
+                cp_async<sizeof(T)>(ring + slot + Sl::kA + lb * sizeof(T), a_base + e * (g.nA * kScalar));
+            if (lane == 0) *reinterpret_cast<int*>(ring + slot + Sl::kA + Sl::kRow) = e;
+            f_p++;
+        } else {
+            while (f_p >= f_end && f_row + 1 < row_hi) {
+                f_row++;
+                f_end = static_cast<int>(offsets[f_row + 1]);
+            }
+            if (f_p < f_end) {
+                if (f_p >= block + 32) next_block();
+                const bool live = f_p + sub < f_end; // (a repeated edge counts as A = 0)
+                const int at = (live ? f_p + sub : f_end - 1) - block;
+                const int ea = __shfl_sync(kFullMask, e0, at & 31), eb = __shfl_sync(kFullMask, e1, at & 31);
+                const int ra = __shfl_sync(kFullMask, g0, at & 31), rb = __shfl_sync(kFullMask, g1, at & 31);
+                const int e = at < 32 ? ea : eb, r = at < 32 ? ra : rb;
+                copy_edge(slot, e, r);
+                unsigned char* a = ring + slot + Sl::kA + sub * Sl::kRow;
+                const unsigned char* a_src = a_base + e * (g.nA * kScalar);
+                for (int x = lb; x < g.nA; x += LP) {
+                    if (live)
+                        cp_async<sizeof(T)>(a + x * sizeof(T), a_src + (x - lb) * kScalar);
+                    else
+                        *reinterpret_cast<T*>(a + x * sizeof(T)) = T(0);
+                }
+                if (lb == 0) *reinterpret_cast<int*>(ring + slot + Sl::kA + S * Sl::kRow + sub * 4) = e;
+                f_p = min(f_p + S, f_end);
+            }
+        }
+        cp_async_commit();
+    };
+    if (p_lo < p_hi) {
+#pragma unroll 1
+        for (int s = 0; s < kDepth - 1; s++) start(s * slot_bytes);
+    }
+
+    int slot = 0, before = (kDepth - 1) * slot_bytes; // byte offsets of this step's slot and the last one's
+    int lo = p_lo;
+    for (int64_t row = row_lo; row < row_hi; row++) {
+        const int hi = static_cast<int>(offsets[row + 1]);
+        begin(row, lo < hi);
+#pragma unroll 1
+        for (int p = lo; p < hi; p += S) {
+            cp_async_wait<kDepth - 2>();
+            __syncwarp();
+            start(before);
+            V w[NC];
+            const unsigned char* from = ring + slot;
+#pragma unroll
+            for (int c = 0; c < NC; c++)
+                w[c] = *reinterpret_cast<const V*>(from + lane_off + c * (32 * sizeof(V)));
+            const V bv = *reinterpret_cast<const V*>(from + lane_off + Sl::kB);
+            const T* a = reinterpret_cast<const T*>(from + Sl::kA + sub * Sl::kRow);
+            const int* e = reinterpret_cast<const int*>(from + Sl::kA + S * Sl::kRow) + sub;
+            step(w, bv, a, e, !kSide || p + sub < hi);
+            before = slot;
+            slot += slot_bytes;
+            if (slot == kDepth * slot_bytes) slot = 0;
+            if (!kSide && f_p == block + 32) next_block();
+        }
+        end(row);
+        lo = hi;
+    }
+    cp_async_wait<0>();
+    __syncwarp();
+}
+
+// The A row of an edge in registers (16-byte loads).
+template <typename T, int NA> __device__ __forceinline__ void load_a(const T* a, T (&out)[NA]) {
+    constexpr int N = 16 / sizeof(T);
+#pragma unroll
+    for (int x = 0; x < NA; x += N) {
+        T v[N];
+        load_vec<T, N>(a + x, v);
+#pragma unroll
+        for (int i = 0; i < N; i++)
+            if (x + i < NA) out[x + i] = v[i];
+    }
+}
+
+// out[o] (+)= sum_{a,c} D[o][a][c0 + c] acc[a][c] for the lane's column, o = 0 .. nOut - 1.
+template <typename T, int VEC, int NA, int NC>
+__device__ __forceinline__ void contract_row(const RowsArgs<T>& g, const T* D, T* out,
+                                             typename Pack<T, VEC>::V (&acc)[NA][NC], int c0, bool store,
+                                             bool add_to) {
+    using P = Pack<T, VEC>;
+    using V = typename P::V;
+    for (int o = 0; o < g.nOut; o += kTableOut) {
+        V v[kTableOut];
+#pragma unroll
+        for (int u = 0; u < kTableOut; u++) v[u] = V(0);
+        const T* d = D + static_cast<size_t>(o) * NA * g.pad_c + c0;
+#pragma unroll
+        for (int a = 0; a < NA; a++)
+#pragma unroll
+            for (int c = 0; c < NC; c++)
+#pragma unroll
+                for (int u = 0; u < kTableOut; u++)
+                    v[u] = P::fma(P::dup(d[(u * NA + a) * g.pad_c + c]), acc[a][c], v[u]);
+#pragma unroll
+        for (int u = 0; u < kTableOut; u++) {
+            for (int x = g.lanes; x < 32; x <<= 1) v[u] = P::add(v[u], P::shift(v[u], x));
+            if (store && o + u < g.nOut) {
+                V* dst = reinterpret_cast<V*>(out + static_cast<int64_t>(o + u) * g.L);
+                *dst = add_to ? P::add(*dst, v[u]) : v[u];
+            }
+        }
+    }
+}
+
+// Forward, and the gW part of the gradients: `out` is [rows][nOut][L].
+template <typename T, int VEC, int NA, int NC, Mode MODE, typename Off>
+__device__ __forceinline__ void outer_rows(const RowsArgs<T>& g, const Off* __restrict__ offsets,
+                                           T* __restrict__ out, int64_t row_lo, int64_t row_hi, const T* D,
+                                           unsigned char* ring, int lane, const Status& st) {
+    using P = Pack<T, VEC>;
+    using V = typename P::V;
+    const int lb = lane & (g.lanes - 1);
+    for (int b0 = 0; b0 < g.L; b0 += 32 * VEC) {
+        const int b = b0 + lb * VEC;
+        const bool store = lane < g.lanes && b < g.L;
+        for (int c0 = 0; c0 < g.nC; c0 += NC) {
+            V acc[NA][NC];
+            walk_rows<T, VEC, NA, NC, MODE>(
+                g, offsets, row_lo, row_hi, b0, c0, ring, lane, st,
+                [&](int64_t, bool) {
+#pragma unroll
+                    for (int a = 0; a < NA; a++)
+#pragma unroll
+                        for (int c = 0; c < NC; c++) acc[a][c] = V(0);
+                },
+                [&](V(&w)[NC], V bv, const T* a_row, const int*, bool) {
+                    T A[NA];
+                    load_a<T, NA>(a_row, A);
+#pragma unroll
+                    for (int c = 0; c < NC; c++) w[c] = P::mul(w[c], bv);
+#pragma unroll
+                    for (int a = 0; a < NA; a++) {
+                        const V av = P::dup(A[a]);
+#pragma unroll
+                        for (int c = 0; c < NC; c++) acc[a][c] = P::fma(av, w[c], acc[a][c]);
+                    }
+                },
+                [&](int64_t row) {
+                    contract_row<T, VEC, NA, NC>(g, D, out + row * g.nOut * g.L + b, acc, c0, store, c0 > 0);
+                });
+        }
+    }
+}
+
+// Adds NP values over the LP lanes of an edge and stores them, dst[0 .. n). While a lane holds several
+// values it hands half of them to its partner and takes the partner's share of the other half, so
+// that NP values cost about NP shuffles and not NP log LP.
+template <int O, typename T, int NP, int LP>
+__device__ __forceinline__ void sum_level(T (&v)[NP], int lb, int& which) {
+    constexpr int kHeld = NP * O * 2 / LP; // values a lane holds at this level, if more than one
+    if constexpr (kHeld > 1) {
+        const bool upper = lb & O;
+#pragma unroll
+        for (int i = 0; i < kHeld / 2; i++) {
+            const T send = upper ? v[i] : v[i + kHeld / 2];
+            const T mine = upper ? v[i + kHeld / 2] : v[i];
+            v[i] = mine + __shfl_xor_sync(kFullMask, send, O);
+        }
+        which += upper ? kHeld / 2 : 0;
+    } else {
+        v[0] += __shfl_xor_sync(kFullMask, v[0], O);
+    }
+    if constexpr (O > 1) sum_level<O / 2, T, NP, LP>(v, lb, which);
+}
+template <typename T, int NP, int LP>
+__device__ __forceinline__ void sum_lanes(T (&v)[NP], int lb, T* dst, int n, bool live, bool first) {
+    int which = 0;
+    sum_level<LP / 2, T, NP, LP>(v, lb, which);
+    constexpr int kLeft = NP > LP ? NP / LP : 1, kCopies = LP > NP ? LP / NP : 1;
+    if (live && (lb & (kCopies - 1)) == 0) {
+#pragma unroll
+        for (int i = 0; i < kLeft; i++)
+            if (which + i < n) dst[which + i] = first ? v[i] : dst[which + i] + v[i];
+    }
+}
+
+// The same without selecting, for one edge per warp: lane `lb` holds its values in the order i ^ mask,
+// with the mask below, so that what it hands over is always the upper half. M of the NA values (a
+// power of two) go this way, the ninth of nine by itself.
+__device__ __forceinline__ int sum_mask(int lane, int m) {
+    int mask = 0;
+    for (int o = 16, h = m / 2; h >= 1; o /= 2, h /= 2)
+        if (lane & o) mask |= h;
+    return mask;
+}
+template <int O, int HELD, typename T, int NA> __device__ __forceinline__ void sum_ordered(T (&v)[NA]) {
+    if constexpr (HELD > 1) {
+#pragma unroll
+        for (int i = 0; i < HELD / 2; i++) v[i] += __shfl_xor_sync(kFullMask, v[i + HELD / 2], O);
+    } else {
+        v[0] += __shfl_xor_sync(kFullMask, v[0], O);
+    }
+    if constexpr (O > 1) sum_ordered<O / 2, (HELD > 1 ? HELD / 2 : 1), T, NA>(v);
+}
+
+// gA and gB. `own` is the matrix of the rows themselves, [rows][nOut][L] (W, where the rows are
+// those of W and g.G is gO).
+template <typename T, int VEC, int NA, int NC, Mode MODE, typename Off>
+__device__ __forceinline__ void edge_gradients(const RowsArgs<T>& g, const Off* __restrict__ offsets,
+                                               T* __restrict__ gA, T* __restrict__ gB,
+                                               const T* __restrict__ own, int64_t row_lo, int64_t row_hi,
+                                               const T* D, unsigned char* ring, int lane, const Status& st) {
+    using P = Pack<T, VEC>;
+    using V = typename P::V;
+    constexpr int NP = NA <= 4 ? 4 : 16;              // values in the sums over lanes, padded
+    constexpr int M = NA <= 4 ? 4 : NA <= 9 ? 8 : 16; // ... that are taken in the lane's own order
+    constexpr bool kOrdered = MODE != kSideBySide;
+    const int LP = g.lanes, lb = lane & (LP - 1);
+    const int mask = kOrdered ? sum_mask(lane, M) : 0;
+    for (int b0 = 0; b0 < g.L; b0 += 32 * VEC) {
+        const int b = b0 + lb * VEC, bc = b < g.L ? b : g.L - VEC;
+        for (int c0 = 0; c0 < g.nC; c0 += NC) {
+            const bool first = b0 == 0 && c0 == 0;
+            V E[NA][NC];
+            walk_rows<T, VEC, NA, NC, MODE>(
+                g, offsets, row_lo, row_hi, b0, c0, ring, lane, st,
+                [&](int64_t row, bool any) {
+                    if (!any) return;
+#pragma unroll
+                    for (int a = 0; a < NA; a++)
+#pragma unroll
+                        for (int c = 0; c < NC; c++) E[a][c] = V(0);
+                    const T* src = own + row * g.nOut * g.L + bc;
+                    V next = *reinterpret_cast<const V*>(src);
+                    for (int o = 0; o < g.nOut; o++) {
+                        const V v = next;
+                        if (o + 1 < g.nOut) next = *reinterpret_cast<const V*>(src + static_cast<int64_t>(o + 1) * g.L);
+                        const T* d = D + static_cast<size_t>(o) * NA * g.pad_c + c0;
+#pragma unroll
+                        for (int a = 0; a < NA; a++)
+#pragma unroll
+                            for (int c = 0; c < NC; c++)
+                                E[a][c] = P::fma(P::dup(d[(a < M ? a ^ mask : a) * g.pad_c + c]), v, E[a][c]);
+                    }
+                },
+                [&](V(&w)[NC], V bv, const T* a_row, const int* edge, bool live) {
+                    const int64_t e = *edge;
+                    V z[NA];
+#pragma unroll
+                    for (int a = 0; a < NA; a++) {
+                        z[a] = P::mul(E[a][0], w[0]);
+#pragma unroll
+                        for (int c = 1; c < NC; c++) z[a] = P::fma(E[a][c], w[c], z[a]);
+                    }
+                    if (gB != nullptr) {
+                        T A[NA];
+                        if constexpr (kOrdered) {
+#pragma unroll
+                            for (int a = 0; a < NA; a++) A[a] = a_row[a < M ? a ^ mask : a];
+                        } else {
+                            load_a<T, NA>(a_row, A);
+                        }
+                        V s0 = P::mul(P::dup(A[0]), z[0]), s1 = V(0);
+#pragma unroll
+                        for (int a = 1; a < NA; a++)
+                            (a & 1 ? s1 : s0) = P::fma(P::dup(A[a]), z[a], a & 1 ? s1 : s0);
+                        s0 = P::add(s0, s1);
+                        if (live && b < g.L) {
+                            V* dst = reinterpret_cast<V*>(gB + e * g.L + b);
+                            *dst = c0 > 0 ? P::add(*dst, s0) : s0;
+                        }
+                    }
+                    if (gA != nullptr) {
+                        T* dst = gA + e * g.nA;
+                        if constexpr (kOrdered) {
+                            T v[NA];
+#pragma unroll
+                            for (int a = 0; a < NA; a++) v[a] = P::sum(P::mul(z[a], bv));
+                            T last = T(0);
+                            if constexpr (NA > M) last = warp_sum(v[M]);
+                            sum_ordered<16, M, T, NA>(v);
+                            if ((lane & (32 / M - 1)) == 0 && mask < g.nA)
+                                dst[mask] = first ? v[0] : dst[mask] + v[0];
+                            if (NA > M && lane == 1 && M < g.nA) dst[M] = first ? last : dst[M] + last;
+                        } else {
+                            T v[NP];
+#pragma unroll
+                            for (int a = 0; a < NP; a++)
+                                v[a] = a < NA ? P::sum(P::mul(z[a < NA ? a : 0], bv)) : T(0);
+                            switch (LP) { // (uniform)
+                            case 16: sum_lanes<T, NP, 16>(v, lb, dst, g.nA, live, first); break;
+                            case 8: sum_lanes<T, NP, 8>(v, lb, dst, g.nA, live, first); break;
+                            default: sum_lanes<T, NP, 4>(v, lb, dst, g.nA, live, first); break;
+                            }
+                        }
+                    }
+                },
+                [&](int64_t) {});
+        }
+    }
+}
+
+// ---- kernels
+// A block owns a range of rows (the blocks share the edges evenly); its warps take them a few at a
+// time, about kChunkEdges edges, so that none waits for another's long rows
+// (60 000 edges, 1000 rows: 63 -> 45 us against rows dealt out beforehand).
+constexpr int kChunkEdges = 256;
+template <typename Off> __device__ __forceinline__ int chunk_rows(const Off* offsets, int64_t lo, int64_t hi) {
+    const int64_t edges = offsets[hi] - offsets[lo], rows = hi - lo;
+    if (edges <= 0) return 256;
+    const int64_t n = kChunkEdges * rows / edges, fair = rows / (2 * kRowWarps);
+    return static_cast<int>(n < 1 || fair < 1 ? 1 : n < fair ? n : fair);
+}
+template <typename Off, typename F>
+__device__ __forceinline__ void for_block_rows(const Off* offsets, int64_t rows, int* counter, int lane, F&& f) {
+    const int64_t lo = balanced_row_split(offsets, rows, blockIdx.x, gridDim.x, lane);
+    const int64_t hi = balanced_row_split(offsets, rows, blockIdx.x + 1, gridDim.x, lane);
+    const int n = chunk_rows(offsets, lo, hi);
+    while (true) {
+        int at = 0;
+        if (lane == 0) at = atomicAdd(counter, n);
+        const int64_t r = lo + __shfl_sync(kFullMask, at, 0);
+        if (r >= hi) break;
+        f(r, r + n < hi ? r + n : hi);
+    }
+}
+
+// Shared memory of the kernels: the table, the rings, and a counter of rows taken.
+template <typename T, int VEC, int NA, int NC> struct RowsShared {
+    T* D;
+    unsigned char* ring;
+    int* counter;
+    __device__ RowsShared(const RowsArgs<T>& g, unsigned char* smem, int* c, int warp) : counter(c) {
+        D = reinterpret_cast<T*>(smem);
+        const int size = g.pad_out * NA * g.pad_c;
+        if (threadIdx.x == 0) *counter = 0;
+        for (int x = threadIdx.x; x < size; x += kRowWarps * 32) D[x] = g.D[x];
+        ring = smem + static_cast<int>(size * sizeof(T) + 127) / 128 * 128 +
+               warp * kDepth * Slot<T, VEC, NA, NC>::bytes(32 / g.lanes);
+        __syncthreads();
+    }
+};
+
+// Forward (rows of the scatter index, `offsets`, or `starts` with a permutation when that turned out not
+// to be sorted) and gW (rows of W, `starts`).
+enum RowsRun { kSorted = 0, kIfUnsorted = 1, kAlways = 2 };
+
+template <typename T, int VEC, int NA, int NC, Mode MODE>
+__global__ void __launch_bounds__(kRowWarps * 32, 1)
+sasaw_sum_rows(const __grid_constant__ RowsArgs<T> g, const int64_t* __restrict__ offsets,
+               const int32_t* __restrict__ starts, T* __restrict__ out, RowsRun run, Status st) {
+    if (run != kAlways && saw_unsorted(st) != (run == kIfUnsorted)) return;
+    __shared__ int counter;
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int warp = __shfl_sync(kFullMask, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    const RowsShared<T, VEC, NA, NC> sh(g, smem, &counter, warp);
+    if (run == kSorted)
+        for_block_rows(offsets, g.rows, sh.counter, lane, [&](int64_t lo, int64_t hi) {
+            outer_rows<T, VEC, NA, NC, MODE>(g, offsets, out, lo, hi, sh.D, sh.ring, lane, st);
+        });
+    else
+        for_block_rows(starts, g.rows, sh.counter, lane, [&](int64_t lo, int64_t hi) {
+            outer_rows<T, VEC, NA, NC, MODE>(g, starts, out, lo, hi, sh.D, sh.ring, lane, st);
+        });
+}
+
+// gA and gB. (A kernel of its own: gathering for gW at the same time in half of the warps saves DRAM
+// traffic, but with both loops in one kernel the registers do not suffice.)
+template <typename T, int VEC, int NA, int NC, Mode MODE>
+__global__ void __launch_bounds__(kRowWarps * 32, 1)
+sasaw_edge_gradients(const __grid_constant__ RowsArgs<T> g, const int32_t* __restrict__ starts, T* __restrict__ gA,
+                     T* __restrict__ gB, const T* __restrict__ W, Status st) {
+    __shared__ int counter;
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int warp = __shfl_sync(kFullMask, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    const RowsShared<T, VEC, NA, NC> sh(g, smem, &counter, warp);
+    for_block_rows(starts, g.rows, sh.counter, lane, [&](int64_t lo, int64_t hi) {
+        edge_gradients<T, VEC, NA, NC, MODE>(g, starts, gA, gB, W, lo, hi, sh.D, sh.ring, lane, st);
+    });
+}
+
+// ---- the order of the edges by a row index: row starts and permutation (a counting sort)
+__global__ void __launch_bounds__(kSortThreads)
+order_edges_grid(EntrySort s, const int32_t* __restrict__ P, int64_t E, int64_t rows, int bit, Status st) {
+    sort_entries(s, P, E, rows, true, st, [] { cooperative_groups::this_grid().sync(); }, bit);
+}
+__global__ void __launch_bounds__(kSortThreads)
+order_edges_block(EntrySort s, const int32_t* __restrict__ P, int64_t E, int64_t rows, int bit, Status st) {
+    sort_entries(s, P, E, rows, true, st, [] { __syncthreads(); }, bit);
+}
+
+// ---- dispatch
+// Channel counts are padded to the next instantiation: A to 4, 9, 16 (spherical harmonics up to
+// l = 1, 2, 3), the other one to at most 81 products, several passes where it is wider.
+inline int pad_a(int n) { return n <= 4 ? 4 : n <= 9 ? 9 : 16; }
+inline int chunk_c(int na, int n) { return n <= 4 ? 4 : na <= 9 ? 9 : n <= 5 || n > 8 ? 5 : 4; }
+
+template <typename T> struct RowsShape {
+    RowsArgs<T> g;
+    int na, nc, vec, blocks;
+    size_t smem;
+    size_t table_bytes;
+};
+
+template <typename T>
+RowsShape<T> rows_shape(const Call& call, const SasawProblem<T>& p, const T* gathered, bool out_is_m2, int vec) {
+    RowsShape<T> s{};
+    s.na = pad_a(p.nA);
+    s.g.nC = out_is_m2 ? p.nO : p.nW;
+    s.g.nOut = out_is_m2 ? p.nW : p.nO;
+    s.nc = chunk_c(s.na, s.g.nC);
+    s.vec = vec;
+    s.g.A = p.A, s.g.B = p.B, s.g.G = gathered;
+    s.g.rows = p.rows, s.g.nA = p.nA, s.g.L = p.L;
+    s.g.pad_c = static_cast<int>(ceil_div(s.g.nC, s.nc)) * s.nc;
+    s.g.pad_out = static_cast<int>(ceil_div(s.g.nOut, kTableOut)) * kTableOut;
+    int lanes = 4;
+    while (lanes < 32 && lanes * vec < p.L) lanes *= 2;
+    s.g.lanes = lanes;
+    s.table_bytes = static_cast<size_t>(s.g.pad_out) * s.na * s.g.pad_c * sizeof(T);
+    // (Slot::bytes)
+    size_t slot = static_cast<size_t>(s.nc + 1) * 32 * vec * sizeof(T) +
+                        (32 / lanes) * ((s.na * sizeof(T) + 15) / 16 * 16) + (32 / lanes * 4 + 15) / 16 * 16;
+    slot = (slot + 127) / 128 * 128;
+    s.smem = (s.table_bytes + 127) / 128 * 128 + slot * kDepth * kRowWarps;
+    return s;
+}
+
+template <typename T, typename F> void for_shape(const RowsShape<T>& s, F&& f) {
+    auto with = [&](auto vec, auto na, auto nc) {
+        constexpr int VEC = decltype(vec)::value, NA = decltype(na)::value, NC = decltype(nc)::value;
+        using I = std::integral_constant<int, VEC>;
+        using A = std::integral_constant<int, NA>;
+        using X = std::integral_constant<int, NC>;
+        if (s.g.L == 32 * VEC)
+            f(I(), A(), X(), std::integral_constant<Mode, kExact>());
+        else if (VEC == 2 || s.g.lanes == 32)
+            f(I(), A(), X(), std::integral_constant<Mode, kOneEdge>());
+        else if constexpr (VEC == 1)
+            f(I(), A(), X(), std::integral_constant<Mode, kSideBySide>());
+    };
+    auto widths = [&](auto vec) {
+        using I4 = std::integral_constant<int, 4>;
+        using I5 = std::integral_constant<int, 5>;
+        using I9 = std::integral_constant<int, 9>;
+        using I16 = std::integral_constant<int, 16>;
+        if (s.na == 4)
+            s.nc == 4 ? with(vec, I4(), I4()) : with(vec, I4(), I9());
+        else if (s.na == 9)
+            s.nc == 4 ? with(vec, I9(), I4()) : with(vec, I9(), I9());
+        else
+            s.nc == 4 ? with(vec, I16(), I4()) : with(vec, I16(), I5());
+    };
+    if constexpr (sizeof(T) == 4) {
+        if (s.vec == 2) {
+            widths(std::integral_constant<int, 2>());
+            return;
+        }
+    }
+    widths(std::integral_constant<int, 1>());
+}
+
+template <typename T> bool rows_apply(const SasawProblem<T>& p) {
+    return p.nA >= 1 && p.nA <= kWidest && p.nW >= 1 && p.nW <= kWidest && p.nO >= 1 && p.nO <= kWidest &&
+           p.L >= 1 && p.E >= 1 && p.E <= INT32_MAX - 64 && p.rows >= 1 && p.N <= (1 << 20);
+}
+
+// Two columns per lane (f32) from 33 columns on, where every operand allows 8-byte accesses.
+template <typename T> int vector_width(int L, std::initializer_list<const void*> operands) {
+    if (sizeof(T) == 8 || L % 2 != 0 || L <= 32) return 1;
+    for (const void* p : operands)
+        if (reinterpret_cast<uintptr_t>(p) % 8 != 0) return 1;
+    return 2;
+}
+
+template <typename T>
+TableRef dense_table(const Call& call, const SasawProblem<T>& p, const RowsShape<T>& s, bool out_is_m2) {
+    TableKey key{};
+    key.kind = kSasawDenseTable;
+    key.scalar_bytes = static_cast<int>(sizeof(T));
+    key.ptr[0] = p.C, key.ptr[1] = p.M1, key.ptr[2] = p.M2, key.ptr[3] = p.M3;
+    key.n[0] = p.N, key.n[1] = p.nA, key.n[2] = p.nW, key.n[3] = p.nO, key.n[4] = out_is_m2 ? 1 : 0;
+    TableRef ref = acquire_table(call, key, s.table_bytes);
+    if (ref.fresh) {
+        const int64_t warps = static_cast<int64_t>(s.g.pad_out) * s.na * s.g.pad_c;
+        sasaw_dense_table<T><<<static_cast<unsigned>(ceil_div(warps, 8)), 256, 0, call.stream>>>(
+            static_cast<T*>(ref.ptr), p.C, p.M1, p.M2, p.M3, p.N, p.nA, p.nW, p.nO, out_is_m2, s.g.pad_out, s.na,
+            s.g.pad_c, call.status);
+        MOPS_CUDA_OK(cudaGetLastError());
+        commit_table(call, ref);
+    }
+    return ref;
+}
+
+// One block per SM, fewer for few rows.
+inline unsigned rows_blocks(const Call& call, int64_t rows) {
+    return static_cast<unsigned>(std::min<int64_t>(rows, sm_count(call.device)));
+}
+
+template <typename T>
+void launch_sums(const Call& call, const RowsShape<T>& s, unsigned blocks, const int64_t* offsets,
+                 const int32_t* starts, T* out, RowsRun when) {
+    for_shape(s, [&](auto vec, auto na, auto nc, auto mode) {
+        auto kernel = sasaw_sum_rows<T, decltype(vec)::value, decltype(na)::value, decltype(nc)::value,
+                                     decltype(mode)::value>;
+        allow_dynamic_smem(kernel, call.device, s.smem);
+        kernel<<<blocks, kRowWarps * 32, s.smem, call.stream>>>(s.g, offsets, starts, out, when, call.status);
+    });
+    MOPS_CUDA_OK(cudaGetLastError());
+}
+
+} // namespace
+
+template <typename T> bool sasaw_forward_rows(const Call& call, const SasawProblem<T>& p, T* O) {
+    if (!rows_apply(p)) return false;
+    RowsShape<T> s = rows_shape(call, p, p.W, false, vector_width<T>(p.L, {p.B, p.W, O}));
+    if (s.smem > static_cast<size_t>(max_optin_smem(call.device))) return false;
+    TableRef table = dense_table(call, p, s, false);
+    SegmentTable seg = segment_table(call, p.I, p.E, p.rows);
+    s.g.gather = p.J, s.g.perm = nullptr, s.g.D = static_cast<const T*>(table.ptr), s.g.bit = kBitJ;
+    const unsigned blocks = rows_blocks(call, p.rows);
+    note_kernel_f("sasaw_sum_rows<%s,VEC=%d,NA=%d,NC=%d>", scalar_name<T>(), s.vec, s.na, s.nc);
+    auto run = [&](RowsRun when, const int32_t* starts) { launch_sums(call, s, blocks, seg.offsets, starts, O, when); };
+    run(kSorted, nullptr);
+    bool unsorted = !seg.known_sorted; // asynchronous calls cannot look: always enqueue
+    if (unsorted && call.wait) {
+        wait_stream(call);
+        unsorted = host_saw_unsorted(call);
+    }
+    if (unsorted) {
+        const int sorters = sort_blocks(call, p.E);
+        void* scratch = scratch_alloc(call, entry_sort_bytes(p.E, p.rows, sorters));
+        const EntrySort sort = entry_sort_at(scratch, p.rows, sorters);
+        launch_sorting(call, sorters, sort_if_unsorted_grid, sort_if_unsorted_block, sort, p.I, p.E, p.rows,
+                       call.status);
+        s.g.perm = sort.perm;
+        run(kIfUnsorted, sort.starts);
+        scratch_free(call, scratch);
+    }
+    release_table(call, seg.ref);
+    release_table(call, table);
+    return true;
+}
+
+template <typename T>
+bool sasaw_backward_rows(const Call& call, const SasawProblem<T>& p, T* gA, T* gB, T* gW, const T* gO) {
+    if (!rows_apply(p)) return false;
+    RowsShape<T> s = rows_shape(call, p, gO, true, vector_width<T>(p.L, {p.B, p.W, gO, gB, gW}));
+    if (s.smem > static_cast<size_t>(max_optin_smem(call.device))) return false;
+    TableRef table = dense_table(call, p, s, true);
+    // the edges in the order of J
+    const int sorters = sort_blocks(call, p.E);
+    TableKey key{};
+    key.kind = kEdgeOrder;
+    key.ptr[0] = p.J;
+    key.n[0] = p.E, key.n[1] = p.rows;
+    TableRef order = acquire_table(call, key, entry_sort_bytes(p.E, p.rows, sorters));
+    const EntrySort sort = entry_sort_at(order.ptr, p.rows, sorters);
+    if (order.fresh) {
+        launch_sorting(call, sorters, order_edges_grid, order_edges_block, sort, p.J, p.E, p.rows,
+                       static_cast<int>(kBitJ), call.status);
+        commit_table(call, order);
+    }
+    s.g.gather = p.I, s.g.perm = sort.perm, s.g.D = static_cast<const T*>(table.ptr), s.g.bit = kBitI;
+    const unsigned blocks = rows_blocks(call, p.rows);
+    if (gW != nullptr) {
+        note_kernel_f("sasaw_sum_rows<%s,VEC=%d,NA=%d,NC=%d>", scalar_name<T>(), s.vec, s.na, s.nc);
+        launch_sums(call, s, blocks, nullptr, sort.starts, gW, kAlways);
+    }
+    if (gA != nullptr || gB != nullptr) {
+        note_kernel_f("sasaw_edge_gradients<%s,VEC=%d,NA=%d,NC=%d>", scalar_name<T>(), s.vec, s.na, s.nc);
+        for_shape(s, [&](auto vec, auto na, auto nc, auto mode) {
+            auto kernel = sasaw_edge_gradients<T, decltype(vec)::value, decltype(na)::value, decltype(nc)::value,
+                                               decltype(mode)::value>;
+            allow_dynamic_smem(kernel, call.device, s.smem);
+            kernel<<<blocks, kRowWarps * 32, s.smem, call.stream>>>(s.g, sort.starts, gA, gB, p.W, call.status);
+        });
+        MOPS_CUDA_OK(cudaGetLastError());
+    }
+    release_table(call, order);
+    release_table(call, table);
+    return true;
+}
+
+#define INSTANTIATE(T)                                                                             \
+    template bool sasaw_forward_rows<T>(const Call&, const SasawProblem<T>&, T*);                  \
+    template bool sasaw_backward_rows<T>(const Call&, const SasawProblem<T>&, T*, T*, T*, const T*);
+INSTANTIATE(float)
+INSTANTIATE(double)
+
+} // namespace mops_b200

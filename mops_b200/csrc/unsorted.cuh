@@ -70,7 +70,8 @@ __device__ __forceinline__ int block_scan(int v, int& exclusive, int32_t* warp_s
 // Out-of-range rows are reported, and left out or (keep_bad) taken for row 0.
 template <typename Sync>
 __device__ __forceinline__ void sort_entries(const EntrySort& s, const int32_t* __restrict__ P, int64_t J,
-                                             int64_t n_rows, bool keep_bad, const Status& st, Sync&& sync) {
+                                             int64_t n_rows, bool keep_bad, const Status& st, Sync&& sync,
+                                             int bit = 0) {
     __shared__ int32_t warp_sums[33];
     const int64_t thread = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     const int64_t threads = static_cast<int64_t>(gridDim.x) * blockDim.x;
@@ -83,7 +84,7 @@ __device__ __forceinline__ void sort_entries(const EntrySort& s, const int32_t* 
     for (int64_t j = thread; j < J; j += threads) {
         const int row = row_of(j);
         if (row >= 0) atomicAdd(s.starts + row, 1);
-        if (static_cast<uint32_t>(__ldg(P + j)) >= static_cast<uint32_t>(n_rows)) report_bad_index(st, 0);
+        if (static_cast<uint32_t>(__ldg(P + j)) >= static_cast<uint32_t>(n_rows)) report_bad_index(st, bit);
     }
     sync();
     // block b scans the rows [b per, (b + 1) per)
