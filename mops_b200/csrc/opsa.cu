@@ -472,12 +472,11 @@ void launch_fwd_mma_l(int L, unsigned blocks, cudaStream_t stream, Args... args)
 
 // ------------------------------------------------------------- streaming kernels, host side
 template <typename T, bool WEIGHTED>
-bool pipe_usable(const T* A, const T* B, const T* W, const void* extra, int K, int L, bool vjp) {
+bool pipe_usable(const T* A, const T* B, const T* W, const void* extra, int K, int L) {
     auto aligned = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
     if (K < 1 || K > 16 || L < 1 || L > 32) return false;
     if (!aligned(A) || !aligned(B) || !aligned(extra)) return false;
     if (WEIGHTED && (!aligned(W) || (L * sizeof(T)) % 16 != 0)) return false;
-    if (vjp && (static_cast<size_t>(K) * L * sizeof(T)) % 16 != 0) return false;
     return true;
 }
 
@@ -536,7 +535,7 @@ void launch_fwd_pipe_l(const Call& call, const PipeLayout& lay, int64_t nO, Args
 template <typename T, bool WEIGHTED>
 bool forward_pipe(const Call& call, T* O, const T* A, const T* B, const T* W, const int32_t* PW,
                   const int64_t* offsets, int64_t J, int K, int L, int64_t nO) {
-    if (!pipe_usable<T, WEIGHTED>(A, B, W, nullptr, K, L, false)) return false;
+    if (!pipe_usable<T, WEIGHTED>(A, B, W, nullptr, K, L)) return false;
     const PipeLayout lay = choose_pipe_layout<T, WEIGHTED>(K, L, false);
     if (static_cast<size_t>(lay.warp_bytes) * kPipeWarps > static_cast<size_t>(max_optin_smem(call.device)))
         return false;
@@ -1262,7 +1261,7 @@ void backward(const Call& call, T* gA, T* gB, T* gW, const T* gO, const T* A, co
     // f64 operands it cannot take (alignment) the kernel that loads its fragments from global
     // memory; otherwise, and whenever the index turns out unsorted, the entry-per-lane kernels
     // below do the work.
-    const bool streaming = pipe_usable<T, WEIGHTED>(A, B, W, gO, K, L, true);
+    const bool streaming = pipe_usable<T, WEIGHTED>(A, B, W, gO, K, L);
     if (K <= 16 && L <= 32 && (streaming || sizeof(T) == 8)) {
         const int sms = sm_count(call.device);
         SegmentTable seg = segment_table(call, P, J, nO);
@@ -1291,10 +1290,11 @@ void backward(const Call& call, T* gA, T* gB, T* gW, const T* gO, const T* A, co
             plan.only_if_unsorted = true; // asynchronous calls cannot look: always enqueue
         }
     }
-    // An index that is not sorted: take the entries in the order of their rows.
+    // An index that is not sorted: take the entries in the order of their rows. (Asynchronous calls
+    // do without: the sort would be one more launch for every call on a sorted index, 3 us each.)
     plan.perm = nullptr;
     void* scratch = nullptr;
-    if (plan.only_if_unsorted && J <= INT32_MAX) {
+    if (plan.only_if_unsorted && call.wait && J <= INT32_MAX) {
         const int blocks = sort_blocks(call, J);
         scratch = scratch_alloc(call, entry_sort_bytes(J, nO, blocks));
         const EntrySort sort = entry_sort_at(scratch, nO, blocks);

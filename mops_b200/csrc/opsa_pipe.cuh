@@ -38,6 +38,29 @@ constexpr int kPipeWarps = 4;
 
 __host__ __device__ constexpr int round16(size_t n) { return static_cast<int>((n + 15) / 16 * 16); }
 
+// A slot of the grad_output ring: rows whose size is no multiple of 16 bytes start up to 15 bytes behind
+// a 16-byte boundary and are copied from that boundary on.
+__host__ __device__ constexpr int grad_slot_bytes(int g_bytes) {
+    return round16(g_bytes) + (g_bytes % 16 != 0 ? 16 : 0);
+}
+
+// Starts the copy of grad_output row r into `slot` (one lane). What a whole number of 16-byte pieces
+// would read behind the end of the array goes by plain stores.
+template <typename S>
+__device__ __forceinline__ void issue_grad_row(unsigned char* slot, const S* gO, int64_t r, int64_t rows,
+                                               int g_bytes, uint64_t* bar) {
+    const int64_t start = r * g_bytes, from = start & ~int64_t(15), total = rows * g_bytes;
+    const int64_t end = (start + g_bytes + 15) & ~int64_t(15);
+    const int64_t whole = end <= total ? end : total & ~int64_t(15); // start of the last, partial piece
+    const unsigned bytes = whole > from ? static_cast<unsigned>(whole - from) : 0;
+    mbarrier_arrive_expect(bar, bytes);
+    const unsigned char* src = reinterpret_cast<const unsigned char*>(gO) + from;
+    if (bytes > 0) bulk_copy_in(slot, src, bytes, bar);
+    if (end > total)
+        for (int64_t x = whole - from; x < total - from; x += sizeof(S))
+            *reinterpret_cast<S*>(slot + x) = *reinterpret_cast<const S*>(src + x);
+}
+
 __host__ __device__ constexpr PipeLayout pipe_layout(size_t s, int K, int L, bool weighted, bool vjp, int ch,
                                                      int stages, int g_slots = 2) {
     PipeLayout p{};
@@ -58,7 +81,7 @@ __host__ __device__ constexpr PipeLayout pipe_layout(size_t s, int K, int L, boo
     p.g_bytes = static_cast<int>(static_cast<size_t>(K) * L * s);
     p.g_off = p.stages * p.stage_bytes;
     p.g_slots = g_slots < 2 ? 1 : 2;
-    p.bar_off = p.g_off + (vjp ? p.g_slots * round16(p.g_bytes) : 0);
+    p.bar_off = p.g_off + (vjp ? p.g_slots * grad_slot_bytes(p.g_bytes) : 0);
     p.warp_bytes = (p.bar_off + 8 * (p.stages + 2) + 127) / 128 * 128;
     return p;
 }
@@ -411,8 +434,10 @@ opsa_vjp_pipe(S* __restrict__ gA, S* __restrict__ gB, S* __restrict__ gW,
 
     const bool want_a = gA != nullptr, want_b = gB != nullptr || (WEIGHTED && gW != nullptr);
     const bool pair_ok = L % 2 == 0 && (gB == nullptr || reinterpret_cast<uintptr_t>(gB) % (2 * sizeof(S)) == 0);
-    const int64_t rowsize = static_cast<int64_t>(K) * L;
-    const int g_slot_bytes = (lay.g_bytes + 15) / 16 * 16;
+    const int g_slot_bytes = grad_slot_bytes(lay.g_bytes);
+    auto grad_row = [&](int64_t r, int slot) { // row r in its slot
+        return area + lay.g_off + slot * g_slot_bytes + static_cast<int>((r * lay.g_bytes) & 15);
+    };
 
     auto load_pw = [&](int c) -> int32_t {
         int32_t pw = 0;
@@ -440,14 +465,13 @@ opsa_vjp_pipe(S* __restrict__ gA, S* __restrict__ gB, S* __restrict__ gW,
     auto issue_g = [&](int64_t r) {
         if (r < w.r1 && lane == 0) {
             const int slot = two_slots ? static_cast<int>(r - w.r0) & 1 : 0;
-            mbarrier_arrive_expect(gbars + slot, static_cast<unsigned>(lay.g_bytes));
-            bulk_copy_in(area + lay.g_off + slot * g_slot_bytes, gO + r * rowsize,
-                         static_cast<unsigned>(lay.g_bytes), gbars + slot);
+            issue_grad_row(area + lay.g_off + slot * g_slot_bytes, gO, r, nO, lay.g_bytes, gbars + slot);
         }
     };
     issue_g(w.r0);
     if (two_slots) issue_g(w.r0 + 1);
     for (int i = 0; i < NS - 1; i++) issue_next();
+    __syncwarp(); // (a last row's end may have been stored by one lane)
 
     int64_t wbase = w.r0;
     auto load_window = [&](int64_t base) {
@@ -477,7 +501,7 @@ opsa_vjp_pipe(S* __restrict__ gA, S* __restrict__ gB, S* __restrict__ gW,
             return;
         }
         if (has_entries) {
-            const S* g = reinterpret_cast<const S*>(area + lay.g_off + slot * g_slot_bytes);
+            const S* g = reinterpret_cast<const S*>(grad_row(r, slot));
 #pragma unroll
             for (int nt = 0; nt < NTK; nt++)
 #pragma unroll
@@ -697,6 +721,7 @@ opsa_fwd_pipe_tf32(float* __restrict__ O, const float* __restrict__ A, const flo
         }
     };
     for (int i = 0; i < NS - 1; i++) issue_next();
+    __syncwarp(); // (a last row's end may have been stored by one lane)
 
     int64_t wbase = w.r0;
     auto load_window = [&](int64_t base) {
@@ -842,8 +867,10 @@ opsa_vjp_pipe_tf32(float* __restrict__ gA, float* __restrict__ gB, const float* 
     const PipeWarp w = pipe_partition_entries(offsets, nO, CH, warp);
     if (w.r0 >= w.r1 || w.nchunks == 0) return;
     const bool want_a = gA != nullptr, want_b = gB != nullptr;
-    const int64_t rowsize = static_cast<int64_t>(K) * L;
-    const int g_slot_bytes = (lay.g_bytes + 15) / 16 * 16;
+    const int g_slot_bytes = grad_slot_bytes(lay.g_bytes);
+    auto grad_row = [&](int64_t r, int slot) { // row r in its slot
+        return area + lay.g_off + slot * g_slot_bytes + static_cast<int>((r * lay.g_bytes) & 15);
+    };
     const bool pair_a = K % 2 == 0 && reinterpret_cast<uintptr_t>(gA) % 8 == 0;
     const bool pair_b = L % 2 == 0 && reinterpret_cast<uintptr_t>(gB) % 8 == 0;
 
@@ -859,14 +886,13 @@ opsa_vjp_pipe_tf32(float* __restrict__ gA, float* __restrict__ gB, const float* 
     auto issue_g = [&](int64_t r) {
         if (r < w.r1 && lane == 0) {
             const int slot = static_cast<int>(r - w.r0) & 1;
-            mbarrier_arrive_expect(gbars + slot, static_cast<unsigned>(lay.g_bytes));
-            bulk_copy_in(area + lay.g_off + slot * g_slot_bytes, gO + r * rowsize,
-                         static_cast<unsigned>(lay.g_bytes), gbars + slot);
+            issue_grad_row(area + lay.g_off + slot * g_slot_bytes, gO, r, nO, lay.g_bytes, gbars + slot);
         }
     };
     issue_g(w.r0);
     issue_g(w.r0 + 1);
     for (int i = 0; i < NS - 1; i++) issue_next();
+    __syncwarp(); // (a last row's end may have been stored by one lane)
 
     int64_t wbase = w.r0;
     auto load_window = [&](int64_t base) {
@@ -894,7 +920,7 @@ opsa_vjp_pipe_tf32(float* __restrict__ gA, float* __restrict__ gB, const float* 
             return;
         }
         if (has_entries) {
-            const float* gs = reinterpret_cast<const float*>(area + lay.g_off + (use & 1) * g_slot_bytes);
+            const float* gs = reinterpret_cast<const float*>(grad_row(r, use & 1));
 #pragma unroll
             for (int ks = 0; ks < LS; ks++)
 #pragma unroll

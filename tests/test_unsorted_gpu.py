@@ -21,3 +21,12 @@ def test_outer_products(oracle, E, n, K, L, dtype):
             po[::3] = n // 2
         d["indices_output"] = po.astype(np.int32)
         compare(op, d, dtype, oracle, what=f"{op} unsorted {E} {n} {K}x{L}")
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("K,L", [(1, 1), (7, 25), (3, 5), (13, 31), (15, 17), (5, 3)])
+def test_gradient_rows_of_odd_sizes(oracle, K, L, dtype):
+    """Sorted index, grad_output rows that are no multiple of 16 bytes: every alignment of a row's
+    start, and the end of the array inside a 16-byte piece (an odd number of rows)."""
+    compare("opsa", workloads.opsa(J=3001, K=K, L=L, nO=57), dtype, oracle, what=f"opsa odd {K}x{L}")
+    compare("opsa", workloads.opsa(J=7, K=K, L=L, nO=1), dtype, oracle, what=f"opsa one row {K}x{L}")
