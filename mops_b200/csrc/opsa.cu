@@ -32,6 +32,7 @@
 #include "bulk.cuh"
 #include "checks.hpp"
 #include "device.cuh"
+#include "opsa_small.cuh"
 #include "unsorted.cuh"
 
 namespace mops_b200 {
@@ -698,6 +699,15 @@ void forward(const Call& call, T* O, const T* A, const T* B, const T* W, const i
         MOPS_CUDA_OK(cudaMemsetAsync(O, 0, nO * KL * sizeof(T), call.stream));
         return;
     }
+    if (small_forward(J, nO, WEIGHTED)) {
+        const int64_t units = nO * ceil_div(K, 8) * ceil_div(L, 32);
+        const int64_t blocks = std::min<int64_t>(ceil_div(units, kSmallWarps), sm_count(call.device) * 8);
+        note_kernel_f("opsa_fwd_small<%s,W=%d>", scalar_name<T>(), WEIGHTED ? 1 : 0);
+        opsa_fwd_small<T, WEIGHTED><<<static_cast<unsigned>(blocks), kSmallWarps * 32, 0, call.stream>>>(
+            O, A, B, W, PW, P, static_cast<int>(J), K, L, static_cast<int>(nO), call.status);
+        MOPS_CUDA_OK(cudaGetLastError());
+        return;
+    }
     const bool aligned = reinterpret_cast<uintptr_t>(O) % 16 == 0;
     FwdPlan plan = plan_forward<T, WEIGHTED>(K, L, aligned);
     const size_t smem = plan.smem_per_warp * kFwdWarps;
@@ -1255,6 +1265,14 @@ void backward(const Call& call, T* gA, T* gB, T* gW, const T* gO, const T* A, co
         return;
     }
 
+    if (J <= kSmallEntries && K <= 16) {
+        note_kernel_f("opsa_vjp_small<%s,W=%d>", scalar_name<T>(), WEIGHTED ? 1 : 0);
+        opsa_vjp_small<T, WEIGHTED>
+            <<<static_cast<unsigned>(ceil_div(J, kSmallWarps)), kSmallWarps * 32, 0, call.stream>>>(
+                gA, gB, gW, gO, A, B, W, PW, P, static_cast<int>(J), K, L, static_cast<int>(nO), call.status);
+        MOPS_CUDA_OK(cudaGetLastError());
+        return;
+    }
     VjpPlan plan;
     plan.only_if_unsorted = false;
     // Sorted scatter index (checked on the device): the streaming tensor-core kernel, or for

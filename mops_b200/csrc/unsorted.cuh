@@ -154,6 +154,45 @@ void launch_sorting(const Call& call, int blocks, void (*grid_kernel)(Params...)
 // ---- forward of OPSA / OPSAW
 constexpr int kGatherEntries = 8; // entries whose rows are in flight at a time
 
+// acc[k] += A[e, kb + k] (B o W)[e, lc] for the `count` (<= 32) entries e that the lanes hold, U at a time.
+template <typename T, int KC, bool WEIGHTED, int U = kGatherEntries>
+__device__ __forceinline__ void add_products(T (&acc)[KC], int my_entry, int my_w, int count,
+                                             const T* __restrict__ A, const T* __restrict__ B,
+                                             const T* __restrict__ W, int K, int L, int kb, int kn, int lc,
+                                             T* stage, int lane) {
+    for (int u0 = 0; u0 < count; u0 += U) {
+        T b[U], w[U];
+#pragma unroll
+        for (int x = lane; x < U * KC; x += 32) {
+            const int u = x / KC, k = x - u * KC;
+            const int64_t e = __shfl_sync(kFullMask, my_entry, u0 + u);
+            stage[x] = k < kn && u0 + u < count ? __ldg(A + e * K + kb + k) : T(0);
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int64_t e = __shfl_sync(kFullMask, my_entry, u0 + u);
+            b[u] = __ldg(B + e * L + lc);
+            if (WEIGHTED)
+                w[u] = __ldg(W + static_cast<int64_t>(__shfl_sync(kFullMask, my_w, u0 + u)) * L + lc);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            if (WEIGHTED) b[u] *= w[u];
+            if (u0 + u >= count) b[u] = T(0);
+            constexpr int V = 16 / sizeof(T);
+#pragma unroll
+            for (int k = 0; k < KC; k += V) {
+                T a[V];
+                load_vec<T, V>(stage + u * KC + k, a);
+#pragma unroll
+                for (int v = 0; v < V; v++) acc[k + v] += a[v] * b[u];
+            }
+        }
+        __syncwarp();
+    }
+}
+
 // One warp per output row and KC by 32 part of it, lane = column l of B. The entries' numbers (and
 // their rows of W) are fetched 32 at a time, one per lane; B rows go to registers and A rows to shared
 // memory eight entries at a time (`stage`: [8][KC] of this warp), where they are read as
@@ -164,7 +203,6 @@ __device__ __forceinline__ void opsa_rows_gathered(T* __restrict__ O, const T* _
                                                    const T* __restrict__ B, const T* __restrict__ W,
                                                    const int32_t* __restrict__ PW, const EntrySort& s, int K,
                                                    int L, int64_t n_rows, T* stage, const Status& st) {
-    constexpr int U = kGatherEntries;
     const int lane = threadIdx.x & 31;
     const int64_t warps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
     const int k_units = (K + KC - 1) / KC, units = k_units * ((L + 31) / 32);
@@ -188,37 +226,7 @@ __device__ __forceinline__ void opsa_rows_gathered(T* __restrict__ O, const T* _
                 my_w = __ldg(PW + my_entry);
                 if (clamp_index(my_w, static_cast<int32_t>(n_rows))) report_bad_index(st, 1);
             }
-            for (int u0 = 0; u0 < count; u0 += U) {
-                T b[U], w[U];
-#pragma unroll
-                for (int x = lane; x < U * KC; x += 32) {
-                    const int u = x / KC, k = x - u * KC;
-                    const int64_t e = __shfl_sync(kFullMask, my_entry, u0 + u);
-                    stage[x] = k < kn && u0 + u < count ? __ldg(A + e * K + kb + k) : T(0);
-                }
-#pragma unroll
-                for (int u = 0; u < U; u++) {
-                    const int64_t e = __shfl_sync(kFullMask, my_entry, u0 + u);
-                    b[u] = __ldg(B + e * L + lc);
-                    if (WEIGHTED)
-                        w[u] = __ldg(W + static_cast<int64_t>(__shfl_sync(kFullMask, my_w, u0 + u)) * L + lc);
-                }
-                __syncwarp();
-#pragma unroll
-                for (int u = 0; u < U; u++) {
-                    if (WEIGHTED) b[u] *= w[u];
-                    if (u0 + u >= count) b[u] = T(0);
-                    constexpr int V = 16 / sizeof(T);
-#pragma unroll
-                    for (int k = 0; k < KC; k += V) {
-                        T a[V];
-                        load_vec<T, V>(stage + u * KC + k, a);
-#pragma unroll
-                        for (int v = 0; v < V; v++) acc[k + v] += a[v] * b[u];
-                    }
-                }
-                __syncwarp();
-            }
+            add_products<T, KC, WEIGHTED>(acc, my_entry, my_w, count, A, B, W, K, L, kb, kn, lc, stage, lane);
         }
         if (l < L) {
 #pragma unroll

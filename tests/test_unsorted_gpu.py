@@ -1,5 +1,5 @@
 """Scatter operations on unsorted indices: one-block and whole-GPU sorts (the line lies at 512
-entries), widths on both sides of a 32-lane row and an 8-row part, rows without entries, one row that
+entries) and the one-launch kernels of small problems (up to 2048 and 4096), widths on both sides of a 32-lane row and an 8-row part, rows without entries, one row that
 receives everything, against the CPU oracle at the parity tolerances."""
 import numpy as np
 import pytest
@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
-@pytest.mark.parametrize("E,n,K,L", [(2, 2, 1, 1), (511, 7, 4, 33), (513, 900, 5, 31), (4097, 1, 9, 32),
+@pytest.mark.parametrize("E,n,K,L", [(2, 2, 1, 1), (511, 7, 4, 33), (2048, 33, 16, 40), (2049, 70, 13, 32), (513, 900, 5, 31), (4097, 1, 9, 32),
                                      (20011, 157, 16, 32), (70001, 40000, 17, 20)])
 def test_outer_products(oracle, E, n, K, L, dtype):
     r = np.random.default_rng(E)
@@ -21,6 +21,12 @@ def test_outer_products(oracle, E, n, K, L, dtype):
             po[::3] = n // 2
         d["indices_output"] = po.astype(np.int32)
         compare(op, d, dtype, oracle, what=f"{op} unsorted {E} {n} {K}x{L}")
+        if E < 4096:
+            order = np.argsort(d["indices_output"], kind="stable")
+            for k in ("A", "B", "indices_output", "indices_W"):
+                if k in d:
+                    d[k] = d[k][order]
+            compare(op, d, dtype, oracle, what=f"{op} sorted {E} {n} {K}x{L}")
 
 
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
