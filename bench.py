@@ -81,19 +81,20 @@ SMALL_CASES = {
 BATCH_KEYS = {"hpe": ("I",), "sap": ("I",), "opsa": ("J", "nO"), "opsaw": ("E", "n"),
               "sasaw": ("E", "n")}
 ROW_KEYS = ("nO", "n")
-# what bounds each case on the SM: HBM bytes, shared-memory
-# wavefronts (every operand is a gather with a run-time index), or FP64 throughput. SASAW also
+# what bounds each case on the SM: HBM bytes, or FP64 throughput (HPE and SAP gather their operands
+# from tensor memory and are bounded by instruction issue and the FP64 pipe). SASAW also
 # reports the DRAM traffic it really causes (`*_traffic_frac_of_hbm`): its W table (151 MB at
-# the benchmark size) does not fit L2, so the gathered W rows and the grad_W additions of every
-# edge go to DRAM and the kernels move 4 to 7 times their algorithmic bytes.
-BOUND = {"hpe": "smem", "sap": "smem", "opsa": "hbm", "opsa_f32": "hbm", "opsaw": "hbm",
+# the benchmark size) does not fit L2, so the gathered W and grad_output rows of every edge go to
+# DRAM and the kernels move several times their algorithmic bytes.
+BOUND = {"hpe": "fp64", "sap": "fp64", "opsa": "hbm", "opsa_f32": "hbm", "opsaw": "hbm",
          "sasaw": "fp64"}
 # kernels of this library launched by one forward / one VJP call of every case (sorted input,
-# waiting calls, no plan bound): a table builder (HPE / SAP plan, segment offsets) + the main
-# kernel; SASAW builds two tables (segment offsets and the grouped coupling) in either call.
+# waiting calls, no plan bound): a table builder (HPE / SAP records, segment offsets) + the main
+# kernel; the HPE forward packs its records itself; SASAW builds the dense coupling and the segment
+# offsets (forward) or the order of the edges (VJP, two main kernels).
 # profiles/launch_list_full_bench.md counts the same 26 launches per step.
-LAUNCHES = {"hpe": (2, 2), "sap": (2, 2), "opsa": (2, 2), "opsa_f32": (2, 2), "opsaw": (2, 2),
-            "sasaw": (3, 3)}
+LAUNCHES = {"hpe": (1, 2), "sap": (2, 2), "opsa": (2, 2), "opsa_f32": (2, 2), "opsaw": (2, 2),
+            "sasaw": (3, 4)}
 
 OP_NAMES = {"hpe": "homogeneous_polynomial_evaluation", "sap": "sparse_accumulation_of_products",
             "opsa": "outer_product_scatter_add", "opsaw": "outer_product_scatter_add_with_weights",
@@ -858,10 +859,6 @@ def main():
                 entry[f"{lvl}_traffic_frac_of_hbm"] = dram / ms / 1e6 / peak
             if BOUND[n] == "hbm":
                 entry[f"{lvl}_frac_of_bound"] = b / ms / 1e6 / peak
-            elif BOUND[n] == "smem":
-                # one shared-memory wavefront per clock per SM
-                entry[f"{lvl}_frac_of_bound"] = None if wavefronts is None else \
-                    wavefronts / (sms * clk_hz * ms / 1e3)
             else:
                 hd = {k2: (v.numpy() if isinstance(v, torch.Tensor) else v)
                       for k2, v in host[n].items()}

@@ -128,9 +128,19 @@ def items(op, w):
 
 def useful_flops(op, level, w):
     """Floating-point operations one call needs when the work is organised the way the kernels
-    organise it (multiply-add = 2). Only SASAW differs from the naive count: the coupling table
-    is first contracted with the edge's A row into a dense nO2 x nW2 matrix T_e (2*cells*nA),
-    which is then applied to the 32-wide rows (2*nO2*nW2*L per product)."""
+    organise it (multiply-add = 2). HPE: products of K factors and a coefficient, for the VJP one of
+    K - 1 factors per incidence. SAP: three operations per triplet; for the VJP one multiply-add per
+    triplet and two per cell (operand column pair). SASAW: the coupling contracted with the edge's A
+    row into a dense nO2 x nW2 matrix T_e (2*cells*nA), which is then applied to the 32-wide rows
+    (2*nO2*nW2*L per product); the kernels that apply the coupling per row do about as much."""
+    if op == "hpe":
+        I = w["A"].shape[0]
+        J, K = w["indices_A"].shape
+        return I * J * (K + 1) if level == "fwd" else I * J * K * K
+    if op == "sap":
+        I, K = w["A"].shape[0], w["C"].shape[0]
+        cells = w["A"].shape[1] * w["B"].shape[1]
+        return 3 * I * K if level == "fwd" else 2 * I * K + 4 * I * cells
     if op != "sasaw":
         raise KeyError(op)
     E, nA = w["A"].shape
