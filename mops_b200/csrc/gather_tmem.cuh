@@ -321,53 +321,71 @@ gather_table(unsigned char* __restrict__ records, int32_t* __restrict__ n_start,
 
 // ---------------------------------------------------------------- the sums
 // The 32-byte sector that ends at `at`: the value `now` of slot r and the ones before it.
-template <int R>
-__device__ __forceinline__ void store_sector(double* at, const double (&past)[3][R], int r, double now) {
-    asm volatile("st.global.v4.f64 [%0], {%1,%2,%3,%4};\n" ::"l"(at - 3), "d"(past[2][r]), "d"(past[1][r]),
-                 "d"(past[0][r]), "d"(now)
+__device__ __forceinline__ void store_sector(double* from, const double (&v)[4]) {
+    asm volatile("st.global.v4.f64 [%0], {%1,%2,%3,%4};\n" ::"l"(from), "d"(v[0]), "d"(v[1]), "d"(v[2]), "d"(v[3])
                  : "memory");
 }
-template <int R>
-__device__ __forceinline__ void store_sector(float* at, const float (&past)[7][R], int r, float now) {
-    asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n" ::"l"(at - 7), "f"(past[6][r]),
-                 "f"(past[5][r]), "f"(past[4][r]), "f"(past[3][r]), "f"(past[2][r]), "f"(past[1][r]),
-                 "f"(past[0][r]), "f"(now)
+__device__ __forceinline__ void store_sector(float* from, const float (&v)[8]) {
+    asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n" ::"l"(from), "f"(v[0]), "f"(v[1]),
+                 "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
                  : "memory");
 }
 
 // Writes results to rows, one column after the other, in whole 32-byte sectors (partial ones cost
-// L2 five times as much: measured 1.1 against 5 TB/s). A lane keeps its row's last E - 1 values
-// and stores them when they end a sector, which depends on the row where the row size is no
-// multiple of 32 bytes; what lies before the first or behind the last whole sector goes out alone.
+// L2 five times as much: measured 1.1 against 5 TB/s). A lane keeps its row's last E values, column n
+// in held[n mod E] (the switch makes that a constant: shifting the values along took 300
+// instructions per column of four rows), and stores them when they end a sector, which depends on the
+// row where the row size is no multiple of 32 bytes; what lies before the first or behind the last
+// whole sector goes out alone.
 template <typename T, int R> struct SectorWriter {
     static constexpr int E = 32 / sizeof(T);
-    T past[E - 1][R];
+    T held[E][R];
 
-    // Column `local` of the `cols` columns of `out` for row0 + 128 r (if live); `lo`: the first column
-    // of the run this lane writes, `last`: the run ends here.
-    __device__ __forceinline__ void put(T* out, int64_t row0, int cols, int local, int lo, bool last,
-                                        const T (&now)[R], const bool (&live)[R]) {
-        T* at = out + row0 * cols + local;
+    // The value at `at` (and at + r row_step for the other rows, if live), column J of E, the `run`-th
+    // (from 0) that this lane writes in a row; `last`: the run ends here.
+    template <int J>
+    __device__ __forceinline__ void put(T* at, int64_t row_step, int run, bool last, const T (&now)[R],
+                                        const bool (&live)[R]) {
+#pragma unroll
+        for (int r = 0; r < R; r++) held[J][r] = now[r];
         const int phase = static_cast<int>(reinterpret_cast<size_t>(at) / sizeof(T)) & (E - 1);
-        const int k = phase == E - 1 || last ? min(phase, local - lo) + 1 : 0; // values to store
+        if (phase == E - 1 && run >= E - 1) {
 #pragma unroll
-        for (int r = 0; r < R; r++) {
-            T* dst = at + r * kSlabRows * static_cast<int64_t>(cols);
-            if (live[r] && k == E) {
-                store_sector(dst, past, r, now[r]);
-            } else if (live[r] && k > 0) {
-                *dst = now[r];
+            for (int r = 0; r < R; r++) {
+                T v[E];
 #pragma unroll
-                for (int e = 1; e < E; e++)
-                    if (e < k) dst[-e] = past[e - 1][r];
+                for (int e = 0; e < E; e++) v[e] = held[(J + 1 + e) & (E - 1)][r];
+                if (live[r]) store_sector(at + r * row_step - (E - 1), v);
             }
+        } else if (phase == E - 1 || last) { // at an end of the run
+            const int k = min(phase, run);
+#pragma unroll
+            for (int e = 0; e < E - 1; e++)
+                if (e <= k) {
+#pragma unroll
+                    for (int r = 0; r < R; r++)
+                        if (live[r]) at[r * row_step - e] = held[(J - e) & (E - 1)][r];
+                }
+            // (a whole sector is complete only with phase == E - 1)
         }
         __syncwarp();
-#pragma unroll
-        for (int r = 0; r < R; r++) {
-#pragma unroll
-            for (int e = E - 2; e > 0; e--) past[e][r] = past[e - 1][r];
-            past[0][r] = now[r];
+    }
+    __device__ __forceinline__ void put(int column, T* at, int64_t row_step, int run, bool last, const T (&now)[R],
+                                        const bool (&live)[R]) {
+        switch (column & (E - 1)) {
+        case 0: put<0>(at, row_step, run, last, now, live); break;
+        case 1: put<1>(at, row_step, run, last, now, live); break;
+        case 2: put<2>(at, row_step, run, last, now, live); break;
+        case 3: put<3>(at, row_step, run, last, now, live); break;
+        default:
+            if constexpr (E > 4) {
+                switch (column & (E - 1)) {
+                case 4: put<4>(at, row_step, run, last, now, live); break;
+                case 5: put<5>(at, row_step, run, last, now, live); break;
+                case 6: put<6>(at, row_step, run, last, now, live); break;
+                default: put<7>(at, row_step, run, last, now, live); break;
+                }
+            }
         }
     }
 };
@@ -516,19 +534,23 @@ gather_sums(const __grid_constant__ Results<T> results, const __grid_constant__ 
             local -= results.cols[which_result++];
         int lo = local; // first column of this result that is the group's
         SectorWriter<T, R> writer{};
+        int cols = results.cols[which_result];
+        T* at = results.data[which_result] + row0 * cols + local;
         auto close = [&] { // column n is complete
-            const int cols = results.cols[which_result];
 #pragma unroll
             for (int r = 0; r < R; r++)
                 if (results.scale && live[r]) acc[r] *= __ldg(results.scale + row0 + r * kSlabRows);
-            writer.put(results.data[which_result], row0, cols, local, lo, n + 1 == n_hi || local + 1 == cols,
-                       acc, live);
+            writer.put(local, at, kSlabRows * static_cast<int64_t>(cols), local - lo,
+                       n + 1 == n_hi || local + 1 == cols, acc, live);
 #pragma unroll
             for (int r = 0; r < R; r++) acc[r] = T(0);
             n++;
-            if (++local == cols) {
+            at++;
+            if (++local == cols && n < n_hi) {
                 local = lo = 0;
                 which_result++;
+                cols = results.cols[which_result];
+                at = results.data[which_result] + row0 * cols;
             }
         };
         if (batches > 0) {

@@ -163,7 +163,8 @@ sap_vjp_cells(T* __restrict__ gT, T* __restrict__ gS, const __grid_constant__ Op
                 if (moved) {
                     c++;
                     if (++s == nS) {
-                        writer.put(gT, row0, nT, t, t_lo, t + 1 == t_hi, sum_t, live);
+                        writer.put(t, gT + row0 * nT + t, kSlabRows * static_cast<int64_t>(nT), t - t_lo, t + 1 == t_hi,
+                                   sum_t, live);
 #pragma unroll
                         for (int r = 0; r < R; r++) sum_t[r] = T(0);
                         s = 0;
