@@ -139,6 +139,9 @@ template <int BYTES, int OFFSET> __device__ __forceinline__ void cp_async_at(uns
     asm volatile("cp.async.ca.shared.global [%0 + %1], [%2], %3;\n" ::"r"(dst), "n"(OFFSET), "l"(src), "n"(BYTES)
                  : "memory");
 }
+__device__ __forceinline__ void cp_async16(unsigned dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
+}
 template <int BYTES, int STEP, int C, int N>
 __device__ __forceinline__ void cp_async_rows(unsigned dst, const unsigned char* src, int64_t row_bytes) {
     if constexpr (C < N) {
@@ -148,7 +151,8 @@ __device__ __forceinline__ void cp_async_rows(unsigned dst, const unsigned char*
 }
 
 // How a warp takes the edges: several side by side (L <= 16 columns and f64 or f32 of one column per lane),
-// one at a time, or one at a time with L = 32 VEC columns (then every offset is a constant).
+// one at a time, or one at a time with L = 32 VEC columns and operands at 16-byte boundaries (then
+// every offset is a constant and the copies are whole 16-byte pieces).
 enum Mode { kSideBySide = 0, kOneEdge = 1, kExact = 2 };
 
 // Walks rows [row_lo, row_hi) for columns [b0, ...) and c in [c0, c0 + nc): begin(row), step(w[NC] and B
@@ -210,8 +214,31 @@ __device__ __forceinline__ void walk_rows(const RowsArgs<T>& g, const Off* __res
     const int64_t g_row = g.nC * (L * kScalar);
     const unsigned char* b_base = reinterpret_cast<const unsigned char*>(g.B + bc);
     const unsigned char* a_base = reinterpret_cast<const unsigned char*>(g.A + lb);
+    const unsigned char* g_piece = reinterpret_cast<const unsigned char*>(g.G + static_cast<int64_t>(c0) * L) + lane * 16;
+    const unsigned char* b_piece = reinterpret_cast<const unsigned char*>(g.B) + lane * 16;
     constexpr int kStep = 32 * sizeof(V);
     auto copy_edge = [&](int slot, int e, int r) { // W (or gO) row and B
+        if constexpr (MODE == kExact) {
+            // Both are contiguous, and so are their places in the slot: 16-byte pieces, spread over
+            // the lanes (gradients of 4.2 10^6 edges, f64: 3.05 -> 2.91 ms).
+            constexpr int kPieces = Sl::kB / 16, kAll = Sl::kA / 16; // with B
+            const unsigned to = ring32 + slot + lane * 16;
+            const unsigned char* g_src = g_piece + r * g_row;
+            const unsigned char* b_src = b_piece + e * (L * kScalar);
+            if (nc == NC) {
+#pragma unroll
+                for (int i = 0; i < kAll; i += 32) {
+                    const bool in_row = i + 32 <= kPieces || i + lane < kPieces;
+                    const unsigned char* src = in_row ? g_src + i * 16 : b_src + (i - kPieces) * 16;
+                    if (i + 32 <= kAll || i + lane < kAll) cp_async16(to + i * 16, src);
+                }
+            } else {
+                for (int i = lane; i < nc * (kStep / 16); i += 32)
+                    cp_async16(ring32 + slot + i * 16, g_src + (i - lane) * 16);
+                if (lane < kStep / 16) cp_async16(to + Sl::kB, b_src);
+            }
+            return;
+        }
         const unsigned dst = ring32 + slot + lane_off;
         const unsigned char* src = g_base + r * g_row;
         if (nc == NC) {
@@ -529,6 +556,13 @@ __device__ __forceinline__ void edge_gradients(const RowsArgs<T>& g, const Off* 
 }
 
 // ---- kernels
+// Blocks per SM: two for f32 with one column per lane, whose sums take 81 registers and not 162. That
+// pays for the edge gradients (200 000 edges, 32 columns, 16 x 9 -> 16 channels: 0.67 -> 0.54 ms) and
+// for short rows (10 edges: sums 0.15 -> 0.12, gradients 0.26 -> 0.19 ms); the sums of 16 channels
+// stay with one block (0.31 against 0.34 ms).
+template <typename T, int VEC> constexpr int kEdgeBlocks = sizeof(T) == 4 && VEC == 1 ? 2 : 1;
+template <typename T, int VEC, int NA> constexpr int kSumBlocks = NA <= 9 ? kEdgeBlocks<T, VEC> : 1;
+
 // A block owns a range of rows (the blocks share the edges evenly); its warps take them a few at a
 // time, about kChunkEdges edges, so that none waits for another's long rows
 // (60 000 edges, 1000 rows: 63 -> 45 us against rows dealt out beforehand).
@@ -574,7 +608,7 @@ template <typename T, int VEC, int NA, int NC> struct RowsShared {
 enum RowsRun { kSorted = 0, kIfUnsorted = 1, kAlways = 2 };
 
 template <typename T, int VEC, int NA, int NC, Mode MODE>
-__global__ void __launch_bounds__(kRowWarps * 32, 1)
+__global__ void __launch_bounds__(kRowWarps * 32, (kSumBlocks<T, VEC, NA>))
 sasaw_sum_rows(const __grid_constant__ RowsArgs<T> g, const int64_t* __restrict__ offsets,
                const int32_t* __restrict__ starts, T* __restrict__ out, RowsRun run, Status st) {
     if (run != kAlways && saw_unsorted(st) != (run == kIfUnsorted)) return;
@@ -595,7 +629,7 @@ sasaw_sum_rows(const __grid_constant__ RowsArgs<T> g, const int64_t* __restrict_
 // gA and gB. (A kernel of its own: gathering for gW at the same time in half of the warps saves DRAM
 // traffic, but with both loops in one kernel the registers do not suffice.)
 template <typename T, int VEC, int NA, int NC, Mode MODE>
-__global__ void __launch_bounds__(kRowWarps * 32, 1)
+__global__ void __launch_bounds__(kRowWarps * 32, (kEdgeBlocks<T, VEC>))
 sasaw_edge_gradients(const __grid_constant__ RowsArgs<T> g, const int32_t* __restrict__ starts, T* __restrict__ gA,
                      T* __restrict__ gB, const T* __restrict__ W, Status st) {
     __shared__ int counter;
@@ -625,7 +659,8 @@ inline int chunk_c(int na, int n) { return n <= 4 ? 4 : na <= 9 ? 9 : n <= 5 || 
 
 template <typename T> struct RowsShape {
     RowsArgs<T> g;
-    int na, nc, vec, blocks;
+    int na, nc, vec;
+    bool aligned; // G and B at 16-byte boundaries
     size_t smem;
     size_t table_bytes;
 };
@@ -640,6 +675,7 @@ RowsShape<T> rows_shape(const Call& call, const SasawProblem<T>& p, const T* gat
     s.vec = vec;
     s.g.A = p.A, s.g.B = p.B, s.g.G = gathered;
     s.g.rows = p.rows, s.g.nA = p.nA, s.g.L = p.L;
+    s.aligned = (reinterpret_cast<uintptr_t>(gathered) | reinterpret_cast<uintptr_t>(p.B)) % 16 == 0;
     s.g.pad_c = static_cast<int>(ceil_div(s.g.nC, s.nc)) * s.nc;
     s.g.pad_out = static_cast<int>(ceil_div(s.g.nOut, kTableOut)) * kTableOut;
     int lanes = 4;
@@ -660,7 +696,7 @@ template <typename T, typename F> void for_shape(const RowsShape<T>& s, F&& f) {
         using I = std::integral_constant<int, VEC>;
         using A = std::integral_constant<int, NA>;
         using X = std::integral_constant<int, NC>;
-        if (s.g.L == 32 * VEC)
+        if (s.g.L == 32 * VEC && s.aligned)
             f(I(), A(), X(), std::integral_constant<Mode, kExact>());
         else if (VEC == 2 || s.g.lanes == 32)
             f(I(), A(), X(), std::integral_constant<Mode, kOneEdge>());
@@ -720,18 +756,21 @@ TableRef dense_table(const Call& call, const SasawProblem<T>& p, const RowsShape
     return ref;
 }
 
-// One block per SM, fewer for few rows.
-inline unsigned rows_blocks(const Call& call, int64_t rows) {
-    return static_cast<unsigned>(std::min<int64_t>(rows, sm_count(call.device)));
+// As many blocks as the SMs hold, fewer for few rows.
+template <typename Kernel> unsigned rows_blocks(const Call& call, Kernel kernel, size_t smem, int64_t rows) {
+    const int64_t sms = sm_count(call.device);
+    int64_t blocks = sms * resident_blocks(kernel, call.device, kRowWarps * 32, smem);
+    if (rows < blocks * kRowWarps) blocks = sms; // (more blocks than rows for their warps: 23 -> 29 us)
+    return static_cast<unsigned>(std::min<int64_t>(rows, blocks));
 }
 
 template <typename T>
-void launch_sums(const Call& call, const RowsShape<T>& s, unsigned blocks, const int64_t* offsets,
-                 const int32_t* starts, T* out, RowsRun when) {
+void launch_sums(const Call& call, const RowsShape<T>& s, const int64_t* offsets, const int32_t* starts,
+                 T* out, RowsRun when) {
     for_shape(s, [&](auto vec, auto na, auto nc, auto mode) {
         auto kernel = sasaw_sum_rows<T, decltype(vec)::value, decltype(na)::value, decltype(nc)::value,
                                      decltype(mode)::value>;
-        allow_dynamic_smem(kernel, call.device, s.smem);
+        const unsigned blocks = rows_blocks(call, kernel, s.smem, s.g.rows);
         kernel<<<blocks, kRowWarps * 32, s.smem, call.stream>>>(s.g, offsets, starts, out, when, call.status);
     });
     MOPS_CUDA_OK(cudaGetLastError());
@@ -746,9 +785,8 @@ template <typename T> bool sasaw_forward_rows(const Call& call, const SasawProbl
     TableRef table = dense_table(call, p, s, false);
     SegmentTable seg = segment_table(call, p.I, p.E, p.rows);
     s.g.gather = p.J, s.g.perm = nullptr, s.g.D = static_cast<const T*>(table.ptr), s.g.bit = kBitJ;
-    const unsigned blocks = rows_blocks(call, p.rows);
     note_kernel_f("sasaw_sum_rows<%s,VEC=%d,NA=%d,NC=%d>", scalar_name<T>(), s.vec, s.na, s.nc);
-    auto run = [&](RowsRun when, const int32_t* starts) { launch_sums(call, s, blocks, seg.offsets, starts, O, when); };
+    auto run = [&](RowsRun when, const int32_t* starts) { launch_sums(call, s, seg.offsets, starts, O, when); };
     run(kSorted, nullptr);
     bool unsorted = !seg.known_sorted; // asynchronous calls cannot look: always enqueue
     if (unsorted && call.wait) {
@@ -790,17 +828,16 @@ bool sasaw_backward_rows(const Call& call, const SasawProblem<T>& p, T* gA, T* g
         commit_table(call, order);
     }
     s.g.gather = p.I, s.g.perm = sort.perm, s.g.D = static_cast<const T*>(table.ptr), s.g.bit = kBitI;
-    const unsigned blocks = rows_blocks(call, p.rows);
     if (gW != nullptr) {
         note_kernel_f("sasaw_sum_rows<%s,VEC=%d,NA=%d,NC=%d>", scalar_name<T>(), s.vec, s.na, s.nc);
-        launch_sums(call, s, blocks, nullptr, sort.starts, gW, kAlways);
+        launch_sums<T>(call, s, nullptr, sort.starts, gW, kAlways);
     }
     if (gA != nullptr || gB != nullptr) {
         note_kernel_f("sasaw_edge_gradients<%s,VEC=%d,NA=%d,NC=%d>", scalar_name<T>(), s.vec, s.na, s.nc);
         for_shape(s, [&](auto vec, auto na, auto nc, auto mode) {
             auto kernel = sasaw_edge_gradients<T, decltype(vec)::value, decltype(na)::value, decltype(nc)::value,
                                                decltype(mode)::value>;
-            allow_dynamic_smem(kernel, call.device, s.smem);
+            const unsigned blocks = rows_blocks(call, kernel, s.smem, s.g.rows);
             kernel<<<blocks, kRowWarps * 32, s.smem, call.stream>>>(s.g, sort.starts, gA, gB, p.W, call.status);
         });
         MOPS_CUDA_OK(cudaGetLastError());

@@ -61,3 +61,17 @@ def test_skipped_gradients(oracle, dtype):
         assert [x is None for x in some] == [i != which for i in range(3)]
         scale = full[which].abs().max()  # (sums of the same terms, the edges of a row in any order)
         assert (some[which] - full[which]).abs().max() <= (1e-12 if dtype == np.float64 else 1e-5) * scale
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("shift", ["", "B", "W", "grad_output"])
+def test_whole_warps(oracle, dtype, shift):
+    """L = 32, rows enough for two blocks per SM; with one operand an element past a 16-byte boundary."""
+    d = workloads.sasaw(E=9000, n=3000, nA=9, nW2=9, nO2=10, L=32, N=80, dtype=dtype)
+    t = to_dev(d, dtype)
+    if shift:
+        flat = t[shift].new_empty(t[shift].numel() + 1)
+        t[shift] = flat[1:].view(t[shift].shape).copy_(t[shift])
+    got, want = run_library("sasaw", t), run_checker(oracle, "sasaw", d, dtype)
+    for k in want:
+        assert_parity(got[k], want[k], f"sasaw L=32 shifted {shift}/{k}")
