@@ -74,13 +74,15 @@ def library():
 
 
 def native_calls(error):
-    """The function ``call`` of ``_calls.so``, which raises ``error`` for a failed call."""
+    """The function ``call`` of ``_calls.so``, which raises ``error`` for a failed call. Without that
+    module (``python -m mops_b200.build --no-torch`` leaves it out) every call takes the general path,
+    to the same kernels."""
     import importlib.machinery
     import importlib.util
     library()  # the same library, already loaded
     path = os.path.join(_HERE, "lib", "_calls.so")
     if not os.path.isfile(path):
-        raise ImportError(f"{path} not found: build it with `python -m mops_b200.build`")
+        return lambda *args: NotImplemented
     loader = importlib.machinery.ExtensionFileLoader("mops_b200._calls", path)
     module = importlib.util.module_from_spec(importlib.util.spec_from_loader(loader.name, loader))
     loader.exec_module(module)

@@ -125,3 +125,9 @@ def test_stream_and_wait_extensions():
     lib.mops_b200_set_wait(1)
     assert lib.mops_b200_get_stream() in (None, 0)
     assert b"sm_100a" in lib.mops_b200_version()
+
+
+def test_calls_on_cuda_tensors_do_without_the_torch_module(tmp_path, monkeypatch):
+    """A build without torch (--no-torch) has no ``_calls.so``: the front end takes its general path."""
+    monkeypatch.setattr(_lib, "_HERE", str(tmp_path))
+    assert _lib.native_calls(_lib.MopsError)(0, None, None, None) is NotImplemented
