@@ -86,6 +86,20 @@ void* get_stream() { return g_thread.stream; }
 void set_wait(bool wait) { g_thread.wait = wait; }
 bool get_wait() { return g_thread.wait; }
 
+namespace {
+// Zeros device words before any kernel can use them. On a stream of its own and waited for: a memset on
+// the legacy default stream is in order with neither the host nor a non-blocking stream, and could
+// wipe out what the first call's kernels have written.
+void zero_words(uint32_t* dev, int words) {
+    cudaStream_t stream = nullptr;
+    MOPS_CUDA_OK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+    cudaError_t err = cudaMemsetAsync(dev, 0, words * sizeof(uint32_t), stream);
+    if (err == cudaSuccess) err = cudaStreamSynchronize(stream);
+    (void)cudaStreamDestroy(stream);
+    MOPS_CUDA_OK(err);
+}
+} // namespace
+
 Call begin_call() {
     Call call;
     MOPS_CUDA_OK(cudaGetDevice(&call.device));
@@ -108,7 +122,7 @@ Call begin_call() {
             block.host = static_cast<uint32_t*>(host);
             MOPS_CUDA_OK(cudaMalloc(reinterpret_cast<void**>(&block.dev),
                                     kStatusWords * sizeof(uint32_t)));
-            MOPS_CUDA_OK(cudaMemset(block.dev, 0, kStatusWords * sizeof(uint32_t)));
+            zero_words(block.dev, kStatusWords);
             state.status = block;
         }
         g_thread.last = &state;

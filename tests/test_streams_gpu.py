@@ -1,0 +1,41 @@
+"""Calls on streams and threads that come and go: the first call of a stream, many short-lived streams,
+threads that end with calls in flight; results against the CPU oracle."""
+import numpy as np
+import pytest
+
+import mops_b200
+from conftest import assert_parity
+from helpers import to_dev
+from mops_b200 import workloads
+
+pytestmark = pytest.mark.gpu
+
+
+def _problem(oracle, J=5000, unsorted=True, seed=0):
+    d = workloads.opsa(J=J, K=5, L=8, nO=97)
+    if unsorted:
+        d["indices_output"] = np.random.default_rng(seed).permutation(d["indices_output"])
+    want = oracle.opsa(d["A"], d["B"], d["indices_output"], d["output_size"])
+    return to_dev(d, np.float64), want
+
+
+def _call(t):
+    return mops_b200.outer_product_scatter_add(t["A"], t["B"], t["indices_output"], t["output_size"])
+
+
+def test_first_call_of_a_stream_while_the_default_stream_is_busy(oracle):
+    """What the call's kernels report to one another (here: the index is not sorted) must not be
+    overwritten by the preparation of the stream's status words."""
+    import torch
+    t, want = _problem(oracle)
+    _call(t)
+    torch.cuda.synchronize()
+    side = [torch.cuda.Stream() for _ in range(4)]
+    torch.cuda._sleep(200_000_000)  # about 0.1 s on the default stream
+    got = []
+    for s in side:
+        with torch.cuda.stream(s):
+            got.append(_call(t))
+    torch.cuda.synchronize()
+    for g in got:
+        assert_parity(g.cpu().numpy(), want, "first call of a stream")
