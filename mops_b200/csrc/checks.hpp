@@ -10,6 +10,7 @@
 #ifndef MOPS_B200_CHECKS_HPP
 #define MOPS_B200_CHECKS_HPP
 
+#include <cstdint>
 #include <stdexcept>
 #include <string>
 
@@ -44,6 +45,11 @@ inline void fits_int32(size_t value, const char* what, const std::string& operat
                                  operation);
     }
 }
+
+// Whether kernels may keep the positions of `n` entries in an int. They look past the last entry before
+// they compare with it: by a block of 32 in the walks over sorted entries (unsorted.cuh), by three
+// blocks and the depth of the ring, 102 in all, in the walks over rows (sasaw_rows.cu).
+constexpr bool positions_fit_int(int64_t n) { return n <= INT32_MAX - 256; }
 
 } // namespace mops_b200
 

@@ -290,15 +290,16 @@ segment_offsets(const int32_t* __restrict__ P, int64_t J, int64_t n_rows, int64_
     for (int q = 0; q < Q; q++) {
         const int32_t prev = v[q], cur = v[1 + q];
         // rows prev + 1 .. cur start at entry j0 + q
-        if (cur > prev) offsets[prev + 1] = j0 + q;
-        unsigned wide = __ballot_sync(kFullMask, cur > prev + 1);
+        if (cur > prev) offsets[int64_t(prev) + 1] = j0 + q;
+        // (64 bits: with 2^31 - 1 rows the sums leave 32)
+        unsigned wide = __ballot_sync(kFullMask, cur > int64_t(prev) + 1);
         while (wide) {
             const int src = __ffs(wide) - 1;
             wide &= wide - 1;
-            const int32_t lo = __shfl_sync(kFullMask, prev, src) + 2;
-            const int32_t hi = __shfl_sync(kFullMask, cur, src);
+            const int64_t lo = int64_t(__shfl_sync(kFullMask, prev, src)) + 2;
+            const int64_t hi = __shfl_sync(kFullMask, cur, src);
             const int64_t at = __shfl_sync(kFullMask, j0, src) + q;
-            for (int32_t r = lo + lane; r <= hi; r += 32) offsets[r] = at;
+            for (int64_t r = lo + lane; r <= hi; r += 32) offsets[r] = at;
         }
     }
 }

@@ -751,7 +751,7 @@ void forward(const Call& call, T* O, const T* A, const T* B, const T* W, const i
             wait_stream(call);
             need_fallback = host_saw_unsorted(call);
         }
-        if (need_fallback && J <= INT32_MAX) {
+        if (need_fallback && positions_fit_int(J)) {
             launch_fwd_unsorted<T, WEIGHTED>(call, O, A, B, W, PW, P, J, K, L, nO);
         } else if (need_fallback) {
             zero_if_unsorted<T><<<grid_generic, 256, 0, call.stream>>>(O, nO * KL, call.status);

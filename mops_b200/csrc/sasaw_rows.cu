@@ -27,6 +27,7 @@
 #include <initializer_list>
 #include <type_traits>
 
+#include "checks.hpp"
 #include "sasaw_rows.hpp"
 #include "unsorted.cuh"
 
@@ -726,7 +727,7 @@ template <typename T, typename F> void for_shape(const RowsShape<T>& s, F&& f) {
 
 template <typename T> bool rows_apply(const SasawProblem<T>& p) {
     return p.nA >= 1 && p.nA <= kWidest && p.nW >= 1 && p.nW <= kWidest && p.nO >= 1 && p.nO <= kWidest &&
-           p.L >= 1 && p.E >= 1 && p.E <= INT32_MAX - 64 && p.rows >= 1 && p.N <= (1 << 20);
+           p.L >= 1 && p.E >= 1 && positions_fit_int(p.E) && p.rows >= 1 && p.N <= (1 << 20);
 }
 
 // Two columns per lane (f32) from 33 columns on, where every operand allows 8-byte accesses.
