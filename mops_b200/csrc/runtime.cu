@@ -29,6 +29,7 @@ struct StreamState {
     unsigned char* workspace = nullptr;
     size_t size = 0, used = 0;
     size_t wanted = 0; // by the previous call
+    bool pending = false; // a call may still be running (it did not wait, or ended with an exception)
 };
 
 namespace {
@@ -47,10 +48,24 @@ struct ThreadState {
     int workspaces = 0;
     std::string kernels; // main kernels dispatched by the current / last call
 
-    // The thread is gone, so are its calls; cudaFree waits for what may still run.
+    // The thread is gone, its kernels may not be: cudaFree does not wait for the users of memory from a
+    // stream-ordered pool. (Relaxed: another thread may be capturing. Where the device cannot be waited
+    // for, the workspace is left behind.)
     ~ThreadState() {
-        for (auto& s : streams)
-            if (s.second.workspace != nullptr) (void)cudaFree(s.second.workspace);
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        int device = 0;
+        if (workspaces == 0 || cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess ||
+            cudaGetDevice(&device) != cudaSuccess)
+            return;
+        for (auto& s : streams) {
+            if (s.second.workspace == nullptr) continue;
+            if (!s.second.pending ||
+                (cudaSetDevice(s.first.first) == cudaSuccess && cudaDeviceSynchronize() == cudaSuccess))
+                (void)cudaFree(s.second.workspace);
+            (void)cudaGetLastError();
+        }
+        (void)cudaSetDevice(device);
+        (void)cudaThreadExchangeStreamCaptureMode(&mode);
     }
 };
 
@@ -130,6 +145,7 @@ Call begin_call() {
     }
     call.state = g_thread.last;
     call.state->used = 0;
+    call.state->pending = true;
     call.status = call.state->status;
     g_thread.epoch += 1;
     if (g_thread.epoch == 0) g_thread.epoch = 1;
@@ -162,6 +178,7 @@ void end_call(const Call& call, const char* operation, const char* const* index_
     MOPS_CUDA_OK(cudaGetLastError());
     if (!call.wait) return;
     MOPS_CUDA_OK(cudaStreamSynchronize(call.stream));
+    call.state->pending = false;
     volatile uint32_t* host = call.status.host;
     if (host[kStalled] == call.status.epoch)
         throw std::runtime_error(std::string("internal error in operation ") + operation +

@@ -39,3 +39,33 @@ def test_first_call_of_a_stream_while_the_default_stream_is_busy(oracle):
     torch.cuda.synchronize()
     for g in got:
         assert_parity(g.cpu().numpy(), want, "first call of a stream")
+
+
+def test_threads_that_end_with_calls_in_flight(oracle):
+    """Asynchronous calls from threads that end at once: their scratch memory stays until the kernels are
+    done with it."""
+    import threading
+
+    import torch
+
+    import mops_b200.torch as mt
+    t, want = _problem(oracle, J=40000)
+    filler = torch.randn(4096, 4096, device="cuda")
+    got = []
+
+    def work(stream):
+        with torch.cuda.stream(stream):
+            for _ in range(3):  # (the second call gets a workspace)
+                filler @ filler
+                got.append(mt.outer_product_scatter_add(t["A"], t["B"], t["indices_output"], t["output_size"]))
+
+    streams = [torch.cuda.Stream() for _ in range(8)]
+    for s in streams:
+        s.wait_stream(torch.cuda.current_stream())
+        thread = threading.Thread(target=work, args=(s,))
+        thread.start()
+        thread.join()
+    torch.cuda.synchronize()
+    assert len(got) == 24
+    for g in got:
+        assert_parity(g.cpu().numpy(), want, "thread that ended")
