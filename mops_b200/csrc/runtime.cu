@@ -1,6 +1,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <algorithm>
 #include <vector>
 #include <map>
 #include <mutex>
@@ -22,20 +23,30 @@ namespace mops_b200 {
 
 // What a thread keeps for a (device, stream): calls on one stream run in order, so a call's status
 // words and workspace cannot be overwritten before its own kernels are done with them, and calls on
-// different streams (which may overlap) never share them. The status block is a few bytes and lives
-// until the process exits.
+// different streams (which may overlap) never share them. Status words are never freed (kernels of
+// captured graphs hold their address) but handed on, with the workspace, to later streams.
 struct StreamState {
     Status status{};
     unsigned char* workspace = nullptr;
     size_t size = 0, used = 0;
     size_t wanted = 0; // by the previous call
     bool pending = false; // a call may still be running (it did not wait, or ended with an exception)
+    bool captured = false; // a graph holds the address of the status words
+    uint64_t last_call = 0;
 };
 
 namespace {
 
+// Lets this thread wait and free while another thread captures a graph.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { (void)cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { (void)cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 constexpr size_t kMostWorkspace = 4 << 20; // bytes per (thread, device, stream)
 constexpr int kMostWorkspaces = 16;        // per thread
+constexpr size_t kMostStreams = 64;        // per thread, before states of old streams are handed on
 
 struct ThreadState {
     cudaStream_t stream = nullptr;
@@ -43,29 +54,28 @@ struct ThreadState {
     uint32_t epoch = 0;
     // by device and stream id: a handle may come back for another stream, an id does not
     std::map<std::pair<int, unsigned long long>, StreamState> streams;
+    std::vector<std::pair<int, StreamState>> spare; // (device, state) of streams that have gone
+    uint64_t calls = 0;
     std::pair<int, unsigned long long> last_key{-1, 0};
     StreamState* last = nullptr; // of the previous call
     int workspaces = 0;
     std::string kernels; // main kernels dispatched by the current / last call
 
     // The thread is gone, its kernels may not be: cudaFree does not wait for the users of memory from a
-    // stream-ordered pool. (Relaxed: another thread may be capturing. Where the device cannot be waited
-    // for, the workspace is left behind.)
+    // stream-ordered pool. (Where the device cannot be waited for, the workspace is left behind.)
     ~ThreadState() {
-        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
         int device = 0;
-        if (workspaces == 0 || cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess ||
-            cudaGetDevice(&device) != cudaSuccess)
-            return;
-        for (auto& s : streams) {
-            if (s.second.workspace == nullptr) continue;
-            if (!s.second.pending ||
-                (cudaSetDevice(s.first.first) == cudaSuccess && cudaDeviceSynchronize() == cudaSuccess))
-                (void)cudaFree(s.second.workspace);
+        if (workspaces == 0 || cudaGetDevice(&device) != cudaSuccess) return;
+        const RelaxedCapture relaxed;
+        auto give_back = [](int on, const StreamState& s) {
+            if (s.workspace == nullptr) return;
+            if (!s.pending || (cudaSetDevice(on) == cudaSuccess && cudaDeviceSynchronize() == cudaSuccess))
+                (void)cudaFree(s.workspace);
             (void)cudaGetLastError();
-        }
+        };
+        for (auto& s : streams) give_back(s.first.first, s.second);
+        for (auto& s : spare) give_back(s.first, s.second);
         (void)cudaSetDevice(device);
-        (void)cudaThreadExchangeStreamCaptureMode(&mode);
     }
 };
 
@@ -113,6 +123,57 @@ void zero_words(uint32_t* dev, int words) {
     (void)cudaStreamDestroy(stream);
     MOPS_CUDA_OK(err);
 }
+
+// Ids of streams never come back, so a program that makes a stream per step would leave a state behind
+// each time. At kMostStreams the older half of them (but for graphs') goes to `spare`, once the device
+// has been waited for if any of their calls may still run: one wait in kMostStreams / 2 new streams.
+// Where it cannot be waited for, the states stay.
+void retire_streams(int device) {
+    std::vector<std::pair<uint64_t, std::pair<int, unsigned long long>>> old;
+    for (const auto& s : g_thread.streams)
+        if (s.first.first == device && !s.second.captured) old.push_back({s.second.last_call, s.first});
+    std::sort(old.begin(), old.end());
+    old.resize(std::min(old.size(), kMostStreams / 2));
+    const RelaxedCapture relaxed;
+    bool pending = false;
+    for (const auto& o : old) pending |= g_thread.streams[o.second].pending;
+    if (old.empty() || (pending && cudaDeviceSynchronize() != cudaSuccess)) {
+        (void)cudaGetLastError();
+        return;
+    }
+    g_thread.last = nullptr;
+    for (const auto& o : old) {
+        StreamState& state = g_thread.streams[o.second];
+        state.pending = false;
+        g_thread.spare.push_back({device, state});
+        g_thread.streams.erase(o.second);
+    }
+}
+
+StreamState& state_of(const std::pair<int, unsigned long long>& key, bool capturing) {
+    auto it = g_thread.streams.find(key);
+    if (it != g_thread.streams.end()) return it->second;
+    if (g_thread.streams.size() >= kMostStreams && !capturing) retire_streams(key.first);
+    // (a spare one with a workspace rather than one without)
+    auto spare = g_thread.spare.end();
+    for (auto s = g_thread.spare.begin(); s != g_thread.spare.end(); ++s)
+        if (s->first == key.first && (spare == g_thread.spare.end() || s->second.workspace != nullptr)) spare = s;
+    StreamState state{};
+    if (spare != g_thread.spare.end()) {
+        state = spare->second;
+        g_thread.spare.erase(spare);
+    } else {
+        void* host = nullptr;
+        // (with unified addressing the host pointer is the device-visible one)
+        MOPS_CUDA_OK(cudaHostAlloc(&host, kStatusWords * sizeof(uint32_t),
+                                   cudaHostAllocMapped | cudaHostAllocPortable));
+        for (int i = 0; i < kStatusWords; i++) static_cast<volatile uint32_t*>(host)[i] = 0;
+        state.status.host = static_cast<uint32_t*>(host);
+        MOPS_CUDA_OK(cudaMalloc(reinterpret_cast<void**>(&state.status.dev), kStatusWords * sizeof(uint32_t)));
+        zero_words(state.status.dev, kStatusWords);
+    }
+    return g_thread.streams.emplace(key, state).first->second;
+}
 } // namespace
 
 Call begin_call() {
@@ -122,30 +183,21 @@ Call begin_call() {
     call.wait = g_thread.wait;
 
     g_thread.kernels.clear();
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(call.stream, &capture) != cudaSuccess) (void)cudaGetLastError();
+    call.capturing = capture != cudaStreamCaptureStatusNone;
     unsigned long long id = 0;
     MOPS_CUDA_OK(cudaStreamGetId(call.stream, &id));
     const auto key = std::make_pair(call.device, id);
     if (g_thread.last == nullptr || key != g_thread.last_key) {
-        StreamState& state = g_thread.streams[key];
-        if (state.status.dev == nullptr) {
-            Status block{};
-            void* host = nullptr;
-            // (with unified addressing the host pointer is the device-visible one)
-            MOPS_CUDA_OK(cudaHostAlloc(&host, kStatusWords * sizeof(uint32_t),
-                                       cudaHostAllocMapped | cudaHostAllocPortable));
-            for (int i = 0; i < kStatusWords; i++) static_cast<volatile uint32_t*>(host)[i] = 0;
-            block.host = static_cast<uint32_t*>(host);
-            MOPS_CUDA_OK(cudaMalloc(reinterpret_cast<void**>(&block.dev),
-                                    kStatusWords * sizeof(uint32_t)));
-            zero_words(block.dev, kStatusWords);
-            state.status = block;
-        }
-        g_thread.last = &state;
+        g_thread.last = &state_of(key, call.capturing);
         g_thread.last_key = key;
     }
     call.state = g_thread.last;
     call.state->used = 0;
     call.state->pending = true;
+    call.state->captured |= call.capturing;
+    call.state->last_call = ++g_thread.calls;
     call.status = call.state->status;
     g_thread.epoch += 1;
     if (g_thread.epoch == 0) g_thread.epoch = 1;
@@ -342,9 +394,7 @@ void* scratch_alloc(const Call& call, size_t bytes) {
     StreamState& w = *call.state;
     bytes = (bytes + 255) / 256 * 256;
     if (bytes <= kMostWorkspace) {
-        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(call.stream, &capture) != cudaSuccess) (void)cudaGetLastError();
-        if (capture == cudaStreamCaptureStatusNone) {
+        if (!call.capturing) {
             if (w.used == 0 && w.size < w.wanted) { // grow between calls, in stream order
                 if (w.workspace != nullptr) {
                     MOPS_CUDA_OK(cudaFreeAsync(w.workspace, call.stream));

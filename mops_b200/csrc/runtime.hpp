@@ -44,6 +44,7 @@ struct Call {
     Status status;
     int device;
     StreamState* state;
+    bool capturing; // into a graph
 };
 
 [[noreturn]] void throw_cuda(cudaError_t err, const char* what, const char* file, int line);

@@ -6,7 +6,7 @@ import pytest
 import mops_b200
 from conftest import assert_parity
 from helpers import to_dev
-from mops_b200 import workloads
+from mops_b200 import _lib, workloads
 
 pytestmark = pytest.mark.gpu
 
@@ -69,3 +69,51 @@ def test_threads_that_end_with_calls_in_flight(oracle):
     assert len(got) == 24
     for g in got:
         assert_parity(g.cpu().numpy(), want, "thread that ended")
+
+
+def test_many_short_lived_streams(oracle):
+    """A stream per step: states of streams that have gone serve later ones (no allocation is left behind
+    per stream), each stream's status words are its own, and calls in flight keep theirs."""
+    import ctypes
+
+    import torch
+
+    import mops_b200.torch as mt
+    rt = ctypes.CDLL("libcudart.so.12")
+    t, want = _problem(oracle)
+    s, want_s = _problem(oracle, unsorted=False)
+
+    def steps(n, wait):
+        got = []
+        for i in range(n):
+            handle = ctypes.c_void_p()
+            assert rt.cudaStreamCreateWithFlags(ctypes.byref(handle), 1) == 0
+            with torch.cuda.stream(torch.cuda.ExternalStream(handle.value)):
+                args = t if i % 3 else s
+                got.append((_call if wait else mt.outer_product_scatter_add)(
+                    *((args,) if wait else (args["A"], args["B"], args["indices_output"], args["output_size"]))))
+            assert rt.cudaStreamDestroy(handle) == 0
+        torch.cuda.synchronize()
+        for i, g in enumerate(got):
+            assert_parity(g.cpu().numpy(), want if i % 3 else want_s, f"stream {i}")
+
+    steps(200, wait=False)
+    steps(200, wait=True)
+    # through the C ABI into one output: torch itself keeps memory for every stream it has seen
+    small = to_dev(workloads.opsa(J=20, K=2, L=2, nO=3), np.float64)
+    out = torch.empty(3, 2, 2, dtype=torch.float64, device="cuda")
+    structs = [_lib.make_struct(x.data_ptr(), x.shape)
+               for x in (out, small["A"], small["B"], small["indices_output"])]
+    lib = _lib.library()
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    for i in range(8000):  # (512 bytes each where they are left behind: 4 MB)
+        handle = ctypes.c_void_p()
+        assert rt.cudaStreamCreateWithFlags(ctypes.byref(handle), 1) == 0
+        lib.mops_b200_set_stream(handle)
+        try:
+            _lib.call("mops_cuda_outer_product_scatter_add_f64", structs)
+        finally:
+            lib.mops_b200_set_stream(None)
+        assert rt.cudaStreamDestroy(handle) == 0
+    assert before - torch.cuda.mem_get_info()[0] < 3 << 20
