@@ -121,10 +121,12 @@ Tensor requested(const Tensor& t) { return t.defined() && t.numel() == 0 ? Tenso
 }
 
 // The gradients of an operation: through the differentiable Function when this backward pass is itself
-// recorded (create_graph), else straight from the kernels, without a node and saved variables that
-// nobody would use.
+// recorded (create_graph) or an argument carries a forward-mode tangent (which Function refuses, and
+// which the kernels would drop), else straight from the kernels, without a node and saved variables
+// that nobody would use.
 template <typename Backward, typename... Args> tensor_list backward_of(const Args&... args) {
-    return at::GradMode::is_enabled() ? Backward::apply(args...) : Backward::run(args...);
+    const bool tangent = (... || (args.defined() && args._fw_grad(/*level=*/0).defined()));
+    return at::GradMode::is_enabled() || tangent ? Backward::apply(args...) : Backward::run(args...);
 }
 
 // =============================================================================== HPE

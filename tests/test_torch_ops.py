@@ -137,6 +137,33 @@ def test_second_derivatives_without_a_kernel_raise():
 
 
 @pytest.mark.gpu
+def test_forward_mode_tangents_are_refused_in_the_backward_pass():
+    """The operators have no forward-mode derivatives: a tangent on grad_output is an error, also in a
+    backward pass that is not recorded, and never dropped."""
+    import torch.autograd.forward_ad as fwAD
+    A, B, W = (torch.rand(*s, dtype=torch.float64, device="cuda", requires_grad=True)
+               for s in ((20, 6), (20, 5), (4, 5)))
+    C = torch.rand(9, dtype=torch.float64, device="cuda")
+    W3 = torch.rand(4, 3, 5, dtype=torch.float64, device="cuda", requires_grad=True)
+    idx = torch.sort(torch.randint(4, (20,), dtype=torch.int32, device="cuda")).values
+    ri = lambda n, *s: torch.randint(n, s, dtype=torch.int32, device="cuda")
+    outs = [
+        (mt.homogeneous_polynomial_evaluation(A, C, ri(6, 9, 3)), [A]),
+        (mt.sparse_accumulation_of_products(A, B, C, ri(6, 9), ri(5, 9), ri(4, 9), 4), [A, B]),
+        (mt.outer_product_scatter_add(A, B, idx, 4), [A, B]),
+        (mt.outer_product_scatter_add_with_weights(A, B, W, idx, idx), [A, B, W]),
+        (mt.sparse_accumulation_scatter_add_with_weights(A, B, C, W3, ri(6, 9), idx, ri(3, 9), idx,
+                                                         ri(4, 9), 4), [A, B, W3]),
+    ]
+    for out, inputs in outs:
+        for create_graph in (True, False):
+            with fwAD.dual_level():
+                g = fwAD.make_dual(torch.ones_like(out), torch.ones_like(out))
+                with pytest.raises(RuntimeError, match="jvp is not implemented"):
+                    torch.autograd.grad(out, inputs, g, create_graph=create_graph, retain_graph=True)
+
+
+@pytest.mark.gpu
 def test_torchscript_round_trip():
     class M(torch.nn.Module):
         def forward(self, A: torch.Tensor, B: torch.Tensor, idx: torch.Tensor) -> torch.Tensor:
