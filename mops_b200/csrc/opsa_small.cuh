@@ -66,7 +66,13 @@ opsa_fwd_small(T* __restrict__ O, const T* __restrict__ A, const T* __restrict__
                 w = __ldg(PW + e);
                 if (clamp_index(w, n_rows)) report_bad_index(st, 1);
             }
-            add_products<T, KC, WEIGHTED, U>(acc, e, w, count, A, B, W, K, L, kb, kn, lc, stage[warp], lane);
+            for (int u0 = 0; u0 < count; u0 += U) {
+                T b[U];
+                load_entries<T, KC, WEIGHTED, U>(b, e, w, u0, count, A, B, W, K, L, kb, kn, lc, stage[warp], lane);
+#pragma unroll
+                for (int u = 0; u < U; u++) add_entry<T, KC>(acc, stage[warp] + u * KC, b[u]);
+                __syncwarp();
+            }
         };
         for (int p0 = lo; p0 < hi; p0 += 32) {
             const int p = p0 + lane;

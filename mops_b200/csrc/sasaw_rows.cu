@@ -795,7 +795,7 @@ template <typename T> bool sasaw_forward_rows(const Call& call, const SasawProbl
         unsorted = host_saw_unsorted(call);
     }
     if (unsorted) {
-        const int sorters = sort_blocks(call, p.E);
+        const int sorters = sort_blocks(call, p.E, p.rows);
         void* scratch = scratch_alloc(call, entry_sort_bytes(p.E, p.rows, sorters));
         const EntrySort sort = entry_sort_at(scratch, p.rows, sorters);
         launch_sorting(call, sorters, sort_if_unsorted_grid, sort_if_unsorted_block, sort, p.I, p.E, p.rows,
@@ -830,7 +830,7 @@ bool sasaw_backward_rows(const Call& call, const SasawProblem<T>& p, T* gA, T* g
     if (s.smem > static_cast<size_t>(max_optin_smem(call.device))) return false;
     TableRef table = dense_table(call, p, s, true);
     // the edges in the order of J
-    const int sorters = sort_blocks(call, p.E);
+    const int sorters = sort_blocks(call, p.E, p.rows);
     TableKey key{};
     key.kind = kEdgeOrder;
     key.ptr[0] = p.J;

@@ -9,6 +9,8 @@
 #ifndef MOPS_B200_UNSORTED_CUH
 #define MOPS_B200_UNSORTED_CUH
 
+#include <algorithm>
+
 #include <cooperative_groups.h>
 
 #include "device.cuh"
@@ -17,7 +19,8 @@ namespace mops_b200 {
 namespace {
 
 constexpr int kSortThreads = 1024;         // one block per SM, 64 registers
-constexpr int64_t kOneBlockEntries = 512;  // up to here one block (and an ordinary launch) will do
+constexpr int64_t kOneBlockEntries = 512;  // up to here one block (and an ordinary launch) will do,
+constexpr int64_t kOneBlockWrites = 8192;  // if it does not have more than this to clear
 
 // Scratch of the sort.
 struct EntrySort {
@@ -128,7 +131,11 @@ sort_if_unsorted_block(EntrySort s, const int32_t* __restrict__ P, int64_t J, in
     sort_entries(s, P, J, n_rows, true, st, [] { __syncthreads(); });
 }
 
-inline int sort_blocks(const Call& call, int64_t J) { return J <= kOneBlockEntries ? 1 : sm_count(call.device); }
+// `writes`: the rows, or the values of the result where the kernel clears it. (500 entries for 100 000 rows
+// of 13 x 32: one block takes as long for the zeros as the whole GPU for 148 times as many.)
+inline int sort_blocks(const Call& call, int64_t J, int64_t writes) {
+    return J <= kOneBlockEntries && writes <= kOneBlockWrites ? 1 : sm_count(call.device);
+}
 
 // Launches `grid_kernel` cooperatively, or `block_kernel` with one block for few entries.
 template <typename... Params, typename... Args>
@@ -154,117 +161,182 @@ void launch_sorting(const Call& call, int blocks, void (*grid_kernel)(Params...)
 // ---- forward of OPSA / OPSAW
 constexpr int kGatherEntries = 8; // entries whose rows are in flight at a time
 
-// acc[k] += A[e, kb + k] (B o W)[e, lc] for the `count` (<= 32) entries e that the lanes hold, U at a time.
-template <typename T, int KC, bool WEIGHTED, int U = kGatherEntries>
-__device__ __forceinline__ void add_products(T (&acc)[KC], int my_entry, int my_w, int count,
+// Entries u0 .. u0 + U - 1 of the `count` (<= 32) that the lanes hold: (B o W)[e, lc] in `b` (0 beyond
+// `count`), A[e, kb .. kb + kn) in `stage`.
+template <typename T, int KC, bool WEIGHTED, int U>
+__device__ __forceinline__ void load_entries(T (&b)[U], int my_entry, int my_w, int u0, int count,
                                              const T* __restrict__ A, const T* __restrict__ B,
                                              const T* __restrict__ W, int K, int L, int kb, int kn, int lc,
                                              T* stage, int lane) {
-    for (int u0 = 0; u0 < count; u0 += U) {
-        T b[U], w[U];
+    T w[U];
 #pragma unroll
-        for (int x = lane; x < U * KC; x += 32) {
-            const int u = x / KC, k = x - u * KC;
-            const int64_t e = __shfl_sync(kFullMask, my_entry, u0 + u);
-            stage[x] = k < kn && u0 + u < count ? __ldg(A + e * K + kb + k) : T(0);
-        }
+    for (int x = lane; x < U * KC; x += 32) {
+        const int u = x / KC, k = x - u * KC;
+        const int64_t e = __shfl_sync(kFullMask, my_entry, u0 + u);
+        stage[x] = k < kn && u0 + u < count ? __ldg(A + e * K + kb + k) : T(0);
+    }
 #pragma unroll
-        for (int u = 0; u < U; u++) {
-            const int64_t e = __shfl_sync(kFullMask, my_entry, u0 + u);
-            b[u] = __ldg(B + e * L + lc);
-            if (WEIGHTED)
-                w[u] = __ldg(W + static_cast<int64_t>(__shfl_sync(kFullMask, my_w, u0 + u)) * L + lc);
-        }
-        __syncwarp();
+    for (int u = 0; u < U; u++) {
+        const int64_t e = __shfl_sync(kFullMask, my_entry, u0 + u);
+        b[u] = __ldg(B + e * L + lc);
+        if (WEIGHTED) w[u] = __ldg(W + static_cast<int64_t>(__shfl_sync(kFullMask, my_w, u0 + u)) * L + lc);
+    }
+    __syncwarp();
 #pragma unroll
-        for (int u = 0; u < U; u++) {
-            if (WEIGHTED) b[u] *= w[u];
-            if (u0 + u >= count) b[u] = T(0);
-            constexpr int V = 16 / sizeof(T);
-#pragma unroll
-            for (int k = 0; k < KC; k += V) {
-                T a[V];
-                load_vec<T, V>(stage + u * KC + k, a);
-#pragma unroll
-                for (int v = 0; v < V; v++) acc[k + v] += a[v] * b[u];
-            }
-        }
-        __syncwarp();
+    for (int u = 0; u < U; u++) {
+        if (WEIGHTED) b[u] *= w[u];
+        if (u0 + u >= count) b[u] = T(0);
     }
 }
 
-// One warp per output row and KC by 32 part of it, lane = column l of B. The entries' numbers (and
-// their rows of W) are fetched 32 at a time, one per lane; B rows go to registers and A rows to shared
-// memory eight entries at a time (`stage`: [8][KC] of this warp), where they are read as
-// broadcasts. Bounded by the latency of the gathers. (Handing A around by shuffles, one per product,
-// took 430 us where this takes 175.)
+// acc[k] += a[k] b
+template <typename T, int KC> __device__ __forceinline__ void add_entry(T (&acc)[KC], const T* a_row, T b) {
+    constexpr int V = 16 / sizeof(T);
+#pragma unroll
+    for (int k = 0; k < KC; k += V) {
+        T a[V];
+        load_vec<T, V>(a_row + k, a);
+#pragma unroll
+        for (int v = 0; v < V; v++) acc[k + v] += a[v] * b;
+    }
+}
+
+// A warp takes a segment of S consecutive positions of the sorted entries and a KC by 32 part of their
+// rows, lane = column l of B. The entries' numbers and rows (of O, of W) are fetched 32 at a time, one
+// per lane; B rows go to registers and A rows to shared memory eight entries at a time (`stage`: [8][KC]
+// of this warp), where they are read as broadcasts. A row that lies in one segment is stored; one
+// that is cut is added up with atomics (zero_cut_rows has cleared it), so that few or uneven rows
+// still occupy every warp: 60 000 entries in 144 rows, f32, 8 x 17: 375 us with a warp per row, 85 with
+// atomics per entry. Bounded by the latency of the gathers. (Handing A around by shuffles, one per
+// product, took 430 us where this takes 175.)
 template <typename T, int KC, bool WEIGHTED>
 __device__ __forceinline__ void opsa_rows_gathered(T* __restrict__ O, const T* __restrict__ A,
                                                    const T* __restrict__ B, const T* __restrict__ W,
-                                                   const int32_t* __restrict__ PW, const EntrySort& s, int K,
-                                                   int L, int64_t n_rows, T* stage, const Status& st) {
+                                                   const int32_t* __restrict__ PW,
+                                                   const int32_t* __restrict__ P, const EntrySort& s, int K,
+                                                   int L, int64_t n_rows, int S, T* stage, const Status& st) {
+    constexpr int U = kGatherEntries;
     const int lane = threadIdx.x & 31;
     const int64_t warps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
     const int k_units = (K + KC - 1) / KC, units = k_units * ((L + 31) / 32);
-    // consecutive warps take the parts of one row: what they both read is in the caches
+    const int total = s.starts[n_rows]; // (bad rows are left out)
+    const int64_t segments = (static_cast<int64_t>(total) + S - 1) / S;
+    // consecutive warps take the parts of one segment: what they both read is in the caches
     for (int64_t unit = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-         unit < n_rows * units; unit += warps) {
-        const int64_t r = unit / units;
-        const int part = static_cast<int>(unit - r * units), lb = part / k_units * 32;
+         unit < segments * units; unit += warps) {
+        const int p_lo = static_cast<int>(unit / units * S), p_hi = p_lo + S < total ? p_lo + S : total;
+        const int part = static_cast<int>(unit % units), lb = part / k_units * 32;
         const int kb = (part - part / k_units * k_units) * KC;
-        const int lo = s.starts[r], hi = s.starts[r + 1];
         const int l = lb + lane, lc = l < L ? l : L - 1;
         const int kn = K - kb < KC ? K - kb : KC;
+        // rows that go on in the neighbouring segments
+        const int before = p_lo > 0 ? __ldg(P + s.perm[p_lo - 1]) : -1;
+        const int after = p_hi < total ? __ldg(P + s.perm[p_hi]) : -1;
         T acc[KC];
 #pragma unroll
         for (int k = 0; k < KC; k++) acc[k] = T(0);
-        for (int p0 = lo; p0 < hi; p0 += 32) {
-            const int count = hi - p0 < 32 ? hi - p0 : 32;
+        int row = -1;
+        auto flush = [&] {
+            T* dst = O + (static_cast<int64_t>(row) * K + kb) * L + l;
+            const bool cut = row == before || row == after;
+#pragma unroll
+            for (int k = 0; k < KC; k++) {
+                if (row >= 0 && l < L && k < kn) {
+                    if (cut)
+                        red_add(dst + static_cast<int64_t>(k) * L, acc[k]);
+                    else
+                        dst[static_cast<int64_t>(k) * L] = acc[k];
+                }
+                acc[k] = T(0);
+            }
+        };
+        for (int p0 = p_lo; p0 < p_hi; p0 += 32) {
+            const int count = p_hi - p0 < 32 ? p_hi - p0 : 32;
             const int my_entry = s.perm[p0 + (lane < count ? lane : 0)];
+            const int my_row = __ldg(P + my_entry);
             int my_w = 0;
             if (WEIGHTED) {
                 my_w = __ldg(PW + my_entry);
                 if (clamp_index(my_w, static_cast<int32_t>(n_rows))) report_bad_index(st, 1);
             }
-            add_products<T, KC, WEIGHTED>(acc, my_entry, my_w, count, A, B, W, K, L, kb, kn, lc, stage, lane);
-        }
-        if (l < L) {
+            for (int u0 = 0; u0 < count; u0 += U) {
+                T b[U];
+                load_entries<T, KC, WEIGHTED, U>(b, my_entry, my_w, u0, count, A, B, W, K, L, kb, kn, lc, stage, lane);
 #pragma unroll
-            for (int k = 0; k < KC; k++)
-                if (k < kn) O[(r * K + kb + k) * L + l] = acc[k];
+                for (int u = 0; u < U; u++) {
+                    const int r = __shfl_sync(kFullMask, my_row, u0 + u);
+                    if (u0 + u < count) {
+                        if (r != row) {
+                            flush();
+                            row = r;
+                        }
+                        add_entry<T, KC>(acc, stage + u * KC, b[u]);
+                    }
+                }
+                __syncwarp();
+            }
         }
+        flush();
+    }
+}
+
+// Clears the rows that nobody stores: those without entries and those that segments of S positions cut.
+template <typename T>
+__device__ __forceinline__ void zero_cut_rows(T* __restrict__ O, const EntrySort& s, int64_t row_size,
+                                              int64_t n_rows, int S) {
+    const int lane = threadIdx.x & 31;
+    const int64_t warps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
+    for (int64_t r = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; r < n_rows; r += warps) {
+        const int lo = s.starts[r], hi = s.starts[r + 1];
+        if (lo < hi && lo / S == (hi - 1) / S) continue;
+        for (int64_t x = lane; x < row_size; x += 32) O[r * row_size + x] = T(0);
     }
 }
 
 template <typename T, int KC, bool WEIGHTED>
 __global__ void __launch_bounds__(kSortThreads)
 opsa_fwd_unsorted_grid(T* O, const T* A, const T* B, const T* W, const int32_t* PW, const int32_t* P,
-                       EntrySort s, int64_t J, int K, int L, int64_t n_rows, Status st) {
+                       EntrySort s, int64_t J, int K, int L, int64_t n_rows, int S, Status st) {
     __shared__ __align__(16) T stage[kSortThreads / 32][kGatherEntries * KC];
     if (!saw_unsorted(st)) return;
-    sort_entries(s, P, J, n_rows, false, st, [] { cooperative_groups::this_grid().sync(); });
-    opsa_rows_gathered<T, KC, WEIGHTED>(O, A, B, W, PW, s, K, L, n_rows, stage[threadIdx.x >> 5], st);
+    auto sync = [] { cooperative_groups::this_grid().sync(); };
+    sort_entries(s, P, J, n_rows, false, st, sync);
+    zero_cut_rows(O, s, static_cast<int64_t>(K) * L, n_rows, S);
+    sync();
+    opsa_rows_gathered<T, KC, WEIGHTED>(O, A, B, W, PW, P, s, K, L, n_rows, S, stage[threadIdx.x >> 5], st);
 }
 template <typename T, int KC, bool WEIGHTED>
 __global__ void __launch_bounds__(kSortThreads)
 opsa_fwd_unsorted_block(T* O, const T* A, const T* B, const T* W, const int32_t* PW, const int32_t* P,
-                        EntrySort s, int64_t J, int K, int L, int64_t n_rows, Status st) {
+                        EntrySort s, int64_t J, int K, int L, int64_t n_rows, int S, Status st) {
     __shared__ __align__(16) T stage[kSortThreads / 32][kGatherEntries * KC];
     if (!saw_unsorted(st)) return;
-    sort_entries(s, P, J, n_rows, false, st, [] { __syncthreads(); });
-    opsa_rows_gathered<T, KC, WEIGHTED>(O, A, B, W, PW, s, K, L, n_rows, stage[threadIdx.x >> 5], st);
+    auto sync = [] { __syncthreads(); };
+    sort_entries(s, P, J, n_rows, false, st, sync);
+    zero_cut_rows(O, s, static_cast<int64_t>(K) * L, n_rows, S);
+    sync();
+    opsa_rows_gathered<T, KC, WEIGHTED>(O, A, B, W, PW, P, s, K, L, n_rows, S, stage[threadIdx.x >> 5], st);
+}
+
+// Positions per segment: one segment and part per warp, within bounds (32 entries are fetched at a time;
+// 512 so that the warps of a large problem end together).
+inline int segment_length(int64_t J, int parts, int blocks) {
+    const int64_t warps = static_cast<int64_t>(blocks) * (kSortThreads / 32);
+    const int64_t S = ceil_div(ceil_div(J * parts, warps), 32) * 32;
+    return static_cast<int>(std::min<int64_t>(std::max<int64_t>(S, 32), 512));
 }
 
 template <typename T, bool WEIGHTED>
 void launch_fwd_unsorted(const Call& call, T* O, const T* A, const T* B, const T* W, const int32_t* PW,
                          const int32_t* P, int64_t J, int K, int L, int64_t n_rows) {
-    const int blocks = sort_blocks(call, J);
+    const int blocks = sort_blocks(call, J, n_rows * K * L);
     void* scratch = scratch_alloc(call, entry_sort_bytes(J, n_rows, blocks));
     const EntrySort s = entry_sort_at(scratch, n_rows, blocks);
 #define MOPS_B200_LAUNCH(KC_)                                                                      \
     launch_sorting(call, blocks, opsa_fwd_unsorted_grid<T, KC_, WEIGHTED>,                         \
                    opsa_fwd_unsorted_block<T, KC_, WEIGHTED>, O, A, B, W, PW, P, s, J, K, L,       \
-                   n_rows, call.status);
+                   n_rows, segment_length(J, static_cast<int>(ceil_div(K, KC_) * ceil_div(L, 32)), blocks), \
+                   call.status);
     if (K <= 4) {
         MOPS_B200_LAUNCH(4)
     } else {

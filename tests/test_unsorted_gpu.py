@@ -4,7 +4,8 @@ receives everything, against the CPU oracle at the parity tolerances."""
 import numpy as np
 import pytest
 
-from mops_b200 import workloads
+from helpers import run_checker, run_library, to_dev
+from mops_b200 import _lib, workloads
 from test_parity_gpu import compare
 
 pytestmark = pytest.mark.gpu
@@ -36,3 +37,35 @@ def test_gradient_rows_of_odd_sizes(oracle, K, L, dtype):
     start, and the end of the array inside a 16-byte piece (an odd number of rows)."""
     compare("opsa", workloads.opsa(J=3001, K=K, L=L, nO=57), dtype, oracle, what=f"opsa odd {K}x{L}")
     compare("opsa", workloads.opsa(J=7, K=K, L=L, nO=1), dtype, oracle, what=f"opsa one row {K}x{L}")
+
+
+def _in_f64(oracle, op, d):
+    """The f32 operands' results in f64."""
+    rounded = {k: v.astype(np.float32).astype(np.float64) if isinstance(v, np.ndarray) and v.dtype == np.float64
+               else v for k, v in d.items()}
+    return run_checker(oracle, op, rounded, np.float64)
+
+
+@pytest.mark.parametrize("op", ["opsa", "opsaw"])
+@pytest.mark.parametrize("kw", [dict(E=60001, n=31, K=8, L=17), dict(E=40003, n=1000, K=13, L=32), dict(E=9001, n=3, K=5, L=70),
+                                dict(E=500, n=90001, K=13, L=32), dict(E=400, n=5, K=3, L=8)])
+@pytest.mark.parametrize("rows", ["even", "half in one", "all in one"])
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+def test_few_and_uneven_rows(oracle, op, kw, rows, dtype):
+    """Rows cut by the segments of the gathering kernel, rows of one segment, empty ones."""
+    kw = dict(kw)
+    E, n = kw.pop("E"), kw.pop("n")
+    d = workloads.opsa(J=E, nO=n, **kw) if op == "opsa" else workloads.opsaw(E=E, n=n, **kw)
+    po = np.random.default_rng(2).permutation(d["indices_output"])
+    if rows != "even":
+        po[: E if rows == "all in one" else E // 2] = n // 2
+        po[0] = n - 1  # (still not sorted)
+    d["indices_output"] = po.astype(np.int32)
+    if dtype == np.float32 and rows != "even":
+        # the oracle's own f32 chains over one row are too long for the tolerance: f64 on the same operands
+        got, want = run_library(op, to_dev(d, dtype)), _in_f64(oracle, op, d)
+        for k in want:
+            scale = np.abs(want[k]).max()
+            assert np.abs(got[k] - want[k]).max() <= 1e-5 * scale, f"{op} {kw} {rows} {k}"
+        return
+    compare(op, d, dtype, oracle, what=f"{op} {E} {n} {kw} {rows}")
