@@ -46,6 +46,18 @@ def _in_f64(oracle, op, d):
     return run_checker(oracle, op, rounded, np.float64)
 
 
+@pytest.mark.parametrize("K,L", [(7, 25), (10, 3), (15, 17), (13, 31)])
+def test_f32_gradients_of_odd_rows_keep_their_precision(oracle, K, L):
+    """grad_output rows that are no multiple of 16 bytes: no less than f32 products (7e-8 of the norm)."""
+    d = workloads.opsa(J=7700, K=K, L=L, nO=57)
+    t = to_dev(d, np.float32)
+    got, want = run_library("opsa", t), _in_f64(oracle, "opsa", d)
+    assert any("opsa_vjp_pipe<f32" in k for k in _lib.last_kernels())
+    for k in ("grad_A", "grad_B"):
+        error = np.linalg.norm(got[k].astype(np.float64) - want[k]) / np.linalg.norm(want[k])
+        assert error < 7e-8, f"{K}x{L} {k}: {error:.1e}"
+
+
 @pytest.mark.parametrize("op", ["opsa", "opsaw"])
 @pytest.mark.parametrize("kw", [dict(E=60001, n=31, K=8, L=17), dict(E=40003, n=1000, K=13, L=32), dict(E=9001, n=3, K=5, L=70),
                                 dict(E=500, n=90001, K=13, L=32), dict(E=400, n=5, K=3, L=8)])
