@@ -8,6 +8,8 @@
 #ifndef MOPS_B200_OPSA_SMALL_CUH
 #define MOPS_B200_OPSA_SMALL_CUH
 
+#include <type_traits>
+
 #include "unsorted.cuh"
 
 namespace mops_b200 {
@@ -16,12 +18,17 @@ namespace {
 constexpr int kSmallEntries = 4096; // 16 KB of index per block
 constexpr int kSmallWarps = 4;
 
+// Products and sums of the weighted operation are f64 at any number of entries, as in the streaming
+// kernels (opsa_pipe.cuh): the precision of a model must not depend on the size of its batch.
+template <typename T, bool WEIGHTED> using SmallSum = std::conditional_t<WEIGHTED, double, T>;
+
 // Forward: a warp per output row and 8 by 32 part of it, as for unsorted input (unsorted.cuh).
 template <typename T, bool WEIGHTED>
 __global__ void __launch_bounds__(kSmallWarps * 32)
 opsa_fwd_small(T* __restrict__ O, const T* __restrict__ A, const T* __restrict__ B, const T* __restrict__ W,
                const int32_t* __restrict__ PW, const int32_t* __restrict__ P, int J, int K, int L, int n_rows,
                Status st) {
+    using S = SmallSum<T, WEIGHTED>;
     constexpr int KC = 8, U = 16; // (latency: more rows in flight than in unsorted.cuh)
     __shared__ int32_t index[kSmallEntries];
     __shared__ int32_t found[kSmallWarps][64];
@@ -55,9 +62,9 @@ opsa_fwd_small(T* __restrict__ O, const T* __restrict__ A, const T* __restrict__
         const int lb = part / k_units * 32, kb = part % k_units * KC;
         const int l = lb + lane, lc = l < L ? l : L - 1, kn = K - kb < KC ? K - kb : KC;
         const int lo = sorted ? lower_bound(r) : 0, hi = sorted ? lower_bound(r + 1) : J;
-        T acc[KC];
+        S acc[KC];
 #pragma unroll
-        for (int k = 0; k < KC; k++) acc[k] = T(0);
+        for (int k = 0; k < KC; k++) acc[k] = S(0);
         int held = 0; // entries of this row found and not yet added
         auto add = [&](int count) {
             const int e = found[warp][lane < count ? lane : 0];
@@ -67,10 +74,10 @@ opsa_fwd_small(T* __restrict__ O, const T* __restrict__ A, const T* __restrict__
                 if (clamp_index(w, n_rows)) report_bad_index(st, 1);
             }
             for (int u0 = 0; u0 < count; u0 += U) {
-                T b[U];
-                load_entries<T, KC, WEIGHTED, U>(b, e, w, u0, count, A, B, W, K, L, kb, kn, lc, stage[warp], lane);
+                S b[U];
+                load_entries<T, KC, WEIGHTED, U, S>(b, e, w, u0, count, A, B, W, K, L, kb, kn, lc, stage[warp], lane);
 #pragma unroll
-                for (int u = 0; u < U; u++) add_entry<T, KC>(acc, stage[warp] + u * KC, b[u]);
+                for (int u = 0; u < U; u++) add_entry<T, KC, S>(acc, stage[warp] + u * KC, b[u]);
                 __syncwarp();
             }
         };
@@ -95,7 +102,7 @@ opsa_fwd_small(T* __restrict__ O, const T* __restrict__ A, const T* __restrict__
         if (l < L) {
 #pragma unroll
             for (int k = 0; k < KC; k++)
-                if (k < kn) O[(static_cast<int64_t>(r) * K + kb + k) * L + l] = acc[k];
+                if (k < kn) O[(static_cast<int64_t>(r) * K + kb + k) * L + l] = static_cast<T>(acc[k]);
         }
     }
 }
@@ -118,28 +125,29 @@ opsa_vjp_small(T* __restrict__ gA, T* __restrict__ gB, T* __restrict__ gW, const
         w_row = __ldg(PW + e);
         if (clamp_index(w_row, n_rows) && lane == 0) report_bad_index(st, 1);
     }
-    T a[KP], ga[KP];
+    using S = SmallSum<T, WEIGHTED>;
+    S a[KP], ga[KP];
 #pragma unroll
     for (int k = 0; k < KP; k++) {
         a[k] = k < K ? __ldg(A + e * K + k) : T(0);
-        ga[k] = T(0);
+        ga[k] = S(0);
     }
     for (int l = lane; l < L; l += 32) {
         const T* g = gO + static_cast<int64_t>(row) * K * L + l;
-        T v[KP];
+        S v[KP];
 #pragma unroll
         for (int k = 0; k < KP; k++) v[k] = k < K ? __ldg(g + k * L) : T(0);
-        const T b = __ldg(B + e * L + l);
-        const T w = WEIGHTED ? __ldg(W + static_cast<int64_t>(w_row) * L + l) : T(1);
-        const T bw = WEIGHTED ? b * w : b;
-        T s = T(0);
+        const S b = __ldg(B + e * L + l);
+        const S w = WEIGHTED ? __ldg(W + static_cast<int64_t>(w_row) * L + l) : T(1);
+        const S bw = WEIGHTED ? b * w : b;
+        S s = S(0);
 #pragma unroll
         for (int k = 0; k < KP; k++) {
             s += v[k] * a[k];
             ga[k] += v[k] * bw;
         }
-        if (gB != nullptr) gB[e * L + l] = WEIGHTED ? s * w : s;
-        if (WEIGHTED && gW != nullptr) red_add(gW + static_cast<int64_t>(w_row) * L + l, s * b);
+        if (gB != nullptr) gB[e * L + l] = static_cast<T>(WEIGHTED ? s * w : s);
+        if (WEIGHTED && gW != nullptr) red_add(gW + static_cast<int64_t>(w_row) * L + l, static_cast<T>(s * b));
     }
     if (gA == nullptr) return;
     int which = 0;
@@ -150,14 +158,14 @@ opsa_vjp_small(T* __restrict__ gA, T* __restrict__ gB, T* __restrict__ gW, const
 #pragma unroll
         for (int i = 0; i < KP / 2; i++) {
             if (i < h) {
-                const T send = upper ? ga[i] : ga[i + h], keep = upper ? ga[i + h] : ga[i];
+                const S send = upper ? ga[i] : ga[i + h], keep = upper ? ga[i + h] : ga[i];
                 ga[i] = keep + __shfl_xor_sync(kFullMask, send, o);
             }
         }
         which += upper ? h : 0;
     }
-    const T sum = ga[0] + __shfl_xor_sync(kFullMask, ga[0], 1);
-    if ((lane & 1) == 0 && which < K) gA[e * K + which] = sum;
+    const S sum = ga[0] + __shfl_xor_sync(kFullMask, ga[0], 1);
+    if ((lane & 1) == 0 && which < K) gA[e * K + which] = static_cast<T>(sum);
 }
 
 // Few enough entries that three launches cost more than one slower kernel (one warp per row, one round

@@ -162,9 +162,9 @@ void launch_sorting(const Call& call, int blocks, void (*grid_kernel)(Params...)
 constexpr int kGatherEntries = 8; // entries whose rows are in flight at a time
 
 // Entries u0 .. u0 + U - 1 of the `count` (<= 32) that the lanes hold: (B o W)[e, lc] in `b` (0 beyond
-// `count`), A[e, kb .. kb + kn) in `stage`.
-template <typename T, int KC, bool WEIGHTED, int U>
-__device__ __forceinline__ void load_entries(T (&b)[U], int my_entry, int my_w, int u0, int count,
+// `count`), A[e, kb .. kb + kn) in `stage`. S: the type of products and sums.
+template <typename T, int KC, bool WEIGHTED, int U, typename S>
+__device__ __forceinline__ void load_entries(S (&b)[U], int my_entry, int my_w, int u0, int count,
                                              const T* __restrict__ A, const T* __restrict__ B,
                                              const T* __restrict__ W, int K, int L, int kb, int kn, int lc,
                                              T* stage, int lane) {
@@ -184,20 +184,21 @@ __device__ __forceinline__ void load_entries(T (&b)[U], int my_entry, int my_w, 
     __syncwarp();
 #pragma unroll
     for (int u = 0; u < U; u++) {
-        if (WEIGHTED) b[u] *= w[u];
-        if (u0 + u >= count) b[u] = T(0);
+        if (WEIGHTED) b[u] *= static_cast<S>(w[u]);
+        if (u0 + u >= count) b[u] = S(0);
     }
 }
 
 // acc[k] += a[k] b
-template <typename T, int KC> __device__ __forceinline__ void add_entry(T (&acc)[KC], const T* a_row, T b) {
+template <typename T, int KC, typename S>
+__device__ __forceinline__ void add_entry(S (&acc)[KC], const T* a_row, S b) {
     constexpr int V = 16 / sizeof(T);
 #pragma unroll
     for (int k = 0; k < KC; k += V) {
         T a[V];
         load_vec<T, V>(a_row + k, a);
 #pragma unroll
-        for (int v = 0; v < V; v++) acc[k + v] += a[v] * b;
+        for (int v = 0; v < V; v++) acc[k + v] += static_cast<S>(a[v]) * b;
     }
 }
 
@@ -261,7 +262,7 @@ __device__ __forceinline__ void opsa_rows_gathered(T* __restrict__ O, const T* _
             }
             for (int u0 = 0; u0 < count; u0 += U) {
                 T b[U];
-                load_entries<T, KC, WEIGHTED, U>(b, my_entry, my_w, u0, count, A, B, W, K, L, kb, kn, lc, stage, lane);
+                load_entries<T, KC, WEIGHTED, U, T>(b, my_entry, my_w, u0, count, A, B, W, K, L, kb, kn, lc, stage, lane);
 #pragma unroll
                 for (int u = 0; u < U; u++) {
                     const int r = __shfl_sync(kFullMask, my_row, u0 + u);
@@ -270,7 +271,7 @@ __device__ __forceinline__ void opsa_rows_gathered(T* __restrict__ O, const T* _
                             flush();
                             row = r;
                         }
-                        add_entry<T, KC>(acc, stage + u * KC, b[u]);
+                        add_entry<T, KC, T>(acc, stage + u * KC, b[u]);
                     }
                 }
                 __syncwarp();

@@ -46,6 +46,23 @@ def _in_f64(oracle, op, d):
     return run_checker(oracle, op, rounded, np.float64)
 
 
+@pytest.mark.parametrize("E", [200, 512, 513, 4096, 4097])
+@pytest.mark.parametrize("order", ["sorted", "one row"])
+def test_weighted_f32_sums_carry_f64(oracle, E, order):
+    """The precision of the weighted operation does not depend on the number of entries: f64 products and
+    sums on both sides of the one-launch kernels' limits, so what is left is the rounding of the
+    results, half of 2^-23 each (1.2e-7 of a norm at most; one f32 chain of 512 terms has 1e-6)."""
+    d = workloads.opsaw(E=E, K=13, L=32, n=70)
+    if order == "one row":
+        d["indices_output"][:] = 33
+    d["B"][1::2] = -d["B"][::2][: d["B"][1::2].shape[0]] * (1 + 1e-3)  # sums that nearly cancel
+    d["A"][1::2] = d["A"][::2][: d["A"][1::2].shape[0]]
+    got, want = run_library("opsaw", to_dev(d, np.float32)), _in_f64(oracle, "opsaw", d)
+    for k in ("output", "grad_A", "grad_B"):  # (grad_W is added up over entries in f32)
+        error = np.linalg.norm(got[k].astype(np.float64) - want[k]) / np.linalg.norm(want[k])
+        assert error < 6e-8, f"{E} {order} {k}: {error:.1e}"
+
+
 @pytest.mark.parametrize("K,L", [(7, 25), (10, 3), (15, 17), (13, 31)])
 def test_f32_gradients_of_odd_rows_keep_their_precision(oracle, K, L):
     """grad_output rows that are no multiple of 16 bytes: no less than f32 products (7e-8 of the norm)."""
