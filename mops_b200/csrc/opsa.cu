@@ -706,7 +706,7 @@ void forward(const Call& call, T* O, const T* A, const T* B, const T* W, const i
     }
     if (small_forward(J, nO, WEIGHTED)) {
         const int64_t units = nO * ceil_div(K, 8) * ceil_div(L, 32);
-        const int64_t blocks = std::min<int64_t>(ceil_div(units, kSmallWarps), sm_count(call.device) * 8);
+        const int64_t blocks = std::min<int64_t>(units, sm_count(call.device) * 8);
         note_kernel_f("opsa_fwd_small<%s,W=%d>", scalar_name<T>(), WEIGHTED ? 1 : 0);
         opsa_fwd_small<T, WEIGHTED><<<static_cast<unsigned>(blocks), kSmallWarps * 32, 0, call.stream>>>(
             O, A, B, W, PW, P, static_cast<int>(J), K, L, static_cast<int>(nO), call.status);

@@ -22,7 +22,10 @@ constexpr int kSmallWarps = 4;
 // kernels (opsa_pipe.cuh): the precision of a model must not depend on the size of its batch.
 template <typename T, bool WEIGHTED> using SmallSum = std::conditional_t<WEIGHTED, double, T>;
 
-// Forward: a warp per output row and 8 by 32 part of it, as for unsorted input (unsorted.cuh).
+// Forward: a block per output row and 8 by 32 part of it. Its warps share the row's entries (or, where the
+// index is not sorted, the search for them), eight or more each, and add their sums up in shared
+// memory: one row with all of 2000 entries of 8 x 20, f64, took one warp 175 us (with three
+// launches 72).
 template <typename T, bool WEIGHTED>
 __global__ void __launch_bounds__(kSmallWarps * 32)
 opsa_fwd_small(T* __restrict__ O, const T* __restrict__ A, const T* __restrict__ B, const T* __restrict__ W,
@@ -33,6 +36,7 @@ opsa_fwd_small(T* __restrict__ O, const T* __restrict__ A, const T* __restrict__
     __shared__ int32_t index[kSmallEntries];
     __shared__ int32_t found[kSmallWarps][64];
     __shared__ __align__(16) T stage[kSmallWarps][U * KC];
+    __shared__ S partial[kSmallWarps - 1][KC][32];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     bool bad = false, descent = false;
     for (int j = tid; j < J; j += kSmallWarps * 32) {
@@ -56,12 +60,13 @@ opsa_fwd_small(T* __restrict__ O, const T* __restrict__ A, const T* __restrict__
     };
     const int k_units = (K + KC - 1) / KC, units = k_units * ((L + 31) / 32);
     const int64_t all = static_cast<int64_t>(n_rows) * units;
-    for (int64_t unit = static_cast<int64_t>(blockIdx.x) * kSmallWarps + warp; unit < all;
-         unit += static_cast<int64_t>(gridDim.x) * kSmallWarps) {
+    for (int64_t unit = blockIdx.x; unit < all; unit += gridDim.x) {
         const int r = static_cast<int>(unit / units), part = static_cast<int>(unit - static_cast<int64_t>(r) * units);
         const int lb = part / k_units * 32, kb = part % k_units * KC;
         const int l = lb + lane, lc = l < L ? l : L - 1, kn = K - kb < KC ? K - kb : KC;
-        const int lo = sorted ? lower_bound(r) : 0, hi = sorted ? lower_bound(r + 1) : J;
+        const int row_lo = sorted ? lower_bound(r) : 0, row_hi = sorted ? lower_bound(r + 1) : J;
+        const int share = ((row_hi - row_lo + kSmallWarps - 1) / kSmallWarps + 7) / 8 * 8;
+        const int lo = row_lo + warp * share, hi = lo + share < row_hi ? lo + share : row_hi;
         S acc[KC];
 #pragma unroll
         for (int k = 0; k < KC; k++) acc[k] = S(0);
@@ -99,7 +104,21 @@ opsa_fwd_small(T* __restrict__ O, const T* __restrict__ A, const T* __restrict__
         }
         if (held > 0) add(held);
         __syncwarp();
-        if (l < L) {
+        if (row_hi - row_lo > share) { // (the same for the whole block)
+            if (warp > 0) {
+#pragma unroll
+                for (int k = 0; k < KC; k++) partial[warp - 1][k][lane] = acc[k];
+            }
+            __syncthreads();
+            if (warp == 0) {
+#pragma unroll
+                for (int w = 0; w < kSmallWarps - 1; w++)
+#pragma unroll
+                    for (int k = 0; k < KC; k++) acc[k] += partial[w][k][lane];
+            }
+            __syncthreads(); // (the next unit writes there again)
+        }
+        if (warp == 0 && l < L) {
 #pragma unroll
             for (int k = 0; k < KC; k++)
                 if (k < kn) O[(static_cast<int64_t>(r) * K + kb + k) * L + l] = static_cast<T>(acc[k]);
@@ -168,9 +187,8 @@ opsa_vjp_small(T* __restrict__ gA, T* __restrict__ gB, T* __restrict__ gW, const
     if ((lane & 1) == 0 && which < K) gA[e * K + which] = static_cast<T>(sum);
 }
 
-// Few enough entries that three launches cost more than one slower kernel (one warp per row, one round
-// trip to memory per 16 entries), rows not long; with a plan there is one launch anyway.
-// (2000 entries in 35 rows, f64: 16 us, with weights 31.)
+// Few enough entries that three launches cost more than one slower kernel (one block per row, one round
+// trip to memory per 16 entries and warp), rows not long; with a plan there is one launch anyway.
 inline bool small_forward(int64_t J, int64_t n_rows, bool weighted) {
     return J <= (weighted ? 512 : 2048) && n_rows <= 4096 && J <= 64 * n_rows && plan_bound() == nullptr;
 }
