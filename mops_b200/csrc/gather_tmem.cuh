@@ -156,6 +156,45 @@ __device__ __forceinline__ void add_terms(const Batch<T, NF, W>& g, const Record
     }
 }
 
+// f32 sums are taken in pieces of 32 records, which are then added up: one chain over a column's records
+// (thousands) lost up to four bits against the kernels that split them among 32 lanes (201 monomials of
+// order 5 in one variable: relative error 3.8e-6 against 2.1e-7). f64 keeps one chain.
+constexpr int kPieceRecords = 32;
+template <typename T, int R> struct PieceSum {
+    static constexpr bool kPieces = sizeof(T) == 4;
+    T total[kPieces ? R : 1];
+    __device__ __forceinline__ void clear() {
+#pragma unroll
+        for (int r = 0; r < (kPieces ? R : 1); r++) total[r] = T(0);
+    }
+    // Behind batch pair i of B records per batch.
+    template <int B> __device__ __forceinline__ void piece(int i, T (&acc)[R]) {
+        if constexpr (kPieces) {
+            constexpr int kBatches = kPieceRecords / B;
+            if ((i & (kBatches - 1)) == kBatches - 2) take(acc);
+        }
+    }
+    __device__ __forceinline__ void take(T (&acc)[R]) {
+        if constexpr (kPieces) {
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                total[r] += acc[r];
+                acc[r] = T(0);
+            }
+        }
+    }
+    // The whole sum, in acc.
+    __device__ __forceinline__ void finish(T (&acc)[R]) {
+        if constexpr (kPieces) {
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                acc[r] += total[r];
+                total[r] = T(0);
+            }
+        }
+    }
+};
+
 // The slabs of the tiles one block works on.
 template <typename T, int W> struct Tiles {
     static constexpr int R = W / words_of(sizeof(T));
@@ -523,6 +562,8 @@ gather_sums(const __grid_constant__ Results<T> results, const __grid_constant__ 
         t.load(tile + step < tiles ? tile + step : -1, base, tid, warp, lane);
         const int64_t row0 = tile * (kSlabRows * R) + (warp & 3) * 32 + lane;
         T acc[R];
+        PieceSum<T, R> sum;
+        sum.clear();
         bool live[R];
 #pragma unroll
         for (int r = 0; r < R; r++) {
@@ -537,6 +578,7 @@ gather_sums(const __grid_constant__ Results<T> results, const __grid_constant__ 
         int cols = results.cols[which_result];
         T* at = results.data[which_result] + row0 * cols + local;
         auto close = [&] { // column n is complete
+            sum.finish(acc);
 #pragma unroll
             for (int r = 0; r < R; r++)
                 if (results.scale && live[r]) acc[r] *= __ldg(results.scale + row0 + r * kSlabRows);
@@ -574,6 +616,7 @@ gather_sums(const __grid_constant__ Results<T> results, const __grid_constant__ 
                 await<T, NF, W>(y);
                 issue<T, NF, W>(x, rx, base);
                 add_terms<T, NF, W>(y, ry, acc);
+                sum.template piece<B>(i, acc);
                 if (__builtin_expect(--left == 0, 0)) {
                     close();
                     left = n < n_hi ? uniform(starts[n + 1] - starts[n]) / (2 * B) : 0;

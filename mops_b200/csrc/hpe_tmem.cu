@@ -115,6 +115,8 @@ hpe_fwd_tmem(T* __restrict__ O, const __grid_constant__ Operands operands, const
     for (int64_t tile = first; tile < tiles; tile += step) {
         t.load(tile + step < tiles ? tile + step : -1, base, tid, warp, lane);
         T acc[R];
+        PieceSum<T, R> sum;
+        sum.clear();
 #pragma unroll
         for (int r = 0; r < R; r++) acc[r] = T(0);
         for (int s = 0; s < stages; s++) {
@@ -143,10 +145,12 @@ hpe_fwd_tmem(T* __restrict__ O, const __grid_constant__ Operands operands, const
                 await<T, K, W>(y);
                 issue<T, K, W>(x, rx, base);
                 add_terms<T, K, W>(y, ry, acc);
+                sum.template piece<B>(i, acc);
                 fetch<T, K, W>(ry, at(i + 3));
             }
             await<T, K, W>(x); // the loads started last are not used
         }
+        sum.finish(acc);
         __syncthreads(); // the stages become the partial sums
         const int own = (warp & 3) * 32 + lane;
 #pragma unroll

@@ -4,6 +4,7 @@ without records, one column, many), against the CPU oracle at the parity toleran
 import numpy as np
 import pytest
 
+from helpers import run_checker, run_library, to_dev
 from mops_b200 import workloads
 from test_parity_gpu import compare
 
@@ -37,3 +38,19 @@ def test_sap(oracle, kw, dtype):
     d["grad_grad_A"] = r.standard_normal(d["A"].shape)
     d["grad_grad_B"] = r.standard_normal(d["B"].shape)
     compare("sap", d, dtype, oracle, second_order=True, what=f"sap {kw}")
+
+
+@pytest.mark.parametrize("op,kw", [("hpe", dict(I=300, N=13, J=6400, K=4)), ("hpe", dict(I=20000, N=8, J=2000, K=3)),
+                                   ("sap", dict(I=100, nA=32, nB=2, nO=3, K=4100)),
+                                   ("sap", dict(I=5000, nA=9, nB=15, nO=2, K=2000))])
+def test_f32_sums_of_thousands_of_records(oracle, op, kw):
+    """Sums in pieces of 32: an error of about eps (sqrt(32) + sqrt(records / 32)) / 2 of the terms' size
+    for records of random sign, 4e-7 of the result's norm at most; one chain had 8e-7."""
+    d = workloads.__dict__[op](**kw)
+    rounded = {k: v.astype(np.float32).astype(np.float64) if isinstance(v, np.ndarray) and v.dtype == np.float64
+               else v for k, v in d.items()}
+    got = run_library(op, to_dev(d, np.float32))
+    want = run_checker(oracle, op, rounded, np.float64)
+    for k in want:
+        error = np.linalg.norm(got[k].astype(np.float64) - want[k]) / np.linalg.norm(want[k])
+        assert error < 4e-7, f"{op} {kw} {k}: {error:.1e}"
