@@ -12,6 +12,7 @@
 
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/torch.h>
 
@@ -236,12 +237,9 @@ PyObject* call(PyObject*, PyObject* const* args, Py_ssize_t n) {
         Py_RETURN_NOTIMPLEMENTED;
     }
     Args rest{args + 1, n - 1};
-    try {
-        return kOperations[which](rest);
-    } catch (const std::exception& e) { // (allocation of the results)
-        if (PyErr_Occurred() == nullptr) PyErr_SetString(PyExc_RuntimeError, e.what());
-        return nullptr;
-    }
+    HANDLE_TH_ERRORS // (allocation of the results: torch.OutOfMemoryError, as from Python)
+    return kOperations[which](rest);
+    END_HANDLE_TH_ERRORS
 }
 
 PyObject* setup(PyObject*, PyObject* error) {

@@ -164,6 +164,17 @@ def test_forward_mode_tangents_are_refused_in_the_backward_pass():
 
 
 @pytest.mark.gpu
+def test_results_that_do_not_fit_raise_torchs_own_error():
+    """A result of 9 TB, through the functions of mops_b200: the error that programs catch to free memory."""
+    import mops_b200
+    A = torch.rand(20, 16, dtype=torch.float64, device="cuda")
+    B = torch.rand(20, 32, dtype=torch.float64, device="cuda")
+    idx = torch.zeros(20, dtype=torch.int32, device="cuda")
+    with pytest.raises(torch.OutOfMemoryError):
+        mops_b200.outer_product_scatter_add(A, B, idx, 2**31 - 1)
+
+
+@pytest.mark.gpu
 def test_torchscript_round_trip():
     class M(torch.nn.Module):
         def forward(self, A: torch.Tensor, B: torch.Tensor, idx: torch.Tensor) -> torch.Tensor:
