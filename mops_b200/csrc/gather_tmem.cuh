@@ -672,7 +672,9 @@ bool choose_gather_shape(const Call& call, int64_t I, const Operands& op, double
             const double waves = static_cast<double>(ceil_div(tiles * parts, sms));
             double share = records / parts;
             if (column > 0) share = std::max(share, std::ceil(records / column / (4 * parts)) * 4 * column);
-            const double cost = waves * (share * record + 1500 + 4.0 * op.total * r);
+            // (blocks of a cluster wait for one another at both ends of every tile)
+            const double together = power_of_two_parts && parts > 1 && waves > 1 ? 2500 : 0;
+            const double cost = waves * (share * record + 1500 + together + 4.0 * op.total * r);
             if (best_cost < 0 || cost < best_cost) {
                 best_cost = cost;
                 best = {w, parts, tiles, fixed_smem + r * slab};

@@ -211,6 +211,16 @@ bool few_terms(const Call& call, int64_t I, int N, int64_t gathers) {
     return fills_gpu(call, I) && gathers < 5 * static_cast<int64_t>(N);
 }
 
+// Very few result columns: one warp group walks all records of a column, where the kernels in hpe.cu
+// split them among the lanes of a warp (batches of up to 8192 rows) or the warps of a block. In products
+// per column: 4800 monomials of order 4 in one variable, 27 rows, take 170 us there and 359 here. The
+// lines cross at about 1200 (25 000 for one column and a batch that fills the GPU); from eight columns
+// on, and for batches between, they do not.
+bool few_columns(const Call& call, int64_t I, int N, int64_t products) {
+    if (fills_gpu(call, I)) return N == 1 && products > 25000;
+    return I <= 8192 && N < 8 && products > 1200 * static_cast<int64_t>(N);
+}
+
 template <typename T, int K>
 bool forward_order(const Call& call, T* O, const T* A, const T* C, const int32_t* P, int64_t I, int N,
                    int64_t J) {
@@ -238,7 +248,7 @@ bool forward_order(const Call& call, T* O, const T* A, const T* C, const int32_t
 template <typename T, int K>
 bool backward_order(const Call& call, T* gA, const T* gO, const T* A, const T* C, const int32_t* P,
                     int64_t I, int N, int64_t J) {
-    if (few_terms(call, I, N, J * K)) return false;
+    if (few_terms(call, I, N, J * K) || few_columns(call, I, N, J * K * (K - 1))) return false;
     Operands op{};
     op.add(A, N);
     Results<T> results{};
