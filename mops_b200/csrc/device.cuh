@@ -296,8 +296,10 @@ segment_offsets(const int32_t* __restrict__ P, int64_t J, int64_t n_rows, int64_
         const int32_t prev = v[q], cur = v[1 + q];
         // rows prev + 1 .. cur start at entry j0 + q
         // (64 bits: with 2^31 - 1 rows the sums leave 32)
+        if (cur > prev) offsets[int64_t(prev) + 1] = j0 + q;
+        if (!__any_sync(kFullMask, cur > int64_t(prev) + 1)) continue; // (no empty rows)
         const int64_t own = min(int64_t(prev) + kOwnRows, int64_t(cur));
-        for (int64_t r = int64_t(prev) + 1; r <= own; r++) offsets[r] = j0 + q;
+        for (int64_t r = int64_t(prev) + 2; r <= own; r++) offsets[r] = j0 + q;
         unsigned wide = __ballot_sync(kFullMask, cur > own);
         while (wide) {
             const int src = __ffs(wide) - 1;

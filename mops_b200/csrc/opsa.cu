@@ -1336,7 +1336,8 @@ void backward(const Call& call, T* gA, T* gB, T* gW, const T* gO, const T* A, co
         const int blocks = sort_blocks(call, J, nO);
         scratch = scratch_alloc(call, entry_sort_bytes(J, nO, blocks));
         const EntrySort sort = entry_sort_at(scratch, nO, blocks);
-        launch_sorting(call, blocks, sort_if_unsorted_grid, sort_if_unsorted_block, sort, P, J, nO, call.status);
+        launch_sorting(call, blocks, sort_if_unsorted_grid, sort_if_unsorted_block, sort, P, J, nO,
+                       static_cast<uint32_t*>(nullptr), static_cast<int64_t>(0), 0, call.status);
         plan.perm = sort.perm;
     }
     const int KP = vjp_tile_k(K);

@@ -28,6 +28,7 @@
 // is not sorted. VJP: one warp per edge (lane = b), independent of the index order; gW is
 // accumulated with RED because indices_W_1 is not sorted.
 #include <algorithm>
+#include <cmath>
 #include <cstdlib>
 #include <mutex>
 #include <type_traits>
@@ -2139,33 +2140,39 @@ int pick_warps_fast(const Call& call, int ncc, int ds, size_t per_warp, size_t* 
 inline int fast_width(int n) { return n >= 1 && n <= 16 ? (n + 3) / 4 * 4 : 0; }
 
 template <typename T, int TP, int NAP>
-bool forward_fast(const Call& call, T* O, const Problem<T>& p) {
+int forward_fast(const Call& call, T* O, const Problem<T>& p, ScatterPart part) {
     const int64_t rowsize = static_cast<int64_t>(p.nO1) * p.L;
     const int ncc = p.nO1 * p.nW1, ds = NAP + 1; // odd row stride: conflict-free row-per-lane reads
-    if (static_cast<int64_t>(p.nO1) * p.nW1 > 1024) return false;
+    if (static_cast<int64_t>(p.nO1) * p.nW1 > 1024) return kNotApplicable;
     const int grid_generic = sm_count(call.device) * 8;
     size_t smem_seg = 0, smem_edge = 0;
     const size_t tsize = round4(static_cast<size_t>(p.nO1) * TP);
     const int warps_seg = pick_warps_fast<T>(call, ncc, ds, tsize + round4(rowsize), &smem_seg);
     const int warps_edge = pick_warps_fast<T>(call, ncc, ds, tsize, &smem_edge);
-    if (warps_seg == 0 || warps_edge == 0) return false;
+    if (warps_seg == 0 || warps_edge == 0) return kNotApplicable;
     Coupling<T> cp{};
     TableRef scratch{};
-    if (!build_coupling(call, p, cp, &scratch, TP, ds)) return false;
-    SegmentTable seg = segment_table(call, p.Io, p.E, p.nW0);
-    const int64_t* offsets = seg.offsets;
-    allow_dynamic_smem(sasaw_fwd_fast<T, TP, NAP, true>, call.device, smem_seg);
-    note_kernel_f("sasaw_fwd_fast<%s,TP=%d,NAP=%d>", scalar_name<T>(), TP, NAP);
-    sasaw_fwd_fast<T, TP, NAP, true><<<static_cast<unsigned>(ceil_div(p.nW0, warps_seg)),
-                                       warps_seg * 32, smem_seg, call.stream>>>(
-        O, p.A, p.B, p.W, p.Jw, p.Io, offsets, cp, p.E, p.nA, p.L, p.nW0, p.nW1, p.nO1, false,
-        call.status);
-    MOPS_CUDA_OK(cudaGetLastError());
-    release_table(call, seg.ref);
-    bool need_fallback = !seg.known_sorted; // asynchronous calls cannot look: always enqueue
-    if (need_fallback && call.wait) {
-        wait_stream(call);
-        need_fallback = host_saw_unsorted(call);
+    if (!build_coupling(call, p, cp, &scratch, TP, ds)) return kNotApplicable;
+    bool need_fallback = true;
+    if (part != ScatterPart::kUnsorted) {
+        SegmentTable seg = segment_table(call, p.Io, p.E, p.nW0);
+        allow_dynamic_smem(sasaw_fwd_fast<T, TP, NAP, true>, call.device, smem_seg);
+        note_kernel_f("sasaw_fwd_fast<%s,TP=%d,NAP=%d>", scalar_name<T>(), TP, NAP);
+        sasaw_fwd_fast<T, TP, NAP, true><<<static_cast<unsigned>(ceil_div(p.nW0, warps_seg)),
+                                           warps_seg * 32, smem_seg, call.stream>>>(
+            O, p.A, p.B, p.W, p.Jw, p.Io, seg.offsets, cp, p.E, p.nA, p.L, p.nW0, p.nW1, p.nO1, false,
+            call.status);
+        MOPS_CUDA_OK(cudaGetLastError());
+        release_table(call, seg.ref);
+        need_fallback = !seg.known_sorted; // asynchronous calls cannot look: always enqueue
+        if (need_fallback && call.wait) {
+            wait_stream(call);
+            need_fallback = host_saw_unsorted(call);
+        }
+    }
+    if (need_fallback && part == ScatterPart::kSorted) {
+        release_table(call, scratch);
+        return kUnsortedLeft;
     }
     if (need_fallback) {
         zero_if_unsorted<T><<<grid_generic, 256, 0, call.stream>>>(O, p.nW0 * rowsize, call.status);
@@ -2178,7 +2185,7 @@ bool forward_fast(const Call& call, T* O, const Problem<T>& p) {
     }
     MOPS_CUDA_OK(cudaGetLastError());
     release_table(call, scratch);
-    return true;
+    return kComplete;
 }
 
 template <typename T, int TP, int NAP>
@@ -2205,25 +2212,23 @@ bool backward_fast(const Call& call, T* gA, T* gB, T* gW, const T* gO, const Pro
 }
 
 // Tensor-core variants (f64, output_size <= 16 as well).
-// `segmented_done`: another kernel has already handled sorted input; only the kernels for an
-// unsorted scatter index are enqueued (they stand down by themselves when it was sorted).
 template <typename T, int TP>
-bool forward_mma_launch(const Call& call, T* O, const Problem<T>& p, bool segmented_done = false) {
+int forward_mma_launch(const Call& call, T* O, const Problem<T>& p, ScatterPart part) {
     using Lay = VjpMma<TP>;
     const int warps = 4;
     const size_t smem =
         (Lay::d_scalars(p.nO1, p.nA) + Lay::per_warp(p.nO1, p.nW1) * warps) * sizeof(T);
-    if (smem > 74 * 1024) return false; // three blocks per SM
+    if (smem > 74 * 1024) return kNotApplicable; // three blocks per SM
     const int64_t rowsize = static_cast<int64_t>(p.nO1) * p.L;
     const int sms = sm_count(call.device);
     Coupling<T> cp{};
     TableRef scratch{};
-    if (!build_coupling(call, p, cp, &scratch, Lay::TS, Lay::d_stride(p.nA), true)) return false;
+    if (!build_coupling(call, p, cp, &scratch, Lay::TS, Lay::d_stride(p.nA), true)) return kNotApplicable;
     const bool wide_copies = p.L % 2 == 0 && reinterpret_cast<uintptr_t>(p.W) % 16 == 0 &&
                              reinterpret_cast<uintptr_t>(p.B) % 16 == 0 &&
                              reinterpret_cast<uintptr_t>(O) % 16 == 0;
     bool known_sorted = false;
-    if (!segmented_done) {
+    if (part != ScatterPart::kUnsorted) {
         SegmentTable seg = segment_table(call, p.Io, p.E, p.nW0);
         const int64_t* offsets = seg.offsets;
         known_sorted = seg.known_sorted;
@@ -2238,9 +2243,13 @@ bool forward_mma_launch(const Call& call, T* O, const Problem<T>& p, bool segmen
         release_table(call, seg.ref);
     }
     bool need_fallback = !known_sorted; // asynchronous calls cannot look: always enqueue
-    if (need_fallback && call.wait && !segmented_done) {
+    if (need_fallback && call.wait && part != ScatterPart::kUnsorted) {
         wait_stream(call);
         need_fallback = host_saw_unsorted(call);
+    }
+    if (need_fallback && part == ScatterPart::kSorted) {
+        release_table(call, scratch);
+        return kUnsortedLeft;
     }
     if (need_fallback) {
         zero_if_unsorted<T><<<sms * 8, 256, 0, call.stream>>>(O, p.nW0 * rowsize, call.status);
@@ -2252,7 +2261,7 @@ bool forward_mma_launch(const Call& call, T* O, const Problem<T>& p, bool segmen
     }
     MOPS_CUDA_OK(cudaGetLastError());
     release_table(call, scratch);
-    return true;
+    return kComplete;
 }
 
 // Sorted scatter index through the quad kernel. Returns 0 when it does not apply, 1 when it
@@ -2308,32 +2317,44 @@ template <typename T> int forward_quad(const Call& call, T* O, const Problem<T>&
     }
 }
 
-template <typename T> bool forward_mma(const Call& call, T* O, const Problem<T>& p) {
+template <typename T> int forward_mma(const Call& call, T* O, const Problem<T>& p, ScatterPart part) {
     if constexpr (!std::is_same<T, double>::value) {
-        return false;
+        return kNotApplicable;
     } else {
         if (fast_width(p.nO1) == 0 || fast_width(p.nA) == 0 || fast_width(p.nW1) == 0)
-            return false;
-        const int quad = forward_quad(call, O, p);
-        if (quad == 1) return true;
-        switch (fast_width(p.nW1)) {
-        case 4: return forward_mma_launch<T, 4>(call, O, p, quad == 2);
-        case 8: return forward_mma_launch<T, 8>(call, O, p, quad == 2);
-        case 12: return forward_mma_launch<T, 12>(call, O, p, quad == 2);
-        case 16: return forward_mma_launch<T, 16>(call, O, p, quad == 2);
-        default: return false;
+            return kNotApplicable;
+        bool sorted_done = false;
+        if (part != ScatterPart::kUnsorted) {
+            const int quad = forward_quad(call, O, p);
+            if (quad == 1) return kComplete;
+            sorted_done = quad == 2;
+            if (sorted_done && part == ScatterPart::kSorted) return kUnsortedLeft;
+            if (sorted_done) part = ScatterPart::kUnsorted;
         }
+        int done = kNotApplicable;
+        switch (fast_width(p.nW1)) {
+        case 4: done = forward_mma_launch<T, 4>(call, O, p, part); break;
+        case 8: done = forward_mma_launch<T, 8>(call, O, p, part); break;
+        case 12: done = forward_mma_launch<T, 12>(call, O, p, part); break;
+        case 16: done = forward_mma_launch<T, 16>(call, O, p, part); break;
+        }
+        return done == kNotApplicable && sorted_done ? kUnsortedLeft : done;
     }
 }
+
+template <int TP> size_t vjp_mma_smem(int nA, int nW1, int nO1) {
+    using Lay = VjpMma<TP>;
+    return (Lay::d_scalars(nO1, nA) + Lay::per_warp(nO1, nW1) * 4) * sizeof(double);
+}
+constexpr size_t kVjpMmaSmem = 74 * 1024; // three blocks per SM
 
 template <typename T, int TP, int KS3>
 bool backward_mma_launch(const Call& call, T* gA, T* gB, T* gW, const T* gO, const Problem<T>& p,
                          bool only_if_unsorted) {
     using Lay = VjpMma<TP>;
     const int warps = 4;
-    const size_t smem =
-        (Lay::d_scalars(p.nO1, p.nA) + Lay::per_warp(p.nO1, p.nW1) * warps) * sizeof(T);
-    if (smem > 74 * 1024) return false; // three blocks per SM
+    const size_t smem = vjp_mma_smem<TP>(p.nA, p.nW1, p.nO1);
+    if (smem > kVjpMmaSmem) return false;
     Coupling<T> cp{};
     TableRef scratch{};
     if (!build_coupling(call, p, cp, &scratch, Lay::TS, Lay::d_stride(p.nA), true)) return false;
@@ -2351,6 +2372,12 @@ bool backward_mma_launch(const Call& call, T* gA, T* gB, T* gW, const T* gO, con
     return true;
 }
 
+// Whether sasaw_vjp_quad has these widths compiled in and takes these operands.
+template <typename T> bool quad_gradients(const Problem<T>& p) {
+    const uintptr_t both = reinterpret_cast<uintptr_t>(p.W) | reinterpret_cast<uintptr_t>(p.B);
+    return sizeof(T) == 8 && p.nA == 9 && p.nW1 == 9 && p.nO1 == 9 && p.L % 2 == 0 && both % 16 == 0;
+}
+
 // VJP through the quad kernel (sorted scatter index, compiled-in widths). Returns 0 when it
 // does not apply, 1 when it ran and the index was seen to be sorted, 2 when it was launched
 // but the edge-by-edge kernel must still be enqueued for the unsorted case.
@@ -2359,9 +2386,8 @@ int backward_quad(const Call& call, T* gA, T* gB, T* gW, const T* gO, const Prob
     if constexpr (!std::is_same<T, double>::value) {
         return 0;
     } else {
-        if (!(p.nA == 9 && p.nW1 == 9 && p.nO1 == 9)) return 0;
         auto aligned = [](const void* ptr) { return reinterpret_cast<uintptr_t>(ptr) % 16 == 0; };
-        if (p.L % 2 != 0 || !aligned(p.W) || !aligned(p.B) || !aligned(gB)) return 0;
+        if (!quad_gradients(p) || !aligned(gB)) return 0;
         constexpr QuadLayout q = quad_layout(9, 9, 9);
         const size_t d_bytes = static_cast<size_t>(q.d_scalars) * sizeof(T);
         const size_t warp_bytes = static_cast<size_t>(q.warp_scalars) * sizeof(T);
@@ -2425,7 +2451,7 @@ bool backward_mma(const Call& call, T* gA, T* gB, T* gW, const T* gO, const Prob
 
 // Dispatch on the two padded widths; returns false when the fast kernels do not apply.
 #define MOPS_B200_SASAW_FAST(FN, ...)                                                              \
-    [&]() -> bool {                                                                                \
+    [&]() -> int {                                                                                 \
         const int tp = fast_width(p.nW1), nap = fast_width(p.nA);                                  \
         if (tp == 0 || nap == 0) return false;                                                     \
         switch (tp * 100 + nap) {                                                                  \
@@ -2452,39 +2478,101 @@ template <typename T> SasawProblem<T> rows_problem(const Problem<T>& p) {
     return {p.A, p.B, p.C, p.W, p.M1, p.Jw, p.M2, p.Io, p.M3, p.E, p.N, p.nW0, p.nA, p.nW1, p.nO1, p.L};
 }
 
-// The row kernels (sasaw_rows.cu) or the ones here, from measurements on B200:
-//   forward   f64 with fewer than 24 edges per row: the coupling per row then costs more than the
-//             coupling per edge of the MMA kernels (200 000 edges, 10 per row, 9 x 9 x 9 channels, 32
-//             columns: 190 against 122 us; 61 per row: 110 against 116 us).
-//   gradients f64, where the MMA kernels apply and W and gW stay in L2, these are faster from 100 000
-//             edges on (10^6 edges, 9 x 9 x 9: 1.20 against 1.37 ms; 60 000: 148 against 120 us;
-//             4.2 10^6 with W and gW of 151 MB each: 5.70 against 4.85 ms).
-//             Output channels in several passes (more than 9) and few of W (up to 4): here it pays
-//             to gather W and to add to gW, f32 0.21 against 0.45 ms, f64 0.15 against 0.42 ms.
-constexpr int64_t kShortRows = 24;
-constexpr int64_t kFewEdges = 100000;
-constexpr double kCacheBytes = 100e6; // of the 126 MB of L2
+// The row kernels (sasaw_rows.cu) or the ones here, by estimates of their time, fitted to the same 750 shapes
+// (sasaw_rows_cost) in every direction. The estimates miss by a third in one of ten, so the family that is
+// usually the faster one gives way only where the other is estimated to be so by kMargin. Of 3000 calls (those
+// shapes, forward and gradients, waiting and not) 5 % then take more than 1.07 and 1 % more than 1.25 times what
+// the better family would; one family alone is up to 8 times slower. Microseconds:
+struct EdgeCost {
+    double call, cell, entry, edge, table, row; // cells, entries, edges and rows in 10^-6, the table 10^-3
+    double few_edge, few_cell;                  // a row's edges one after the other: 10^-2, 10^-5
+};
+template <typename T> double edge_cost(const Problem<T>& p, const EdgeCost& c) {
+    const double E = static_cast<double>(p.E), N = static_cast<double>(p.N), rows = static_cast<double>(p.nW0);
+    const double cells = static_cast<double>(p.nO1) * ((p.nW1 + 3) / 4 * 4) * static_cast<double>(ceil_div(p.L, 32));
+    const double few = std::max(0.0, 1 - rows / 2368);
+    return c.call + E * (c.cell * cells + c.entry * N + c.edge) * 1e-6 + N * c.table * 1e-3 +
+           rows * p.nO1 * p.L * c.row * 1e-6 + few * E / rows * (c.few_edge * 1e-2 + c.few_cell * cells * 1e-5);
+}
+constexpr double kMargin = 1.3;
+constexpr int64_t kShortRows = 24; // edges; from here on the forward by rows is usually the faster one
+template <typename T> double rows_margin(const Problem<T>& p) {
+    return p.E >= kShortRows * p.nW0 ? kMargin : 1 / kMargin;
+}
+template <typename T> bool sorted_by_rows(const Problem<T>& p) {
+    const EdgeCost cost = sizeof(T) == 4 ? EdgeCost{33.2, 4.1, 0, 342, 32.1, 2.02, 91.9, 720}
+                          : p.L % 2 == 0 ? EdgeCost{46.2, 4.04, 0.0252, 403, 78.6, 4.15, 28, 568}
+                                         : EdgeCost{37.7, 7.7, 0, 337, 0, 10.8, 45.7, 998};
+    double us = edge_cost(p, cost);
+    if (sizeof(T) == 8 && p.L % 2 == 0) { // wide channels leave the quad kernel fewer than eight warps
+        const QuadLayout q = quad_layout(p.nA, p.nW1, p.nO1);
+        const double room = 227.0 * 1024 / sizeof(T) - q.d_scalars, warps = std::max(1.0, std::floor(room / q.warp_scalars));
+        us *= std::max(1.0, 8 / warps);
+    }
+    return p.E >= p.nW0 && sasaw_rows_cost(rows_problem(p), RowsWork::kSorted) < us * rows_margin(p);
+}
+template <typename T> bool unsorted_by_rows(const Problem<T>& p) {
+    const EdgeCost cost = sizeof(T) == 4 ? EdgeCost{25.4, 3.54, 0.0224, 413, 18.5, 2.09, 0, 0}
+                          : p.L % 2 == 0 ? EdgeCost{39.4, 6.25, 0, 439, 49.2, 2.39, 0, 0}
+                                         : EdgeCost{33.7, 1.73, 0, 1110, 23.6, 106, 0, 0};
+    return sasaw_rows_cost(rows_problem(p), RowsWork::kUnsorted) < edge_cost(p, cost) * rows_margin(p);
+}
+// The f64 gradients have three kernels by edge. The one with compiled-in widths adds to gW from all over it,
+// which costs more where W and gW are larger than L2 (4.2 10^6 edges, 151 MB each: 5.70 against 4.85 ms),
+// and gives a row of the output to one warp, however long (60 000 edges in one: 45 against 0.16 ms).
+template <typename T> bool gradients_by_rows(const Problem<T>& p) {
+    constexpr double kCacheBytes = 100e6; // of the 126 MB of L2
+    double us, margin;
+    if (sizeof(T) == 4) {
+        us = edge_cost(p, EdgeCost{16.7, 16.7, 0, 620, 23.1, 1.18, 0, 0});
+        margin = p.nW0 >= 2000 ? 1 : 1 / kMargin; // (rows enough for the warps)
+    } else if (quad_gradients(p)) {
+        const double tables = 2.0 * p.nW0 * p.nW1 * p.L * sizeof(T);
+        us = std::min(80.0, 50 + p.E * 600e-6) + edge_cost(p, EdgeCost{0, 10, 0.05, 0, 11, 3.77, 0, 0});
+        us *= 1 + 0.8 * std::max(0.0, 1 - kCacheBytes / tables);
+        margin = kMargin;
+    } else {
+        size_t smem = 0;
+        switch (fast_width(p.nW1)) {
+        case 4: smem = vjp_mma_smem<4>(p.nA, p.nW1, p.nO1); break;
+        case 8: smem = vjp_mma_smem<8>(p.nA, p.nW1, p.nO1); break;
+        case 12: smem = vjp_mma_smem<12>(p.nA, p.nW1, p.nO1); break;
+        default: smem = vjp_mma_smem<16>(p.nA, p.nW1, p.nO1);
+        }
+        const bool mma = smem <= kVjpMmaSmem;
+        us = edge_cost(p, mma ? EdgeCost{24.2, 13.6, 0, 541, 45.1, 5.47, 0, 0}
+                              : EdgeCost{21.9, 25.6, 0.034, 2510, 12.2, 1.09, 0, 0});
+        margin = mma ? 1 / 1.5 : 1 / 1.1;
+    }
+    return sasaw_rows_cost(rows_problem(p), RowsWork::kGradients) < us * margin;
+}
 
-template <typename T> bool rows_first_backward(const Problem<T>& p) {
-    const bool long_rows = p.E >= kShortRows * p.nW0;
-    if (p.nW1 <= 4 && p.nO1 > 9) return false;
-    if (sizeof(T) == 4) return true;
-    const double tables = 2.0 * p.nW0 * p.nW1 * p.L * sizeof(T);
-    return long_rows && (tables > kCacheBytes || (p.E < kFewEdges && p.nW1 == 9 && p.nO1 == 9 && p.nA == 9));
+template <typename T> int forward_by_edge(const Call& call, T* O, const Problem<T>& p, ScatterPart part) {
+    const int done = forward_mma(call, O, p, part);
+    return done != kNotApplicable ? done : MOPS_B200_SASAW_FAST(forward_fast, call, O, p, part);
 }
 
 template <typename T> void forward(const Call& call, T* O, const Problem<T>& p) {
-    const bool short_rows = sizeof(T) == 8 && p.E < kShortRows * p.nW0;
     const int64_t rowsize = static_cast<int64_t>(p.nO1) * p.L;
     if (p.nW0 == 0 || rowsize == 0) return;
     if (p.E == 0 || p.N == 0) {
         MOPS_CUDA_OK(cudaMemsetAsync(O, 0, p.nW0 * rowsize * sizeof(T), call.stream));
         return;
     }
-    if (!short_rows && sasaw_forward_rows<T>(call, rows_problem(p), O)) return;
-    if (forward_mma(call, O, p)) return;
-    if (short_rows && sasaw_forward_rows<T>(call, rows_problem(p), O)) return;
-    if (MOPS_B200_SASAW_FAST(forward_fast, call, O, p)) return;
+    const bool sorted_rows = sorted_by_rows(p), unsorted_rows = unsorted_by_rows(p);
+    // (an asynchronous call enqueues both parts, and would build both families' tables for them)
+    const bool mixed = sorted_rows != unsorted_rows && call.wait;
+    const ScatterPart first = mixed ? ScatterPart::kSorted : ScatterPart::kBoth;
+    int done = kNotApplicable;
+    if (sorted_rows) done = sasaw_forward_rows<T>(call, rows_problem(p), O, first);
+    if (done == kNotApplicable) done = forward_by_edge(call, O, p, sorted_rows ? ScatterPart::kBoth : first);
+    if (done == kUnsortedLeft) { // (by edge also where the other family was asked and does not apply)
+        done = kNotApplicable;
+        if (!unsorted_rows) done = forward_by_edge(call, O, p, ScatterPart::kUnsorted);
+        if (done == kNotApplicable) done = sasaw_forward_rows<T>(call, rows_problem(p), O, ScatterPart::kUnsorted);
+        if (done == kNotApplicable) done = forward_by_edge(call, O, p, ScatterPart::kUnsorted);
+    }
+    if (done != kNotApplicable) return;
     const int grid_generic = sm_count(call.device) * 8;
     Coupling<T> cp{};
     TableRef scratch{};
@@ -2531,13 +2619,12 @@ void backward(const Call& call, T* gA, T* gB, T* gW, const T* gO, const Problem<
     if (gA == nullptr && gB == nullptr && gW == nullptr) return;
     const int64_t wsize = p.nW0 * static_cast<int64_t>(p.nW1) * p.L;
     const bool some = p.E > 0 && p.N > 0 && p.L > 0;
-    if (some && rows_first_backward(p) && sasaw_backward_rows<T>(call, rows_problem(p), gA, gB, gW, gO)) return;
+    if (some && gradients_by_rows(p) && sasaw_backward_rows<T>(call, rows_problem(p), gA, gB, gW, gO)) return;
     if (gW != nullptr && wsize > 0)
         MOPS_CUDA_OK(cudaMemsetAsync(gW, 0, wsize * sizeof(T), call.stream));
     if (p.E == 0) return;
     const bool empty = p.N == 0 || p.L == 0 || p.nO1 == 0 || p.nW1 == 0 || p.nA == 0;
     if (!empty && backward_mma(call, gA, gB, gW, gO, p)) return;
-    if (some && !(p.nW1 <= 4 && p.nO1 > 9) && sasaw_backward_rows<T>(call, rows_problem(p), gA, gB, gW, gO)) return;
     if (!empty && MOPS_B200_SASAW_FAST(backward_fast, call, gA, gB, gW, gO, p)) return;
     Coupling<T> cp{};
     TableRef scratch{};

@@ -24,6 +24,7 @@
 // -> 45 + 120 us. Half the products per warp and three warps per scheduler were slower (62 -> 111 us):
 // what an edge costs beside its products then counts twice.
 #include <algorithm>
+#include <cmath>
 #include <initializer_list>
 #include <type_traits>
 
@@ -50,6 +51,7 @@ template <typename T> struct Pack<T, 1> {
     static __device__ __forceinline__ V add(V a, V b) { return a + b; }
     static __device__ __forceinline__ T sum(V a) { return a; }
     static __device__ __forceinline__ V shift(V a, int o) { return __shfl_xor_sync(kFullMask, a, o); }
+    static __device__ __forceinline__ void add_at(T* p, V a) { red_add(p, a); }
 };
 template <> struct Pack<float, 2> { // FFMA2: two multiply-adds per instruction
     using V = unsigned long long;
@@ -79,6 +81,12 @@ template <> struct Pack<float, 2> { // FFMA2: two multiply-adds per instruction
         return x + y;
     }
     static __device__ __forceinline__ V shift(V a, int o) { return __shfl_xor_sync(kFullMask, a, o); }
+    static __device__ __forceinline__ void add_at(float* p, V a) {
+        float x, y;
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a));
+        red_add(p, x);
+        red_add(p + 1, y);
+    }
 };
 
 // ---- the dense coupling table D[out][a][c], padded with zeros: `out` is m3 (forward) or m2
@@ -122,6 +130,21 @@ template <typename T> struct RowsArgs {
     int pad_out, pad_c;
     int lanes;                   // lanes per edge (a power of two); 32 / lanes edges side by side
     int bit;                     // status bit of `gather`
+    const int32_t* longest;      // with a permutation: where its rows are longer than `limit`, they are
+    int limit, chunk;            // taken in chunks of this many edges, whatever rows these belong to
+};
+
+// Some rows. CUT: and of their edges those at positions [p_lo, p_hi); other warps have others, so that sums
+// are added to what is there. (Instantiated for both: with the choice at run time the even case took 3 %
+// longer, f32, 250 000 edges.)
+template <bool CUT> struct Part {
+    static constexpr bool kCut = CUT;
+    int64_t row_lo, row_hi;
+};
+template <> struct Part<true> {
+    static constexpr bool kCut = true;
+    int64_t row_lo, row_hi;
+    int p_lo, p_hi;
 };
 
 // One slot of a warp's ring: NC rows of 32 lanes, B, the A rows of the edges side by side, their numbers.
@@ -156,16 +179,17 @@ __device__ __forceinline__ void cp_async_rows(unsigned dst, const unsigned char*
 // every offset is a constant and the copies are whole 16-byte pieces).
 enum Mode { kSideBySide = 0, kOneEdge = 1, kExact = 2 };
 
-// Walks rows [row_lo, row_hi) for columns [b0, ...) and c in [c0, c0 + nc): begin(row), step(w[NC] and B
+// Walks a part for columns [b0, ...) and c in [c0, c0 + nc): begin(row), step(w[NC] and B
 // of this lane, A row, edge, live), end(row) in order. All lanes together.
 //
 // One edge at a time the copies do not care about rows: they run along the positions, and a step is
 // straight-line code (wait, start the copies of the step seven ahead, read, multiply), which the
 // compiler can interleave: at 9 x 9 channels, f64, 337 -> 210 instructions per edge of the sums,
 // 640 -> 450 us at 10^6 edges.
-template <typename T, int VEC, int NA, int NC, Mode MODE, typename Off, typename Begin, typename Step, typename End>
-__device__ __forceinline__ void walk_rows(const RowsArgs<T>& g, const Off* __restrict__ offsets, int64_t row_lo,
-                                          int64_t row_hi, int b0, int c0, unsigned char* ring, int lane,
+template <typename T, int VEC, int NA, int NC, Mode MODE, typename Off, bool CUT, typename Begin, typename Step,
+          typename End>
+__device__ __forceinline__ void walk_rows(const RowsArgs<T>& g, const Off* __restrict__ offsets,
+                                          const Part<CUT>& part, int b0, int c0, unsigned char* ring, int lane,
                                           const Status& st, Begin&& begin, Step&& step, End&& end) {
     using P = Pack<T, VEC>;
     using V = typename P::V;
@@ -185,7 +209,13 @@ __device__ __forceinline__ void walk_rows(const RowsArgs<T>& g, const Off* __res
     for (int x = lane * 4; x < kDepth * slot_bytes; x += 128) *reinterpret_cast<int*>(ring + x) = 0;
     __syncwarp();
 
-    const int p_lo = static_cast<int>(offsets[row_lo]), p_hi = static_cast<int>(offsets[row_hi]);
+    const int64_t row_lo = part.row_lo, row_hi = part.row_hi;
+    int p_lo = static_cast<int>(offsets[row_lo]), p_hi = static_cast<int>(offsets[row_hi]);
+    if constexpr (CUT) p_lo = max(p_lo, part.p_lo), p_hi = min(p_hi, part.p_hi);
+    auto row_end = [&](int64_t row) {
+        const int end = static_cast<int>(offsets[row + 1]);
+        return CUT ? min(end, p_hi) : end;
+    };
     // Edge numbers and gathered rows, 32 positions per register: the block that the copies have
     // reached (0), the next (1), and of the one after that the edge numbers only (2).
     auto load_edge = [&](int base) {
@@ -252,7 +282,7 @@ __device__ __forceinline__ void walk_rows(const RowsArgs<T>& g, const Off* __res
 
     // the copies: the next step to start
     int64_t f_row = row_lo;
-    int f_p = p_lo, f_end = row_lo < row_hi ? static_cast<int>(offsets[row_lo + 1]) : p_lo;
+    int f_p = p_lo, f_end = row_lo < row_hi ? row_end(row_lo) : p_lo;
     auto start = [&](int slot) { // slot: byte offset in the ring
         if constexpr (!kSide) { // (behind the last edge it is copied again: nobody reads it)
             const int at = f_p - block;
@@ -265,7 +295,7 @@ __device__ __forceinline__ void walk_rows(const RowsArgs<T>& g, const Off* __res
         } else {
             while (f_p >= f_end && f_row + 1 < row_hi) {
                 f_row++;
-                f_end = static_cast<int>(offsets[f_row + 1]);
+                f_end = row_end(f_row);
             }
             if (f_p < f_end) {
                 if (f_p >= block + 32) next_block();
@@ -297,8 +327,9 @@ __device__ __forceinline__ void walk_rows(const RowsArgs<T>& g, const Off* __res
     int slot = 0, before = (kDepth - 1) * slot_bytes; // byte offsets of this step's slot and the last one's
     int lo = p_lo;
     for (int64_t row = row_lo; row < row_hi; row++) {
-        const int hi = static_cast<int>(offsets[row + 1]);
-        begin(row, lo < hi);
+        const int hi = row_end(row);
+        const bool any = lo < hi;
+        begin(row, any);
 #pragma unroll 1
         for (int p = lo; p < hi; p += S) {
             cp_async_wait<kDepth - 2>();
@@ -318,7 +349,7 @@ __device__ __forceinline__ void walk_rows(const RowsArgs<T>& g, const Off* __res
             if (slot == kDepth * slot_bytes) slot = 0;
             if (!kSide && f_p == block + 32) next_block();
         }
-        end(row);
+        end(row, any);
         lo = hi;
     }
     cp_async_wait<0>();
@@ -338,8 +369,8 @@ template <typename T, int NA> __device__ __forceinline__ void load_a(const T* a,
     }
 }
 
-// out[o] (+)= sum_{a,c} D[o][a][c0 + c] acc[a][c] for the lane's column, o = 0 .. nOut - 1.
-template <typename T, int VEC, int NA, int NC>
+// out[o] (+)= sum_{a,c} D[o][a][c0 + c] acc[a][c] for the lane's column, o = 0 .. nOut - 1. CUT: by atomics.
+template <typename T, int VEC, int NA, int NC, bool CUT>
 __device__ __forceinline__ void contract_row(const RowsArgs<T>& g, const T* D, T* out,
                                              typename Pack<T, VEC>::V (&acc)[NA][NC], int c0, bool store,
                                              bool add_to) {
@@ -361,17 +392,21 @@ __device__ __forceinline__ void contract_row(const RowsArgs<T>& g, const T* D, T
         for (int u = 0; u < kTableOut; u++) {
             for (int x = g.lanes; x < 32; x <<= 1) v[u] = P::add(v[u], P::shift(v[u], x));
             if (store && o + u < g.nOut) {
-                V* dst = reinterpret_cast<V*>(out + static_cast<int64_t>(o + u) * g.L);
-                *dst = add_to ? P::add(*dst, v[u]) : v[u];
+                T* at = out + static_cast<int64_t>(o + u) * g.L;
+                V* dst = reinterpret_cast<V*>(at);
+                if constexpr (CUT)
+                    P::add_at(at, v[u]);
+                else
+                    *dst = add_to ? P::add(*dst, v[u]) : v[u];
             }
         }
     }
 }
 
 // Forward, and the gW part of the gradients: `out` is [rows][nOut][L].
-template <typename T, int VEC, int NA, int NC, Mode MODE, typename Off>
+template <typename T, int VEC, int NA, int NC, Mode MODE, typename Off, bool CUT>
 __device__ __forceinline__ void outer_rows(const RowsArgs<T>& g, const Off* __restrict__ offsets,
-                                           T* __restrict__ out, int64_t row_lo, int64_t row_hi, const T* D,
+                                           T* __restrict__ out, const Part<CUT>& part, const T* D,
                                            unsigned char* ring, int lane, const Status& st) {
     using P = Pack<T, VEC>;
     using V = typename P::V;
@@ -381,8 +416,8 @@ __device__ __forceinline__ void outer_rows(const RowsArgs<T>& g, const Off* __re
         const bool store = lane < g.lanes && b < g.L;
         for (int c0 = 0; c0 < g.nC; c0 += NC) {
             V acc[NA][NC];
-            walk_rows<T, VEC, NA, NC, MODE>(
-                g, offsets, row_lo, row_hi, b0, c0, ring, lane, st,
+            walk_rows<T, VEC, NA, NC, MODE, Off, CUT>(
+                g, offsets, part, b0, c0, ring, lane, st,
                 [&](int64_t, bool) {
 #pragma unroll
                     for (int a = 0; a < NA; a++)
@@ -401,8 +436,9 @@ __device__ __forceinline__ void outer_rows(const RowsArgs<T>& g, const Off* __re
                         for (int c = 0; c < NC; c++) acc[a][c] = P::fma(av, w[c], acc[a][c]);
                     }
                 },
-                [&](int64_t row) {
-                    contract_row<T, VEC, NA, NC>(g, D, out + row * g.nOut * g.L + b, acc, c0, store, c0 > 0);
+                [&](int64_t row, bool any) {
+                    T* at = out + row * g.nOut * g.L + b;
+                    if (!CUT || any) contract_row<T, VEC, NA, NC, CUT>(g, D, at, acc, c0, store, c0 > 0);
                 });
         }
     }
@@ -461,11 +497,11 @@ template <int O, int HELD, typename T, int NA> __device__ __forceinline__ void s
 
 // gA and gB. `own` is the matrix of the rows themselves, [rows][nOut][L] (W, where the rows are
 // those of W and g.G is gO).
-template <typename T, int VEC, int NA, int NC, Mode MODE, typename Off>
+template <typename T, int VEC, int NA, int NC, Mode MODE, typename Off, bool CUT>
 __device__ __forceinline__ void edge_gradients(const RowsArgs<T>& g, const Off* __restrict__ offsets,
                                                T* __restrict__ gA, T* __restrict__ gB,
-                                               const T* __restrict__ own, int64_t row_lo, int64_t row_hi,
-                                               const T* D, unsigned char* ring, int lane, const Status& st) {
+                                               const T* __restrict__ own, const Part<CUT>& part, const T* D,
+                                               unsigned char* ring, int lane, const Status& st) {
     using P = Pack<T, VEC>;
     using V = typename P::V;
     constexpr int NP = NA <= 4 ? 4 : 16;              // values in the sums over lanes, padded
@@ -478,8 +514,8 @@ __device__ __forceinline__ void edge_gradients(const RowsArgs<T>& g, const Off* 
         for (int c0 = 0; c0 < g.nC; c0 += NC) {
             const bool first = b0 == 0 && c0 == 0;
             V E[NA][NC];
-            walk_rows<T, VEC, NA, NC, MODE>(
-                g, offsets, row_lo, row_hi, b0, c0, ring, lane, st,
+            walk_rows<T, VEC, NA, NC, MODE, Off, CUT>(
+                g, offsets, part, b0, c0, ring, lane, st,
                 [&](int64_t row, bool any) {
                     if (!any) return;
 #pragma unroll
@@ -551,7 +587,7 @@ __device__ __forceinline__ void edge_gradients(const RowsArgs<T>& g, const Off* 
                         }
                     }
                 },
-                [&](int64_t) {});
+                [&](int64_t, bool) {});
         }
     }
 }
@@ -568,23 +604,43 @@ template <typename T, int VEC, int NA> constexpr int kSumBlocks = NA <= 9 ? kEdg
 // time, about kChunkEdges edges, so that none waits for another's long rows
 // (60 000 edges, 1000 rows: 63 -> 45 us against rows dealt out beforehand).
 constexpr int kChunkEdges = 256;
+constexpr int kLeastChunk = 32;
 template <typename Off> __device__ __forceinline__ int chunk_rows(const Off* offsets, int64_t lo, int64_t hi) {
     const int64_t edges = offsets[hi] - offsets[lo], rows = hi - lo;
     if (edges <= 0) return 256;
     const int64_t n = kChunkEdges * rows / edges, fair = rows / (2 * kRowWarps);
     return static_cast<int>(n < 1 || fair < 1 ? 1 : n < fair ? n : fair);
 }
-template <typename Off, typename F>
-__device__ __forceinline__ void for_block_rows(const Off* offsets, int64_t rows, int* counter, int lane, F&& f) {
-    const int64_t lo = balanced_row_split(offsets, rows, blockIdx.x, gridDim.x, lane);
-    const int64_t hi = balanced_row_split(offsets, rows, blockIdx.x + 1, gridDim.x, lane);
-    const int n = chunk_rows(offsets, lo, hi);
-    while (true) {
+//
+// Rows longer than the limit (or few of them) would leave warps waiting for one another: then the blocks
+// share out chunks of edges instead, and rows are cut where a chunk ends (sums of 60 000 edges, half of
+// them in one of 1000 rows, f32, 9 x 9 x 9 channels: 9.3 ms without).
+template <bool CUT, typename Off, typename F>
+__device__ __forceinline__ void for_parts(const Off* offsets, int64_t rows, int chunk, int* counter, int lane, F&& f) {
+    auto take = [&](int n) {
         int at = 0;
         if (lane == 0) at = atomicAdd(counter, n);
-        const int64_t r = lo + __shfl_sync(kFullMask, at, 0);
-        if (r >= hi) break;
-        f(r, r + n < hi ? r + n : hi);
+        return __shfl_sync(kFullMask, at, 0);
+    };
+    if constexpr (!CUT) {
+        const int64_t lo = balanced_row_split(offsets, rows, blockIdx.x, gridDim.x, lane);
+        const int64_t hi = balanced_row_split(offsets, rows, blockIdx.x + 1, gridDim.x, lane);
+        const int n = chunk_rows(offsets, lo, hi);
+        while (true) {
+            const int64_t r = lo + take(n);
+            if (r >= hi) break;
+            f(Part<false>{r, r + n < hi ? r + n : hi});
+        }
+    } else {
+        const int edges = static_cast<int>(offsets[rows]);
+        while (true) {
+            const int64_t p = (blockIdx.x + static_cast<int64_t>(take(1)) * gridDim.x) * chunk;
+            if (p >= edges) break;
+            const int end = p + chunk < edges ? static_cast<int>(p) + chunk : edges;
+            // the rows of the first and of the last edge
+            f(Part<true>{warp_count_weighted_le(offsets, rows + 1, 0, p, lane) - 1,
+                         warp_count_weighted_le(offsets, rows + 1, 0, end - 1, lane), static_cast<int>(p), end});
+        }
     }
 }
 
@@ -617,14 +673,15 @@ sasaw_sum_rows(const __grid_constant__ RowsArgs<T> g, const int64_t* __restrict_
     extern __shared__ __align__(128) unsigned char smem[];
     const int warp = __shfl_sync(kFullMask, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const RowsShared<T, VEC, NA, NC> sh(g, smem, &counter, warp);
+    auto sum = [&](const auto* at, const auto& part) {
+        outer_rows<T, VEC, NA, NC, MODE>(g, at, out, part, sh.D, sh.ring, lane, st);
+    };
     if (run == kSorted)
-        for_block_rows(offsets, g.rows, sh.counter, lane, [&](int64_t lo, int64_t hi) {
-            outer_rows<T, VEC, NA, NC, MODE>(g, offsets, out, lo, hi, sh.D, sh.ring, lane, st);
-        });
-    else
-        for_block_rows(starts, g.rows, sh.counter, lane, [&](int64_t lo, int64_t hi) {
-            outer_rows<T, VEC, NA, NC, MODE>(g, starts, out, lo, hi, sh.D, sh.ring, lane, st);
-        });
+        for_parts<false>(offsets, g.rows, 0, sh.counter, lane, [&](const auto& part) { sum(offsets, part); });
+    else if (*g.longest <= g.limit)
+        for_parts<false>(starts, g.rows, 0, sh.counter, lane, [&](const auto& part) { sum(starts, part); });
+    else // (`out` has been cleared by a kernel before)
+        for_parts<true>(starts, g.rows, g.chunk, sh.counter, lane, [&](const auto& part) { sum(starts, part); });
 }
 
 // gA and gB. (A kernel of its own: gathering for gW at the same time in half of the warps saves DRAM
@@ -632,14 +689,25 @@ sasaw_sum_rows(const __grid_constant__ RowsArgs<T> g, const int64_t* __restrict_
 template <typename T, int VEC, int NA, int NC, Mode MODE>
 __global__ void __launch_bounds__(kRowWarps * 32, (kEdgeBlocks<T, VEC>))
 sasaw_edge_gradients(const __grid_constant__ RowsArgs<T> g, const int32_t* __restrict__ starts, T* __restrict__ gA,
-                     T* __restrict__ gB, const T* __restrict__ W, Status st) {
+                     T* __restrict__ gB, T* __restrict__ gW, const T* __restrict__ W, Status st) {
     __shared__ int counter;
     extern __shared__ __align__(128) unsigned char smem[];
     const int warp = __shfl_sync(kFullMask, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const RowsShared<T, VEC, NA, NC> sh(g, smem, &counter, warp);
-    for_block_rows(starts, g.rows, sh.counter, lane, [&](int64_t lo, int64_t hi) {
-        edge_gradients<T, VEC, NA, NC, MODE>(g, starts, gA, gB, W, lo, hi, sh.D, sh.ring, lane, st);
-    });
+    auto gradients = [&](const auto& part) {
+        edge_gradients<T, VEC, NA, NC, MODE>(g, starts, gA, gB, W, part, sh.D, sh.ring, lane, st);
+    };
+    if (*g.longest <= g.limit) {
+        for_parts<false>(starts, g.rows, 0, sh.counter, lane, gradients);
+        return;
+    }
+    if (gW != nullptr) { // for the sums, which come next and will add to it
+        const int64_t n = g.rows * g.nOut * g.L;
+        for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
+             i += static_cast<int64_t>(gridDim.x) * blockDim.x)
+            gW[i] = T(0);
+    }
+    for_parts<true>(starts, g.rows, g.chunk, sh.counter, lane, gradients);
 }
 
 // ---- the order of the edges by a row index: row starts and permutation (a counting sort)
@@ -757,21 +825,36 @@ TableRef dense_table(const Call& call, const SasawProblem<T>& p, const RowsShape
     return ref;
 }
 
-// As many blocks as the SMs hold, fewer for few rows.
-template <typename Kernel> unsigned rows_blocks(const Call& call, Kernel kernel, size_t smem, int64_t rows) {
+// As many blocks as the SMs hold, fewer for few rows (more blocks than rows for their warps: 23 -> 29 us).
+// With a permutation rows may be cut, so that it is the edges that count.
+template <typename Kernel, typename T>
+unsigned rows_blocks(const Call& call, Kernel kernel, const RowsShape<T>& s, int64_t edges) {
     const int64_t sms = sm_count(call.device);
-    int64_t blocks = sms * resident_blocks(kernel, call.device, kRowWarps * 32, smem);
-    if (rows < blocks * kRowWarps) blocks = sms; // (more blocks than rows for their warps: 23 -> 29 us)
-    return static_cast<unsigned>(std::min<int64_t>(rows, blocks));
+    int64_t blocks = sms * resident_blocks(kernel, call.device, kRowWarps * 32, s.smem);
+    if (s.g.rows < blocks * kRowWarps) blocks = sms;
+    const int64_t most = s.g.perm == nullptr ? s.g.rows : std::max(s.g.rows, ceil_div(edges, kLeastChunk));
+    return static_cast<unsigned>(std::min(most, blocks));
+}
+
+// Rows longer than twice the average are cut in chunks, two or more for every warp; where there are few
+// rows for the warps, those longer than kFewRowsLimit.
+constexpr int kFewRowsLimit = 96;
+template <typename T> void set_chunks(const Call& call, RowsShape<T>& s, const EntrySort& sort, int64_t edges) {
+    const int64_t warps = static_cast<int64_t>(sm_count(call.device)) * kRowWarps;
+    const int64_t average = edges / s.g.rows;
+    s.g.longest = sort.longest;
+    s.g.limit = s.g.rows < 2 * warps ? kFewRowsLimit : static_cast<int>(std::max<int64_t>(128, 2 * average));
+    s.g.chunk = static_cast<int>(std::min<int64_t>(
+        std::max<int64_t>(ceil_div(edges, 2 * warps * kLeastChunk) * kLeastChunk, kLeastChunk), kChunkEdges));
 }
 
 template <typename T>
 void launch_sums(const Call& call, const RowsShape<T>& s, const int64_t* offsets, const int32_t* starts,
-                 T* out, RowsRun when) {
+                 T* out, RowsRun when, int64_t edges) {
     for_shape(s, [&](auto vec, auto na, auto nc, auto mode) {
         auto kernel = sasaw_sum_rows<T, decltype(vec)::value, decltype(na)::value, decltype(nc)::value,
                                      decltype(mode)::value>;
-        const unsigned blocks = rows_blocks(call, kernel, s.smem, s.g.rows);
+        const unsigned blocks = rows_blocks(call, kernel, s, edges);
         kernel<<<blocks, kRowWarps * 32, s.smem, call.stream>>>(s.g, offsets, starts, out, when, call.status);
     });
     MOPS_CUDA_OK(cudaGetLastError());
@@ -779,54 +862,84 @@ void launch_sums(const Call& call, const RowsShape<T>& s, const int64_t* offsets
 
 } // namespace
 
-template <typename T> bool sasaw_forward_rows(const Call& call, const SasawProblem<T>& p, T* O) {
-    if (!rows_apply(p)) return false;
+// Microseconds, fitted to 750 shapes up to 2 10^6 edges with 1 to 16 channels, 1 to 100 columns and rows of
+// a fraction of an edge to thousands; nine in ten estimates are within a third where a call takes more
+// than 80 us. A step is an edge (or the edges side by side) in one pass over columns and channels.
+template <typename T> double sasaw_rows_cost(const SasawProblem<T>& p, RowsWork work) {
+    if (!rows_apply(p)) return INFINITY;
+    struct Cost {
+        double call, product, step, exact_product, exact_step; // products and steps in 10^-6
+        double contract, contract_once, table, pass, edge, row; // 10^-6, 10^-3, 10^-5, 1, 10^-6, 10^-3
+        double few_step, few_product; // a row's steps one after the other: 10^-2, 10^-4
+    };
+    constexpr bool f32 = sizeof(T) == 4;
+    constexpr Cost sorted = f32 ? Cost{22.3, 1.92, 247, 3.51, 79.4, 4.61, 0, 0.369, 1.27, 10.3, 0, 16.8, 18.3}
+                                : Cost{20.8, 4.46, 145, 3, 163, 4.81, 0, 0.739, 1.14, 51.1, 1.02, 16, 21.7};
+    constexpr Cost unsorted = f32 ? Cost{33.9, 4.21, 210, 2.79, 152, 4.3, 4.59, 1.7, 3.19, 32.5, 0, 0, 0}
+                                  : Cost{30.3, 4.66, 139, 2.38, 109, 4.41, 3.32, 0.0769, 8.66, 178, 0.922, 0, 0};
+    constexpr Cost gradients = f32 ? Cost{31.4, 6.26, 741, 8.67, 352, 5.62, 6.84, 1.01, 23.3, 0, 0.113, 0, 0}
+                                   : Cost{38.3, 14.2, 743, 10.5, 539, 9.55, 2.48, 0.897, 15.7, 29.7, 0, 0, 0};
+    const Cost& c = work == RowsWork::kSorted ? sorted : work == RowsWork::kUnsorted ? unsorted : gradients;
+    const bool forward = work != RowsWork::kGradients;
+    const int nC = forward ? p.nW : p.nO, nOut = forward ? p.nO : p.nW;
+    const int na = pad_a(p.nA), nc = chunk_c(na, nC), vec = vector_width<T>(p.L, {});
+    int lanes = 4;
+    while (lanes < 32 && lanes * vec < p.L) lanes *= 2;
+    const double E = static_cast<double>(p.E), rows = static_cast<double>(p.rows), side = 32 / lanes;
+    const double passes = static_cast<double>(ceil_div(nC, nc) * ceil_div(p.L, lanes * vec));
+    const double products = na * nc, contract = products * (ceil_div(nOut, kTableOut) * kTableOut);
+    // (a row's last step is half empty)
+    const double steps = E / side + std::min(E, rows) * (1 - 1 / side);
+    const bool exact = p.L == 32 * vec;
+    const double busy = std::max(rows, 1184.0); // (a row for each of the warps)
+    double us = c.call + passes * c.pass + E * c.edge * 1e-6 + contract * static_cast<double>(p.N) * c.table * 1e-5 +
+                passes * contract * (busy * c.contract * 1e-6 + c.contract_once * 1e-3) + passes * busy * c.row * 1e-3;
+    us += passes * steps * 1e-6 * (exact ? products * c.exact_product + c.exact_step : products * c.product + c.step);
+    const double few = std::max(0.0, 1 - rows / 2368); // (two rows for each of the warps)
+    if (exact && na == 16 && (vec == 2 || !f32)) us *= 1.25; // (what the fit leaves over)
+    us += few * passes * (E / rows / side) * (c.few_step * 1e-2 + products * c.few_product * 1e-4);
+    return us;
+}
+
+template <typename T> int sasaw_forward_rows(const Call& call, const SasawProblem<T>& p, T* O, ScatterPart part) {
+    if (!rows_apply(p)) return kNotApplicable;
     RowsShape<T> s = rows_shape(call, p, p.W, false, vector_width<T>(p.L, {p.B, p.W, O}));
-    if (s.smem > static_cast<size_t>(max_optin_smem(call.device))) return false;
+    if (s.smem > static_cast<size_t>(max_optin_smem(call.device))) return kNotApplicable;
     TableRef table = dense_table(call, p, s, false);
-    SegmentTable seg = segment_table(call, p.I, p.E, p.rows);
     s.g.gather = p.J, s.g.perm = nullptr, s.g.D = static_cast<const T*>(table.ptr), s.g.bit = kBitJ;
-    note_kernel_f("sasaw_sum_rows<%s,VEC=%d,NA=%d,NC=%d>", scalar_name<T>(), s.vec, s.na, s.nc);
-    auto run = [&](RowsRun when, const int32_t* starts) { launch_sums(call, s, seg.offsets, starts, O, when); };
-    run(kSorted, nullptr);
-    bool unsorted = !seg.known_sorted; // asynchronous calls cannot look: always enqueue
-    if (unsorted && call.wait) {
-        wait_stream(call);
-        unsorted = host_saw_unsorted(call);
+    bool unsorted = true;
+    if (part != ScatterPart::kUnsorted) {
+        note_kernel_f("sasaw_sum_rows<%s,VEC=%d,NA=%d,NC=%d>", scalar_name<T>(), s.vec, s.na, s.nc);
+        SegmentTable seg = segment_table(call, p.I, p.E, p.rows);
+        launch_sums<T>(call, s, seg.offsets, nullptr, O, kSorted, p.E);
+        unsorted = !seg.known_sorted; // asynchronous calls cannot look: always enqueue
+        release_table(call, seg.ref);
+        if (unsorted && call.wait) {
+            wait_stream(call);
+            unsorted = host_saw_unsorted(call);
+        }
     }
-    if (unsorted) {
+    if (unsorted && part != ScatterPart::kSorted) {
         const int sorters = sort_blocks(call, p.E, p.rows);
         void* scratch = scratch_alloc(call, entry_sort_bytes(p.E, p.rows, sorters));
         const EntrySort sort = entry_sort_at(scratch, p.rows, sorters);
-        launch_sorting(call, sorters, sort_if_unsorted_grid, sort_if_unsorted_block, sort, p.I, p.E, p.rows,
-                       call.status);
         s.g.perm = sort.perm;
-        run(kIfUnsorted, sort.starts);
+        set_chunks(call, s, sort, p.E);
+        launch_sorting(call, sorters, sort_if_unsorted_grid, sort_if_unsorted_block, sort, p.I, p.E, p.rows,
+                       reinterpret_cast<uint32_t*>(O), p.rows * p.nO * p.L * static_cast<int64_t>(sizeof(T) / 4),
+                       s.g.limit, call.status);
+        launch_sums<T>(call, s, nullptr, sort.starts, O, kIfUnsorted, p.E);
         scratch_free(call, scratch);
+        unsorted = false;
     }
-    release_table(call, seg.ref);
     release_table(call, table);
-    return true;
-}
-
-// A warp walks its rows alone, once per pass over columns and output channels: with few rows most
-// warps stay idle, and padding to the instantiations multiplies the work. Over 400 shapes up to 10^6
-// edges the gradients by edge are the faster ones below these rows, above these passes and above this
-// ratio of padded to useful products (10 to 700 rows, 16 x 9 -> 16 channels: 2 to 6 times as fast).
-template <typename T> bool gradients_by_rows(const RowsShape<T>& s, const SasawProblem<T>& p) {
-    const int columns = s.g.L > 16 ? 32 * s.vec : s.g.lanes;
-    const int64_t wide = ceil_div(p.L, columns), deep = ceil_div(s.g.nC, s.nc);
-    const double padded = static_cast<double>(wide * columns) * (deep * s.nc) * s.na;
-    const bool single = sizeof(T) == 4;
-    return p.rows >= (single ? 2000 : 600) && wide * deep <= (single ? 3 : 4) &&
-           padded <= (single ? 3.0 : 2.5) * p.nA * p.nW * p.L;
+    return unsorted ? kUnsortedLeft : kComplete;
 }
 
 template <typename T>
 bool sasaw_backward_rows(const Call& call, const SasawProblem<T>& p, T* gA, T* gB, T* gW, const T* gO) {
     if (!rows_apply(p)) return false;
     RowsShape<T> s = rows_shape(call, p, gO, true, vector_width<T>(p.L, {p.B, p.W, gO, gB, gW}));
-    if (!gradients_by_rows(s, p)) return false;
     if (s.smem > static_cast<size_t>(max_optin_smem(call.device))) return false;
     TableRef table = dense_table(call, p, s, true);
     // the edges in the order of J
@@ -843,19 +956,22 @@ bool sasaw_backward_rows(const Call& call, const SasawProblem<T>& p, T* gA, T* g
         commit_table(call, order);
     }
     s.g.gather = p.I, s.g.perm = sort.perm, s.g.D = static_cast<const T*>(table.ptr), s.g.bit = kBitI;
-    if (gW != nullptr) {
-        note_kernel_f("sasaw_sum_rows<%s,VEC=%d,NA=%d,NC=%d>", scalar_name<T>(), s.vec, s.na, s.nc);
-        launch_sums<T>(call, s, nullptr, sort.starts, gW, kAlways);
-    }
+    set_chunks(call, s, sort, p.E);
     if (gA != nullptr || gB != nullptr) {
         note_kernel_f("sasaw_edge_gradients<%s,VEC=%d,NA=%d,NC=%d>", scalar_name<T>(), s.vec, s.na, s.nc);
         for_shape(s, [&](auto vec, auto na, auto nc, auto mode) {
             auto kernel = sasaw_edge_gradients<T, decltype(vec)::value, decltype(na)::value, decltype(nc)::value,
                                                decltype(mode)::value>;
-            const unsigned blocks = rows_blocks(call, kernel, s.smem, s.g.rows);
-            kernel<<<blocks, kRowWarps * 32, s.smem, call.stream>>>(s.g, sort.starts, gA, gB, p.W, call.status);
+            const unsigned blocks = rows_blocks(call, kernel, s, p.E);
+            kernel<<<blocks, kRowWarps * 32, s.smem, call.stream>>>(s.g, sort.starts, gA, gB, gW, p.W, call.status);
         });
         MOPS_CUDA_OK(cudaGetLastError());
+    } else if (gW != nullptr) {
+        MOPS_CUDA_OK(cudaMemsetAsync(gW, 0, p.rows * p.nW * p.L * sizeof(T), call.stream));
+    }
+    if (gW != nullptr) {
+        note_kernel_f("sasaw_sum_rows<%s,VEC=%d,NA=%d,NC=%d>", scalar_name<T>(), s.vec, s.na, s.nc);
+        launch_sums<T>(call, s, nullptr, sort.starts, gW, kAlways, p.E);
     }
     release_table(call, order);
     release_table(call, table);
@@ -863,7 +979,8 @@ bool sasaw_backward_rows(const Call& call, const SasawProblem<T>& p, T* gA, T* g
 }
 
 #define INSTANTIATE(T)                                                                             \
-    template bool sasaw_forward_rows<T>(const Call&, const SasawProblem<T>&, T*);                  \
+    template double sasaw_rows_cost<T>(const SasawProblem<T>&, RowsWork);                          \
+    template int sasaw_forward_rows<T>(const Call&, const SasawProblem<T>&, T*, ScatterPart);      \
     template bool sasaw_backward_rows<T>(const Call&, const SasawProblem<T>&, T*, T*, T*, const T*);
 INSTANTIATE(float)
 INSTANTIATE(double)

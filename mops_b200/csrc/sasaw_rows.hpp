@@ -13,9 +13,20 @@ template <typename T> struct SasawProblem {
     int nA, nW, nO, L;
 };
 
+// Which kernels of a forward to enqueue: for a scatter index that is sorted, for one that is not (they
+// stand down on the device where the index is the other), or both.
+enum class ScatterPart { kBoth, kSorted, kUnsorted };
+// What a forward then returns: its kernels do not apply; the result is complete; the sorted part is
+// enqueued, and the one for an unsorted index is still to come.
+enum : int { kNotApplicable = 0, kComplete = 1, kUnsortedLeft = 2 };
+
+// Microseconds that the row kernels take, as fitted to measurements; infinite where they do not apply.
+enum class RowsWork { kSorted, kUnsorted, kGradients };
+template <typename T> double sasaw_rows_cost(const SasawProblem<T>& p, RowsWork work);
+
 // Enqueue the operation on the call's stream and return true, or return false when its channel
-// counts are too large for these kernels. Gradients that are nullptr are skipped.
-template <typename T> bool sasaw_forward_rows(const Call& call, const SasawProblem<T>& p, T* O);
+// counts are too large for these kernels (the forward: as above). Gradients that are nullptr are skipped.
+template <typename T> int sasaw_forward_rows(const Call& call, const SasawProblem<T>& p, T* O, ScatterPart part);
 template <typename T>
 bool sasaw_backward_rows(const Call& call, const SasawProblem<T>& p, T* gA, T* gB, T* gW, const T* gO);
 

@@ -27,18 +27,21 @@ struct EntrySort {
     int32_t* starts; // [n_rows + 1] first position of every row in `perm`
     int32_t* cursor; // [n_rows + 1]
     int32_t* sums;   // [blocks]
+    int32_t* longest; // entries of the longest row, if more than kEvenRow, else 0
     int32_t* perm;   // [J] entries in the order of their rows
 };
+constexpr int kEvenRow = 32;
 
 inline size_t entry_sort_bytes(int64_t J, int64_t n_rows, int blocks) {
-    return (2 * static_cast<size_t>(n_rows + 1) + blocks + static_cast<size_t>(J)) * sizeof(int32_t);
+    return (2 * static_cast<size_t>(n_rows + 1) + blocks + 1 + static_cast<size_t>(J)) * sizeof(int32_t);
 }
 inline EntrySort entry_sort_at(void* p, int64_t n_rows, int blocks) {
     EntrySort s;
     s.starts = static_cast<int32_t*>(p);
     s.cursor = s.starts + n_rows + 1;
     s.sums = s.cursor + n_rows + 1;
-    s.perm = s.sums + blocks;
+    s.longest = s.sums + blocks;
+    s.perm = s.longest + 1;
     return s;
 }
 
@@ -76,6 +79,7 @@ __device__ __forceinline__ void sort_entries(const EntrySort& s, const int32_t* 
                                              int64_t n_rows, bool keep_bad, const Status& st, Sync&& sync,
                                              int bit = 0) {
     __shared__ int32_t warp_sums[33];
+    __shared__ int32_t block_longest;
     const int64_t thread = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     const int64_t threads = static_cast<int64_t>(gridDim.x) * blockDim.x;
     auto row_of = [&](int64_t j) {
@@ -83,6 +87,8 @@ __device__ __forceinline__ void sort_entries(const EntrySort& s, const int32_t* 
         return static_cast<uint32_t>(row) < static_cast<uint32_t>(n_rows) ? row : keep_bad ? 0 : -1;
     };
     for (int64_t r = thread; r <= n_rows; r += threads) s.starts[r] = 0;
+    if (thread == 0) *s.longest = 0;
+    if (threadIdx.x == 0) block_longest = 0;
     sync();
     for (int64_t j = thread; j < J; j += threads) {
         const int row = row_of(j);
@@ -102,14 +108,20 @@ __device__ __forceinline__ void sort_entries(const EntrySort& s, const int32_t* 
     int before = 0;
     for (int b = threadIdx.x; b < static_cast<int>(blockIdx.x); b += blockDim.x) before += s.sums[b];
     int run = block_scan(before, unused, warp_sums);
+    int most = 0;
     for (int64_t r0 = lo; r0 < hi; r0 += blockDim.x) {
         const int64_t r = r0 + threadIdx.x;
         const int v = r < hi ? s.starts[r] : 0;
+        most = max(most, v);
         int exclusive;
         const int all = block_scan(v, exclusive, warp_sums);
         if (r < hi) s.starts[r] = s.cursor[r] = run + exclusive;
         run += all;
     }
+    most = __reduce_max_sync(kFullMask, most);
+    if ((threadIdx.x & 31) == 0 && most > kEvenRow) atomicMax(&block_longest, most);
+    __syncthreads();
+    if (threadIdx.x == 0 && block_longest > 0) atomicMax(s.longest, block_longest);
     if (hi == n_rows && (lo < hi || blockIdx.x == 0) && threadIdx.x == 0) s.starts[n_rows] = run;
     sync();
     for (int64_t j = thread; j < J; j += threads) {
@@ -119,16 +131,28 @@ __device__ __forceinline__ void sort_entries(const EntrySort& s, const int32_t* 
     sync();
 }
 
-// The sort alone (for the VJP, whose kernel reads `perm`).
-__global__ void __launch_bounds__(kSortThreads)
-sort_if_unsorted_grid(EntrySort s, const int32_t* __restrict__ P, int64_t J, int64_t n_rows, Status st) {
+// The sort alone, for kernels that read `perm`. Where rows are longer than `limit`, `zero` (n words, or
+// nullptr) is cleared for kernels that will then add to it.
+template <typename Sync>
+__device__ __forceinline__ void sort_if_unsorted(const EntrySort& s, const int32_t* __restrict__ P, int64_t J,
+                                                 int64_t n_rows, uint32_t* zero, int64_t n, int limit,
+                                                 const Status& st, Sync&& sync) {
     if (!saw_unsorted(st)) return;
-    sort_entries(s, P, J, n_rows, true, st, [] { cooperative_groups::this_grid().sync(); });
+    sort_entries(s, P, J, n_rows, true, st, sync);
+    if (zero != nullptr && *s.longest > limit)
+        for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
+             i += static_cast<int64_t>(gridDim.x) * blockDim.x)
+            zero[i] = 0;
 }
 __global__ void __launch_bounds__(kSortThreads)
-sort_if_unsorted_block(EntrySort s, const int32_t* __restrict__ P, int64_t J, int64_t n_rows, Status st) {
-    if (!saw_unsorted(st)) return;
-    sort_entries(s, P, J, n_rows, true, st, [] { __syncthreads(); });
+sort_if_unsorted_grid(EntrySort s, const int32_t* __restrict__ P, int64_t J, int64_t n_rows, uint32_t* zero,
+                      int64_t n, int limit, Status st) {
+    sort_if_unsorted(s, P, J, n_rows, zero, n, limit, st, [] { cooperative_groups::this_grid().sync(); });
+}
+__global__ void __launch_bounds__(kSortThreads)
+sort_if_unsorted_block(EntrySort s, const int32_t* __restrict__ P, int64_t J, int64_t n_rows, uint32_t* zero,
+                       int64_t n, int limit, Status st) {
+    sort_if_unsorted(s, P, J, n_rows, zero, n, limit, st, [] { __syncthreads(); });
 }
 
 // `writes`: the rows, or the values of the result where the kernel clears it. (500 entries for 100 000 rows

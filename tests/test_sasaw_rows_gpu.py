@@ -7,7 +7,7 @@ import pytest
 
 from conftest import assert_parity
 from helpers import run_checker, run_library, to_dev
-from mops_b200 import workloads
+from mops_b200 import _lib, workloads
 from test_parity_gpu import compare
 
 import mops_b200
@@ -75,3 +75,80 @@ def test_whole_warps(oracle, dtype, shift):
     got, want = run_library("sasaw", t), run_checker(oracle, "sasaw", d, dtype)
     for k in want:
         assert_parity(got[k], want[k], f"sasaw L=32 shifted {shift}/{k}")
+
+
+def _by_rows(d, dtype, oracle, what):
+    """All results against the oracle in f64 on the same operands (its f32 chains are too long for the f32
+    tolerance); the gradients must have come from the row kernels."""
+    t = to_dev(d, dtype)
+    got = run_library("sasaw", t)
+    assert any("sasaw_edge_gradients" in k for k in _lib.last_kernels()), (what, _lib.last_kernels())
+    rounded = {k: v.astype(dtype).astype(np.float64) if isinstance(v, np.ndarray) and v.dtype == np.float64 else v
+               for k, v in d.items()}
+    want = run_checker(oracle, "sasaw", rounded, np.float64)
+    for k in want:
+        assert_parity(got[k], want[k].astype(dtype), f"{what}/{k}")
+    return t, got
+
+
+# shapes that the gradients take by rows: edges side by side (L <= 16), one column per lane, two (f32), whole
+# rows of 16-byte pieces (32 and 64), 4, 9 and 16 A channels, one pass over the output channels and several
+GRADIENTS = [(np.float32, (4, 9, 16), L) for L in (3, 8, 16, 32, 64, 66)] + \
+            [(np.float32, (9, 9, 9), L) for L in (3, 8, 16, 64, 66)] + \
+            [(np.float64, (4, 9, 16), L) for L in (3, 8, 16, 32, 33, 64, 66)] + \
+            [(np.float64, (9, 9, 9), L) for L in (8, 16)] + [(np.float64, (16, 16, 9), L) for L in (3, 8)]
+
+
+@pytest.mark.parametrize("dtype,channels,L", GRADIENTS)
+@pytest.mark.parametrize("rows", ["even", "half in one", "cubic"])
+def test_gradients_by_rows(oracle, dtype, channels, L, rows):
+    """The rows of W with about equal numbers of edges, and with so many in some that they are cut."""
+    nA, nW2, nO2 = channels
+    d = workloads.sasaw(E=30000, n=2500, nA=nA, nW2=nW2, nO2=nO2, L=L, N=100)
+    r = np.random.default_rng(4)
+    if rows == "half in one":
+        d["indices_W_1"][r.permutation(30000)[:15000]] = 77
+    elif rows == "cubic":
+        d["indices_W_1"][:] = (r.random(30000) ** 3 * 2500).astype(np.int32)
+    what = f"sasaw {channels} L={L} {rows}"
+    t, got = _by_rows(d, dtype, oracle, what)
+    if L != 8:
+        return
+    idx = [t[k] for k in ("indices_A", "indices_W_1", "indices_W_2", "indices_output_1", "indices_output_2")]
+    for which, name in enumerate(("grad_A", "grad_B", "grad_W")):  # one at a time
+        some = mops_b200.sparse_accumulation_scatter_add_with_weights_vjp(
+            t["grad_output"], t["A"], t["B"], t["C"], t["W"], *idx,
+            **{f"compute_grad_{x}": i == which for i, x in enumerate("ABW")})
+        assert [x is None for x in some] == [i != which for i in range(3)]
+        tol = 1e-12 if dtype == np.float64 else 1e-5
+        assert np.abs(some[which].cpu().numpy() - got[name]).max() <= tol * np.abs(got[name]).max(), what
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("kw", [dict(E=20000, n=40, L=32), dict(E=9000, n=2, L=66), dict(E=30000, n=900, L=16),
+                                dict(E=700, n=3000, L=8)])
+@pytest.mark.parametrize("rows", ["even", "half in one", "all in one"])
+def test_unsorted_rows(oracle, dtype, kw, rows):
+    """Rows of an unsorted index, few, long, cut or without edges; waiting and not."""
+    import torch
+
+    import mops_b200.torch as mt
+    d = workloads.sasaw(nA=9, nW2=9, nO2=9, N=100, **kw)
+    r = np.random.default_rng(6)
+    p = r.permutation(d["indices_output_1"])
+    if rows != "even":
+        p[: kw["E"] // (1 if rows == "all in one" else 2)] = kw["n"] // 2
+        p[0] = kw["n"] - 1
+    d["indices_output_1"] = p
+    t = to_dev(d, dtype)
+    rounded = {k: v.astype(dtype).astype(np.float64) if isinstance(v, np.ndarray) and v.dtype == np.float64 else v
+               for k, v in d.items()}
+    want = run_checker(oracle, "sasaw", rounded, np.float64)
+    got = run_library("sasaw", t)
+    for k in want:
+        assert_parity(got[k], want[k].astype(dtype), f"sasaw unsorted {kw} {rows}/{k}")
+    out = mt.sparse_accumulation_scatter_add_with_weights(
+        t["A"], t["B"], t["C"], t["W"], t["indices_A"], t["indices_W_1"], t["indices_W_2"],
+        t["indices_output_1"], t["indices_output_2"], t["output_size"])
+    torch.cuda.synchronize()
+    assert_parity(out.cpu().numpy(), want["output"].astype(dtype), f"sasaw unsorted {kw} {rows} asynchronous")
