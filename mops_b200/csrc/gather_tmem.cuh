@@ -359,7 +359,7 @@ gather_table(unsigned char* __restrict__ records, int32_t* __restrict__ n_start,
 }
 
 // ---------------------------------------------------------------- the sums
-// The 32-byte sector that ends at `at`: the value `now` of slot r and the ones before it.
+// A whole 32-byte sector, from a 32-byte boundary on, in one store.
 __device__ __forceinline__ void store_sector(double* from, const double (&v)[4]) {
     asm volatile("st.global.v4.f64 [%0], {%1,%2,%3,%4};\n" ::"l"(from), "d"(v[0]), "d"(v[1]), "d"(v[2]), "d"(v[3])
                  : "memory");

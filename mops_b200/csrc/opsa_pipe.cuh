@@ -721,7 +721,6 @@ opsa_fwd_pipe_tf32(float* __restrict__ O, const float* __restrict__ A, const flo
         }
     };
     for (int i = 0; i < NS - 1; i++) issue_next();
-    __syncwarp(); // (a last row's end may have been stored by one lane)
 
     int64_t wbase = w.r0;
     auto load_window = [&](int64_t base) {
