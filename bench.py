@@ -464,20 +464,18 @@ def load_traffic():
 
 
 def measured(traffic, name, level, launched):
-    """(DRAM bytes per launch, shared-memory wavefronts per launch) of the captured kernel,
-    scaled to this run's size, or (None, None, why) when the capture is of another
-    instantiation than the one this run launched."""
+    """DRAM bytes per launch of the captured kernels, scaled to this run's size, or (None, why) when the
+    capture is of other instantiations than this run launched. `kernel` names them all, as
+    mops_b200_last_kernels does."""
     e = traffic.get(f"{name}/{level}")
     if e is None:
-        return None, None, "no capture"
-    if not any(e["kernel"] in k for k in launched):
-        return None, None, f"capture is of {e['kernel']}, this run launched {'; '.join(launched)}"
+        return None, "no capture"
+    if not all(any(part in k for k in launched) for part in e["kernel"].split("; ")):
+        return None, f"capture is of {e['kernel']}, this run launched {'; '.join(launched)}"
     if bool(e.get("keep_rows", False)) != KEEP_ROWS and SCALE != 1:
-        return None, None, "capture and run scale their output rows differently"
+        return None, "capture and run scale their output rows differently"
     f = e["scale"] / SCALE
-    wf = e.get("smem_wavefronts")
-    return (e["dram_read_bytes"] + e["dram_write_bytes"]) * f, None if wf is None else wf * f, \
-        e.get("note")
+    return (e["dram_read_bytes"] + e["dram_write_bytes"]) * f, e.get("note")
 
 
 # ------------------------------------------------------------------------------ main
@@ -851,7 +849,7 @@ def main():
         for lvl, ms, b in (("fwd", f_ms, bf), ("vjp", v_ms, bv)):
             k = launched.get((n, lvl), [])
             entry[f"{lvl}_kernels"] = k
-            dram, wavefronts, note = measured(traffic, n, lvl, k)
+            dram, note = measured(traffic, n, lvl, k)
             entry[f"{lvl}_traffic"] = dram
             if note:
                 entry[f"{lvl}_traffic_note"] = note
