@@ -2481,8 +2481,8 @@ template <typename T> SasawProblem<T> rows_problem(const Problem<T>& p) {
 // The row kernels (sasaw_rows.cu) or the ones here, by estimates of their time, fitted to the same 750 shapes
 // (sasaw_rows_cost) in every direction. The estimates miss by a third in one of ten, so the family that is
 // usually the faster one gives way only where the other is estimated to be so by kMargin. Of 3000 calls (those
-// shapes, forward and gradients, waiting and not) 5 % then take more than 1.07 and 1 % more than 1.25 times what
-// the better family would; one family alone is up to 8 times slower. Microseconds:
+// shapes, forward and gradients, waiting and not) 16 % then take more than 1.07 and 5 % more than 1.25 times
+// what the better family would; one family alone is up to 8 times slower. Microseconds:
 struct EdgeCost {
     double call, cell, entry, edge, table, row; // cells, entries, edges and rows in 10^-6, the table 10^-3
     double few_edge, few_cell;                  // a row's edges one after the other: 10^-2, 10^-5
