@@ -68,14 +68,341 @@ bool run(const Call& call, const SapProblem<T>& p, const Family* families, int c
     return run_gather<T, 2>(call, key, source, p.K * count, op, results, p.I, name);
 }
 
-// ---------------------------------------------------------------- VJP by cells
-// With S the narrower of A, B and T the wider one, both gradients are sums over the cells (t, s) of
+// ---------------------------------------------------------------- large batches
+// Two kernels for batches that give every SM a tile. The triplets' records stay in shared memory for all
+// tiles of a block, and results are collected there, to leave as one bulk copy per tile: the ring, its
+// meetings and the stores of single sectors of the kernels of gather_tmem.cuh cost half of the time of
+// 1000 triplets (2^22 rows, 20 x 6 -> 50, f64: 25 700 clocks per 256 rows in the forward, 11 600 of them
+// whatever the number of triplets; VJP 42 600 and 24 000).
+
+// Records in batches of four, coefficients and 16-bit TMEM columns apart.
+constexpr int kLot = 4;
+template <typename T, int NF, int W> struct Lot {
+    static constexpr int R = W / words_of(sizeof(T)); // rows per lane
+    uint32_t v[kLot][NF][W];
+};
+template <typename T, int NF> struct LotRecords {
+    T c[kLot];
+    uint32_t q[kLot * NF / 2];
+};
+
+template <typename T, int NF> struct ResidentRecords {
+    T* c;
+    uint16_t* q;
+    static __host__ __device__ size_t bytes(int capacity) { return static_cast<size_t>(capacity) * (sizeof(T) + 2 * NF); }
+
+    __device__ ResidentRecords(unsigned char* smem, int capacity)
+        : c(reinterpret_cast<T*>(smem)), q(reinterpret_cast<uint16_t*>(smem + capacity * sizeof(T))) {}
+    // Once per block: `count` records as the table builder wrote them; zeros (column 0) behind them, which
+    // are fetched ahead but not used.
+    __device__ void load(const unsigned char* records, int count, int capacity, int tid) {
+        static_assert(tmem_record_bytes(sizeof(T), NF) == 16, "one 16-byte piece per record");
+        for (int x = tid; x < capacity; x += kTmemThreads) {
+            uint4 v = make_uint4(0u, 0u, 0u, 0u);
+            if (x < count) v = __ldg(reinterpret_cast<const uint4*>(records) + x);
+            uint32_t columns;
+            if constexpr (sizeof(T) == 8) {
+                c[x] = __hiloint2double(static_cast<int>(v.y), static_cast<int>(v.x));
+                columns = v.z;
+            } else {
+                c[x] = __uint_as_float(v.x);
+                columns = v.y;
+            }
+#pragma unroll
+            for (int k = 0; k < NF; k++) q[x * NF + k] = static_cast<uint16_t>(columns >> (16 * k));
+        }
+    }
+    __device__ __forceinline__ void fetch(LotRecords<T, NF>& r, int lot) const {
+        constexpr int V = 16 / sizeof(T);
+#pragma unroll
+        for (int i = 0; i < kLot; i += V) {
+            T v[V];
+            load_vec<T, V>(c + lot * kLot + i, v);
+#pragma unroll
+            for (int j = 0; j < V; j++) r.c[i + j] = v[j];
+        }
+        const uint2* src = reinterpret_cast<const uint2*>(q + lot * (kLot * NF));
+#pragma unroll
+        for (int i = 0; i < NF; i++) {
+            const uint2 u = src[i];
+            r.q[2 * i] = u.x, r.q[2 * i + 1] = u.y;
+        }
+    }
+};
+
+template <typename T, int NF, int W>
+__device__ __forceinline__ void issue(Lot<T, NF, W>& g, const LotRecords<T, NF>& r, uint32_t base) {
+#pragma unroll
+    for (int b = 0; b < kLot; b++)
+#pragma unroll
+        for (int k = 0; k < NF; k++) {
+            const int i = b * NF + k;
+            tmem_load(__byte_perm(r.q[i / 2], base, (i & 1) ? 0x7632 : 0x7610), g.v[b][k]);
+        }
+}
+template <typename T, int NF, int W> __device__ __forceinline__ void await(Lot<T, NF, W>& g) {
+    tmem_wait_load();
+#pragma unroll
+    for (int b = 0; b < kLot; b++)
+#pragma unroll
+        for (int k = 0; k < NF; k++) tmem_pin(g.v[b][k]);
+}
+// Two chains of sums: even and odd records of the batches.
+template <typename T, int NF, int W>
+__device__ __forceinline__ void add_terms(const Lot<T, NF, W>& g, const LotRecords<T, NF>& rec,
+                                          T (&acc)[2][Lot<T, NF, W>::R]) {
+#pragma unroll
+    for (int b = 0; b < kLot; b++)
+#pragma unroll
+        for (int r = 0; r < Lot<T, NF, W>::R; r++) {
+            T p = rec.c[b];
+#pragma unroll
+            for (int k = 0; k + 1 < NF; k++) p *= tmem_value<T>(g.v[b][k], r);
+            acc[b & 1][r] += p * tmem_value<T>(g.v[b][NF - 1], r);
+        }
+}
+
+// The batches [first, first + count) in order, added to acc; after(i) behind batch i (from 0).
+template <typename T, int NF, int W, typename After>
+__device__ __forceinline__ void walk_lots(const ResidentRecords<T, NF>& records, int first, int count, uint32_t base,
+                                          T (&acc)[2][Lot<T, NF, W>::R], After&& after) {
+    if (count <= 0) return;
+    Lot<T, NF, W> x, y;
+    LotRecords<T, NF> rx, ry;
+    records.fetch(rx, first);
+    issue(x, rx, base);
+    records.fetch(ry, first + 1);
+#pragma unroll 1
+    for (int i = 0; i < count; i += 2) {
+        await(x);
+        issue(y, ry, base);
+        add_terms(x, rx, acc);
+        records.fetch(rx, first + i + 2);
+        after(i);
+        await(y);
+        issue(x, rx, base);
+        add_terms(y, ry, acc); // (an odd count's last batch is not the group's: everything is closed by then)
+        records.fetch(ry, first + i + 3);
+        after(i + 1);
+    }
+    await(x);
+}
+
+// Results of a tile in shared memory, rows side by side as in HBM (or 16 bytes further apart, where lanes
+// that store a column would otherwise meet in the same banks: then they leave row by row).
+struct ResultStage {
+    int columns, stride; // bytes from row to row
+    int offset;          // in shared memory
+};
+template <typename T> ResultStage result_stage(int columns, int rows, size_t& smem) {
+    const int bytes = columns * static_cast<int>(sizeof(T));
+    const bool crowded = bytes % (sizeof(T) == 8 ? 64 : 32) == 0; // more than four lanes to a bank
+    ResultStage s{columns, bytes + (crowded ? 16 : 0), static_cast<int>(smem)};
+    smem += static_cast<size_t>(rows) * s.stride;
+    return s;
+}
+__device__ __forceinline__ void bulk_copy_out(void* global_dst, const void* smem_src, unsigned bytes) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n" ::"l"(global_dst),
+                 "r"(smem_address(smem_src)), "r"(bytes)
+                 : "memory");
+}
+// One warp, when all of the tile's results are there (and fence_results has been called by who wrote them).
+template <typename T>
+__device__ __forceinline__ void send_results(const ResultStage& s, const unsigned char* smem, T* out, int64_t row0,
+                                             int rows, int lane) {
+    const int bytes = s.columns * static_cast<int>(sizeof(T));
+    T* dst = out + row0 * s.columns;
+    const unsigned char* src = smem + s.offset;
+    if (s.stride == bytes) {
+        const int all = rows * bytes, whole = all & ~15;
+        if (lane == 0 && whole > 0) bulk_copy_out(dst, src, static_cast<unsigned>(whole));
+        const int x = whole + lane * static_cast<int>(sizeof(T));
+        if (x < all) dst[x / sizeof(T)] = *reinterpret_cast<const T*>(src + x);
+    } else {
+        for (int r = lane; r < rows; r += 32) bulk_copy_out(dst + static_cast<int64_t>(r) * s.columns, src + r * s.stride, bytes);
+    }
+    asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
+}
+__device__ __forceinline__ void fence_results() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
+__device__ __forceinline__ void await_results_read() { asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory"); }
+__device__ __forceinline__ void await_results_sent() { asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory"); }
+
+// The stage may be written again when the copies of the tile before have read it: warp 0, which issued
+// them, says so on a barrier, and every warp waits there before its first result of a tile.
+struct StageGuard {
+    uint64_t* bar;
+    int tile = 0;       // how many tiles this block has begun
+    bool passed = false;
+    __device__ void begin_tile() { passed = false; }
+    __device__ __forceinline__ void pass(int warp, int lane, const Status& st) {
+        if (passed) return;
+        passed = true;
+        if (tile == 0) return;
+        if (warp == 0) {
+            await_results_read();
+            __syncwarp();
+            if (lane == 0) mbarrier_arrive_expect(bar, 0);
+        } else if (!mbarrier_wait(bar, (tile - 1) & 1) && lane == 0) {
+            report_stalled(st);
+        }
+        __syncwarp();
+    }
+};
+
+// ---- forward: by products of operand columns (NF = 1: the records' columns are the cells (a, b) of A x B,
+// whose products are formed once per row on the way into TMEM), where those fit, else by pairs (NF = 2).
+template <typename T> struct ProductSource {
+    const T* C;
+    const int32_t *PA, *PB, *PO;
+    int nA, nB, nO;
+    __device__ int key(int x, unsigned& bad) const {
+        int32_t a = __ldg(PA + x), b = __ldg(PB + x), o = __ldg(PO + x);
+        if (clamp_index(a, nA)) bad |= 1u << kA;
+        if (clamp_index(b, nB)) bad |= 1u << kB;
+        if (clamp_index(o, nO)) bad |= 1u << kO;
+        return o;
+    }
+    __device__ T coefficient(int x) const { return __ldg(C + x); }
+    __device__ int column(int x, int) const {
+        int32_t a = __ldg(PA + x), b = __ldg(PB + x);
+        clamp_index(a, nA);
+        clamp_index(b, nB);
+        return a * nB + b;
+    }
+};
+
+template <typename T, int NF, int W>
+__global__ void __launch_bounds__(kTmemThreads, 1)
+sap_fwd_resident(T* __restrict__ O, const __grid_constant__ Operands operands, const unsigned char* __restrict__ table,
+                 const int32_t* __restrict__ o_start, const ResultStage stage, int capacity, int slab_offset,
+                 int64_t I, int64_t tiles, Status st) {
+    constexpr int R = W / words_of(sizeof(T));
+    const int nA = operands.cols[0], nB = operands.cols[1], nO = stage.columns;
+    extern __shared__ __align__(16) unsigned char smem[];
+    // layout: records | starts [nO + 1] | results | slabs
+    ResidentRecords<T, NF> records(smem, capacity);
+    int32_t* starts = reinterpret_cast<int32_t*>(smem + (records.bytes(capacity) + 15) / 16 * 16);
+    __shared__ uint32_t tmem_s;
+    __shared__ uint64_t stage_free;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(kFullMask, tid >> 5, 0), group = warp >> 2;
+
+    Tiles<T, W> t{operands, I, operands.template slab_bytes<T>(), smem + slab_offset};
+    t.start(blockIdx.x, tid);
+    if (warp == 0) tmem_alloc(&tmem_s, kTmemColumns);
+    if (tid == 0) {
+        mbarrier_init(&stage_free, 1);
+        mbarrier_init_fence();
+    }
+    for (int n = tid; n <= nO; n += kTmemThreads) starts[n] = __ldg(o_start + n);
+    records.load(table, __ldg(o_start + nO), capacity, tid);
+    tmem_fence_before_sync();
+    __syncthreads();
+    tmem_fence_after_sync();
+    const uint32_t base = tmem_quadrant(tmem_s, warp);
+    if (warp < 4) // the column of ones
+        for (int r = 0; r < R; r++)
+            tmem_store(base + (NF == 1 ? nA * nB : nA + nB) * W + r * words_of(sizeof(T)), T(1));
+    const int n_lo = uniform(group_column(starts, nO, 1, group, kTmemGroups));
+    const int n_hi = uniform(group_column(starts, nO, 1, group + 1, kTmemGroups));
+    const int first = uniform(starts[n_lo]) / kLot, count = uniform(starts[n_hi]) / kLot - first;
+    const int own = (warp & 3) * 32 + lane;
+    unsigned char* own_results = smem + stage.offset + own * stage.stride;
+    StageGuard guard{&stage_free};
+
+    int64_t before = -1;
+    for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        cp_async_wait<0>();
+        tmem_fence_before_sync();
+        __syncthreads(); // this tile's rows are there, the results of the one before, too
+        tmem_fence_after_sync();
+        if (warp == 0 && before >= 0) send_results(stage, smem, O, before, kSlabRows * R, lane);
+        before = tile * (kSlabRows * R);
+        const int a_stride = slab_stride(nA * static_cast<int>(sizeof(T)));
+        const int b_stride = slab_stride(nB * static_cast<int>(sizeof(T)));
+        if constexpr (NF == 1) {
+            const unsigned char* a_row = t.slabs + own * a_stride;
+            const unsigned char* b_row = t.slabs + kSlabRows * a_stride + own * b_stride;
+            for (int a = group; a < nA; a += kTmemGroups) {
+                T va[R];
+#pragma unroll
+                for (int r = 0; r < R; r++) va[r] = reinterpret_cast<const T*>(a_row + r * t.slab)[a];
+                for (int b = 0; b < nB; b++) {
+                    uint32_t w[W];
+#pragma unroll
+                    for (int r = 0; r < R; r++)
+                        put_coefficient<T>(w + r * words_of(sizeof(T)),
+                                           va[r] * reinterpret_cast<const T*>(b_row + r * t.slab)[b]);
+                    tmem_store(base + (a * nB + b) * W, w);
+                }
+            }
+        } else {
+            slabs_to_tmem<T, W>(t.slabs, t.slab, a_stride, nA, base, warp, lane);
+            slabs_to_tmem<T, W>(t.slabs + kSlabRows * a_stride, t.slab, b_stride, nB, base + nA * W, warp, lane);
+        }
+        tmem_wait_store();
+        tmem_fence_before_sync();
+        __syncthreads();
+        tmem_fence_after_sync();
+        if (tile + gridDim.x < tiles) t.start(tile + gridDim.x, tid);
+
+        guard.begin_tile();
+        if (count == 0) guard.pass(warp, lane, st);
+        T acc[2][R];
+        PieceSum<T, R> sum;
+        sum.clear();
+#pragma unroll
+        for (int r = 0; r < R; r++) acc[0][r] = acc[1][r] = T(0);
+        int n = n_lo, left = n_lo < n_hi ? uniform(starts[n_lo + 1] - starts[n_lo]) / kLot : 0;
+        walk_lots<T, NF, W>(records, first, count, base, acc, [&](int i) {
+            if constexpr (sizeof(T) == 4) { // (PieceSum: pieces of 32 records)
+                if ((i & (kPieceRecords / kLot - 1)) == kPieceRecords / kLot - 1) {
+#pragma unroll
+                    for (int r = 0; r < R; r++) {
+                        sum.total[r] += acc[0][r] + acc[1][r];
+                        acc[0][r] = acc[1][r] = T(0);
+                    }
+                }
+            }
+            if (__builtin_expect(--left == 0, 0)) { // column n is complete
+                guard.pass(warp, lane, st);
+#pragma unroll
+                for (int r = 0; r < R; r++) {
+                    T v = acc[0][r] + acc[1][r];
+                    if constexpr (sizeof(T) == 4) {
+                        v += sum.total[r];
+                        sum.total[r] = T(0);
+                    }
+                    reinterpret_cast<T*>(own_results + r * kSlabRows * stage.stride)[n] = v;
+                    acc[0][r] = acc[1][r] = T(0);
+                }
+                n++;
+                left = n < n_hi ? uniform(starts[n + 1] - starts[n]) / kLot : 0;
+            }
+        });
+        guard.tile++;
+        fence_results();
+    }
+    cp_async_wait<0>();
+    tmem_fence_before_sync();
+    __syncthreads();
+    tmem_fence_after_sync();
+    if (warp == 0) {
+        if (before >= 0)
+            send_results(stage, smem, O, before, static_cast<int>(min(static_cast<int64_t>(kSlabRows * R), I - before)), lane);
+        tmem_free(tmem_s, kTmemColumns);
+        await_results_sent();
+    }
+}
+
+// ---- VJP by cells. With S the narrower of A, B and T the wider one, both gradients are sums over the
+// cells (t, s) of
 //
 //   X = sum of C gO[PO] over the triplets of the cell:    gT[t] += X S[s],    gS[s] += X T[t],
 //
 // so a triplet costs one gather and one FMA per row instead of two records of two factors. The
-// cells are sorted by t, then s; a warp group owns whole t: gT[t] is summed in registers, gS in
-// shared memory, by every group for itself, and the groups' sums are added at the end of a tile.
+// cells are sorted by t, then s; a warp group owns whole t: gT[t] is summed in registers, gS in TMEM
+// columns that every group has for itself; the groups' sums are added at the end of a tile.
 template <typename T> struct CellSource {
     const T* C;
     const int32_t *PT, *PS, *PO;
@@ -95,33 +422,33 @@ template <typename T> struct CellSource {
     }
 };
 
-// Operands: gO (nO columns), T, S; starts[t * nS + s] in records.
+// Operands: gO (nO columns), T, S; cell_start[t * nS + s] in records.
 template <typename T, int W>
 __global__ void __launch_bounds__(kTmemThreads, 1)
-sap_vjp_cells(T* __restrict__ gT, T* __restrict__ gS, const __grid_constant__ Operands operands,
-              const unsigned char* __restrict__ records, const int32_t* __restrict__ cell_start, int64_t I,
-              int64_t tiles, Status st) {
-    using G = Batch<T, 1, W>;
-    constexpr int B = G::B, R = G::R, RB = G::RB;
-    using Ring = RecordRing<1024>;
-    constexpr int kPerStage = 1024 / (B * RB);
-    static_assert(kPerStage % 2 == 0, "pairs of batches do not straddle stages");
+sap_vjp_resident(T* __restrict__ gT, T* __restrict__ gS, const __grid_constant__ Operands operands,
+                 const unsigned char* __restrict__ table, const int32_t* __restrict__ cell_start,
+                 const ResultStage t_stage, const ResultStage s_stage, int capacity, int slab_offset, int64_t I,
+                 int64_t tiles, Status st) {
+    constexpr int R = W / words_of(sizeof(T));
     const int nO = operands.cols[0], nT = operands.cols[1], nS = operands.cols[2], cells = nT * nS;
     extern __shared__ __align__(16) unsigned char smem[];
-    // layout: ring | starts [cells + 1], padded | gS sums [group][nS][128 R] | slabs
-    int32_t* starts = reinterpret_cast<int32_t*>(smem + kStageBytes);
-    T* sums = reinterpret_cast<T*>(smem + kStageBytes + (static_cast<size_t>(cells + 1) * 4 + 15) / 16 * 16);
-    unsigned char* slabs = reinterpret_cast<unsigned char*>(sums + kTmemGroups * nS * kSlabRows * R);
+    // layout: records | starts [cells + 1] | results | slabs
+    ResidentRecords<T, 1> records(smem, capacity);
+    int32_t* starts = reinterpret_cast<int32_t*>(smem + (records.bytes(capacity) + 15) / 16 * 16);
     __shared__ uint32_t tmem_s;
-    __shared__ uint64_t full[kTmemGroups][2];
+    __shared__ uint64_t stage_free;
     const int tid = threadIdx.x, lane = tid & 31;
     const int warp = __shfl_sync(kFullMask, tid >> 5, 0), group = warp >> 2;
 
-    Tiles<T, W> tile_of{operands, I, operands.template slab_bytes<T>(), slabs};
+    Tiles<T, W> tile_of{operands, I, operands.template slab_bytes<T>(), smem + slab_offset};
     tile_of.start(blockIdx.x, tid);
     if (warp == 0) tmem_alloc(&tmem_s, kTmemColumns);
-    Ring::prepare(smem, full, tid);
+    if (tid == 0) {
+        mbarrier_init(&stage_free, 1);
+        mbarrier_init_fence();
+    }
     for (int c = tid; c <= cells; c += kTmemThreads) starts[c] = __ldg(cell_start + c);
+    records.load(table, __ldg(cell_start + cells), capacity, tid);
     tmem_fence_before_sync();
     __syncthreads();
     tmem_fence_after_sync();
@@ -131,185 +458,274 @@ sap_vjp_cells(T* __restrict__ gT, T* __restrict__ gS, const __grid_constant__ Op
     const int t_lo = uniform(group_column(starts, nT, nS, group, kTmemGroups));
     const int t_hi = uniform(group_column(starts, nT, nS, group + 1, kTmemGroups));
     const int c_hi = t_hi * nS;
-    const int x_lo = uniform(starts[t_lo * nS]), batches = uniform(starts[c_hi] - starts[t_lo * nS]) / B;
-    Ring ring(smem + group * 2048, full[group], group, (warp & 3) == 0 && lane == 0,
-              records + static_cast<size_t>(x_lo) * RB, batches * B * RB);
+    const int first = uniform(starts[t_lo * nS]) / kLot, count = uniform(starts[c_hi]) / kLot - first;
     const int own = (warp & 3) * 32 + lane;
-    T* mine = sums + static_cast<size_t>(group) * nS * kSlabRows * R + own; // [s][slot][128]
+    unsigned char* own_t = smem + t_stage.offset + own * t_stage.stride;
+    unsigned char* own_s = smem + s_stage.offset + own * s_stage.stride;
+    // the groups' sums of gS: [group][s], behind the operands and the column of ones
+    const uint32_t all_sums = base + (operands.total + 1) * W, sums = all_sums + group * nS * W;
+    StageGuard guard{&stage_free};
 
+    int64_t before = -1;
     for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        tile_of.load(tile + gridDim.x < tiles ? tile + gridDim.x : -1, base, tid, warp, lane);
-        const int64_t row0 = tile * (kSlabRows * R) + own;
-        bool live[R];
-        T acc[R], sum_t[R];
-#pragma unroll
-        for (int r = 0; r < R; r++) {
-            live[r] = row0 + r * kSlabRows < I;
-            acc[r] = sum_t[r] = T(0);
+        cp_async_wait<0>();
+        tmem_fence_before_sync();
+        __syncthreads(); // this tile's rows are there, the results of the one before, too
+        tmem_fence_after_sync();
+        if (warp == 0 && before >= 0) {
+            send_results(t_stage, smem, gT, before, kSlabRows * R, lane);
+            send_results(s_stage, smem, gS, before, kSlabRows * R, lane);
         }
-        for (int s = 0; s < nS * R; s++) mine[s * kSlabRows] = T(0);
-        SectorWriter<T, R> writer{};
+        before = tile * (kSlabRows * R);
+        {
+            const unsigned char* src = tile_of.slabs;
+            uint32_t column = base;
+            for (int q = 0; q < 3; q++) {
+                const int stride = slab_stride(operands.cols[q] * static_cast<int>(sizeof(T)));
+                slabs_to_tmem<T, W>(src, tile_of.slab, stride, operands.cols[q], column, warp, lane);
+                src += kSlabRows * stride;
+                column += operands.cols[q] * W;
+            }
+            uint32_t zero[W];
+#pragma unroll
+            for (int i = 0; i < W; i++) zero[i] = 0;
+            for (int s = 0; s < nS; s++) tmem_store(sums + s * W, zero);
+        }
+        tmem_wait_store();
+        tmem_fence_before_sync();
+        __syncthreads();
+        tmem_fence_after_sync();
+        if (tile + gridDim.x < tiles) tile_of.start(tile + gridDim.x, tid);
+
+        guard.begin_tile();
+        if (t_lo == t_hi) guard.pass(warp, lane, st);
+        T acc[2][R], sum_t[R];
+#pragma unroll
+        for (int r = 0; r < R; r++) acc[0][r] = acc[1][r] = sum_t[r] = T(0);
         int t = t_lo, s = 0, c = t_lo * nS;
-        uint32_t value_t[1][W];
+        uint32_t value_t[W];
         auto load_t = [&] { // T[t] of the lane's rows
-            tmem_load(base + (nO + t) * W, value_t[0]);
+            tmem_load(base + (nO + t) * W, value_t);
             tmem_wait_load();
-            tmem_pin(value_t[0]);
+            tmem_pin(value_t);
         };
-        // Moves on to the next cell that has records (or to the end), storing gT[t] on the way.
+        // Moves on to the next cell that has records (or to the end), keeping gT[t] on the way.
         // Returns its number of batches.
         auto next_cell = [&](bool moved) {
             for (; c < c_hi; moved = true) {
                 if (moved) {
                     c++;
                     if (++s == nS) {
-                        writer.put(t, gT + row0 * nT + t, kSlabRows * static_cast<int64_t>(nT), t - t_lo, t + 1 == t_hi,
-                                   sum_t, live);
+                        guard.pass(warp, lane, st);
 #pragma unroll
-                        for (int r = 0; r < R; r++) sum_t[r] = T(0);
+                        for (int r = 0; r < R; r++) {
+                            reinterpret_cast<T*>(own_t + r * kSlabRows * t_stage.stride)[t] = sum_t[r];
+                            sum_t[r] = T(0);
+                        }
                         s = 0;
                         t++;
                         if (t < t_hi) load_t();
                     }
                     if (c == c_hi) break;
                 }
-                const int n = uniform(starts[c + 1] - starts[c]) / B;
+                const int n = uniform(starts[c + 1] - starts[c]) / kLot;
                 if (n > 0) return n;
             }
             return -1;
         };
-        auto end_cell = [&] {
-            uint32_t value_s[W];
-            tmem_load(base + (nO + nT + s) * W, value_s);
-            tmem_wait_load();
-            tmem_pin(value_s);
-#pragma unroll
-            for (int r = 0; r < R; r++) {
-                sum_t[r] += acc[r] * tmem_value<T>(value_s, r);
-                mine[(s * R + r) * kSlabRows] += acc[r] * tmem_value<T>(value_t[0], r);
-                acc[r] = T(0);
-            }
-        };
         if (t < t_hi) load_t();
-        ring.start_tile();
         int left = next_cell(false);
-        if (batches > 0) {
-            G x, y;
-            Records<T, 1, W> rx, ry;
-            auto add = [&](const G& g, const Records<T, 1, W>& rec) {
-                add_terms<T, 1, W>(g, rec, acc);
-                if (--left == 0) {
-                    end_cell();
-                    left = next_cell(true);
-                }
-            };
-            ring.enter_stage(0, lane, st);
-            fetch<T, 1, W>(rx, ring.template at<B * RB>(0));
-            issue<T, 1, W>(x, rx, base);
-            fetch<T, 1, W>(ry, ring.template at<B * RB>(1));
-            for (int i = 0; i < batches; i += 2) {
-                await<T, 1, W>(x);
-                issue<T, 1, W>(y, ry, base);
-                add(x, rx);
-                if ((i & (kPerStage - 1)) == kPerStage - 2 && i + 2 < batches)
-                    ring.enter_stage((i + 2) / kPerStage, lane, st);
-                fetch<T, 1, W>(rx, ring.template at<B * RB>(i + 2));
-                await<T, 1, W>(y);
-                issue<T, 1, W>(x, rx, base);
-                add(y, ry); // (behind the last batch: all cells are done, nothing is kept)
-                fetch<T, 1, W>(ry, ring.template at<B * RB>(i + 3));
-            }
-            await<T, 1, W>(x);
-        }
-        tmem_fence_before_sync();
-        __syncthreads(); // all sums are complete; before the next tile overwrites TMEM
-        tmem_fence_after_sync();
-        // gS: the tile's rows are contiguous in memory
-        const int64_t first_row = tile * (kSlabRows * R);
-        const int64_t have = I - first_row < kSlabRows * R ? I - first_row : kSlabRows * R;
-        for (int y = tid; y < have * nS; y += kTmemThreads) {
-            const int row = y / nS, s2 = y - row * nS;
-            T v = T(0);
+        walk_lots<T, 1, W>(records, first, count, base, acc, [&](int) {
+            if (--left == 0) {
+                uint32_t value_s[W], sum_s[W];
+                tmem_wait_store(); // (the sum that was stored last may be this one)
+                tmem_load(base + (nO + nT + s) * W, value_s);
+                tmem_load(sums + s * W, sum_s);
+                tmem_wait_load();
+                tmem_pin(value_s);
+                tmem_pin(sum_s);
 #pragma unroll
-            for (int g = 0; g < kTmemGroups; g++)
-                v += sums[(static_cast<size_t>(g) * nS + s2) * kSlabRows * R + row];
-            gS[first_row * nS + y] = v;
+                for (int r = 0; r < R; r++) {
+                    const T x = acc[0][r] + acc[1][r];
+                    sum_t[r] += x * tmem_value<T>(value_s, r);
+                    put_coefficient<T>(sum_s + r * words_of(sizeof(T)),
+                                       tmem_value<T>(sum_s, r) + x * tmem_value<T>(value_t, r));
+                    acc[0][r] = acc[1][r] = T(0);
+                }
+                tmem_store(sums + s * W, sum_s);
+                left = next_cell(true);
+            }
+        });
+        guard.tile++;
+        // gS: the sums of the four groups
+        tmem_wait_store();
+        tmem_fence_before_sync();
+        __syncthreads();
+        tmem_fence_after_sync();
+        for (int s2 = group; s2 < nS; s2 += kTmemGroups) {
+            uint32_t part[kTmemGroups][W];
+#pragma unroll
+            for (int g = 0; g < kTmemGroups; g++) tmem_load(all_sums + (g * nS + s2) * W, part[g]);
+            tmem_wait_load();
+#pragma unroll
+            for (int g = 0; g < kTmemGroups; g++) tmem_pin(part[g]);
+#pragma unroll
+            for (int r = 0; r < R; r++)
+                reinterpret_cast<T*>(own_s + r * kSlabRows * s_stage.stride)[s2] =
+                    (tmem_value<T>(part[0], r) + tmem_value<T>(part[1], r)) +
+                    (tmem_value<T>(part[2], r) + tmem_value<T>(part[3], r));
         }
-        // (the barriers of the next tile's load come before the sums are cleared)
+        fence_results();
     }
     cp_async_wait<0>();
+    tmem_fence_before_sync();
     __syncthreads();
-    if (warp == 0) tmem_free(tmem_s, kTmemColumns);
+    tmem_fence_after_sync();
+    if (warp == 0) {
+        if (before >= 0) {
+            const int rows = static_cast<int>(min(static_cast<int64_t>(kSlabRows * R), I - before));
+            send_results(t_stage, smem, gT, before, rows, lane);
+            send_results(s_stage, smem, gS, before, rows, lane);
+        }
+        tmem_free(tmem_s, kTmemColumns);
+        await_results_sent();
+    }
+}
+
+inline bool at_16_bytes(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
+
+// Builds (or takes from the plan) the table of records over `columns` result columns, each a whole number
+// of batches, and calls go(records, starts).
+template <typename T, int NF, typename Source, typename Go>
+void with_lots(const Call& call, TableKey key, const Source& source, int64_t K, int columns, int w, int least,
+               int ones, Go&& go) {
+    const size_t b_rec = (static_cast<size_t>(K) + static_cast<size_t>(columns) * kLot) * tmem_record_bytes(sizeof(T), NF);
+    key.scalar_bytes = static_cast<int>(sizeof(T));
+    key.n[8] = w;
+    TableRef ref = acquire_table(call, key, b_rec + (static_cast<size_t>(columns) + 1) * sizeof(int32_t));
+    unsigned char* records = static_cast<unsigned char*>(ref.ptr);
+    int32_t* starts = reinterpret_cast<int32_t*>(records + b_rec);
+    if (ref.fresh) {
+        auto build = gather_table<T, NF, Source>;
+        const size_t builder = table_smem(K, columns);
+        allow_dynamic_smem(build, call.device, builder);
+        build<<<1, kTableThreads, builder, call.stream>>>(records, starts, source, static_cast<int>(K), columns, w,
+                                                          kLot, least, ones, call.status);
+        MOPS_CUDA_OK(cudaGetLastError());
+        commit_table(call, ref);
+    }
+    go(static_cast<const unsigned char*>(records), static_cast<const int32_t*>(starts));
+    release_table(call, ref);
+}
+
+template <typename T> TableKey triplet_key(const SapProblem<T>& p, int64_t level) {
+    TableKey key{};
+    key.kind = kSapTable;
+    key.ptr[0] = p.C, key.ptr[1] = p.PA, key.ptr[2] = p.PB, key.ptr[3] = p.PO;
+    key.n[0] = p.K, key.n[1] = p.nA, key.n[2] = p.nB, key.n[3] = p.nO, key.n[4] = level;
+    return key;
+}
+
+// Where a block's shared memory goes; `capacity` records (with the batches fetched ahead).
+inline size_t resident_smem(size_t record_bytes, int capacity, int columns) {
+    return (record_bytes * capacity + 15) / 16 * 16 + (static_cast<size_t>(columns + 1) * 4 + 15) / 16 * 16;
+}
+
+template <typename T, int NF>
+bool forward_resident(const Call& call, const SapProblem<T>& p, T* O, int max_columns) {
+    const int operand_columns = NF == 1 ? p.nA * p.nB : p.nA + p.nB;
+    const size_t limit = static_cast<size_t>(max_optin_smem(call.device)) - 1024;
+    if (table_smem(p.K, p.nO) > limit || !at_16_bytes(O) || p.K > (1 << 14)) return false;
+    Operands op{};
+    op.add(p.A, p.nA);
+    op.add(p.B, p.nB);
+    const int capacity = static_cast<int>(ceil_div(p.K + static_cast<int64_t>(p.nO) * kLot, kLot) + 3) * kLot;
+    for (int w : {4, 2}) {
+        const int rows = kSlabRows * w / words_of(sizeof(T));
+        const int64_t tiles = ceil_div(p.I, static_cast<int64_t>(rows));
+        if (operand_columns + 1 > max_columns / w || tiles < sm_count(call.device)) continue;
+        size_t smem = resident_smem(sizeof(T) + 2 * NF, capacity, p.nO);
+        const ResultStage stage = result_stage<T>(p.nO, rows, smem);
+        smem = (smem + 15) / 16 * 16;
+        const int slabs = static_cast<int>(smem);
+        smem += static_cast<size_t>(w / words_of(sizeof(T))) * op.template slab_bytes<T>();
+        if (smem > limit) continue;
+        note_kernel_f("sap_fwd_resident<%s,NF=%d,W=%d>", scalar_name<T>(), NF, w);
+        const GatherShape shape{w, 1, tiles, smem};
+        auto run = [&](const unsigned char* records, const int32_t* starts) {
+            auto go = [&](auto kernel) {
+                launch_gather(call, kernel, shape, 1, O, op, records, starts, stage, capacity, slabs, p.I, tiles,
+                              call.status);
+            };
+            if (w == 4)
+                go(sap_fwd_resident<T, NF, 4>);
+            else
+                go(sap_fwd_resident<T, NF, 2>);
+        };
+        if constexpr (NF == 1) {
+            with_lots<T, 1>(call, triplet_key(p, -2), ProductSource<T>{p.C, p.PA, p.PB, p.PO, p.nA, p.nB, p.nO}, p.K,
+                            p.nO, w, 1, operand_columns, run);
+        } else {
+            SapSource<T> source{p.C, {p.PA, p.PB, p.PO}, {p.nA, p.nB, p.nO}, static_cast<int>(p.K), {}};
+            source.family[0] = {kO, 0, {kA, kB}, {0, p.nA}};
+            with_lots<T, 2>(call, triplet_key(p, -3), source, p.K, p.nO, w, 1, operand_columns, run);
+        }
+        return true;
+    }
+    return false;
 }
 
 template <typename T>
-bool backward_cells(const Call& call, const SapProblem<T>& p, T* gA, T* gB, const T* gO) {
+bool backward_resident(const Call& call, const SapProblem<T>& p, T* gA, T* gB, const T* gO) {
     const bool b_narrow = p.nB <= p.nA;
     const int nS = b_narrow ? p.nB : p.nA, nT = b_narrow ? p.nA : p.nB, cells = nS * nT;
-    const size_t builder = table_smem(p.K, cells);
-    if (builder > static_cast<size_t>(max_optin_smem(call.device)) - 1024) return false;
+    const size_t limit = static_cast<size_t>(max_optin_smem(call.device)) - 1024;
+    if (table_smem(p.K, cells) > limit || !at_16_bytes(gA) || !at_16_bytes(gB) || p.K > (1 << 14)) return false;
     Operands op{};
     op.add(gO, p.nO);
     op.add(b_narrow ? p.A : p.B, nT);
     op.add(b_narrow ? p.B : p.A, nS);
+    const int64_t padded = p.K + 3 * std::min<int64_t>(p.K, cells);
+    const int capacity = static_cast<int>(ceil_div(padded, kLot) + 3) * kLot;
     // rows per lane: as many as fit and still give every SM a tile
-    int w = 0;
-    int64_t tiles = 0;
-    size_t smem = 0;
-    for (int candidate : {4, 2}) {
-        const int r = candidate / words_of(sizeof(T));
-        tiles = ceil_div(p.I, static_cast<int64_t>(kSlabRows) * r);
-        smem = kStageBytes + (static_cast<size_t>(cells + 1) * 4 + 15) / 16 * 16 +
-               static_cast<size_t>(kTmemGroups) * nS * kSlabRows * r * sizeof(T) +
-               static_cast<size_t>(r) * op.template slab_bytes<T>();
-        if ((op.total + 1) * candidate <= kTmemColumns &&
-            smem <= static_cast<size_t>(max_optin_smem(call.device)) - 1024 &&
-            tiles >= sm_count(call.device)) {
-            w = candidate;
-            break;
-        }
-    }
-    if (w == 0) return false;
-    const int batch = batch_of(1, w);
-    constexpr int RB = tmem_record_bytes(sizeof(T), 1);
-    const size_t b_rec = (static_cast<size_t>(p.K) + static_cast<size_t>(cells) * batch) * RB;
-    TableKey key{};
-    key.kind = kSapTable;
-    key.scalar_bytes = static_cast<int>(sizeof(T));
-    key.ptr[0] = p.C, key.ptr[1] = p.PA, key.ptr[2] = p.PB, key.ptr[3] = p.PO;
-    key.n[0] = p.K, key.n[1] = p.nA, key.n[2] = p.nB, key.n[3] = p.nO, key.n[4] = -1, key.n[8] = w;
-    TableRef ref = acquire_table(call, key, b_rec + (static_cast<size_t>(cells) + 1) * sizeof(int32_t));
-    unsigned char* records = static_cast<unsigned char*>(ref.ptr);
-    int32_t* starts = reinterpret_cast<int32_t*>(records + b_rec);
-    if (ref.fresh) {
-        auto build = gather_table<T, 1, CellSource<T>>;
-        allow_dynamic_smem(build, call.device, builder);
+    for (int w : {4, 2}) {
+        const int rows = kSlabRows * w / words_of(sizeof(T));
+        const int64_t tiles = ceil_div(p.I, static_cast<int64_t>(rows));
+        if (op.total + 1 + kTmemGroups * nS > kTmemColumns / w || tiles < sm_count(call.device)) continue;
+        size_t smem = resident_smem(sizeof(T) + 2, capacity, cells);
+        const ResultStage t_stage = result_stage<T>(nT, rows, smem);
+        smem = (smem + 15) / 16 * 16;
+        const ResultStage s_stage = result_stage<T>(nS, rows, smem);
+        smem = (smem + 15) / 16 * 16;
+        const int slabs = static_cast<int>(smem);
+        smem += static_cast<size_t>(w / words_of(sizeof(T))) * op.template slab_bytes<T>();
+        if (smem > limit) continue;
+        note_kernel_f("sap_vjp_resident<%s,W=%d>", scalar_name<T>(), w);
+        const GatherShape shape{w, 1, tiles, smem};
         const CellSource<T> source{p.C, b_narrow ? p.PA : p.PB, b_narrow ? p.PB : p.PA, p.PO, nT, nS, p.nO,
                                    b_narrow ? 0 : 1, b_narrow ? 1 : 0};
-        build<<<1, kTableThreads, builder, call.stream>>>(records, starts, source, static_cast<int>(p.K),
-                                                          cells, w, batch, 0, op.total, call.status);
-        MOPS_CUDA_OK(cudaGetLastError());
-        commit_table(call, ref);
+        with_lots<T, 1>(call, triplet_key(p, -1), source, p.K, cells, w, 0, op.total,
+                        [&](const unsigned char* records, const int32_t* starts) {
+                            auto go = [&](auto kernel) {
+                                launch_gather(call, kernel, shape, 1, b_narrow ? gA : gB, b_narrow ? gB : gA, op,
+                                              records, starts, t_stage, s_stage, capacity, slabs, p.I, tiles,
+                                              call.status);
+                            };
+                            if (w == 4)
+                                go(sap_vjp_resident<T, 4>);
+                            else
+                                go(sap_vjp_resident<T, 2>);
+                        });
+        return true;
     }
-    note_kernel_f("sap_vjp_cells<%s,W=%d>", scalar_name<T>(), w);
-    const GatherShape shape{w, 1, tiles, smem};
-    auto go = [&](auto kernel) {
-        launch_gather(call, kernel, shape, 1, b_narrow ? gA : gB, b_narrow ? gB : gA, op,
-                      static_cast<const unsigned char*>(records), static_cast<const int32_t*>(starts), p.I,
-                      tiles, call.status);
-    };
-    if (w == 4)
-        go(sap_vjp_cells<T, 4>);
-    else
-        go(sap_vjp_cells<T, 2>);
-    release_table(call, ref);
-    return true;
+    return false;
 }
 
 } // namespace
 
 template <typename T> bool sap_forward_tmem(const Call& call, const SapProblem<T>& p, T* O) {
     if (fills_gpu(call, p.I) && p.K < kForwardTriplets * static_cast<int64_t>(p.nA + p.nB + p.nO)) return false;
+    if (forward_resident<T, 1>(call, p, O, kTmemColumns) || forward_resident<T, 2>(call, p, O, kTmemColumns)) return true;
     Operands op{};
     op.add(p.A, p.nA);
     op.add(p.B, p.nB);
@@ -323,7 +739,7 @@ template <typename T>
 bool sap_backward_tmem(const Call& call, const SapProblem<T>& p, T* gA, T* gB, const T* gO) {
     if (fills_gpu(call, p.I) && p.K < kBackwardTriplets * static_cast<int64_t>(p.nA + p.nB + p.nO)) return false;
     // Both gradients of a batch with a tile for every SM: by cells.
-    if (gA != nullptr && gB != nullptr && backward_cells(call, p, gA, gB, gO)) return true;
+    if (gA != nullptr && gB != nullptr && backward_resident(call, p, gA, gB, gO)) return true;
     Operands op{};
     Results<T> results{};
     Family f[2];

@@ -90,6 +90,9 @@ __device__ __forceinline__ void tmem_store(uint32_t a, double v) {
                  : "memory");
 }
 // N consecutive columns.
+__device__ __forceinline__ void tmem_store(uint32_t a, const uint32_t (&r)[2]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1,%2};\n" ::"r"(a), "r"(r[0]), "r"(r[1]) : "memory");
+}
 __device__ __forceinline__ void tmem_store(uint32_t a, const uint32_t (&r)[4]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};\n" ::"r"(a),
                  "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3])

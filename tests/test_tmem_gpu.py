@@ -40,6 +40,24 @@ def test_sap(oracle, kw, dtype):
     compare("sap", d, dtype, oracle, second_order=True, what=f"sap {kw}")
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("kw", [
+    dict(I=148 * 256, nA=20, nB=6, nO=64, K=1000),         # result rows of whole 128-byte lines: one copy each
+    dict(I=148 * 512 + 1, nA=16, nB=4, nO=32, K=600),      # f32: four rows per lane
+    dict(I=2 * 148 * 256 + 255, nA=9, nB=14, nO=3, K=400),  # 126 products, few result columns
+    dict(I=148 * 128 + 1, nA=16, nB=8, nO=9, K=500),       # 128 products: by pairs, two or four rows per lane
+    dict(I=40001, nA=1, nB=1, nO=2, K=50),                 # one cell: three warp groups have nothing to do
+    dict(I=40003, nA=7, nB=11, nO=33, K=511),              # odd rows; the last tile ends inside a 16-byte piece
+    dict(I=20011, nA=32, nB=16, nO=100, K=2000),
+])
+def test_sap_resident(oracle, kw, dtype):
+    """Batches that fill the GPU: records and results in shared memory (sap_fwd_resident, sap_vjp_resident)."""
+    d = workloads.sap(**kw)
+    r = np.random.default_rng(7)
+    d["indices_output"] = r.permutation(d["indices_output"])
+    compare("sap", d, dtype, oracle, what=f"sap {kw}")
+
+
 @pytest.mark.parametrize("op,kw", [("hpe", dict(I=300, N=13, J=6400, K=4)), ("hpe", dict(I=20000, N=8, J=2000, K=3)),
                                    ("sap", dict(I=100, nA=32, nB=2, nO=3, K=4100)),
                                    ("sap", dict(I=5000, nA=9, nB=15, nO=2, K=2000))])
