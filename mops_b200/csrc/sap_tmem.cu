@@ -7,9 +7,8 @@
 //   gA2[a]  : C gO[PO] ggB[PB]                   (PA = a)     gB2[b] : C gO[PO] ggA[PA] (PB = b)
 //
 // 2^22 rows, 20 x 6 -> 50, 1000 triplets, f64, against the kernels that gather from shared memory:
-// forward 2.99 -> 1.6 ms, VJP 3.04 -> 2.6 ms (a tile's way in and out takes nearly half of that: the
-// time per triplet is 3 times less). 1000 rows: forward 12 -> 9 us, VJP 39 -> 13 us, second order
-// 109 -> 19 us.
+// forward 2.99 -> 1.17 ms, VJP 3.04 -> 1.67 ms (the second order by gather_sums). 1000 rows: forward 12 -> 9 us,
+// VJP 39 -> 13 us, second order 109 -> 19 us.
 #include "gather_tmem.cuh"
 #include "sap_tmem.hpp"
 
@@ -73,14 +72,16 @@ bool run(const Call& call, const SapProblem<T>& p, const Family* families, int c
 // tiles of a block, and results are collected there, to leave as one bulk copy per tile: the ring, its
 // meetings and the stores of single sectors of the kernels of gather_tmem.cuh cost half of the time of
 // 1000 triplets (2^22 rows, 20 x 6 -> 50, f64: 25 700 clocks per 256 rows in the forward, 11 600 of them
-// whatever the number of triplets; VJP 42 600 and 24 000).
+// whatever the number of triplets; VJP 42 600 and 24 000). Now 19 700 and 10 500, VJP 29 000 and 20 000: forward
+// 1.51 -> 1.17 ms, VJP 2.48 -> 1.67 ms. What bounds them is instruction issue (64 %), then latency with four
+// warps per scheduler: a record takes 7.3 instructions (9.5 clocks) for two rows, 4 clocks of them FP64.
 
 // Records in batches of four, coefficients and 16-bit TMEM columns apart.
 constexpr int kLot = 4;
 template <typename T, int NF, int W> struct Lot {
-    static constexpr int R = W / words_of(sizeof(T)); // rows per lane
     uint32_t v[kLot][NF][W];
 };
+template <typename T, int W> constexpr int kLaneRows = W / words_of(sizeof(T));
 template <typename T, int NF> struct LotRecords {
     T c[kLot];
     uint32_t q[kLot * NF / 2];
@@ -150,11 +151,11 @@ template <typename T, int NF, int W> __device__ __forceinline__ void await(Lot<T
 // Two chains of sums: even and odd records of the batches.
 template <typename T, int NF, int W>
 __device__ __forceinline__ void add_terms(const Lot<T, NF, W>& g, const LotRecords<T, NF>& rec,
-                                          T (&acc)[2][Lot<T, NF, W>::R]) {
+                                          T (&acc)[2][kLaneRows<T, W>]) {
 #pragma unroll
     for (int b = 0; b < kLot; b++)
 #pragma unroll
-        for (int r = 0; r < Lot<T, NF, W>::R; r++) {
+        for (int r = 0; r < kLaneRows<T, W>; r++) {
             T p = rec.c[b];
 #pragma unroll
             for (int k = 0; k + 1 < NF; k++) p *= tmem_value<T>(g.v[b][k], r);
@@ -165,7 +166,7 @@ __device__ __forceinline__ void add_terms(const Lot<T, NF, W>& g, const LotRecor
 // The batches [first, first + count) in order, added to acc; after(i) behind batch i (from 0).
 template <typename T, int NF, int W, typename After>
 __device__ __forceinline__ void walk_lots(const ResidentRecords<T, NF>& records, int first, int count, uint32_t base,
-                                          T (&acc)[2][Lot<T, NF, W>::R], After&& after) {
+                                          T (&acc)[2][kLaneRows<T, W>], After&& after) {
     if (count <= 0) return;
     Lot<T, NF, W> x, y;
     LotRecords<T, NF> rx, ry;
@@ -188,15 +189,21 @@ __device__ __forceinline__ void walk_lots(const ResidentRecords<T, NF>& records,
     await(x);
 }
 
-// Results of a tile in shared memory, rows side by side as in HBM (or 16 bytes further apart, where lanes
-// that store a column would otherwise meet in the same banks: then they leave row by row).
+// Results of a tile in shared memory, rows side by side as in HBM: they leave as one bulk copy. Where the
+// lanes that store a column would meet in the same banks, eight or more of them, rows are 16 bytes further
+// apart and all threads copy them out (a bulk copy per row took 40 clocks each: 2 10^6 rows, 5 x 10 -> 16,
+// 954 triplets, f64, forward: 610 -> 830 us).
 struct ResultStage {
     int columns, stride; // bytes from row to row
     int offset;          // in shared memory
+    template <typename T> __device__ __forceinline__ bool whole() const {
+        return stride == columns * static_cast<int>(sizeof(T));
+    }
 };
 template <typename T> ResultStage result_stage(int columns, int rows, size_t& smem) {
     const int bytes = columns * static_cast<int>(sizeof(T));
-    const bool crowded = bytes % (sizeof(T) == 8 ? 64 : 32) == 0; // more than four lanes to a bank
+    const bool crowded = bytes % (sizeof(T) == 8 ? 64 : 32) == 0;
+    smem = (smem + 15) / 16 * 16;
     ResultStage s{columns, bytes + (crowded ? 16 : 0), static_cast<int>(smem)};
     smem += static_cast<size_t>(rows) * s.stride;
     return s;
@@ -206,32 +213,45 @@ __device__ __forceinline__ void bulk_copy_out(void* global_dst, const void* smem
                  "r"(smem_address(smem_src)), "r"(bytes)
                  : "memory");
 }
-// One warp, when all of the tile's results are there (and fence_results has been called by who wrote them).
+// All threads, when all of the tile's results are there (and fence_results has been called by who wrote
+// them); a barrier has to follow before the next results.
 template <typename T>
 __device__ __forceinline__ void send_results(const ResultStage& s, const unsigned char* smem, T* out, int64_t row0,
-                                             int rows, int lane) {
+                                             int rows, int tid) {
     const int bytes = s.columns * static_cast<int>(sizeof(T));
-    T* dst = out + row0 * s.columns;
+    unsigned char* dst = reinterpret_cast<unsigned char*>(out + row0 * s.columns);
     const unsigned char* src = smem + s.offset;
-    if (s.stride == bytes) {
+    if (s.whole<T>()) {
         const int all = rows * bytes, whole = all & ~15;
-        if (lane == 0 && whole > 0) bulk_copy_out(dst, src, static_cast<unsigned>(whole));
-        const int x = whole + lane * static_cast<int>(sizeof(T));
-        if (x < all) dst[x / sizeof(T)] = *reinterpret_cast<const T*>(src + x);
+        if (tid == 0 && whole > 0) bulk_copy_out(dst, src, static_cast<unsigned>(whole));
+        const int x = whole + tid * static_cast<int>(sizeof(T));
+        if (x < all) *reinterpret_cast<T*>(dst + x) = *reinterpret_cast<const T*>(src + x);
     } else {
-        for (int r = lane; r < rows; r += 32) bulk_copy_out(dst + static_cast<int64_t>(r) * s.columns, src + r * s.stride, bytes);
+        const int per_row = bytes / 16, total = rows * per_row;
+        const int dr = kTmemThreads / per_row, dc = kTmemThreads - dr * per_row;
+        int row = tid / per_row, c = tid - row * per_row;
+        for (int x = tid; x < total; x += kTmemThreads) {
+            *reinterpret_cast<uint4*>(dst + static_cast<int64_t>(x) * 16) =
+                *reinterpret_cast<const uint4*>(src + row * s.stride + c * 16);
+            row += dr;
+            c += dc;
+            if (c >= per_row) {
+                c -= per_row;
+                row++;
+            }
+        }
     }
-    asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
+    if (tid == 0) asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
 }
 __device__ __forceinline__ void fence_results() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
 __device__ __forceinline__ void await_results_read() { asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory"); }
 __device__ __forceinline__ void await_results_sent() { asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory"); }
 
-// The stage may be written again when the copies of the tile before have read it: warp 0, which issued
-// them, says so on a barrier, and every warp waits there before its first result of a tile.
+// The stage may be written again when the copies of the tile before have read it: warp 0, whose first
+// lane issued them, says so on a barrier, and every warp waits there before its first result of a tile.
 struct StageGuard {
     uint64_t* bar;
-    int tile = 0;       // how many tiles this block has begun
+    int tile = 0; // how many tiles this block has begun
     bool passed = false;
     __device__ void begin_tile() { passed = false; }
     __device__ __forceinline__ void pass(int warp, int lane, const Status& st) {
@@ -250,7 +270,9 @@ struct StageGuard {
 };
 
 // ---- forward: by products of operand columns (NF = 1: the records' columns are the cells (a, b) of A x B,
-// whose products are formed once per row on the way into TMEM), where those fit, else by pairs (NF = 2).
+// whose products are formed once per row on the way into TMEM), where those fit, else, f32 only, by pairs
+// (NF = 2; f64 has half the rows per lane here, which gather_sums does not: 10^6 rows, 24 x 11 -> 56, 1321
+// triplets: 520 -> 690 us).
 template <typename T> struct ProductSource {
     const T* C;
     const int32_t *PA, *PB, *PO;
@@ -276,7 +298,7 @@ __global__ void __launch_bounds__(kTmemThreads, 1)
 sap_fwd_resident(T* __restrict__ O, const __grid_constant__ Operands operands, const unsigned char* __restrict__ table,
                  const int32_t* __restrict__ o_start, const ResultStage stage, int capacity, int slab_offset,
                  int64_t I, int64_t tiles, Status st) {
-    constexpr int R = W / words_of(sizeof(T));
+    constexpr int R = kLaneRows<T, W>;
     const int nA = operands.cols[0], nB = operands.cols[1], nO = stage.columns;
     extern __shared__ __align__(16) unsigned char smem[];
     // layout: records | starts [nO + 1] | results | slabs
@@ -316,24 +338,45 @@ sap_fwd_resident(T* __restrict__ O, const __grid_constant__ Operands operands, c
         tmem_fence_before_sync();
         __syncthreads(); // this tile's rows are there, the results of the one before, too
         tmem_fence_after_sync();
-        if (warp == 0 && before >= 0) send_results(stage, smem, O, before, kSlabRows * R, lane);
+        if (before >= 0) send_results(stage, smem, O, before, kSlabRows * R, tid);
         before = tile * (kSlabRows * R);
         const int a_stride = slab_stride(nA * static_cast<int>(sizeof(T)));
         const int b_stride = slab_stride(nB * static_cast<int>(sizeof(T)));
         if constexpr (NF == 1) {
             const unsigned char* a_row = t.slabs + own * a_stride;
             const unsigned char* b_row = t.slabs + kSlabRows * a_stride + own * b_stride;
-            for (int a = group; a < nA; a += kTmemGroups) {
-                T va[R];
+            constexpr int words = words_of(sizeof(T)), kHeld = 8;
+            for (int a0 = group; a0 < nA; a0 += kHeld * kTmemGroups) {
+                T va[kHeld][R];
 #pragma unroll
-                for (int r = 0; r < R; r++) va[r] = reinterpret_cast<const T*>(a_row + r * t.slab)[a];
-                for (int b = 0; b < nB; b++) {
-                    uint32_t w[W];
+                for (int i = 0; i < kHeld; i++)
 #pragma unroll
                     for (int r = 0; r < R; r++)
-                        put_coefficient<T>(w + r * words_of(sizeof(T)),
-                                           va[r] * reinterpret_cast<const T*>(b_row + r * t.slab)[b]);
-                    tmem_store(base + (a * nB + b) * W, w);
+                        if (a0 + i * kTmemGroups < nA)
+                            va[i][r] = reinterpret_cast<const T*>(a_row + r * t.slab)[a0 + i * kTmemGroups];
+                for (int b = 0; b < nB; b += 2) { // (behind an odd last column a row is padded)
+                    T vb[R][2];
+#pragma unroll
+                    for (int r = 0; r < R; r++) load_vec<T, 2>(reinterpret_cast<const T*>(b_row + r * t.slab) + b, vb[r]);
+#pragma unroll
+                    for (int i = 0; i < kHeld; i++) {
+                        const int a = a0 + i * kTmemGroups;
+                        if (a >= nA) break;
+                        uint32_t w[2 * W];
+#pragma unroll
+                        for (int c = 0; c < 2; c++)
+#pragma unroll
+                            for (int r = 0; r < R; r++) put_coefficient<T>(w + c * W + r * words, va[i][r] * vb[r][c]);
+                        const uint32_t at = base + (a * nB + b) * W;
+                        if (b + 1 < nB) {
+                            tmem_store(at, w);
+                        } else {
+                            uint32_t one[W];
+#pragma unroll
+                            for (int j = 0; j < W; j++) one[j] = w[j];
+                            tmem_store(at, one);
+                        }
+                    }
                 }
             }
         } else {
@@ -387,9 +430,9 @@ sap_fwd_resident(T* __restrict__ O, const __grid_constant__ Operands operands, c
     tmem_fence_before_sync();
     __syncthreads();
     tmem_fence_after_sync();
+    if (before >= 0)
+        send_results(stage, smem, O, before, static_cast<int>(min(static_cast<int64_t>(kSlabRows * R), I - before)), tid);
     if (warp == 0) {
-        if (before >= 0)
-            send_results(stage, smem, O, before, static_cast<int>(min(static_cast<int64_t>(kSlabRows * R), I - before)), lane);
         tmem_free(tmem_s, kTmemColumns);
         await_results_sent();
     }
@@ -401,8 +444,10 @@ sap_fwd_resident(T* __restrict__ O, const __grid_constant__ Operands operands, c
 //   X = sum of C gO[PO] over the triplets of the cell:    gT[t] += X S[s],    gS[s] += X T[t],
 //
 // so a triplet costs one gather and one FMA per row instead of two records of two factors. The
-// cells are sorted by t, then s; a warp group owns whole t: gT[t] is summed in registers, gS in TMEM
-// columns that every group has for itself; the groups' sums are added at the end of a tile.
+// cells are sorted by t, then s; a warp group owns whole t. It keeps the X of one t in TMEM columns and takes
+// them from there together, two s at a time (from a cell's end alone the gradients took 75 instructions, a
+// triplet 7); gS is summed in TMEM columns that every group has for itself, which are added at the end
+// of a tile.
 template <typename T> struct CellSource {
     const T* C;
     const int32_t *PT, *PS, *PO;
@@ -429,12 +474,13 @@ sap_vjp_resident(T* __restrict__ gT, T* __restrict__ gS, const __grid_constant__
                  const unsigned char* __restrict__ table, const int32_t* __restrict__ cell_start,
                  const ResultStage t_stage, const ResultStage s_stage, int capacity, int slab_offset, int64_t I,
                  int64_t tiles, Status st) {
-    constexpr int R = W / words_of(sizeof(T));
+    constexpr int R = kLaneRows<T, W>;
     const int nO = operands.cols[0], nT = operands.cols[1], nS = operands.cols[2], cells = nT * nS;
     extern __shared__ __align__(16) unsigned char smem[];
-    // layout: records | starts [cells + 1] | results | slabs
+    // layout: records | starts [cells + 1] | list [cells + 1] | results | slabs
     ResidentRecords<T, 1> records(smem, capacity);
     int32_t* starts = reinterpret_cast<int32_t*>(smem + (records.bytes(capacity) + 15) / 16 * 16);
+    uint4* list = reinterpret_cast<uint4*>(starts + (cells + 4) / 4 * 4);
     __shared__ uint32_t tmem_s;
     __shared__ uint64_t stage_free;
     const int tid = threadIdx.x, lane = tid & 31;
@@ -457,13 +503,34 @@ sap_vjp_resident(T* __restrict__ gT, T* __restrict__ gS, const __grid_constant__
 
     const int t_lo = uniform(group_column(starts, nT, nS, group, kTmemGroups));
     const int t_hi = uniform(group_column(starts, nT, nS, group + 1, kTmemGroups));
-    const int c_hi = t_hi * nS;
-    const int first = uniform(starts[t_lo * nS]) / kLot, count = uniform(starts[c_hi]) / kLot - first;
+    const int c_lo = t_lo * nS, c_hi = t_hi * nS;
+    const int first = uniform(starts[c_lo]) / kLot, count = uniform(starts[c_hi]) / kLot - first;
+    // The group's columns behind the operands and the column of ones: X [s], sums of gS [s], for an even
+    // number of s.
+    const int pairs = (nS + 1) / 2, group_columns = (operands.total + 1 + group * 4 * pairs) * W;
+    // Its cells that have records: batches, whether the last one of its t; column of X, t; which s t has.
+    if ((warp & 3) == 0) {
+        int n = 0;
+        for (int c0 = c_lo; c0 < c_hi; c0 += 32) {
+            const int c = c0 + lane, t = c / nS, s = c - t * nS;
+            const int batches = c < c_hi ? (starts[c + 1] - starts[c]) / kLot : 0;
+            const unsigned some = __ballot_sync(kFullMask, batches > 0);
+            if (batches > 0)
+            {
+                uint32_t present = 0;
+                for (int s2 = 0; s2 < nS; s2++)
+                    present |= starts[t * nS + s2 + 1] > starts[t * nS + s2] ? 1u << s2 : 0u;
+                list[c_lo + n + __popc(some & ((1u << lane) - 1))] =
+                    make_uint4(static_cast<uint32_t>(batches) | (starts[c + 1] == starts[(t + 1) * nS] ? 1u << 31 : 0u),
+                               static_cast<uint32_t>(group_columns + s * W) | static_cast<uint32_t>(t) << 16, present, 0u);
+            }
+            n += __popc(some);
+        }
+    }
     const int own = (warp & 3) * 32 + lane;
     unsigned char* own_t = smem + t_stage.offset + own * t_stage.stride;
     unsigned char* own_s = smem + s_stage.offset + own * s_stage.stride;
-    // the groups' sums of gS: [group][s], behind the operands and the column of ones
-    const uint32_t all_sums = base + (operands.total + 1) * W, sums = all_sums + group * nS * W;
+    const uint32_t X = base + group_columns, sums = X + 2 * pairs * W;
     StageGuard guard{&stage_free};
 
     int64_t before = -1;
@@ -472,9 +539,9 @@ sap_vjp_resident(T* __restrict__ gT, T* __restrict__ gS, const __grid_constant__
         tmem_fence_before_sync();
         __syncthreads(); // this tile's rows are there, the results of the one before, too
         tmem_fence_after_sync();
-        if (warp == 0 && before >= 0) {
-            send_results(t_stage, smem, gT, before, kSlabRows * R, lane);
-            send_results(s_stage, smem, gS, before, kSlabRows * R, lane);
+        if (before >= 0) {
+            send_results(t_stage, smem, gT, before, kSlabRows * R, tid);
+            send_results(s_stage, smem, gS, before, kSlabRows * R, tid);
         }
         before = tile * (kSlabRows * R);
         {
@@ -486,10 +553,10 @@ sap_vjp_resident(T* __restrict__ gT, T* __restrict__ gS, const __grid_constant__
                 src += kSlabRows * stride;
                 column += operands.cols[q] * W;
             }
-            uint32_t zero[W];
+            uint32_t zeros[2 * W];
 #pragma unroll
-            for (int i = 0; i < W; i++) zero[i] = 0;
-            for (int s = 0; s < nS; s++) tmem_store(sums + s * W, zero);
+            for (int i = 0; i < 2 * W; i++) zeros[i] = 0;
+            for (int s = 0; s < nS; s += 2) tmem_store(sums + s * W, zeros);
         }
         tmem_wait_store();
         tmem_fence_before_sync();
@@ -499,61 +566,72 @@ sap_vjp_resident(T* __restrict__ gT, T* __restrict__ gS, const __grid_constant__
 
         guard.begin_tile();
         if (t_lo == t_hi) guard.pass(warp, lane, st);
-        T acc[2][R], sum_t[R];
+        auto keep_t = [&](int t, const T (&v)[R]) {
+            guard.pass(warp, lane, st);
 #pragma unroll
-        for (int r = 0; r < R; r++) acc[0][r] = acc[1][r] = sum_t[r] = T(0);
-        int t = t_lo, s = 0, c = t_lo * nS;
-        uint32_t value_t[W];
-        auto load_t = [&] { // T[t] of the lane's rows
+            for (int r = 0; r < R; r++) reinterpret_cast<T*>(own_t + r * kSlabRows * t_stage.stride)[t] = v[r];
+        };
+        T acc[2][R];
+#pragma unroll
+        for (int r = 0; r < R; r++) acc[0][r] = acc[1][r] = T(0);
+        for (int t = t_lo; t < t_hi; t++)
+            if (starts[t * nS] == starts[(t + 1) * nS]) keep_t(t, acc[0]); // zeros
+        // gT[t], and t's part of gS
+        auto end_t = [&](int t, uint32_t present) {
+            uint32_t value_t[W];
+            T sum_t[R];
+#pragma unroll
+            for (int r = 0; r < R; r++) sum_t[r] = T(0);
+            tmem_wait_store(); // (X)
             tmem_load(base + (nO + t) * W, value_t);
-            tmem_wait_load();
-            tmem_pin(value_t);
-        };
-        // Moves on to the next cell that has records (or to the end), keeping gT[t] on the way.
-        // Returns its number of batches.
-        auto next_cell = [&](bool moved) {
-            for (; c < c_hi; moved = true) {
-                if (moved) {
-                    c++;
-                    if (++s == nS) {
-                        guard.pass(warp, lane, st);
-#pragma unroll
-                        for (int r = 0; r < R; r++) {
-                            reinterpret_cast<T*>(own_t + r * kSlabRows * t_stage.stride)[t] = sum_t[r];
-                            sum_t[r] = T(0);
-                        }
-                        s = 0;
-                        t++;
-                        if (t < t_hi) load_t();
-                    }
-                    if (c == c_hi) break;
-                }
-                const int n = uniform(starts[c + 1] - starts[c]) / kLot;
-                if (n > 0) return n;
-            }
-            return -1;
-        };
-        if (t < t_hi) load_t();
-        int left = next_cell(false);
-        walk_lots<T, 1, W>(records, first, count, base, acc, [&](int) {
-            if (--left == 0) {
-                uint32_t value_s[W], sum_s[W];
-                tmem_wait_store(); // (the sum that was stored last may be this one)
+#pragma unroll 1
+            for (int s = 0; s < nS; s += 2, present >>= 2) {
+                uint32_t x[2 * W], value_s[2 * W], sum_s[2 * W];
+                tmem_load(X + s * W, x);
                 tmem_load(base + (nO + nT + s) * W, value_s);
                 tmem_load(sums + s * W, sum_s);
                 tmem_wait_load();
+                tmem_pin(value_t);
+                tmem_pin(x);
                 tmem_pin(value_s);
                 tmem_pin(sum_s);
 #pragma unroll
-                for (int r = 0; r < R; r++) {
-                    const T x = acc[0][r] + acc[1][r];
-                    sum_t[r] += x * tmem_value<T>(value_s, r);
-                    put_coefficient<T>(sum_s + r * words_of(sizeof(T)),
-                                       tmem_value<T>(sum_s, r) + x * tmem_value<T>(value_t, r));
-                    acc[0][r] = acc[1][r] = T(0);
+                for (int c = 0; c < 2; c++) {
+                    if (!(present >> c & 1)) continue; // (no such cell: its X is an older one)
+#pragma unroll
+                    for (int r = 0; r < R; r++) {
+                        const int i = c * R + r;
+                        const T v = tmem_value<T>(x, i);
+                        sum_t[r] += v * tmem_value<T>(value_s, i);
+                        put_coefficient<T>(sum_s + i * words_of(sizeof(T)),
+                                           tmem_value<T>(sum_s, i) + v * tmem_value<T>(value_t, r));
+                    }
                 }
                 tmem_store(sums + s * W, sum_s);
-                left = next_cell(true);
+            }
+            keep_t(t, sum_t);
+        };
+        const uint4* next = list + c_lo;
+        uint4 cell = make_uint4(0u, 0u, 0u, 0u), ahead = count > 0 ? *next++ : cell;
+        int left = 0, batches_left = count;
+        auto next_cell = [&] {
+            cell.x = uniform(ahead.x), cell.y = uniform(ahead.y), cell.z = uniform(ahead.z);
+            left = cell.x & 0x7fffffff;
+            ahead = *next++; // (behind the list: not used)
+        };
+        if (count > 0) next_cell();
+        walk_lots<T, 1, W>(records, first, count, base, acc, [&](int) {
+            batches_left--;
+            if (--left == 0) {
+                uint32_t x[W];
+#pragma unroll
+                for (int r = 0; r < R; r++) {
+                    put_coefficient<T>(x + r * words_of(sizeof(T)), acc[0][r] + acc[1][r]);
+                    acc[0][r] = acc[1][r] = T(0);
+                }
+                tmem_store(__byte_perm(cell.y, base, 0x7610), x);
+                if (cell.x >> 31) end_t(static_cast<int>(cell.y >> 16), cell.z);
+                if (batches_left > 0) next_cell();
             }
         });
         guard.tile++;
@@ -565,7 +643,8 @@ sap_vjp_resident(T* __restrict__ gT, T* __restrict__ gS, const __grid_constant__
         for (int s2 = group; s2 < nS; s2 += kTmemGroups) {
             uint32_t part[kTmemGroups][W];
 #pragma unroll
-            for (int g = 0; g < kTmemGroups; g++) tmem_load(all_sums + (g * nS + s2) * W, part[g]);
+            for (int g = 0; g < kTmemGroups; g++)
+                tmem_load(base + (operands.total + 1 + (4 * g + 2) * pairs + s2) * W, part[g]);
             tmem_wait_load();
 #pragma unroll
             for (int g = 0; g < kTmemGroups; g++) tmem_pin(part[g]);
@@ -581,12 +660,12 @@ sap_vjp_resident(T* __restrict__ gT, T* __restrict__ gS, const __grid_constant__
     tmem_fence_before_sync();
     __syncthreads();
     tmem_fence_after_sync();
+    if (before >= 0) {
+        const int rows = static_cast<int>(min(static_cast<int64_t>(kSlabRows * R), I - before));
+        send_results(t_stage, smem, gT, before, rows, tid);
+        send_results(s_stage, smem, gS, before, rows, tid);
+    }
     if (warp == 0) {
-        if (before >= 0) {
-            const int rows = static_cast<int>(min(static_cast<int64_t>(kSlabRows * R), I - before));
-            send_results(t_stage, smem, gT, before, rows, lane);
-            send_results(s_stage, smem, gS, before, rows, lane);
-        }
         tmem_free(tmem_s, kTmemColumns);
         await_results_sent();
     }
@@ -632,10 +711,12 @@ inline size_t resident_smem(size_t record_bytes, int capacity, int columns) {
 }
 
 template <typename T, int NF>
-bool forward_resident(const Call& call, const SapProblem<T>& p, T* O, int max_columns) {
+bool forward_resident(const Call& call, const SapProblem<T>& p, T* O) {
     const int operand_columns = NF == 1 ? p.nA * p.nB : p.nA + p.nB;
     const size_t limit = static_cast<size_t>(max_optin_smem(call.device)) - 1024;
     if (table_smem(p.K, p.nO) > limit || !at_16_bytes(O) || p.K > (1 << 14)) return false;
+    // Most products have to be used (3.5 10^6 rows, 25 x 5 -> 5, 141 triplets, f64: 410 -> 440 us).
+    if (NF == 1 && 2 * p.K < 3 * static_cast<int64_t>(operand_columns)) return false;
     Operands op{};
     op.add(p.A, p.nA);
     op.add(p.B, p.nB);
@@ -643,7 +724,7 @@ bool forward_resident(const Call& call, const SapProblem<T>& p, T* O, int max_co
     for (int w : {4, 2}) {
         const int rows = kSlabRows * w / words_of(sizeof(T));
         const int64_t tiles = ceil_div(p.I, static_cast<int64_t>(rows));
-        if (operand_columns + 1 > max_columns / w || tiles < sm_count(call.device)) continue;
+        if (operand_columns + 1 > kTmemColumns / w || tiles < sm_count(call.device)) continue;
         size_t smem = resident_smem(sizeof(T) + 2 * NF, capacity, p.nO);
         const ResultStage stage = result_stage<T>(p.nO, rows, smem);
         smem = (smem + 15) / 16 * 16;
@@ -691,10 +772,9 @@ bool backward_resident(const Call& call, const SapProblem<T>& p, T* gA, T* gB, c
     for (int w : {4, 2}) {
         const int rows = kSlabRows * w / words_of(sizeof(T));
         const int64_t tiles = ceil_div(p.I, static_cast<int64_t>(rows));
-        if (op.total + 1 + kTmemGroups * nS > kTmemColumns / w || tiles < sm_count(call.device)) continue;
-        size_t smem = resident_smem(sizeof(T) + 2, capacity, cells);
+        if (op.total + 1 + kTmemGroups * ((nS + 1) / 2 * 4) > kTmemColumns / w || nS > 32 || tiles < sm_count(call.device)) continue;
+        size_t smem = resident_smem(sizeof(T) + 2, capacity, 5 * cells + 8); // (bounds and list)
         const ResultStage t_stage = result_stage<T>(nT, rows, smem);
-        smem = (smem + 15) / 16 * 16;
         const ResultStage s_stage = result_stage<T>(nS, rows, smem);
         smem = (smem + 15) / 16 * 16;
         const int slabs = static_cast<int>(smem);
@@ -725,7 +805,9 @@ bool backward_resident(const Call& call, const SapProblem<T>& p, T* gA, T* gB, c
 
 template <typename T> bool sap_forward_tmem(const Call& call, const SapProblem<T>& p, T* O) {
     if (fills_gpu(call, p.I) && p.K < kForwardTriplets * static_cast<int64_t>(p.nA + p.nB + p.nO)) return false;
-    if (forward_resident<T, 1>(call, p, O, kTmemColumns) || forward_resident<T, 2>(call, p, O, kTmemColumns)) return true;
+    if (forward_resident<T, 1>(call, p, O)) return true;
+    if constexpr (sizeof(T) == 4)
+        if (forward_resident<T, 2>(call, p, O)) return true;
     Operands op{};
     op.add(p.A, p.nA);
     op.add(p.B, p.nB);
