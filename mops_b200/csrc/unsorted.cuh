@@ -4,8 +4,9 @@
 // ones and return at once when those did the work. Otherwise the entries are sorted by output row
 // first (a counting sort: histogram, scan, scatter) and then processed row by row: every output
 // row is written once, by one warp, and the entries that share a grad_output row are neighbours.
-// 300 000 entries of 16 x 32, f32: forward 735 us with atomics -> 205 us (30 of them the sort), VJP
-// 209 us in the order of the entries -> 30 + 103 us.
+// 300 000 entries of 16 x 32, f32: forward 735 us with atomics -> 165 us (23 of them the sort), VJP
+// 209 us in the order of the entries -> 23 + 103 us. (Calls that wait for the result stream the sorted
+// entries instead: opsa_gathered.cu.)
 #ifndef MOPS_B200_UNSORTED_CUH
 #define MOPS_B200_UNSORTED_CUH
 
@@ -25,7 +26,7 @@ constexpr int64_t kOneBlockWrites = 8192;  // if it does not have more than this
 // Scratch of the sort.
 struct EntrySort {
     int32_t* starts; // [n_rows + 1] first position of every row in `perm`
-    int32_t* cursor; // [n_rows + 1]
+    int32_t* cursor; // [n_rows + 1] entries per row
     int32_t* sums;   // [blocks]
     int32_t* longest; // entries of the longest row, if more than kEvenRow, else 0
     int32_t* perm;   // [J] entries in the order of their rows
@@ -73,7 +74,15 @@ __device__ __forceinline__ int block_scan(int v, int& exclusive, int32_t* warp_s
     return warp_sums[32];
 }
 
-// Out-of-range rows are reported, and left out or (keep_bad) taken for row 0.
+// Out-of-range rows are reported, and left out or (keep_bad) taken for row 0. `starts` and `longest` are complete
+// for every thread when it returns, `perm` behind the next sync.
+//
+// Bounded by the latencies between the grid barriers (about 3 us each), so there are three: up to kHeldEntries
+// per thread the count of a row gives every entry its place in the row (no second round of atomics), and up to
+// kRowsAtOnce rows every block adds up the rows before its own by itself (300 000 entries, 5003 rows:
+// 29 -> 22 us).
+constexpr int kHeldEntries = 8;
+constexpr int64_t kRowsAtOnce = 1 << 14;
 template <typename Sync>
 __device__ __forceinline__ void sort_entries(const EntrySort& s, const int32_t* __restrict__ P, int64_t J,
                                              int64_t n_rows, bool keep_bad, const Status& st, Sync&& sync,
@@ -84,38 +93,56 @@ __device__ __forceinline__ void sort_entries(const EntrySort& s, const int32_t* 
     const int64_t threads = static_cast<int64_t>(gridDim.x) * blockDim.x;
     auto row_of = [&](int64_t j) {
         const int32_t row = __ldg(P + j);
-        return static_cast<uint32_t>(row) < static_cast<uint32_t>(n_rows) ? row : keep_bad ? 0 : -1;
+        const bool good = static_cast<uint32_t>(row) < static_cast<uint32_t>(n_rows);
+        if (!good) report_bad_index(st, bit);
+        return good ? row : keep_bad ? 0 : -1;
     };
-    for (int64_t r = thread; r <= n_rows; r += threads) s.starts[r] = 0;
+    int32_t* const counts = s.cursor;
+    for (int64_t r = thread; r <= n_rows; r += threads) counts[r] = 0;
     if (thread == 0) *s.longest = 0;
     if (threadIdx.x == 0) block_longest = 0;
+    const bool held = J <= kHeldEntries * threads;
+    int row[kHeldEntries], rank[kHeldEntries];
+#pragma unroll
+    for (int q = 0; q < kHeldEntries; q++) {
+        const int64_t j = thread + q * threads;
+        row[q] = held && j < J ? row_of(j) : -1;
+    }
     sync();
-    for (int64_t j = thread; j < J; j += threads) {
-        const int row = row_of(j);
-        if (row >= 0) atomicAdd(s.starts + row, 1);
-        if (static_cast<uint32_t>(__ldg(P + j)) >= static_cast<uint32_t>(n_rows)) report_bad_index(st, bit);
+    if (held) {
+#pragma unroll
+        for (int q = 0; q < kHeldEntries; q++) rank[q] = row[q] >= 0 ? atomicAdd(counts + row[q], 1) : 0;
+    } else {
+        for (int64_t j = thread; j < J; j += threads) {
+            const int r = row_of(j);
+            if (r >= 0) atomicAdd(counts + r, 1);
+        }
     }
     sync();
     // block b scans the rows [b per, (b + 1) per)
     const int64_t per = ceil_div(n_rows, gridDim.x);
     const int64_t lo = blockIdx.x * per < n_rows ? blockIdx.x * per : n_rows;
     const int64_t hi = lo + per < n_rows ? lo + per : n_rows;
-    int mine = 0, unused;
-    for (int64_t r = lo + threadIdx.x; r < hi; r += blockDim.x) mine += s.starts[r];
-    const int total = block_scan(mine, unused, warp_sums);
-    if (threadIdx.x == 0) s.sums[blockIdx.x] = total;
-    sync();
-    int before = 0;
-    for (int b = threadIdx.x; b < static_cast<int>(blockIdx.x); b += blockDim.x) before += s.sums[b];
+    int unused, before = 0;
+    if (n_rows <= kRowsAtOnce) {
+        for (int64_t r = threadIdx.x; r < lo; r += blockDim.x) before += counts[r];
+    } else {
+        int mine = 0;
+        for (int64_t r = lo + threadIdx.x; r < hi; r += blockDim.x) mine += counts[r];
+        const int total = block_scan(mine, unused, warp_sums);
+        if (threadIdx.x == 0) s.sums[blockIdx.x] = total;
+        sync();
+        for (int b = threadIdx.x; b < static_cast<int>(blockIdx.x); b += blockDim.x) before += s.sums[b];
+    }
     int run = block_scan(before, unused, warp_sums);
     int most = 0;
     for (int64_t r0 = lo; r0 < hi; r0 += blockDim.x) {
         const int64_t r = r0 + threadIdx.x;
-        const int v = r < hi ? s.starts[r] : 0;
+        const int v = r < hi ? counts[r] : 0;
         most = max(most, v);
         int exclusive;
         const int all = block_scan(v, exclusive, warp_sums);
-        if (r < hi) s.starts[r] = s.cursor[r] = run + exclusive;
+        if (r < hi) s.starts[r] = run + exclusive;
         run += all;
     }
     most = __reduce_max_sync(kFullMask, most);
@@ -124,11 +151,16 @@ __device__ __forceinline__ void sort_entries(const EntrySort& s, const int32_t* 
     if (threadIdx.x == 0 && block_longest > 0) atomicMax(s.longest, block_longest);
     if (hi == n_rows && (lo < hi || blockIdx.x == 0) && threadIdx.x == 0) s.starts[n_rows] = run;
     sync();
-    for (int64_t j = thread; j < J; j += threads) {
-        const int row = row_of(j);
-        if (row >= 0) s.perm[atomicAdd(s.cursor + row, 1)] = static_cast<int32_t>(j);
+    if (held) {
+#pragma unroll
+        for (int q = 0; q < kHeldEntries; q++)
+            if (row[q] >= 0) s.perm[s.starts[row[q]] + rank[q]] = static_cast<int32_t>(thread + q * threads);
+    } else {
+        for (int64_t j = thread; j < J; j += threads) {
+            const int r = row_of(j);
+            if (r >= 0) s.perm[s.starts[r] + atomicSub(counts + r, 1) - 1] = static_cast<int32_t>(j);
+        }
     }
-    sync();
 }
 
 // The sort alone, for kernels that read `perm`. Where rows are longer than `limit`, `zero` (n words, or
