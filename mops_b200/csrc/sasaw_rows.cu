@@ -91,32 +91,38 @@ template <> struct Pack<float, 2> { // FFMA2: two multiply-adds per instruction
 
 // ---- the dense coupling table D[out][a][c], padded with zeros: `out` is m3 (forward) or m2
 // (gradients), c the other one. A warp per entry of the table, lanes over the coupling entries in a
-// fixed order, so the sums are reproducible.
+// fixed order, so the sums are reproducible. A block turns the coupling's indices into places in the table
+// once, in shared memory (each warp by itself, from global memory: 9.6 us for 729 places and 500 entries).
 template <typename T>
 __global__ void __launch_bounds__(256)
 sasaw_dense_table(T* __restrict__ D, const T* __restrict__ C, const int32_t* __restrict__ M1,
                   const int32_t* __restrict__ M2, const int32_t* __restrict__ M3, int64_t N, int nA, int nW,
                   int nO, bool out_is_m2, int pad_out, int pad_a, int pad_c, Status st) {
+    constexpr int kAtOnce = 1024;
+    __shared__ int32_t places[kAtOnce];
     const int lane = threadIdx.x & 31;
     const int slot = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (slot >= pad_out * pad_a * pad_c) return;
-    const int c = slot % pad_c, a = slot / pad_c % pad_a, o = slot / (pad_c * pad_a);
     T sum = T(0);
-    if (o < (out_is_m2 ? nW : nO) && a < nA && c < (out_is_m2 ? nO : nW)) {
-        const int want2 = out_is_m2 ? o : c, want3 = out_is_m2 ? c : o;
-        for (int64_t n = lane; n < N; n += 32) {
-            int32_t m1 = __ldg(M1 + n), m2 = __ldg(M2 + n), m3 = __ldg(M3 + n);
+    for (int64_t n0 = 0; n0 < N; n0 += kAtOnce) {
+        const int count = N - n0 < kAtOnce ? static_cast<int>(N - n0) : kAtOnce;
+        for (int x = threadIdx.x; x < count; x += blockDim.x) {
+            int32_t m1 = __ldg(M1 + n0 + x), m2 = __ldg(M2 + n0 + x), m3 = __ldg(M3 + n0 + x);
             const bool b1 = clamp_index(m1, nA), b2 = clamp_index(m2, nW), b3 = clamp_index(m3, nO);
-            if (slot == 0) {
+            if (blockIdx.x == 0) {
                 if (b1) report_bad_index(st, kBitM1);
                 if (b2) report_bad_index(st, kBitM2);
                 if (b3) report_bad_index(st, kBitM3);
             }
-            if (m1 == a && m2 == want2 && m3 == want3) sum += __ldg(C + n);
+            places[x] = ((out_is_m2 ? m2 : m3) * pad_a + m1) * pad_c + (out_is_m2 ? m3 : m2);
         }
+        __syncthreads();
+#pragma unroll 4
+        for (int x = lane; x < count; x += 32)
+            if (places[x] == slot) sum += __ldg(C + n0 + x);
+        __syncthreads();
     }
     sum = warp_sum(sum);
-    if (lane == 0) D[slot] = sum;
+    if (lane == 0 && slot < pad_out * pad_a * pad_c) D[slot] = sum;
 }
 
 // ---- walking the edges of a range of rows
@@ -242,7 +248,9 @@ __device__ __forceinline__ void walk_rows(const RowsArgs<T>& g, const Off* __res
     };
     constexpr int64_t kScalar = sizeof(T);
     const unsigned char* g_base = reinterpret_cast<const unsigned char*>(g.G + static_cast<int64_t>(c0) * L + bc);
-    const int64_t g_row = g.nC * (L * kScalar);
+    // (row sizes fit 32 bits, rows_apply: an address is one multiply-add)
+    const int g_row = g.nC * L * static_cast<int>(kScalar), l_row = L * static_cast<int>(kScalar);
+    const int a_size = g.nA * static_cast<int>(kScalar);
     const unsigned char* b_base = reinterpret_cast<const unsigned char*>(g.B + bc);
     const unsigned char* a_base = reinterpret_cast<const unsigned char*>(g.A + lb);
     const unsigned char* g_piece = reinterpret_cast<const unsigned char*>(g.G + static_cast<int64_t>(c0) * L) + lane * 16;
@@ -254,8 +262,8 @@ __device__ __forceinline__ void walk_rows(const RowsArgs<T>& g, const Off* __res
             // the lanes (gradients of 4.2 10^6 edges, f64: 3.05 -> 2.91 ms).
             constexpr int kPieces = Sl::kB / 16, kAll = Sl::kA / 16; // with B
             const unsigned to = ring32 + slot + lane * 16;
-            const unsigned char* g_src = g_piece + r * g_row;
-            const unsigned char* b_src = b_piece + e * (L * kScalar);
+            const unsigned char* g_src = g_piece + static_cast<int64_t>(r) * g_row;
+            const unsigned char* b_src = b_piece + static_cast<int64_t>(e) * l_row;
             if (nc == NC) {
 #pragma unroll
                 for (int i = 0; i < kAll; i += 32) {
@@ -271,13 +279,13 @@ __device__ __forceinline__ void walk_rows(const RowsArgs<T>& g, const Off* __res
             return;
         }
         const unsigned dst = ring32 + slot + lane_off;
-        const unsigned char* src = g_base + r * g_row;
+        const unsigned char* src = g_base + static_cast<int64_t>(r) * g_row;
         if (nc == NC) {
-            cp_async_rows<sizeof(V), kStep, 0, NC>(dst, src, L * kScalar);
+            cp_async_rows<sizeof(V), kStep, 0, NC>(dst, src, l_row);
         } else {
-            for (int c = 0; c < nc; c++) cp_async_at<sizeof(V), 0>(dst + c * kStep, src + c * (L * kScalar));
+            for (int c = 0; c < nc; c++) cp_async_at<sizeof(V), 0>(dst + c * kStep, src + c * l_row);
         }
-        if (valid) cp_async_at<sizeof(V), Sl::kB>(dst, b_base + e * (L * kScalar));
+        if (valid) cp_async_at<sizeof(V), Sl::kB>(dst, b_base + static_cast<int64_t>(e) * l_row);
     };
 
     // the copies: the next step to start
@@ -289,7 +297,7 @@ __device__ __forceinline__ void walk_rows(const RowsArgs<T>& g, const Off* __res
             const int e = __shfl_sync(kFullMask, e0, at), r = __shfl_sync(kFullMask, g0, at);
             copy_edge(slot, e, r);
             if (lb < g.nA)
-                cp_async<sizeof(T)>(ring + slot + Sl::kA + lb * sizeof(T), a_base + e * (g.nA * kScalar));
+                cp_async<sizeof(T)>(ring + slot + Sl::kA + lb * sizeof(T), a_base + static_cast<int64_t>(e) * a_size);
             if (lane == 0) *reinterpret_cast<int*>(ring + slot + Sl::kA + Sl::kRow) = e;
             f_p++;
         } else {
@@ -306,7 +314,7 @@ __device__ __forceinline__ void walk_rows(const RowsArgs<T>& g, const Off* __res
                 const int e = at < 32 ? ea : eb, r = at < 32 ? ra : rb;
                 copy_edge(slot, e, r);
                 unsigned char* a = ring + slot + Sl::kA + sub * Sl::kRow;
-                const unsigned char* a_src = a_base + e * (g.nA * kScalar);
+                const unsigned char* a_src = a_base + static_cast<int64_t>(e) * a_size;
                 for (int x = lb; x < g.nA; x += LP) {
                     if (live)
                         cp_async<sizeof(T)>(a + x * sizeof(T), a_src + (x - lb) * kScalar);
@@ -795,7 +803,7 @@ template <typename T, typename F> void for_shape(const RowsShape<T>& s, F&& f) {
 
 template <typename T> bool rows_apply(const SasawProblem<T>& p) {
     return p.nA >= 1 && p.nA <= kWidest && p.nW >= 1 && p.nW <= kWidest && p.nO >= 1 && p.nO <= kWidest &&
-           p.L >= 1 && p.E >= 1 && positions_fit_int(p.E) && p.rows >= 1 && p.N <= (1 << 20);
+           p.L >= 1 && p.L <= (1 << 20) && p.E >= 1 && positions_fit_int(p.E) && p.rows >= 1 && p.N <= (1 << 20);
 }
 
 // Two columns per lane (f32) from 33 columns on, where every operand allows 8-byte accesses.
