@@ -612,7 +612,9 @@ gather_sums(const __grid_constant__ Results<T> results, const __grid_constant__ 
                 add_terms<T, NF, W>(x, rx, acc);
                 if ((i & (kPerStage - 1)) == kPerStage - 2 && i + 2 < batches)
                     ring.enter_stage((i + 2) / kPerStage, lane, st);
-                fetch<T, NF, W>(rx, ring.template at<B * RB>(i + 2));
+                // (batches i + 2 and i + 3 are neighbours: pairs do not straddle stages)
+                const unsigned char* ahead = ring.template at<B * RB>(i + 2);
+                fetch<T, NF, W>(rx, ahead);
                 await<T, NF, W>(y);
                 issue<T, NF, W>(x, rx, base);
                 add_terms<T, NF, W>(y, ry, acc);
@@ -621,7 +623,7 @@ gather_sums(const __grid_constant__ Results<T> results, const __grid_constant__ 
                     close();
                     left = n < n_hi ? uniform(starts[n + 1] - starts[n]) / (2 * B) : 0;
                 }
-                fetch<T, NF, W>(ry, ring.template at<B * RB>(i + 3));
+                fetch<T, NF, W>(ry, ahead + B * RB);
             }
             await<T, NF, W>(x);
         }

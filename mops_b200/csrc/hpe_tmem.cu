@@ -141,12 +141,13 @@ hpe_fwd_tmem(T* __restrict__ O, const __grid_constant__ Operands operands, const
                 await<T, K, W>(x);
                 issue<T, K, W>(y, ry, base);
                 add_terms<T, K, W>(x, rx, acc);
-                fetch<T, K, W>(rx, at(i + 2));
+                const unsigned char* ahead = at(i + 2); // (batch i + 3 comes next: kBatches is even)
+                fetch<T, K, W>(rx, ahead);
                 await<T, K, W>(y);
                 issue<T, K, W>(x, rx, base);
                 add_terms<T, K, W>(y, ry, acc);
                 sum.template piece<B>(i, acc);
-                fetch<T, K, W>(ry, at(i + 3));
+                fetch<T, K, W>(ry, ahead + kTmemGroups * (B * RB));
             }
             await<T, K, W>(x); // the loads started last are not used
         }
