@@ -28,8 +28,8 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ARCH + ["-lineinfo", "-O3", "-std=c++17", "-ccbin", HOST_CXX, "-Xcompiler",
                      "-fPIC,-fvisibility=hidden", "--expt-relaxed-constexpr"]
 
-KERNEL_SOURCES = ["runtime.cu", "hpe.cu", "hpe_tmem.cu", "sap.cu", "sap_tmem.cu", "opsa.cu", "sasaw.cu", "sasaw_rows.cu", "sort.cu", "capi.cu",
-                  "host_stubs.cpp"]
+KERNEL_SOURCES = ["runtime.cu", "hpe.cu", "hpe_tmem.cu", "sap.cu", "sap_tmem.cu", "opsa.cu", "opsa_gathered.cu",
+                  "sasaw.cu", "sasaw_rows.cu", "sort.cu", "capi.cu", "host_stubs.cpp"]
 
 
 def _newer(target, deps):

@@ -32,6 +32,7 @@
 #include "bulk.cuh"
 #include "checks.hpp"
 #include "device.cuh"
+#include "opsa_gathered.hpp"
 #include "opsa_small.cuh"
 #include "unsorted.cuh"
 
@@ -472,19 +473,6 @@ void launch_fwd_mma_l(int L, unsigned blocks, cudaStream_t stream, Args... args)
 }
 
 // ------------------------------------------------------------- streaming kernels, host side
-template <typename T, bool WEIGHTED>
-bool pipe_usable(const T* A, const T* B, const T* W, const void* extra, int K, int L) {
-    auto aligned = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
-    if (K < 1 || K > 16 || L < 1 || L > 32) return false;
-    if (!aligned(A) || !aligned(B) || !aligned(extra)) return false;
-    if (WEIGHTED && (!aligned(W) || (L * sizeof(T)) % 16 != 0)) return false;
-    return true;
-}
-
-// Shapes of the weighted operation that have kernels with K and L fixed at compile time:
-// L = 32 columns and K = 9, 13 or 16 (angular channels up to l = 4, 6, and (l + 1)^2 for l = 3).
-inline bool fixed_shape(int K, int L) { return L == 32 && (K == 9 || K == 13 || K == 16); }
-
 template <typename T, bool WEIGHTED> PipeLayout choose_pipe_layout(int K, int L, bool vjp) {
     // Measured on B200 (J = 2^24 / E = 2^22): without weights two stages of 32 entries per
     // warp are best for f64 (forward 0.92 ms, VJP 1.60 ms against 0.97 / 1.84 with four stages
@@ -520,7 +508,7 @@ void launch_fwd_pipe_l(const Call& call, const PipeLayout& lay, int64_t nO, Args
     {                                                                                              \
         auto kernel = opsa_fwd_pipe<T, MT, NT_, WEIGHTED>;                                         \
         const unsigned blocks = pipe_grid(call, kernel, smem, nO);                                 \
-        kernel<<<blocks, kPipeWarps * 32, smem, call.stream>>>(args..., lay, call.status);         \
+        kernel<<<blocks, kPipeWarps * 32, smem, call.stream>>>(args..., nullptr, 0, lay, call.status); \
     }
     switch ((lay.L + 7) / 8) {
     case 1: MOPS_B200_CASE(1) break;
@@ -574,7 +562,7 @@ bool forward_pipe(const Call& call, T* O, const T* A, const T* B, const T* W, co
         auto kernel = opsa_fwd_pipe<T, 2, 4, true, K_, 32>;                                        \
         const unsigned blocks = pipe_grid(call, kernel, smem, nO);                                 \
         kernel<<<blocks, kPipeWarps * 32, smem, call.stream>>>(O, A, B, W, PW, offsets, J, nO, nO, \
-                                                               lay, call.status);                 \
+                                                               nullptr, 0, lay, call.status);     \
     }
             switch (K) {
             case 9: MOPS_B200_CASE(9) break;
@@ -603,7 +591,7 @@ void launch_vjp_pipe_l(const Call& call, const PipeLayout& lay, int64_t J, Args.
     {                                                                                              \
         auto kernel = opsa_vjp_pipe<T, KT, LT_, WEIGHTED>;                                         \
         const unsigned blocks = pipe_grid_entries(call, kernel, smem, J, lay.ch);                  \
-        kernel<<<blocks, kPipeWarps * 32, smem, call.stream>>>(args..., lay, call.status);         \
+        kernel<<<blocks, kPipeWarps * 32, smem, call.stream>>>(args..., nullptr, lay, call.status); \
     }
     switch ((lay.L + 7) / 8) {
     case 1: MOPS_B200_CASE(1) break;
@@ -668,7 +656,7 @@ bool backward_pipe(const Call& call, T* gA, T* gB, T* gW, const T* gO, const T* 
         auto kernel = opsa_vjp_pipe<T, (K_ + 3) / 4, 4, true, K_, 32>;                             \
         const unsigned blocks = pipe_grid_entries(call, kernel, smem, J, lay.ch);                  \
         kernel<<<blocks, kPipeWarps * 32, smem, call.stream>>>(gA, gB, gW, gO, A, B, W, PW,        \
-                                                               offsets, J, nO, nO, lay,           \
+                                                               offsets, J, nO, nO, nullptr, lay,  \
                                                                call.status);                      \
     }
             switch (K) {
@@ -759,7 +747,9 @@ void forward(const Call& call, T* O, const T* A, const T* B, const T* W, const i
         // Few products: atomics per entry are done before the sort is (its six grid barriers are 15 us;
         // 2700 entries of 6 x 80: 39 against 56 us, 8800 of 4 x 64: 46 against 57).
         if (need_fallback && positions_fit_int(J) && J * KL > kFewProducts) {
-            launch_fwd_unsorted<T, WEIGHTED>(call, O, A, B, W, PW, P, J, K, L, nO);
+            // (Asynchronous calls, which mostly have nothing to do here, make do with one launch.)
+            if (!call.wait || !opsa_forward_gathered<T, WEIGHTED>(call, O, A, B, W, PW, P, J, K, L, nO))
+                launch_fwd_unsorted<T, WEIGHTED>(call, O, A, B, W, PW, P, J, K, L, nO);
         } else if (need_fallback) {
             zero_if_unsorted<T><<<grid_generic, 256, 0, call.stream>>>(O, nO * KL, call.status);
             opsa_fwd_atomic<T, WEIGHTED><<<grid_generic, 256, 0, call.stream>>>(
@@ -1332,6 +1322,9 @@ void backward(const Call& call, T* gA, T* gB, T* gW, const T* gO, const T* A, co
     // do without: the sort would be one more launch for every call on a sorted index, 3 us each.)
     plan.perm = nullptr;
     void* scratch = nullptr;
+    if (plan.only_if_unsorted && call.wait && positions_fit_int(J) &&
+        opsa_backward_gathered<T, WEIGHTED>(call, gA, gB, gW, gO, A, B, W, PW, P, J, K, L, nO))
+        return;
     if (plan.only_if_unsorted && call.wait && J <= INT32_MAX) {
         const int blocks = sort_blocks(call, J, nO);
         scratch = scratch_alloc(call, entry_sort_bytes(J, nO, blocks));

@@ -25,7 +25,7 @@ struct PipeLayout {
     int ch;       // entries per chunk: a multiple of 4 (at most 32 with weights: a lane per entry)
     int stages;   // chunks in flight per warp + 1: a power of two
     int stages_log2;
-    int a_off, b_off, w_off, pw_off; // byte offsets inside a stage (16-byte aligned)
+    int a_off, b_off, w_off, pw_off, e_off; // byte offsets inside a stage (16-byte aligned)
     int stage_bytes;
     int g_off;    // grad_output ring (VJP): g_slots rows of g_bytes each; unused in the forward
     int g_bytes;
@@ -62,7 +62,7 @@ __device__ __forceinline__ void issue_grad_row(unsigned char* slot, const S* gO,
 }
 
 __host__ __device__ constexpr PipeLayout pipe_layout(size_t s, int K, int L, bool weighted, bool vjp, int ch,
-                                                     int stages, int g_slots = 2) {
+                                                     int stages, int g_slots = 2, bool gathered = false) {
     PipeLayout p{};
     p.K = K, p.L = L;
     p.LP = weighted ? L + 4 : L;
@@ -77,7 +77,8 @@ __host__ __device__ constexpr PipeLayout pipe_layout(size_t s, int K, int L, boo
     p.b_off = round16(static_cast<size_t>(ch) * K * s);
     p.w_off = p.b_off + round16(static_cast<size_t>(ch) * p.LP * s);
     p.pw_off = weighted ? p.w_off + round16(static_cast<size_t>(ch) * p.LP * s) : p.w_off;
-    p.stage_bytes = weighted ? p.pw_off + round16(static_cast<size_t>(ch) * 4) : p.pw_off;
+    p.e_off = weighted ? p.pw_off + round16(static_cast<size_t>(ch) * 4) : p.pw_off;
+    p.stage_bytes = gathered ? p.e_off + round16(static_cast<size_t>(ch) * 4) : p.e_off;
     p.g_bytes = static_cast<int>(static_cast<size_t>(K) * L * s);
     p.g_off = p.stages * p.stage_bytes;
     p.g_slots = g_slots < 2 ? 1 : 2;
@@ -145,6 +146,58 @@ __device__ __forceinline__ void pipe_issue_chunk(const PipeLayout& lay, unsigned
         for (int i = b_bulk / sizeof(S) + lane; i < n * L; i += 32) Bs[i] = B[e0 * L + i];
 }
 
+// The same for entries that are not neighbours in memory (a sorted order of them, e_lane: lane i holds the
+// entry at position e0 + i of it): every row goes by copies of its own, 4 to 16 bytes per lane.
+template <int UNIT>
+__device__ __forceinline__ void gather_rows_units(unsigned char* dst, int dst_stride, const unsigned char* src,
+                                                  int bytes, const int32_t* rows, int n, int lane) {
+    const int per_row = bytes / UNIT, total = n * per_row;
+    const int dr = 32 / per_row, dc = 32 - dr * per_row;
+    int row = lane / per_row, c = lane - row * per_row;
+    for (int x = lane; x < total; x += 32) {
+        const unsigned char* from = src + static_cast<int64_t>(rows[row]) * bytes + c * UNIT;
+        if constexpr (UNIT == 16)
+            lane_copy16(dst + row * dst_stride + c * UNIT, from);
+        else
+            cp_async<UNIT>(dst + row * dst_stride + c * UNIT, from);
+        row += dr;
+        c += dc;
+        if (c >= per_row) {
+            c -= per_row;
+            row++;
+        }
+    }
+}
+__device__ __forceinline__ void gather_rows(unsigned char* dst, int dst_stride, const void* src, int bytes,
+                                            const int32_t* rows, int n, int lane) {
+    const unsigned char* s = static_cast<const unsigned char*>(src);
+    if (bytes % 16 == 0)
+        gather_rows_units<16>(dst, dst_stride, s, bytes, rows, n, lane);
+    else if (bytes % 8 == 0)
+        gather_rows_units<8>(dst, dst_stride, s, bytes, rows, n, lane);
+    else
+        gather_rows_units<4>(dst, dst_stride, s, bytes, rows, n, lane);
+}
+template <typename S, bool WEIGHTED>
+__device__ __forceinline__ void pipe_gather_chunk(const PipeLayout& lay, unsigned char* stage, uint64_t* bar,
+                                                  const S* __restrict__ A, const S* __restrict__ B,
+                                                  const S* __restrict__ W, int n, int32_t e_lane, int32_t pw_lane,
+                                                  int lane) {
+    constexpr int s = sizeof(S);
+    int32_t* es = reinterpret_cast<int32_t*>(stage + lay.e_off);
+    int32_t* pws = reinterpret_cast<int32_t*>(stage + lay.pw_off);
+    if (lane == 0) mbarrier_arrive_expect(bar, 0);
+    if (lane < n) {
+        es[lane] = e_lane;
+        if (WEIGHTED) pws[lane] = pw_lane;
+    }
+    __syncwarp();
+    gather_rows(stage + lay.a_off, lay.K * s, A, lay.K * s, es, n, lane);
+    gather_rows(stage + lay.b_off, lay.LP * s, B, lay.L * s, es, n, lane);
+    if (WEIGHTED) gather_rows(stage + lay.w_off, lay.LP * s, W, lay.L * s, pws, n, lane);
+    lane_copies_arrive(bar);
+}
+
 // State shared by the two kernels: which rows and entries the warp owns, the ring, and the
 // window of segment offsets (32 at a time, one per lane).
 struct PipeWarp {
@@ -175,15 +228,19 @@ __device__ __forceinline__ PipeWarp pipe_partition(const int64_t* __restrict__ o
 // inside a row. One very long row, or fewer rows than warps, still occupies the whole GPU.
 // r0 .. r1 are then the rows the warp's entries fall into (the first and the last one possibly
 // shared with its neighbours).
-__device__ __forceinline__ PipeWarp pipe_partition_entries(const int64_t* __restrict__ offsets,
-                                                           int64_t nO, int ch, int warp) {
+//
+// `segment` > 0: so many entries per warp instead (a multiple of four), so that others know where rows are cut.
+template <typename Off>
+__device__ __forceinline__ PipeWarp pipe_partition_entries(const Off* __restrict__ offsets,
+                                                           int64_t nO, int ch, int warp, int64_t segment = 0) {
     PipeWarp w;
     const int lane = threadIdx.x & 31;
     const int64_t total = static_cast<int64_t>(gridDim.x) * kPipeWarps;
     const int64_t gwarp = static_cast<int64_t>(blockIdx.x) * kPipeWarps + warp;
     const int64_t J = offsets[nO], quads = (J + 3) / 4;
-    const int64_t lo = quads / total * gwarp + quads % total * gwarp / total;
-    const int64_t hi = quads / total * (gwarp + 1) + quads % total * (gwarp + 1) / total;
+    const int64_t lo = segment > 0 ? segment / 4 * gwarp : quads / total * gwarp + quads % total * gwarp / total;
+    const int64_t hi =
+        segment > 0 ? lo + segment / 4 : quads / total * (gwarp + 1) + quads % total * (gwarp + 1) / total;
     w.e_begin = w.e_first = 4 * lo < J ? 4 * lo : J;
     w.e_last = 4 * hi < J ? 4 * hi : J;
     w.r0 = w.r1 = 0;
@@ -208,10 +265,14 @@ __device__ __forceinline__ PipeWarp pipe_partition_entries(const int64_t* __rest
 // the fixed one; lay_rt is then ignored.
 template <bool WEIGHTED> constexpr int kFixedChunk = WEIGHTED ? 8 : 32;
 
-template <typename S, bool WEIGHTED, bool VJP, int KC, int LC>
+// Bounds of the rows: segment_offsets' or, GATHERED, those of the entry sort.
+template <bool GATHERED> using PipeOffset = std::conditional_t<GATHERED, int32_t, int64_t>;
+
+template <typename S, bool WEIGHTED, bool VJP, int KC, int LC, bool GATHERED = false>
 __device__ __forceinline__ PipeLayout fixed_layout_or(const PipeLayout& run_time) {
     if constexpr (KC > 0) {
-        constexpr PipeLayout fixed = pipe_layout(sizeof(S), KC, LC, WEIGHTED, VJP, kFixedChunk<WEIGHTED>, 2);
+        constexpr PipeLayout fixed =
+            pipe_layout(sizeof(S), KC, LC, WEIGHTED, VJP, kFixedChunk<WEIGHTED>, 2, 2, GATHERED);
         PipeLayout lay = fixed;
         // the depth of the grad_output ring is the host's choice: it moves what lies behind it
         lay.g_slots = run_time.g_slots, lay.bar_off = run_time.bar_off, lay.warp_bytes = run_time.warp_bytes;
@@ -221,16 +282,20 @@ __device__ __forceinline__ PipeLayout fixed_layout_or(const PipeLayout& run_time
     }
 }
 
-template <typename S, int MT, int NT, bool WEIGHTED, int KC = 0, int LC = 0>
-__global__ void __launch_bounds__(kPipeWarps * 32, (KC > 0 && WEIGHTED) ? 5 : 4)
+//
+// GATHERED: an index that is not sorted. The positions are those of a sorted order, `perm`, and the warps
+// split them (`segment` each), not the rows: what a warp has of a row that others share it adds to what is
+// there (zeros: zero_cut_rows).
+template <typename S, int MT, int NT, bool WEIGHTED, int KC = 0, int LC = 0, bool GATHERED = false>
+__global__ void __launch_bounds__(kPipeWarps * 32, (KC > 0 && WEIGHTED && !GATHERED) ? 5 : 4)
 opsa_fwd_pipe(S* __restrict__ O, const S* __restrict__ A, const S* __restrict__ B,
               const S* __restrict__ W, const int32_t* __restrict__ PW,
-              const int64_t* __restrict__ offsets, int64_t J, int64_t nO, int64_t nW,
-              PipeLayout lay_rt, Status st) {
+              const PipeOffset<GATHERED>* __restrict__ offsets, int64_t J, int64_t nO, int64_t nW,
+              const int32_t* __restrict__ perm, int64_t segment, PipeLayout lay_rt, Status st) {
     using T = double;
-    const PipeLayout lay = fixed_layout_or<S, WEIGHTED, false, KC, LC>(lay_rt);
+    const PipeLayout lay = fixed_layout_or<S, WEIGHTED, false, KC, LC, GATHERED>(lay_rt);
     extern __shared__ __align__(128) unsigned char pipe_smem[];
-    if (saw_unsorted(st)) return; // the atomic kernel of the same call does the work
+    if (saw_unsorted(st) != GATHERED) return; // another kernel of the same call does the work
     const int lane = threadIdx.x & 31;
     const int warp = __shfl_sync(kFullMask, threadIdx.x >> 5, 0); // uniform for the compiler
     const int qr = lane >> 2, qc = lane & 3;
@@ -238,32 +303,46 @@ opsa_fwd_pipe(S* __restrict__ O, const S* __restrict__ A, const S* __restrict__ 
     unsigned char* area = pipe_smem + static_cast<size_t>(warp) * lay.warp_bytes;
     uint64_t* bars = reinterpret_cast<uint64_t*>(area + lay.bar_off);
     if (lane == 0) {
-        for (int s = 0; s < NS; s++) mbarrier_init(bars + s, WEIGHTED ? 33 : 1);
+        for (int s = 0; s < NS; s++) mbarrier_init(bars + s, WEIGHTED || GATHERED ? 33 : 1);
         mbarrier_init_fence();
     }
     __syncwarp();
-    const PipeWarp w = pipe_partition(offsets, nO, CH, warp);
+    PipeWarp w;
+    if constexpr (GATHERED)
+        w = pipe_partition_entries(offsets, nO, CH, warp, segment);
+    else
+        w = pipe_partition(offsets, nO, CH, warp);
     if (w.r0 >= w.r1) return;
 
-    auto load_pw = [&](int c) -> int32_t {
-        int32_t pw = 0;
+    // Numbers of chunk c, one entry per lane: its entries (GATHERED), their W rows. They are looked at when the
+    // chunk is issued, not here, where a warp would wait for them.
+    auto load_entries = [&](int c) -> int32_t {
         const int64_t e = w.e_first + static_cast<int64_t>(c) * CH + lane;
-        if (WEIGHTED && lane < CH && e < J) {
-            pw = __ldg(PW + e);
-            if (clamp_index(pw, static_cast<int32_t>(nW))) report_bad_index(st, 1);
-        }
-        return pw;
+        return GATHERED && lane < CH && e < w.e_last ? __ldg(perm + e) : 0;
+    };
+    auto load_pw = [&](int c, int32_t entry) -> int32_t {
+        const int64_t e = w.e_first + static_cast<int64_t>(c) * CH + lane;
+        if (!WEIGHTED || lane >= CH || e >= (GATHERED ? w.e_last : J)) return 0;
+        return __ldg(PW + (GATHERED ? entry : e));
     };
     int issued = 0;
-    int32_t pw_reg = load_pw(0);
+    int32_t entries = load_entries(0), entries_next = load_entries(1);
+    int32_t pw_reg = load_pw(0, entries);
     auto issue_next = [&]() {
         if (issued < w.nchunks) {
             const int s = issued & (NS - 1);
-            pipe_issue_chunk<S, WEIGHTED>(lay, area + s * lay.stage_bytes, bars + s, A, B, W,
-                                          w.e_first + static_cast<int64_t>(issued) * CH, J, pw_reg,
-                                          lane);
+            const int64_t e0 = w.e_first + static_cast<int64_t>(issued) * CH;
+            if (WEIGHTED && clamp_index(pw_reg, static_cast<int32_t>(nW))) report_bad_index(st, 1);
+            if constexpr (GATHERED)
+                pipe_gather_chunk<S, WEIGHTED>(lay, area + s * lay.stage_bytes, bars + s, A, B, W,
+                                               static_cast<int>(w.e_last - e0 < CH ? w.e_last - e0 : CH), entries,
+                                               pw_reg, lane);
+            else
+                pipe_issue_chunk<S, WEIGHTED>(lay, area + s * lay.stage_bytes, bars + s, A, B, W, e0, J, pw_reg, lane);
             issued++;
-            if (WEIGHTED && issued < w.nchunks) pw_reg = load_pw(issued);
+            entries = entries_next;
+            pw_reg = load_pw(issued, entries);
+            entries_next = load_entries(issued + 1);
         }
     };
     for (int i = 0; i < NS - 1; i++) issue_next();
@@ -272,7 +351,7 @@ opsa_fwd_pipe(S* __restrict__ O, const S* __restrict__ A, const S* __restrict__ 
     int64_t wbase = w.r0;
     auto load_window = [&](int64_t base) {
         const int64_t i = base + 1 + lane;
-        return offsets[i < nO ? i : nO];
+        return static_cast<int64_t>(offsets[i < nO ? i : nO]);
     };
     int64_t win = load_window(wbase);
     auto row_end = [&](int64_t r) -> int64_t {
@@ -292,9 +371,11 @@ opsa_fwd_pipe(S* __restrict__ O, const S* __restrict__ A, const S* __restrict__ 
     };
     const int64_t rowsize = static_cast<int64_t>(K) * L;
     const bool pair_ok = L % 2 == 0 && reinterpret_cast<uintptr_t>(O) % (2 * sizeof(S)) == 0;
+    const bool first_cut = GATHERED && offsets[w.r0] < w.e_begin, last_cut = GATHERED && offsets[w.r1] > w.e_last;
     // element (mt, nt, h) is O[r, k = 8 mt + qr, l = 8 nt + 2 qc + h]
     auto flush = [&](int64_t r) {
         S* dst = O + r * rowsize;
+        const bool cut = GATHERED && ((first_cut && r == w.r0) || (last_cut && r + 1 == w.r1));
 #pragma unroll
         for (int mt = 0; mt < MT; mt++) {
             const int k = 8 * mt + qr;
@@ -304,7 +385,10 @@ opsa_fwd_pipe(S* __restrict__ O, const S* __restrict__ A, const S* __restrict__ 
                 const int l = 8 * nt + 2 * qc;
                 if (l >= L) continue;
                 S* d2 = dst + k * L + l;
-                if (pair_ok) {
+                if (GATHERED && cut) {
+                    red_add(d2, static_cast<S>(acc[mt][nt][0]));
+                    if (l + 1 < L) red_add(d2 + 1, static_cast<S>(acc[mt][nt][1]));
+                } else if (pair_ok) {
                     typename VecOf<S, 2>::type v2;
                     v2.x = static_cast<S>(acc[mt][nt][0]), v2.y = static_cast<S>(acc[mt][nt][1]);
                     *reinterpret_cast<typename VecOf<S, 2>::type*>(d2) = v2;
@@ -321,14 +405,19 @@ opsa_fwd_pipe(S* __restrict__ O, const S* __restrict__ A, const S* __restrict__ 
     int64_t row = w.r0;
     int e = static_cast<int>(w.e_begin - w.e_first);
     const int e_stop = static_cast<int>(w.e_last - w.e_first);
-    int hi = static_cast<int>(row_end(row) - w.e_first);
+    // (of a row that goes on behind the warp's entries: their end)
+    auto stop_of = [&](int64_t r) {
+        const int end = static_cast<int>(row_end(r) - w.e_first);
+        return GATHERED && end > e_stop ? e_stop : end;
+    };
+    int hi = stop_of(row);
     // Rows whose last entry has been consumed (and rows without entries) are written out.
     auto finish_rows = [&] {
         while (row < w.r1 && e == hi) {
             flush(row);
             clear();
             row++;
-            if (row < w.r1) hi = static_cast<int>(row_end(row) - w.e_first);
+            if (row < w.r1) hi = stop_of(row);
         }
     };
     // which fragment rows (k) and columns (l) of this lane exist
@@ -399,22 +488,22 @@ opsa_fwd_pipe(S* __restrict__ O, const S* __restrict__ A, const S* __restrict__ 
 // (grad_B = X * W, grad_W[PW] += X * B) with gO[r] as the common factor, kept in registers as
 // MMA fragments while the row lasts; entries are the MMA's m dimension, eight per tile.
 // KT = ceil(K / 4), LT8 = ceil(L / 8).
-template <typename S, int KT, int LT8, bool WEIGHTED, int KC = 0, int LC = 0>
+template <typename S, int KT, int LT8, bool WEIGHTED, int KC = 0, int LC = 0, bool GATHERED = false>
 __global__ void __launch_bounds__(kPipeWarps * 32, (KC > 0 && WEIGHTED) ? 4 : 3)
 opsa_vjp_pipe(S* __restrict__ gA, S* __restrict__ gB, S* __restrict__ gW,
               const S* __restrict__ gO, const S* __restrict__ A, const S* __restrict__ B,
               const S* __restrict__ W, const int32_t* __restrict__ PW,
-              const int64_t* __restrict__ offsets, int64_t J, int64_t nO, int64_t nW,
-              PipeLayout lay_rt, Status st) {
+              const PipeOffset<GATHERED>* __restrict__ offsets, int64_t J, int64_t nO, int64_t nW,
+              const int32_t* __restrict__ perm, PipeLayout lay_rt, Status st) {
     using T = double;
-    const PipeLayout lay = fixed_layout_or<S, WEIGHTED, true, KC, LC>(lay_rt);
+    const PipeLayout lay = fixed_layout_or<S, WEIGHTED, true, KC, LC, GATHERED>(lay_rt);
     using S2 = typename VecOf<S, 2>::type;
     constexpr int NTK = (KT + 1) / 2; // 8-wide tiles over K
     constexpr int KSL = 2 * LT8;      // k-steps over L
     constexpr int NTL = LT8;          // 8-wide tiles over L
     constexpr int KSK = KT;           // k-steps over K
     extern __shared__ __align__(128) unsigned char pipe_smem[];
-    if (saw_unsorted(st)) return; // the entry-per-lane kernel of the same call does the work
+    if (saw_unsorted(st) != GATHERED) return; // another kernel of the same call does the work
     const int lane = threadIdx.x & 31;
     const int warp = __shfl_sync(kFullMask, threadIdx.x >> 5, 0);
     const int qr = lane >> 2, qc = lane & 3;
@@ -423,7 +512,7 @@ opsa_vjp_pipe(S* __restrict__ gA, S* __restrict__ gB, S* __restrict__ gW,
     uint64_t* bars = reinterpret_cast<uint64_t*>(area + lay.bar_off);
     uint64_t* gbars = bars + NS;
     if (lane == 0) {
-        for (int s = 0; s < NS; s++) mbarrier_init(bars + s, WEIGHTED ? 33 : 1);
+        for (int s = 0; s < NS; s++) mbarrier_init(bars + s, WEIGHTED || GATHERED ? 33 : 1);
         mbarrier_init(gbars, 1);
         mbarrier_init(gbars + 1, 1);
         mbarrier_init_fence();
@@ -439,25 +528,35 @@ opsa_vjp_pipe(S* __restrict__ gA, S* __restrict__ gB, S* __restrict__ gW,
         return area + lay.g_off + slot * g_slot_bytes + static_cast<int>((r * lay.g_bytes) & 15);
     };
 
-    auto load_pw = [&](int c) -> int32_t {
-        int32_t pw = 0;
+    // Numbers of chunk c, one entry per lane: its entries (GATHERED), their W rows. They are looked at when the
+    // chunk is issued, not here, where a warp would wait for them.
+    auto load_entries = [&](int c) -> int32_t {
         const int64_t e = w.e_first + static_cast<int64_t>(c) * CH + lane;
-        if (WEIGHTED && lane < CH && e < J) {
-            pw = __ldg(PW + e);
-            if (clamp_index(pw, static_cast<int32_t>(nW))) report_bad_index(st, 1);
-        }
-        return pw;
+        return GATHERED && lane < CH && e < w.e_last ? __ldg(perm + e) : 0;
+    };
+    auto load_pw = [&](int c, int32_t entry) -> int32_t {
+        const int64_t e = w.e_first + static_cast<int64_t>(c) * CH + lane;
+        if (!WEIGHTED || lane >= CH || e >= (GATHERED ? w.e_last : J)) return 0;
+        return __ldg(PW + (GATHERED ? entry : e));
     };
     int issued = 0;
-    int32_t pw_reg = load_pw(0);
+    int32_t entries = load_entries(0), entries_next = load_entries(1);
+    int32_t pw_reg = load_pw(0, entries);
     auto issue_next = [&]() {
         if (issued < w.nchunks) {
             const int s = issued & (NS - 1);
-            pipe_issue_chunk<S, WEIGHTED>(lay, area + s * lay.stage_bytes, bars + s, A, B, W,
-                                          w.e_first + static_cast<int64_t>(issued) * CH, J, pw_reg,
-                                          lane);
+            const int64_t e0 = w.e_first + static_cast<int64_t>(issued) * CH;
+            if (WEIGHTED && clamp_index(pw_reg, static_cast<int32_t>(nW))) report_bad_index(st, 1);
+            if constexpr (GATHERED)
+                pipe_gather_chunk<S, WEIGHTED>(lay, area + s * lay.stage_bytes, bars + s, A, B, W,
+                                               static_cast<int>(w.e_last - e0 < CH ? w.e_last - e0 : CH), entries,
+                                               pw_reg, lane);
+            else
+                pipe_issue_chunk<S, WEIGHTED>(lay, area + s * lay.stage_bytes, bars + s, A, B, W, e0, J, pw_reg, lane);
             issued++;
-            if (WEIGHTED && issued < w.nchunks) pw_reg = load_pw(issued);
+            entries = entries_next;
+            pw_reg = load_pw(issued, entries);
+            entries_next = load_entries(issued + 1);
         }
     };
     // grad_output rows r0, r0 + 1, ... go through a ring of two slots
@@ -476,7 +575,7 @@ opsa_vjp_pipe(S* __restrict__ gA, S* __restrict__ gB, S* __restrict__ gW,
     int64_t wbase = w.r0;
     auto load_window = [&](int64_t base) {
         const int64_t i = base + 1 + lane;
-        return offsets[i < nO ? i : nO];
+        return static_cast<int64_t>(offsets[i < nO ? i : nO]);
     };
     int64_t win = load_window(wbase);
     auto row_end = [&](int64_t r) -> int64_t {
@@ -551,6 +650,7 @@ opsa_vjp_pipe(S* __restrict__ gA, S* __restrict__ gB, S* __restrict__ gW,
         const S* Bs = reinterpret_cast<const S*>(stage + lay.b_off);
         const S* Ws = reinterpret_cast<const S*>(stage + lay.w_off);
         const int32_t* pws = reinterpret_cast<const int32_t*>(stage + lay.pw_off);
+        const int32_t* es = reinterpret_cast<const int32_t*>(stage + lay.e_off);
         const int c_hi = c_lo + CH < e_stop ? c_lo + CH : e_stop;
         while (true) {
             next_rows();
@@ -562,7 +662,7 @@ opsa_vjp_pipe(S* __restrict__ gA, S* __restrict__ gB, S* __restrict__ gW,
                 constexpr bool kRagged = decltype(ragged)::value;
                 const int idx = t0 + qr; // this lane's entry of the tile, within the chunk
                 const bool valid = !kRagged || idx < last;
-                const int64_t eg = w.e_first + c_lo + idx;
+                const int64_t eg = !GATHERED ? w.e_first + c_lo + idx : valid ? es[idx] : 0;
                 const S* brow = Bs + idx * LP;
                 const S* wrow_s = Ws + idx * LP;
                 if (want_a) {
@@ -1077,3 +1177,17 @@ opsa_vjp_pipe_tf32(float* __restrict__ gA, float* __restrict__ gB, const float* 
     }
     next_rows();
 }
+
+// ------------------------------------------------------------- host side, shared
+template <typename T, bool WEIGHTED>
+bool pipe_usable(const T* A, const T* B, const T* W, const void* extra, int K, int L) {
+    auto aligned = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
+    if (K < 1 || K > 16 || L < 1 || L > 32) return false;
+    if (!aligned(A) || !aligned(B) || !aligned(extra)) return false;
+    if (WEIGHTED && (!aligned(W) || (L * sizeof(T)) % 16 != 0)) return false;
+    return true;
+}
+
+// Shapes of the weighted operation that have kernels with K and L fixed at compile time:
+// L = 32 columns and K = 9, 13 or 16 (angular channels up to l = 4, 6, and (l + 1)^2 for l = 3).
+inline bool fixed_shape(int K, int L) { return L == 32 && (K == 9 || K == 13 || K == 16); }

@@ -98,3 +98,27 @@ def test_few_and_uneven_rows(oracle, op, kw, rows, dtype):
             assert np.abs(got[k] - want[k]).max() <= 1e-5 * scale, f"{op} {kw} {rows} {k}"
         return
     compare(op, d, dtype, oracle, what=f"{op} {E} {n} {kw} {rows}")
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("E,n,K,L", [(9001, 160, 16, 32), (9003, 5000, 13, 32), (12005, 77, 9, 32), (30011, 900, 8, 16),
+                                     (21001, 300, 9, 20), (70001, 3000, 5, 12), (16007, 1, 7, 28), (3300000, 9, 1, 1)])
+def test_streamed_in_sorted_order(oracle, E, n, K, L, dtype):
+    """The streaming kernels over a sorted order: rows cut by the warps' shares and rows between them, a
+    third of the entries in one row, the last chunk of a share, rows of 4-, 8- and 16-byte pieces."""
+    r = np.random.default_rng(E)
+    for op, d in (("opsa", workloads.opsa(J=E, K=K, L=L, nO=n)), ("opsaw", workloads.opsaw(E=E, K=K, L=L, n=n))):
+        if E > 1000000 and op == "opsaw":
+            continue
+        po = r.permutation(d["indices_output"])
+        po[::3] = n // 2
+        po[0], po[1] = n - 1, 0
+        d["indices_output"] = po.astype(np.int32)
+        t = to_dev(d, dtype)
+        got, want = run_library(op, t), _in_f64(oracle, op, d) if dtype == np.float32 else run_checker(oracle, op, d, dtype)
+        if n > 1 and L * np.dtype(dtype).itemsize % 16 == 0:
+            assert any("gathered" in k for k in _lib.last_kernels())
+        for k in want:  # (sums over thousands of entries: see test_few_and_uneven_rows)
+            scale = np.abs(want[k]).max()
+            tolerance = (1e-12 if dtype == np.float64 else 1e-5) * scale
+            assert np.abs(got[k].astype(np.float64) - want[k]).max() <= tolerance, f"{op} {E} {n} {K}x{L} {k}"
