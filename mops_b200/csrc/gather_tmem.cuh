@@ -602,18 +602,23 @@ gather_sums(const __grid_constant__ Results<T> results, const __grid_constant__ 
             // (a column has an even number of batches: it can only end behind a y, and the code that
             // closes it is there once)
             int left = uniform(starts[n_lo + 1] - starts[n_lo]) / (2 * B); // pairs of column n
+            constexpr int kPairs = kPerStage / 2;                          // of a stage
+            int stage = 0, in_stage = kPairs; // pairs until the batches fetched ahead are the next stage's
             ring.enter_stage(0, lane, st);
-            fetch<T, NF, W>(rx, ring.template at<B * RB>(0));
+            const unsigned char* ahead = ring.template at<B * RB>(0);
+            fetch<T, NF, W>(rx, ahead);
             issue<T, NF, W>(x, rx, base);
-            fetch<T, NF, W>(ry, ring.template at<B * RB>(1));
-            for (int i = 0; i < batches; i += 2) {
+            fetch<T, NF, W>(ry, ahead + B * RB);
+            for (int i = 0;; i += 2) {
                 await<T, NF, W>(x);
                 issue<T, NF, W>(y, ry, base);
                 add_terms<T, NF, W>(x, rx, acc);
-                if ((i & (kPerStage - 1)) == kPerStage - 2 && i + 2 < batches)
-                    ring.enter_stage((i + 2) / kPerStage, lane, st);
-                // (batches i + 2 and i + 3 are neighbours: pairs do not straddle stages)
-                const unsigned char* ahead = ring.template at<B * RB>(i + 2);
+                ahead += 2 * B * RB;
+                if (__builtin_expect(--in_stage == 0, 0)) {
+                    if (i + 2 < batches) ring.enter_stage(++stage, lane, st);
+                    ahead = ring.template at<B * RB>(i + 2);
+                    in_stage = kPairs;
+                }
                 fetch<T, NF, W>(rx, ahead);
                 await<T, NF, W>(y);
                 issue<T, NF, W>(x, rx, base);
@@ -621,7 +626,8 @@ gather_sums(const __grid_constant__ Results<T> results, const __grid_constant__ 
                 sum.template piece<B>(i, acc);
                 if (__builtin_expect(--left == 0, 0)) {
                     close();
-                    left = n < n_hi ? uniform(starts[n + 1] - starts[n]) / (2 * B) : 0;
+                    if (n == n_hi) break; // (the last column ends with the last batch)
+                    left = uniform(starts[n + 1] - starts[n]) / (2 * B);
                 }
                 fetch<T, NF, W>(ry, ahead + B * RB);
             }
