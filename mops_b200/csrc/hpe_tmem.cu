@@ -2,8 +2,8 @@
 // and VJP for operands of up to about 200 (f64) / 250 (f32) columns and any batch size.
 //
 // 2^20 rows, 100 columns, 2000 monomials of order 4, f64, against the kernels that gather from
-// shared memory (hpe.cu), which its pipe bounds: forward 2.32 -> 1.06 ms, VJP 6.84 -> 3.7 ms (FP64
-// pipe 44 % / 39 % busy, issue slots 75 %). 1000 rows: forward 20 -> 12 us, VJP 115 -> 18 us.
+// shared memory (hpe.cu), which its pipe bounds: forward and VJP 9.16 -> 3.95 ms together (instruction issue;
+// about 20 instructions per record of the VJP and two rows). 1000 rows: forward 20 -> 12 us, VJP 115 -> 17 us.
 #include "checks.hpp"
 #include "gather_tmem.cuh"
 #include "hpe_tmem.hpp"

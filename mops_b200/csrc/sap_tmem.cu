@@ -49,9 +49,17 @@ template <typename T> struct SapSource {
     }
 };
 
-// Fewer triplets per column of a large batch than this and the kernels of sap.cu are as fast
-// (measured at 76 columns, f64: the lines cross at about 260 triplets in the forward, 770 in the VJP).
-constexpr int kForwardTriplets = 4, kBackwardTriplets = 10; // per column
+// Large batches: fewer triplets per column than this and the kernels of sap.cu are as fast. Measured over
+// drawn widths, 20 000 to 4 10^6 rows, against them: forward, f64 from one triplet per column on 1.0 to 4 times
+// as fast (f32 0.75 to 1.25 at one, 1.2 to 1.5 from one and a half on); VJP from three on 1.1 to 1.7 times where
+// rows are whole 16-byte pieces, else 0.88 to 0.98 at three to five (their copies are 4 or 8 bytes each).
+template <typename T> bool few_forward_triplets(const SapProblem<T>& p) {
+    return 2 * p.K < (sizeof(T) == 8 ? 2 : 3) * static_cast<int64_t>(p.nA + p.nB + p.nO);
+}
+template <typename T> bool few_backward_triplets(const SapProblem<T>& p) {
+    const bool pieces = (p.nA | p.nB | p.nO) * static_cast<int>(sizeof(T)) % 16 == 0;
+    return p.K < (pieces ? 3 : 5) * static_cast<int64_t>(p.nA + p.nB + p.nO);
+}
 
 template <typename T>
 bool run(const Call& call, const SapProblem<T>& p, const Family* families, int count, const Operands& op,
@@ -717,6 +725,8 @@ bool forward_resident(const Call& call, const SapProblem<T>& p, T* O) {
     if (table_smem(p.K, p.nO) > limit || !at_16_bytes(O) || p.K > (1 << 14)) return false;
     // Most products have to be used (3.5 10^6 rows, 25 x 5 -> 5, 141 triplets, f64: 410 -> 440 us).
     if (NF == 1 && 2 * p.K < 3 * static_cast<int64_t>(operand_columns)) return false;
+    // f64, products for one row per lane only: 130 000 rows, 14 x 10 -> 8, 254 triplets: 34 -> 38 us.
+    if (NF == 1 && sizeof(T) == 8 && operand_columns + 1 > kTmemColumns / 4) return false;
     Operands op{};
     op.add(p.A, p.nA);
     op.add(p.B, p.nB);
@@ -804,7 +814,7 @@ bool backward_resident(const Call& call, const SapProblem<T>& p, T* gA, T* gB, c
 } // namespace
 
 template <typename T> bool sap_forward_tmem(const Call& call, const SapProblem<T>& p, T* O) {
-    if (fills_gpu(call, p.I) && p.K < kForwardTriplets * static_cast<int64_t>(p.nA + p.nB + p.nO)) return false;
+    if (fills_gpu(call, p.I) && few_forward_triplets(p)) return false;
     if (forward_resident<T, 1>(call, p, O)) return true;
     if constexpr (sizeof(T) == 4)
         if (forward_resident<T, 2>(call, p, O)) return true;
@@ -819,7 +829,7 @@ template <typename T> bool sap_forward_tmem(const Call& call, const SapProblem<T
 
 template <typename T>
 bool sap_backward_tmem(const Call& call, const SapProblem<T>& p, T* gA, T* gB, const T* gO) {
-    if (fills_gpu(call, p.I) && p.K < kBackwardTriplets * static_cast<int64_t>(p.nA + p.nB + p.nO)) return false;
+    if (fills_gpu(call, p.I) && few_backward_triplets(p)) return false;
     // Both gradients of a batch with a tile for every SM: by cells.
     if (gA != nullptr && gB != nullptr && backward_resident(call, p, gA, gB, gO)) return true;
     Operands op{};
