@@ -156,23 +156,23 @@ template <typename T, int NF, int W> __device__ __forceinline__ void await(Lot<T
 #pragma unroll
         for (int k = 0; k < NF; k++) tmem_pin(g.v[b][k]);
 }
-// Two chains of sums: even and odd records of the batches.
-template <typename T, int NF, int W>
+// CHAINS = 2: two chains of sums, even and odd records of the batches.
+template <int CHAINS, typename T, int NF, int W>
 __device__ __forceinline__ void add_terms(const Lot<T, NF, W>& g, const LotRecords<T, NF>& rec,
                                           T (&acc)[2][kLaneRows<T, W>]) {
 #pragma unroll
     for (int b = 0; b < kLot; b++)
 #pragma unroll
         for (int r = 0; r < kLaneRows<T, W>; r++) {
-            T p = rec.c[b];
+            T p = tmem_value<T>(g.v[b][0], r);
 #pragma unroll
-            for (int k = 0; k + 1 < NF; k++) p *= tmem_value<T>(g.v[b][k], r);
-            acc[b & 1][r] += p * tmem_value<T>(g.v[b][NF - 1], r);
+            for (int k = 1; k < NF; k++) p *= tmem_value<T>(g.v[b][k], r);
+            acc[b & (CHAINS - 1)][r] += rec.c[b] * p;
         }
 }
 
 // The batches [first, first + count) in order, added to acc; after(i) behind batch i (from 0).
-template <typename T, int NF, int W, typename After>
+template <int CHAINS, typename T, int NF, int W, typename After>
 __device__ __forceinline__ void walk_lots(const ResidentRecords<T, NF>& records, int first, int count, uint32_t base,
                                           T (&acc)[2][kLaneRows<T, W>], After&& after) {
     if (count <= 0) return;
@@ -185,12 +185,12 @@ __device__ __forceinline__ void walk_lots(const ResidentRecords<T, NF>& records,
     for (int i = 0; i < count; i += 2) {
         await(x);
         issue(y, ry, base);
-        add_terms(x, rx, acc);
+        add_terms<CHAINS>(x, rx, acc);
         records.fetch(rx, first + i + 2);
         after(i);
         await(y);
         issue(x, rx, base);
-        add_terms(y, ry, acc); // (an odd count's last batch is not the group's: everything is closed by then)
+        add_terms<CHAINS>(y, ry, acc); // (an odd count's last batch is not the group's: everything is closed by then)
         records.fetch(ry, first + i + 3);
         after(i + 1);
     }
@@ -405,7 +405,8 @@ sap_fwd_resident(T* __restrict__ O, const __grid_constant__ Operands operands, c
 #pragma unroll
         for (int r = 0; r < R; r++) acc[0][r] = acc[1][r] = T(0);
         int n = n_lo, left = n_lo < n_hi ? uniform(starts[n_lo + 1] - starts[n_lo]) / kLot : 0;
-        walk_lots<T, NF, W>(records, first, count, base, acc, [&](int i) {
+        // f64: one chain, in the order of gather_sums, so that a row's results do not depend on the batch
+        walk_lots<sizeof(T) == 8 ? 1 : 2, T, NF, W>(records, first, count, base, acc, [&](int i) {
             if constexpr (sizeof(T) == 4) { // (PieceSum: pieces of 32 records)
                 if ((i & (kPieceRecords / kLot - 1)) == kPieceRecords / kLot - 1) {
 #pragma unroll
@@ -628,7 +629,7 @@ sap_vjp_resident(T* __restrict__ gT, T* __restrict__ gS, const __grid_constant__
             ahead = *next++; // (behind the list: not used)
         };
         if (count > 0) next_cell();
-        walk_lots<T, 1, W>(records, first, count, base, acc, [&](int) {
+        walk_lots<2, T, 1, W>(records, first, count, base, acc, [&](int) {
             batches_left--;
             if (--left == 0) {
                 uint32_t x[W];
