@@ -122,3 +122,52 @@ def test_streamed_in_sorted_order(oracle, E, n, K, L, dtype):
             scale = np.abs(want[k]).max()
             tolerance = (1e-12 if dtype == np.float64 else 1e-5) * scale
             assert np.abs(got[k].astype(np.float64) - want[k]).max() <= tolerance, f"{op} {E} {n} {K}x{L} {k}"
+
+
+def _with_a_gap(op, E, n, K, L):
+    """Entries in the first and the last hundred of n rows, in no order, and none between them."""
+    d = workloads.opsa(J=E, K=K, L=L, nO=n) if op == "opsa" else workloads.opsaw(E=E, K=K, L=L, n=n)
+    r = np.random.default_rng(E)
+    rows = r.integers(0, 200, E)
+    d["indices_output"] = np.where(rows < 100, rows, n - 200 + rows).astype(np.int32)
+    return d
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("op", ["opsa", "opsaw"])
+@pytest.mark.parametrize("E,n,K,L", [(70001, 30001, 5, 12), (9001, 3000, 13, 32), (9002, 231, 16, 32)])
+def test_rows_without_entries_in_between(oracle, op, E, n, K, L, dtype):
+    d = _with_a_gap(op, E, n, K, L)
+    got = run_library(op, to_dev(d, dtype))
+    assert any("gathered" in k for k in _lib.last_kernels())
+    want = _in_f64(oracle, op, d) if dtype == np.float32 else run_checker(oracle, op, d, dtype)
+    for k in want:  # (sums over hundreds of entries: see test_few_and_uneven_rows)
+        tolerance = (1e-12 if dtype == np.float64 else 1e-5) * np.abs(want[k]).max()
+        assert np.abs(got[k].astype(np.float64) - want[k]).max() <= tolerance, k
+
+
+@pytest.mark.parametrize("op", ["opsa", "opsaw"])
+def test_rows_without_entries_take_no_time_of_their_own(op):
+    """300 000 entries with 199 800 empty rows between them, against the same entries in 200 rows: the whole
+    GPU clears the rows (7 us); a warp that walks over them one by one needs 40 ms."""
+    import torch
+
+    def time(d):
+        t = to_dev(d, np.float32)
+        calls = []
+        for _ in range(6):
+            start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            start.record()
+            run_library(op, t, to_host=False)
+            end.record()
+            end.synchronize()
+            calls.append(start.elapsed_time(end))
+        return min(calls)
+
+    d = _with_a_gap(op, 300000, 200000, 5, 12)
+    few = dict(d, indices_output=np.where(d["indices_output"] < 100, d["indices_output"],
+                                          d["indices_output"] - 199800).astype(np.int32))
+    if op == "opsa":
+        few["output_size"] = 200
+        few["grad_output"] = np.concatenate([d["grad_output"][:100], d["grad_output"][-100:]])
+    assert time(d) < 5 * time(few)
