@@ -2,7 +2,7 @@
 // order of the entries. A, B and W rows are gathered into the same rings by asynchronous copies, so that the
 // latency of the gathers is hidden as in the sorted case; the kernels with a lane per column or entry
 // (unsorted.cuh, opsa_vjp_entries), which wait for eight rows at a time, remain for widths and alignments that
-// cannot be streamed and for asynchronous calls.
+// cannot be streamed, for asynchronous calls, and for gradients of short rows (least_per_row).
 //
 // 300 000 entries of 16 x 32 in 5003 rows, f32, weighted, without the sort: forward 140 -> 33 us, VJP 104 -> 62 us
 // (60 and 245 instructions per entry became 53 and 92).
@@ -44,8 +44,27 @@ template <typename T, bool WEIGHTED> PipeLayout gathered_layout(int K, int L, bo
     return pipe_layout(sizeof(T), K, L, WEIGHTED, vjp, WEIGHTED ? kFixedChunk<true> : 16, 2, 2, true);
 }
 
-// Calls f with a kernel's widths: fixed ones, or tiles that hold K and L.
-template <bool WEIGHTED, typename F> void for_widths(int K, int L, F&& f) {
+// Gradients: entries per output row from which the streaming kernel is the faster one (0: never). It copies a
+// row's grad_output to shared memory and takes its fragments before the first of the row's entries, where
+// opsa_vjp_entries reads it from the caches, so short rows and few products per entry do not pay; f32 pays
+// for FP64 products of operands that move half the bytes. Streaming / entries, 20 000 to 500 000 entries, at
+// the line and one step (a factor of 2 to 4 in entries per row) below it:
+//
+//   f64, K L >= 400          0.50 - 0.95 from 1 on (weighted: 0.71 - 0.94 from 4 on, 0.91 - 1.15 at 2)
+//   f64, 256 <= K L < 400    0.70 - 1.06 from 8 on, 0.85 - 1.12 at 4
+//   f64, 128 <= K L < 256    0.79 - 1.05 from 32 on, 0.81 - 1.11 at 16; fewer products: 0.85 - 1.5 at any length
+//   f32, K L >= 400          0.84 - 0.99 from 32 on, 0.95 - 1.05 at 16
+//   f32, 256 <= K L < 400    0.91 - 1.05 from 64 on, 0.96 - 1.03 at 32; fewer products: 0.9 - 3.2
+//   f32, weighted            fixed widths 0.91 - 1.03 from 16 on, 1.03 - 1.22 at 8; others 1.01 - 3.4
+template <typename T, bool WEIGHTED> int64_t least_per_row(int K, int L) {
+    const int products = K * L;
+    if (sizeof(T) == 4 && WEIGHTED) return fixed_shape(K, L) ? 16 : 0;
+    if (sizeof(T) == 4) return products >= 400 ? 32 : products >= 256 ? 64 : 0;
+    return products >= 400 ? (WEIGHTED ? 4 : 1) : products >= 256 ? 8 : products >= 128 ? 32 : 0;
+}
+
+// Calls f with a kernel's widths: fixed ones, or (TILES) tiles that hold K and L.
+template <bool WEIGHTED, bool TILES, typename F> void for_widths(int K, int L, F&& f) {
     using std::integral_constant;
     if constexpr (WEIGHTED) {
         if (fixed_shape(K, L)) {
@@ -58,16 +77,18 @@ template <bool WEIGHTED, typename F> void for_widths(int K, int L, F&& f) {
             return;
         }
     }
-    auto tiles = [&](auto k) {
-        if (L <= 16)
-            f(k, integral_constant<int, 2>(), integral_constant<int, 0>());
+    if constexpr (TILES) {
+        auto tiles = [&](auto k) {
+            if (L <= 16)
+                f(k, integral_constant<int, 2>(), integral_constant<int, 0>());
+            else
+                f(k, integral_constant<int, 4>(), integral_constant<int, 0>());
+        };
+        if (K <= 8)
+            tiles(integral_constant<int, 8>());
         else
-            f(k, integral_constant<int, 4>(), integral_constant<int, 0>());
-    };
-    if (K <= 8)
-        tiles(integral_constant<int, 8>());
-    else
-        tiles(integral_constant<int, 16>());
+            tiles(integral_constant<int, 16>());
+    }
 }
 
 } // namespace
@@ -79,7 +100,7 @@ bool opsa_forward_gathered(const Call& call, T* O, const T* A, const T* B, const
     const PipeLayout lay = gathered_layout<T, WEIGHTED>(K, L, false);
     const size_t smem = static_cast<size_t>(lay.warp_bytes) * kPipeWarps;
     if (smem > static_cast<size_t>(max_optin_smem(call.device))) return false;
-    for_widths<WEIGHTED>(K, L, [&](auto k, auto nt, auto kc) {
+    for_widths<WEIGHTED, true>(K, L, [&](auto k, auto nt, auto kc) {
         constexpr int MT = (decltype(k)::value + 7) / 8, NT = decltype(nt)::value, KC = decltype(kc)::value;
         auto kernel = opsa_fwd_pipe<T, MT, NT, WEIGHTED, KC, (KC > 0 ? 32 : 0), true>;
         // every warp the same number of positions
@@ -104,6 +125,8 @@ template <typename T, bool WEIGHTED>
 bool opsa_backward_gathered(const Call& call, T* gA, T* gB, T* gW, const T* gO, const T* A, const T* B, const T* W,
                             const int32_t* PW, const int32_t* P, int64_t J, int K, int L, int64_t nO) {
     if (!pipe_usable<T, WEIGHTED>(A, B, W, gO, K, L)) return false;
+    const int64_t least = least_per_row<T, WEIGHTED>(K, L);
+    if (least == 0 || J < least * nO) return false;
     const PipeLayout lay = gathered_layout<T, WEIGHTED>(K, L, true);
     const size_t smem = static_cast<size_t>(lay.warp_bytes) * kPipeWarps;
     if (smem > static_cast<size_t>(max_optin_smem(call.device))) return false;
@@ -112,7 +135,7 @@ bool opsa_backward_gathered(const Call& call, T* gA, T* gB, T* gW, const T* gO, 
     const EntrySort sort = entry_sort_at(scratch, nO, sorters);
     launch_sorting(call, sorters, sort_if_unsorted_grid, sort_if_unsorted_block, sort, P, J, nO,
                    static_cast<uint32_t*>(nullptr), static_cast<int64_t>(0), 0, call.status);
-    for_widths<WEIGHTED>(K, L, [&](auto k, auto lt, auto kc) {
+    for_widths<WEIGHTED, !(sizeof(T) == 4 && WEIGHTED)>(K, L, [&](auto k, auto lt, auto kc) {
         constexpr int KT = (decltype(k)::value + 3) / 4, LT = decltype(lt)::value, KC = decltype(kc)::value;
         auto kernel = opsa_vjp_pipe<T, KT, LT, WEIGHTED, KC, (KC > 0 ? 32 : 0), true>;
         const int64_t held = static_cast<int64_t>(sm_count(call.device)) *

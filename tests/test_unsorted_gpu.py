@@ -8,6 +8,8 @@ from helpers import run_checker, run_library, to_dev
 from mops_b200 import _lib, workloads
 from test_parity_gpu import compare
 
+import mops_b200 as M
+
 pytestmark = pytest.mark.gpu
 
 
@@ -100,6 +102,32 @@ def test_few_and_uneven_rows(oracle, op, kw, rows, dtype):
     compare(op, d, dtype, oracle, what=f"{op} {E} {n} {kw} {rows}")
 
 
+def _streamed(op, t):
+    """Which of the two calls take the streaming kernels over a sorted order: forward, gradients."""
+    if op == "opsa":
+        M.outer_product_scatter_add(t["A"], t["B"], t["indices_output"], t["output_size"])
+    else:
+        M.outer_product_scatter_add_with_weights(t["A"], t["B"], t["W"], t["indices_W"], t["indices_output"])
+    forward = any("gathered" in k for k in _lib.last_kernels())
+    if op == "opsa":
+        M.outer_product_scatter_add_vjp(t["grad_output"], t["A"], t["B"], t["indices_output"])
+    else:
+        M.outer_product_scatter_add_with_weights_vjp(t["grad_output"], t["A"], t["B"], t["W"], t["indices_W"],
+                                                     t["indices_output"])
+    return forward, any("gathered" in k for k in _lib.last_kernels())
+
+
+def _long_rows(op, E, n, K, L, dtype):
+    """Rows for whose gradients the streaming kernels are the faster ones (least_per_row)."""
+    if dtype == np.float32 and op == "opsaw":
+        least = 16 if L == 32 and K in (9, 13, 16) else None
+    elif dtype == np.float32:
+        least = 32 if K * L >= 400 else 64 if K * L >= 256 else None
+    else:
+        least = (4 if op == "opsaw" else 1) if K * L >= 400 else 8 if K * L >= 256 else 32 if K * L >= 128 else None
+    return least is not None and E >= least * n
+
+
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
 @pytest.mark.parametrize("E,n,K,L", [(9001, 160, 16, 32), (9003, 5000, 13, 32), (12005, 77, 9, 32), (30011, 900, 8, 16),
                                      (21001, 300, 9, 20), (70001, 3000, 5, 12), (16007, 1, 7, 28), (3300000, 9, 1, 1)])
@@ -117,7 +145,7 @@ def test_streamed_in_sorted_order(oracle, E, n, K, L, dtype):
         t = to_dev(d, dtype)
         got, want = run_library(op, t), _in_f64(oracle, op, d) if dtype == np.float32 else run_checker(oracle, op, d, dtype)
         if n > 1 and L * np.dtype(dtype).itemsize % 16 == 0:
-            assert any("gathered" in k for k in _lib.last_kernels())
+            assert _streamed(op, t) == (True, _long_rows(op, E, n, K, L, dtype))
         for k in want:  # (sums over thousands of entries: see test_few_and_uneven_rows)
             scale = np.abs(want[k]).max()
             tolerance = (1e-12 if dtype == np.float64 else 1e-5) * scale
@@ -135,11 +163,12 @@ def _with_a_gap(op, E, n, K, L):
 
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
 @pytest.mark.parametrize("op", ["opsa", "opsaw"])
-@pytest.mark.parametrize("E,n,K,L", [(70001, 30001, 5, 12), (9001, 3000, 13, 32), (9002, 231, 16, 32)])
+@pytest.mark.parametrize("E,n,K,L", [(70001, 30001, 5, 12), (70001, 1501, 13, 32), (9002, 231, 16, 32)])
 def test_rows_without_entries_in_between(oracle, op, E, n, K, L, dtype):
     d = _with_a_gap(op, E, n, K, L)
-    got = run_library(op, to_dev(d, dtype))
-    assert any("gathered" in k for k in _lib.last_kernels())
+    t = to_dev(d, dtype)
+    assert _streamed(op, t) == (True, K > 5)
+    got = run_library(op, t)
     want = _in_f64(oracle, op, d) if dtype == np.float32 else run_checker(oracle, op, d, dtype)
     for k in want:  # (sums over hundreds of entries: see test_few_and_uneven_rows)
         tolerance = (1e-12 if dtype == np.float64 else 1e-5) * np.abs(want[k]).max()
@@ -171,3 +200,19 @@ def test_rows_without_entries_take_no_time_of_their_own(op):
         few["output_size"] = 200
         few["grad_output"] = np.concatenate([d["grad_output"][:100], d["grad_output"][-100:]])
     assert time(d) < 5 * time(few)
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("op", ["opsa", "opsaw"])
+@pytest.mark.parametrize("K,L", [(13, 32), (16, 20), (8, 16), (5, 8), (12, 32), (1, 4)])
+@pytest.mark.parametrize("per_row", [1, 5, 17, 40, 70])
+def test_gradients_by_the_lengths_of_rows(oracle, op, K, L, per_row, dtype):
+    """Both sides of the lines between the two gradient kernels. (All rows streamed: 300 000 entries of 1 x 4 in as
+    many rows, f32, took 197 us instead of 72.)"""
+    E = 6007
+    n = E // per_row
+    d = workloads.opsa(J=E, K=K, L=L, nO=n) if op == "opsa" else workloads.opsaw(E=E, K=K, L=L, n=n)
+    d["indices_output"] = np.random.default_rng(1).permutation(d["indices_output"])
+    t = to_dev(d, dtype)
+    assert _streamed(op, t)[1] == _long_rows(op, E, n, K, L, dtype)
+    compare(op, d, dtype, oracle, what=f"{op} {K}x{L} {per_row}")
