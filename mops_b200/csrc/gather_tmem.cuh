@@ -148,14 +148,11 @@ __device__ __forceinline__ void add_terms(const Batch<T, NF, W>& g, const Record
             c = __uint_as_float(rec.w[b][0]);
 #pragma unroll
         for (int r = 0; r < Batch<T, NF, W>::R; r++) {
-            if constexpr (NF == 2) { // (as sap_fwd_resident does it: a row's results do not depend on the batch)
-                acc[r] += c * (tmem_value<T>(g.v[b][0], r) * tmem_value<T>(g.v[b][1], r));
-            } else {
-                T p = c;
+            // (the coefficient first: a product of operands alone may leave the range where the term does not)
+            T p = c;
 #pragma unroll
-                for (int k = 0; k + 1 < NF; k++) p *= tmem_value<T>(g.v[b][k], r);
-                acc[r] += p * tmem_value<T>(g.v[b][NF - 1], r);
-            }
+            for (int k = 0; k + 1 < NF; k++) p *= tmem_value<T>(g.v[b][k], r);
+            acc[r] += p * tmem_value<T>(g.v[b][NF - 1], r);
         }
     }
 }

@@ -164,10 +164,10 @@ __device__ __forceinline__ void add_terms(const Lot<T, NF, W>& g, const LotRecor
     for (int b = 0; b < kLot; b++)
 #pragma unroll
         for (int r = 0; r < kLaneRows<T, W>; r++) {
-            T p = tmem_value<T>(g.v[b][0], r);
+            T p = rec.c[b];
 #pragma unroll
-            for (int k = 1; k < NF; k++) p *= tmem_value<T>(g.v[b][k], r);
-            acc[b & (CHAINS - 1)][r] += rec.c[b] * p;
+            for (int k = 0; k + 1 < NF; k++) p *= tmem_value<T>(g.v[b][k], r);
+            acc[b & (CHAINS - 1)][r] += p * tmem_value<T>(g.v[b][NF - 1], r);
         }
 }
 
@@ -277,10 +277,80 @@ struct StageGuard {
     }
 };
 
+// Exponents of the values of a row that are not zero: whether all products with another row's are normal
+// numbers. (Conservative by one; infinities and NaN come out of c (a b) as they do of (c a) b.)
+template <typename T> struct ExponentRange {
+    static constexpr int kMantissa = sizeof(T) == 8 ? 20 : 23, kBias = sizeof(T) == 8 ? 1023 : 127;
+    uint32_t least = 0xffffffffu, most = 0; // of |v|'s upper word; `least` less one, so that zeros do not count
+    __device__ __forceinline__ void add(T v) {
+        uint32_t word;
+        if constexpr (sizeof(T) == 8) // (a lower word alone makes a value that is not zero)
+            word = (static_cast<uint32_t>(__double2hiint(v)) & 0x7fffffffu) | min(static_cast<uint32_t>(__double2loint(v)), 1u);
+        else
+            word = __float_as_uint(v) & 0x7fffffffu;
+        least = min(least, word - 1);
+        most = max(most, word);
+    }
+    __device__ __forceinline__ bool products_are_normal(const ExponentRange& o) const {
+        if (most == 0 || o.most == 0) return true; // zeros only
+        const int lo = static_cast<int>((least + 1) >> kMantissa), o_lo = static_cast<int>((o.least + 1) >> kMantissa);
+        return lo > 0 && o_lo > 0 && lo + o_lo > kBias + 1 &&
+               static_cast<int>((most >> kMantissa) + (o.most >> kMantissa)) < 3 * kBias;
+    }
+};
+
+// The columns [n_lo, n_hi) of a tile by factors: the records are those of products (NF = 1), but TMEM holds the
+// operands, A's columns, then B's; the coefficient comes first in every term. (`cell / nB` by multiplication is
+// exact up to 256 cells.) A call of its own, so that the loop over products keeps its registers.
+template <typename T, int W>
+__device__ __noinline__ void sum_by_factors(const ResidentRecords<T, 1> records, const int32_t* starts, int n_lo, int n_hi,
+                                            uint32_t base, int nA, int nB, int ones, unsigned char* results, int row_step) {
+    constexpr int R = kLaneRows<T, W>;
+    const uint32_t reciprocal = (65536u + nB - 1) / nB;
+    for (int n = n_lo; n < n_hi; n++) {
+        const int first = uniform(starts[n]) / kLot, end = uniform(starts[n + 1]) / kLot;
+        T sum[R], part[R]; // (PieceSum: f32 in pieces of 32 records)
+#pragma unroll
+        for (int r = 0; r < R; r++) sum[r] = part[r] = T(0);
+        for (int i = first; i < end; i++) {
+            Lot<T, 2, W> g;
+            LotRecords<T, 1> rec;
+            records.fetch(rec, i);
+#pragma unroll
+            for (int b = 0; b < kLot; b++) {
+                const uint32_t cell = ((b & 1) ? rec.q[b / 2] >> 16 : rec.q[b / 2] & 0xffffu) / W, a = cell * reciprocal >> 16;
+                const bool padding = cell == static_cast<uint32_t>(ones);
+                tmem_load(base + (padding ? cell : a) * W, g.v[b][0]);
+                tmem_load(base + (padding ? cell : nA + cell - a * nB) * W, g.v[b][1]);
+            }
+            await(g);
+#pragma unroll
+            for (int b = 0; b < kLot; b++)
+#pragma unroll
+                for (int r = 0; r < R; r++)
+                    part[r] += rec.c[b] * tmem_value<T>(g.v[b][0], r) * tmem_value<T>(g.v[b][1], r);
+            if (sizeof(T) == 4 && ((i - first) & (kPieceRecords / kLot - 1)) == kPieceRecords / kLot - 1) {
+#pragma unroll
+                for (int r = 0; r < R; r++) {
+                    sum[r] += part[r];
+                    part[r] = T(0);
+                }
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < R; r++) reinterpret_cast<T*>(results + r * row_step)[n] = sum[r] + part[r];
+    }
+}
+
 // ---- forward: by products of operand columns (NF = 1: the records' columns are the cells (a, b) of A x B,
 // whose products are formed once per row on the way into TMEM), where those fit, else, f32 only, by pairs
 // (NF = 2; f64 has half the rows per lane here, which gather_sums does not: 10^6 rows, 24 x 11 -> 56, 1321
 // triplets: 520 -> 690 us).
+//
+// A product a b may overflow or lose bits to underflow where the term C a b does neither (f32: C = 1e-30,
+// a = b = 1e25). A tile with a row for which that is possible is done by factors, C a first, as everywhere else.
+// 2^20 rows, 20 x 6 -> 50, 1000 triplets: looking at the operands' exponents makes 305 us 317 (f64) and 198 us
+// 210 (f32); with such a row in every tile it is 640 and 400 (all by gather_sums: 365, 360).
 template <typename T> struct ProductSource {
     const T* C;
     const int32_t *PA, *PB, *PO;
@@ -300,6 +370,11 @@ template <typename T> struct ProductSource {
         return a * nB + b;
     }
 };
+
+// Behind the products (NF = 1) and, for either way of taking them, the operands.
+__host__ __device__ inline int ones_column(int nf, int nA, int nB) {
+    return nf == 1 && nA * nB > nA + nB ? nA * nB : nA + nB;
+}
 
 template <typename T, int NF, int W>
 __global__ void __launch_bounds__(kTmemThreads, 1)
@@ -330,9 +405,9 @@ sap_fwd_resident(T* __restrict__ O, const __grid_constant__ Operands operands, c
     __syncthreads();
     tmem_fence_after_sync();
     const uint32_t base = tmem_quadrant(tmem_s, warp);
-    if (warp < 4) // the column of ones
-        for (int r = 0; r < R; r++)
-            tmem_store(base + (NF == 1 ? nA * nB : nA + nB) * W + r * words_of(sizeof(T)), T(1));
+    const int ones = ones_column(NF, nA, nB);
+    if (warp < 4)
+        for (int r = 0; r < R; r++) tmem_store(base + ones * W + r * words_of(sizeof(T)), T(1));
     const int n_lo = uniform(group_column(starts, nO, 1, group, kTmemGroups));
     const int n_hi = uniform(group_column(starts, nO, 1, group + 1, kTmemGroups));
     const int first = uniform(starts[n_lo]) / kLot, count = uniform(starts[n_hi]) / kLot - first;
@@ -350,10 +425,12 @@ sap_fwd_resident(T* __restrict__ O, const __grid_constant__ Operands operands, c
         before = tile * (kSlabRows * R);
         const int a_stride = slab_stride(nA * static_cast<int>(sizeof(T)));
         const int b_stride = slab_stride(nB * static_cast<int>(sizeof(T)));
+        int out_of_range = 0; // products of this thread's
         if constexpr (NF == 1) {
             const unsigned char* a_row = t.slabs + own * a_stride;
             const unsigned char* b_row = t.slabs + kSlabRows * a_stride + own * b_stride;
             constexpr int words = words_of(sizeof(T)), kHeld = 8;
+            ExponentRange<T> range_a[R], range_b[R];
             for (int a0 = group; a0 < nA; a0 += kHeld * kTmemGroups) {
                 T va[kHeld][R];
 #pragma unroll
@@ -365,11 +442,19 @@ sap_fwd_resident(T* __restrict__ O, const __grid_constant__ Operands operands, c
                 for (int b = 0; b < nB; b += 2) { // (behind an odd last column a row is padded)
                     T vb[R][2];
 #pragma unroll
-                    for (int r = 0; r < R; r++) load_vec<T, 2>(reinterpret_cast<const T*>(b_row + r * t.slab) + b, vb[r]);
+                    for (int r = 0; r < R; r++) {
+                        load_vec<T, 2>(reinterpret_cast<const T*>(b_row + r * t.slab) + b, vb[r]);
+                        if (b + 1 == nB) vb[r][1] = T(0);
+                    }
+#pragma unroll
+                    for (int r = 0; r < R; r++) range_b[r].add(vb[r][0]), range_b[r].add(vb[r][1]);
 #pragma unroll
                     for (int i = 0; i < kHeld; i++) {
                         const int a = a0 + i * kTmemGroups;
                         if (a >= nA) break;
+                        if (b == 0)
+#pragma unroll
+                            for (int r = 0; r < R; r++) range_a[r].add(va[i][r]);
                         uint32_t w[2 * W];
 #pragma unroll
                         for (int c = 0; c < 2; c++)
@@ -387,14 +472,25 @@ sap_fwd_resident(T* __restrict__ O, const __grid_constant__ Operands operands, c
                     }
                 }
             }
+#pragma unroll
+            for (int r = 0; r < R; r++) // (rows behind the last one hold anything)
+                out_of_range |= !range_a[r].products_are_normal(range_b[r]) && before + r * kSlabRows + own < I;
         } else {
             slabs_to_tmem<T, W>(t.slabs, t.slab, a_stride, nA, base, warp, lane);
             slabs_to_tmem<T, W>(t.slabs + kSlabRows * a_stride, t.slab, b_stride, nB, base + nA * W, warp, lane);
         }
         tmem_wait_store();
         tmem_fence_before_sync();
-        __syncthreads();
+        const bool by_factors = uniform(__syncthreads_or(out_of_range)) != 0;
         tmem_fence_after_sync();
+        if (NF == 1 && by_factors) {
+            slabs_to_tmem<T, W>(t.slabs, t.slab, a_stride, nA, base, warp, lane);
+            slabs_to_tmem<T, W>(t.slabs + kSlabRows * a_stride, t.slab, b_stride, nB, base + nA * W, warp, lane);
+            tmem_wait_store();
+            tmem_fence_before_sync();
+            __syncthreads();
+            tmem_fence_after_sync();
+        }
         if (tile + gridDim.x < tiles) t.start(tile + gridDim.x, tid);
 
         guard.begin_tile();
@@ -405,8 +501,7 @@ sap_fwd_resident(T* __restrict__ O, const __grid_constant__ Operands operands, c
 #pragma unroll
         for (int r = 0; r < R; r++) acc[0][r] = acc[1][r] = T(0);
         int n = n_lo, left = n_lo < n_hi ? uniform(starts[n_lo + 1] - starts[n_lo]) / kLot : 0;
-        // f64: one chain, in the order of gather_sums, so that a row's results do not depend on the batch
-        walk_lots<sizeof(T) == 8 ? 1 : 2, T, NF, W>(records, first, count, base, acc, [&](int i) {
+        auto after = [&](int i) {
             if constexpr (sizeof(T) == 4) { // (PieceSum: pieces of 32 records)
                 if ((i & (kPieceRecords / kLot - 1)) == kPieceRecords / kLot - 1) {
 #pragma unroll
@@ -431,7 +526,15 @@ sap_fwd_resident(T* __restrict__ O, const __grid_constant__ Operands operands, c
                 n++;
                 left = n < n_hi ? uniform(starts[n + 1] - starts[n]) / kLot : 0;
             }
-        });
+        };
+        constexpr int kChains = sizeof(T) == 8 ? 1 : 2;
+        if constexpr (NF == 1) {
+            if (by_factors) {
+                guard.pass(warp, lane, st);
+                sum_by_factors<T, W>(records, starts, n_lo, n_hi, base, nA, nB, ones, own_results, kSlabRows * stage.stride);
+            }
+        }
+        walk_lots<kChains, T, NF, W>(records, first, NF == 1 && by_factors ? 0 : count, base, acc, after);
         guard.tile++;
         fence_results();
     }
@@ -727,7 +830,8 @@ bool forward_resident(const Call& call, const SapProblem<T>& p, T* O) {
     // Most products have to be used (3.5 10^6 rows, 25 x 5 -> 5, 141 triplets, f64: 410 -> 440 us).
     if (NF == 1 && 2 * p.K < 3 * static_cast<int64_t>(operand_columns)) return false;
     // f64, products for one row per lane only: 130 000 rows, 14 x 10 -> 8, 254 triplets: 34 -> 38 us.
-    if (NF == 1 && sizeof(T) == 8 && operand_columns + 1 > kTmemColumns / 4) return false;
+    const int columns = ones_column(NF, p.nA, p.nB) + 1;
+    if (NF == 1 && sizeof(T) == 8 && columns > kTmemColumns / 4) return false;
     Operands op{};
     op.add(p.A, p.nA);
     op.add(p.B, p.nB);
@@ -735,7 +839,7 @@ bool forward_resident(const Call& call, const SapProblem<T>& p, T* O) {
     for (int w : {4, 2}) {
         const int rows = kSlabRows * w / words_of(sizeof(T));
         const int64_t tiles = ceil_div(p.I, static_cast<int64_t>(rows));
-        if (operand_columns + 1 > kTmemColumns / w || tiles < sm_count(call.device)) continue;
+        if (columns > kTmemColumns / w || tiles < sm_count(call.device)) continue;
         size_t smem = resident_smem(sizeof(T) + 2 * NF, capacity, p.nO);
         const ResultStage stage = result_stage<T>(p.nO, rows, smem);
         smem = (smem + 15) / 16 * 16;
@@ -756,11 +860,11 @@ bool forward_resident(const Call& call, const SapProblem<T>& p, T* O) {
         };
         if constexpr (NF == 1) {
             with_lots<T, 1>(call, triplet_key(p, -2), ProductSource<T>{p.C, p.PA, p.PB, p.PO, p.nA, p.nB, p.nO}, p.K,
-                            p.nO, w, 1, operand_columns, run);
+                            p.nO, w, 1, columns - 1, run);
         } else {
             SapSource<T> source{p.C, {p.PA, p.PB, p.PO}, {p.nA, p.nB, p.nO}, static_cast<int>(p.K), {}};
             source.family[0] = {kO, 0, {kA, kB}, {0, p.nA}};
-            with_lots<T, 2>(call, triplet_key(p, -3), source, p.K, p.nO, w, 1, operand_columns, run);
+            with_lots<T, 2>(call, triplet_key(p, -3), source, p.K, p.nO, w, 1, columns - 1, run);
         }
         return true;
     }

@@ -4,9 +4,12 @@ without records, one column, many), against the CPU oracle at the parity toleran
 import numpy as np
 import pytest
 
+from conftest import assert_parity
 from helpers import run_checker, run_library, to_dev
-from mops_b200 import workloads
+from mops_b200 import _lib, workloads
 from test_parity_gpu import compare
+
+import mops_b200 as M
 
 pytestmark = pytest.mark.gpu
 DTYPES = [np.float64, np.float32]
@@ -56,6 +59,53 @@ def test_sap_resident(oracle, kw, dtype):
     r = np.random.default_rng(7)
     d["indices_output"] = r.permutation(d["indices_output"])
     compare("sap", d, dtype, oracle, what=f"sap {kw}")
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("large", [True, False])
+@pytest.mark.parametrize("every", [1, 700])
+@pytest.mark.parametrize("op,kw,kernel", [
+    ("sap", dict(I=300, nA=20, nB=6, nO=50, K=600), "sap_fwd_tmem"),
+    ("sap", dict(I=148 * 512 + 77, nA=20, nB=6, nO=50, K=600), "sap_fwd_resident<f%d,NF=1,W=4>"),
+    ("sap", dict(I=148 * 512 + 3, nA=7, nB=1, nO=11, K=700), "sap_fwd_resident<f%d,NF=1,W=4>"),  # more operands than products
+    ("sap", dict(I=148 * 256, nA=3, nB=5, nO=60, K=900), "sap_fwd_resident<f%d,NF=1"),
+    ("sap", dict(I=148 * 512 + 1, nA=32, nB=16, nO=20, K=900), {4: "sap_fwd_resident<f32,NF=2,W=4>", 8: "sap_fwd_tmem"}),
+    ("hpe", dict(I=300, N=20, J=300, K=2), "hpe_fwd_tmem"), ("hpe", dict(I=20001, N=20, J=300, K=3), "hpe_fwd_tmem"),
+])
+def test_products_of_operands_out_of_range(oracle, op, kw, kernel, every, large, dtype):
+    """Terms C a b within the range of the type with products a b that are not: A and B times 2^k, C over 2^k, for
+    all rows or for few of a tile, which multiplies their sums by exactly 2^k (the other rows' by 2^-k);
+    `large` False: -k, where the products underflow. HPE: the forward of order 2, the gradients of order 3."""
+    size = np.dtype(dtype).itemsize
+    k = (83 if size == 4 else 660) * (1 if large else -1)
+    d = workloads.__dict__[op](**kw)
+    if op == "hpe":
+        d["grad_output"] = np.ones_like(d["grad_output"])
+    d = {n: v.astype(dtype) if isinstance(v, np.ndarray) and v.dtype == np.float64 else v for n, v in d.items()}
+    d["A"][::5, 0] = 0
+    want = run_checker(oracle, op, {n: v.astype(np.float64) if isinstance(v, np.ndarray) and v.dtype == dtype else v
+                                    for n, v in d.items()}, np.float64)
+    scaled = np.zeros(kw["I"], dtype=bool)
+    scaled[kw["I"] // 3 % every::every] = True
+    d["C"] = np.ldexp(d["C"], -k)
+    for name in ("A", "B") if op == "sap" else ("A",):
+        d[name][scaled] = np.ldexp(d[name][scaled], k)
+    t = to_dev(d, dtype)
+    if op == "sap":
+        got = M.sparse_accumulation_of_products(t["A"], t["B"], t["C"], t["indices_A"], t["indices_B"],
+                                                t["indices_output"], t["output_size"])
+        name = kernel[size] if isinstance(kernel, dict) else kernel % (8 * size) if "%" in kernel else kernel
+        want = want["output"]
+    elif kw["K"] == 2:
+        got, name = M.homogeneous_polynomial_evaluation(t["A"], t["C"], t["indices_A"]), kernel
+        want = want["output"]
+    else:
+        got, name = M.homogeneous_polynomial_evaluation_vjp(t["grad_output"], t["A"], t["C"], t["indices_A"]), "hpe_vjp_tmem"
+        want = want["grad_A"]
+    assert any(x.startswith(name) for x in _lib.last_kernels()), _lib.last_kernels()
+    got = got.cpu().numpy().astype(np.float64)
+    got = np.ldexp(got, np.where(scaled, -k, k).reshape((-1,) + (1,) * (got.ndim - 1)))
+    assert_parity(got.astype(dtype), want.astype(dtype), f"{op} {kw}")
 
 
 @pytest.mark.parametrize("op,kw", [("hpe", dict(I=300, N=13, J=6400, K=4)), ("hpe", dict(I=20000, N=8, J=2000, K=3)),
