@@ -783,6 +783,156 @@ sap_vjp_resident(T* __restrict__ gT, T* __restrict__ gS, const __grid_constant__
     }
 }
 
+// The same with the records streamed, gT stored as it comes and gS summed in shared memory: for records, results or
+// addresses that sap_vjp_resident does not take. A cell's end is dearer here (75 instructions), so gather_sums is
+// faster up to about ten triplets per cell. 800 000 rows, f64: 32 x 8 -> 60, 8000 triplets, 5.4 ms by gather_sums,
+// 3.2 here; 25 x 25 -> 30 with 1500 (2.4 per cell), 100 000 rows, 164 us there, 335 here.
+template <typename T, int W>
+__global__ void __launch_bounds__(kTmemThreads, 1)
+sap_vjp_cells(T* __restrict__ gT, T* __restrict__ gS, const __grid_constant__ Operands operands,
+              const unsigned char* __restrict__ records, const int32_t* __restrict__ cell_start, int64_t I,
+              int64_t tiles, Status st) {
+    using G = Batch<T, 1, W>;
+    constexpr int B = G::B, R = G::R, RB = G::RB;
+    using Ring = RecordRing<1024>;
+    constexpr int kPerStage = 1024 / (B * RB);
+    static_assert(kPerStage % 2 == 0, "pairs of batches do not straddle stages");
+    const int nO = operands.cols[0], nT = operands.cols[1], nS = operands.cols[2], cells = nT * nS;
+    extern __shared__ __align__(16) unsigned char smem[];
+    // layout: ring | starts [cells + 1], padded | gS sums [group][nS][128 R] | slabs
+    int32_t* starts = reinterpret_cast<int32_t*>(smem + kStageBytes);
+    T* sums = reinterpret_cast<T*>(smem + kStageBytes + (static_cast<size_t>(cells + 1) * 4 + 15) / 16 * 16);
+    unsigned char* slabs = reinterpret_cast<unsigned char*>(sums + kTmemGroups * nS * kSlabRows * R);
+    __shared__ uint32_t tmem_s;
+    __shared__ uint64_t full[kTmemGroups][2];
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(kFullMask, tid >> 5, 0), group = warp >> 2;
+
+    Tiles<T, W> tile_of{operands, I, operands.template slab_bytes<T>(), slabs};
+    tile_of.start(blockIdx.x, tid);
+    if (warp == 0) tmem_alloc(&tmem_s, kTmemColumns);
+    Ring::prepare(smem, full, tid);
+    for (int c = tid; c <= cells; c += kTmemThreads) starts[c] = __ldg(cell_start + c);
+    tmem_fence_before_sync();
+    __syncthreads();
+    tmem_fence_after_sync();
+    const uint32_t base = tmem_quadrant(tmem_s, warp);
+    tile_of.ones(base, warp);
+
+    const int t_lo = uniform(group_column(starts, nT, nS, group, kTmemGroups));
+    const int t_hi = uniform(group_column(starts, nT, nS, group + 1, kTmemGroups));
+    const int c_hi = t_hi * nS;
+    const int x_lo = uniform(starts[t_lo * nS]), batches = uniform(starts[c_hi] - starts[t_lo * nS]) / B;
+    Ring ring(smem + group * 2048, full[group], group, (warp & 3) == 0 && lane == 0,
+              records + static_cast<size_t>(x_lo) * RB, batches * B * RB);
+    const int own = (warp & 3) * 32 + lane;
+    T* mine = sums + static_cast<size_t>(group) * nS * kSlabRows * R + own; // [s][slot][128]
+
+    for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        tile_of.load(tile + gridDim.x < tiles ? tile + gridDim.x : -1, base, tid, warp, lane);
+        const int64_t row0 = tile * (kSlabRows * R) + own;
+        bool live[R];
+        T acc[R], sum_t[R];
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            live[r] = row0 + r * kSlabRows < I;
+            acc[r] = sum_t[r] = T(0);
+        }
+        for (int s = 0; s < nS * R; s++) mine[s * kSlabRows] = T(0);
+        SectorWriter<T, R> writer{};
+        int t = t_lo, s = 0, c = t_lo * nS;
+        uint32_t value_t[1][W];
+        auto load_t = [&] { // T[t] of the lane's rows
+            tmem_load(base + (nO + t) * W, value_t[0]);
+            tmem_wait_load();
+            tmem_pin(value_t[0]);
+        };
+        // Moves on to the next cell that has records (or to the end), storing gT[t] on the way.
+        // Returns its number of batches.
+        auto next_cell = [&](bool moved) {
+            for (; c < c_hi; moved = true) {
+                if (moved) {
+                    c++;
+                    if (++s == nS) {
+                        writer.put(t, gT + row0 * nT + t, kSlabRows * static_cast<int64_t>(nT), t - t_lo, t + 1 == t_hi,
+                                   sum_t, live);
+#pragma unroll
+                        for (int r = 0; r < R; r++) sum_t[r] = T(0);
+                        s = 0;
+                        t++;
+                        if (t < t_hi) load_t();
+                    }
+                    if (c == c_hi) break;
+                }
+                const int n = uniform(starts[c + 1] - starts[c]) / B;
+                if (n > 0) return n;
+            }
+            return -1;
+        };
+        auto end_cell = [&] {
+            uint32_t value_s[W];
+            tmem_load(base + (nO + nT + s) * W, value_s);
+            tmem_wait_load();
+            tmem_pin(value_s);
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                sum_t[r] += acc[r] * tmem_value<T>(value_s, r);
+                mine[(s * R + r) * kSlabRows] += acc[r] * tmem_value<T>(value_t[0], r);
+                acc[r] = T(0);
+            }
+        };
+        if (t < t_hi) load_t();
+        ring.start_tile();
+        int left = next_cell(false);
+        if (batches > 0) {
+            G x, y;
+            Records<T, 1, W> rx, ry;
+            auto add = [&](const G& g, const Records<T, 1, W>& rec) {
+                add_terms<T, 1, W>(g, rec, acc);
+                if (--left == 0) {
+                    end_cell();
+                    left = next_cell(true);
+                }
+            };
+            ring.enter_stage(0, lane, st);
+            fetch<T, 1, W>(rx, ring.template at<B * RB>(0));
+            issue<T, 1, W>(x, rx, base);
+            fetch<T, 1, W>(ry, ring.template at<B * RB>(1));
+            for (int i = 0; i < batches; i += 2) {
+                await<T, 1, W>(x);
+                issue<T, 1, W>(y, ry, base);
+                add(x, rx);
+                if ((i & (kPerStage - 1)) == kPerStage - 2 && i + 2 < batches)
+                    ring.enter_stage((i + 2) / kPerStage, lane, st);
+                fetch<T, 1, W>(rx, ring.template at<B * RB>(i + 2));
+                await<T, 1, W>(y);
+                issue<T, 1, W>(x, rx, base);
+                add(y, ry); // (behind the last batch: all cells are done, nothing is kept)
+                fetch<T, 1, W>(ry, ring.template at<B * RB>(i + 3));
+            }
+            await<T, 1, W>(x);
+        }
+        tmem_fence_before_sync();
+        __syncthreads(); // all sums are complete; before the next tile overwrites TMEM
+        tmem_fence_after_sync();
+        // gS: the tile's rows are contiguous in memory
+        const int64_t first_row = tile * (kSlabRows * R);
+        const int64_t have = I - first_row < kSlabRows * R ? I - first_row : kSlabRows * R;
+        for (int y = tid; y < have * nS; y += kTmemThreads) {
+            const int row = y / nS, s2 = y - row * nS;
+            T v = T(0);
+#pragma unroll
+            for (int g = 0; g < kTmemGroups; g++)
+                v += sums[(static_cast<size_t>(g) * nS + s2) * kSlabRows * R + row];
+            gS[first_row * nS + y] = v;
+        }
+        // (the barriers of the next tile's load come before the sums are cleared)
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+    if (warp == 0) tmem_free(tmem_s, kTmemColumns);
+}
+
 inline bool at_16_bytes(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
 
 // Builds (or takes from the plan) the table of records over `columns` result columns, each a whole number
@@ -871,49 +1021,70 @@ bool forward_resident(const Call& call, const SapProblem<T>& p, T* O) {
     return false;
 }
 
-template <typename T>
-bool backward_resident(const Call& call, const SapProblem<T>& p, T* gA, T* gB, const T* gO) {
-    const bool b_narrow = p.nB <= p.nA;
-    const int nS = b_narrow ? p.nB : p.nA, nT = b_narrow ? p.nA : p.nB, cells = nS * nT;
-    const size_t limit = static_cast<size_t>(max_optin_smem(call.device)) - 1024;
-    if (table_smem(p.K, cells) > limit || !at_16_bytes(gA) || !at_16_bytes(gB) || p.K > (1 << 14)) return false;
+// The VJP's operands, in the kernels' order, and the source of its records.
+template <typename T> struct CellProblem {
+    bool b_narrow;
+    int nS, nT, cells;
     Operands op{};
-    op.add(gO, p.nO);
-    op.add(b_narrow ? p.A : p.B, nT);
-    op.add(b_narrow ? p.B : p.A, nS);
-    const int64_t padded = p.K + 3 * std::min<int64_t>(p.K, cells);
-    const int capacity = static_cast<int>(ceil_div(padded, kLot) + 3) * kLot;
-    // rows per lane: as many as fit and still give every SM a tile
-    for (int w : {4, 2}) {
-        const int rows = kSlabRows * w / words_of(sizeof(T));
-        const int64_t tiles = ceil_div(p.I, static_cast<int64_t>(rows));
-        if (op.total + 1 + kTmemGroups * ((nS + 1) / 2 * 4) > kTmemColumns / w || nS > 32 || tiles < sm_count(call.device)) continue;
-        size_t smem = resident_smem(sizeof(T) + 2, capacity, 5 * cells + 8); // (bounds and list)
-        const ResultStage t_stage = result_stage<T>(nT, rows, smem);
-        const ResultStage s_stage = result_stage<T>(nS, rows, smem);
-        smem = (smem + 15) / 16 * 16;
-        const int slabs = static_cast<int>(smem);
-        smem += static_cast<size_t>(w / words_of(sizeof(T))) * op.template slab_bytes<T>();
-        if (smem > limit) continue;
-        note_kernel_f("sap_vjp_resident<%s,W=%d>", scalar_name<T>(), w);
-        const GatherShape shape{w, 1, tiles, smem};
-        const CellSource<T> source{p.C, b_narrow ? p.PA : p.PB, b_narrow ? p.PB : p.PA, p.PO, nT, nS, p.nO,
-                                   b_narrow ? 0 : 1, b_narrow ? 1 : 0};
-        with_lots<T, 1>(call, triplet_key(p, -1), source, p.K, cells, w, 0, op.total,
-                        [&](const unsigned char* records, const int32_t* starts) {
-                            auto go = [&](auto kernel) {
-                                launch_gather(call, kernel, shape, 1, b_narrow ? gA : gB, b_narrow ? gB : gA, op,
-                                              records, starts, t_stage, s_stage, capacity, slabs, p.I, tiles,
-                                              call.status);
-                            };
-                            if (w == 4)
-                                go(sap_vjp_resident<T, 4>);
-                            else
-                                go(sap_vjp_resident<T, 2>);
-                        });
-        return true;
+    CellSource<T> source;
+    CellProblem(const SapProblem<T>& p, const T* gO)
+        : b_narrow(p.nB <= p.nA), nS(b_narrow ? p.nB : p.nA), nT(b_narrow ? p.nA : p.nB), cells(nS * nT),
+          source{p.C, b_narrow ? p.PA : p.PB, b_narrow ? p.PB : p.PA, p.PO, nT, nS, p.nO, b_narrow ? 0 : 1, b_narrow ? 1 : 0} {
+        op.add(gO, p.nO);
+        op.add(b_narrow ? p.A : p.B, nT);
+        op.add(b_narrow ? p.B : p.A, nS);
     }
-    return false;
+};
+
+// Rows per lane: W / words(T). Both kernels read the same table.
+template <typename T, int W>
+bool backward_resident(const Call& call, const SapProblem<T>& p, const CellProblem<T>& c, T* gA, T* gB) {
+    constexpr int rows = kSlabRows * kLaneRows<T, W>;
+    const size_t limit = static_cast<size_t>(max_optin_smem(call.device)) - 1024;
+    const int64_t tiles = ceil_div(p.I, static_cast<int64_t>(rows));
+    if (table_smem(p.K, c.cells) > limit || !at_16_bytes(gA) || !at_16_bytes(gB) || p.K > (1 << 14)) return false;
+    if (c.op.total + 1 + kTmemGroups * ((c.nS + 1) / 2 * 4) > kTmemColumns / W || c.nS > 32 || tiles < sm_count(call.device))
+        return false;
+    const int64_t padded = p.K + 3 * std::min<int64_t>(p.K, c.cells);
+    const int capacity = static_cast<int>(ceil_div(padded, kLot) + 3) * kLot;
+    size_t smem = resident_smem(sizeof(T) + 2, capacity, 5 * c.cells + 8); // (bounds and list)
+    const ResultStage t_stage = result_stage<T>(c.nT, rows, smem);
+    const ResultStage s_stage = result_stage<T>(c.nS, rows, smem);
+    smem = (smem + 15) / 16 * 16;
+    const int slabs = static_cast<int>(smem);
+    smem += static_cast<size_t>(kLaneRows<T, W>) * c.op.template slab_bytes<T>();
+    if (smem > limit) return false;
+    note_kernel_f("sap_vjp_resident<%s,W=%d>", scalar_name<T>(), W);
+    with_lots<T, 1>(call, triplet_key(p, -1), c.source, p.K, c.cells, W, 0, c.op.total,
+                    [&](const unsigned char* records, const int32_t* starts) {
+                        launch_gather(call, sap_vjp_resident<T, W>, GatherShape{W, 1, tiles, smem}, 1, c.b_narrow ? gA : gB,
+                                      c.b_narrow ? gB : gA, c.op, records, starts, t_stage, s_stage, capacity, slabs,
+                                      p.I, tiles, call.status);
+                    });
+    return true;
+}
+
+template <typename T, int W>
+bool backward_cells(const Call& call, const SapProblem<T>& p, const CellProblem<T>& c, T* gA, T* gB) {
+    constexpr int rows = kSlabRows * kLaneRows<T, W>;
+    static_assert(batch_of(1, W) == kLot, "the table's batches");
+    const size_t limit = static_cast<size_t>(max_optin_smem(call.device)) - 1024;
+    const int64_t tiles = ceil_div(p.I, static_cast<int64_t>(rows));
+    const size_t smem = kStageBytes + (static_cast<size_t>(c.cells + 1) * 4 + 15) / 16 * 16 +
+                        static_cast<size_t>(kTmemGroups) * c.nS * rows * sizeof(T) +
+                        static_cast<size_t>(kLaneRows<T, W>) * c.op.template slab_bytes<T>();
+    if (table_smem(p.K, c.cells) > limit || c.op.total + 1 > kTmemColumns / W || smem > limit || tiles < sm_count(call.device))
+        return false;
+    // cells / gather_sums, 140 drawn shapes: 0.60 - 1.18 from 12 triplets per cell on (longer: down to 0.25),
+    // 0.69 - 1.26 at 8 to 12, 0.85 - 1.37 at 4 to 6, 0.94 - 3.8 below 2
+    if (p.K < 12 * static_cast<int64_t>(c.cells)) return false;
+    note_kernel_f("sap_vjp_cells<%s,W=%d>", scalar_name<T>(), W);
+    with_lots<T, 1>(call, triplet_key(p, -1), c.source, p.K, c.cells, W, 0, c.op.total,
+                    [&](const unsigned char* records, const int32_t* starts) {
+                        launch_gather(call, sap_vjp_cells<T, W>, GatherShape{W, 1, tiles, smem}, 1, c.b_narrow ? gA : gB,
+                                      c.b_narrow ? gB : gA, c.op, records, starts, p.I, tiles, call.status);
+                    });
+    return true;
 }
 
 } // namespace
@@ -936,7 +1107,12 @@ template <typename T>
 bool sap_backward_tmem(const Call& call, const SapProblem<T>& p, T* gA, T* gB, const T* gO) {
     if (fills_gpu(call, p.I) && few_backward_triplets(p)) return false;
     // Both gradients of a batch with a tile for every SM: by cells.
-    if (gA != nullptr && gB != nullptr && backward_resident(call, p, gA, gB, gO)) return true;
+    if (gA != nullptr && gB != nullptr) {
+        const CellProblem<T> cells(p, gO);
+        if (backward_resident<T, 4>(call, p, cells, gA, gB) || backward_resident<T, 2>(call, p, cells, gA, gB) ||
+            backward_cells<T, 4>(call, p, cells, gA, gB) || backward_cells<T, 2>(call, p, cells, gA, gB))
+            return true;
+    }
     Operands op{};
     Results<T> results{};
     Family f[2];

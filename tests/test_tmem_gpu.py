@@ -61,6 +61,60 @@ def test_sap_resident(oracle, kw, dtype):
     compare("sap", d, dtype, oracle, what=f"sap {kw}")
 
 
+def _sap_kernels(t):
+    """The main kernels of a forward call and of one for both gradients."""
+    idx = (t["indices_A"], t["indices_B"], t["indices_output"])
+    M.sparse_accumulation_of_products(t["A"], t["B"], t["C"], *idx, t["output_size"])
+    forward = _lib.last_kernels()
+    M.sparse_accumulation_of_products_vjp(t["grad_output"], t["A"], t["B"], t["C"], *idx)
+    return forward[0], _lib.last_kernels()[0]
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("kw,kernel", [
+    (dict(I=37889, nA=8, nB=3, nO=9, K=17000), "sap_vjp_cells"),    # records larger than shared memory
+    (dict(I=38001, nA=2, nB=7, nO=60, K=16500), "sap_vjp_cells"),   # B the wider operand, the last tile ragged
+    (dict(I=37889, nA=25, nB=25, nO=30, K=900), "sap_vjp_tmem"),    # few triplets per cell
+])
+def test_sap_gradients_by_streamed_cells(oracle, kw, kernel, dtype):
+    d = workloads.sap(**kw)
+    d["indices_output"] = np.random.default_rng(7).permutation(d["indices_output"])
+    assert _sap_kernels(to_dev(d, dtype))[1].startswith(kernel)
+    if dtype == np.float32:  # (sums of thousands of terms: see test_f32_sums_of_thousands_of_records)
+        rounded = {k: v.astype(np.float32).astype(np.float64) if isinstance(v, np.ndarray) and v.dtype == np.float64
+                   else v for k, v in d.items()}
+        got, want = run_library("sap", to_dev(d, dtype)), run_checker(oracle, "sap", rounded, np.float64)
+        for k in want:
+            assert np.abs(got[k] - want[k]).max() <= 1e-5 * np.abs(want[k]).max(), k
+        return
+    compare("sap", d, dtype, oracle, what=f"sap {kw}")
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_sap_results_at_odd_addresses(oracle, dtype):
+    """Results that start one scalar into an allocation: no bulk copies out of shared memory."""
+    import torch
+    d = workloads.sap(I=148 * 256 + 5, nA=6, nB=4, nO=9, K=600)
+    t = to_dev(d, dtype)
+    want = run_checker(oracle, "sap", d, dtype)
+    odd = {k: t[x].new_empty(t[x].numel() + 1)[1:].view(t[x].shape)
+           for k, x in (("output", "grad_output"), ("grad_A", "A"), ("grad_B", "B"))}
+    suffix = "f64" if dtype == np.float64 else "f32"
+
+    def call(name, *tensors):
+        _lib.call(f"mops_cuda_{name}_{suffix}", [_lib.make_struct(x.data_ptr(), x.shape) for x in tensors])
+        torch.cuda.synchronize()
+        return _lib.last_kernels()[0]
+
+    torch.cuda.synchronize()
+    rest = (t["A"], t["B"], t["C"], t["indices_A"], t["indices_B"], t["indices_output"])
+    assert call("sparse_accumulation_of_products", odd["output"], *rest).startswith("sap_fwd_tmem")
+    assert call("sparse_accumulation_of_products_vjp", odd["grad_A"], odd["grad_B"], t["grad_output"],
+                *rest).startswith("sap_vjp_cells")
+    for k in want:
+        assert_parity(odd[k].cpu().numpy(), want[k], k)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("large", [True, False])
 @pytest.mark.parametrize("every", [1, 700])
