@@ -61,6 +61,25 @@ template <typename T> bool few_backward_triplets(const SapProblem<T>& p) {
     return p.K < (pieces ? 3 : 5) * static_cast<int64_t>(p.nA + p.nB + p.nO);
 }
 
+// And so are they for narrow operands with few triplets, whatever the triplets per column: a tile's way in and
+// out costs the same then, while their tables are small. Measured on 165 shapes (widths 1 to 32 and 1 to 16, 2 to
+// 100 results, 20 to 3000 triplets, 25 000 to 800 000 rows) that the lines above leave to these kernels: sap.cu's
+// take 0.54 to 1.27 times as long in the forward on their side of this line (one shape 1.55), 0.47 to 1.16 for both
+// gradients, 0.59 to 1.27 for one; on the other side 0.83, 0.92 and 0.78 at least, mostly more than 1. 4 x 4 -> 8,
+// 40 triplets, 800 000 rows, f64, forward: 72 against 111 us; both gradients, 120 triplets: 94 against 130. With
+// both operands wider than 16 columns sap.cu has no register kernels.
+template <typename T> bool narrow_forward(const SapProblem<T>& p) {
+    const int64_t cells = static_cast<int64_t>(p.nA) * p.nB;
+    if (std::min(p.nA, p.nB) > 16) return false;
+    return sizeof(T) == 8 ? 2 * p.K + cells + 16 * static_cast<int64_t>(p.nO) < 384 : p.K + cells + 8 * static_cast<int64_t>(p.nO) < 300;
+}
+template <typename T> bool narrow_backward(const SapProblem<T>& p, bool both) {
+    const int64_t cells = static_cast<int64_t>(p.nA) * p.nB, columns = static_cast<int64_t>(p.nA) + p.nB + p.nO;
+    if (std::min(p.nA, p.nB) > 16) return false;
+    if (both) return sizeof(T) == 8 ? p.K + 6 * columns < 324 : p.K + 2 * cells + 6 * columns < 543;
+    return sizeof(T) == 8 ? p.K + 6 * cells + 8 * columns < 454 : p.K + 8 * cells + 3 * columns < 590;
+}
+
 template <typename T>
 bool run(const Call& call, const SapProblem<T>& p, const Family* families, int count, const Operands& op,
          const Results<T>& results, int level, const char* name) {
@@ -1090,7 +1109,7 @@ bool backward_cells(const Call& call, const SapProblem<T>& p, const CellProblem<
 } // namespace
 
 template <typename T> bool sap_forward_tmem(const Call& call, const SapProblem<T>& p, T* O) {
-    if (fills_gpu(call, p.I) && few_forward_triplets(p)) return false;
+    if (fills_gpu(call, p.I) && (few_forward_triplets(p) || narrow_forward(p))) return false;
     if (forward_resident<T, 1>(call, p, O)) return true;
     if constexpr (sizeof(T) == 4)
         if (forward_resident<T, 2>(call, p, O)) return true;
@@ -1105,9 +1124,10 @@ template <typename T> bool sap_forward_tmem(const Call& call, const SapProblem<T
 
 template <typename T>
 bool sap_backward_tmem(const Call& call, const SapProblem<T>& p, T* gA, T* gB, const T* gO) {
-    if (fills_gpu(call, p.I) && few_backward_triplets(p)) return false;
+    const bool both = gA != nullptr && gB != nullptr;
+    if (fills_gpu(call, p.I) && (few_backward_triplets(p) || narrow_backward(p, both))) return false;
     // Both gradients of a batch with a tile for every SM: by cells.
-    if (gA != nullptr && gB != nullptr) {
+    if (both) {
         const CellProblem<T> cells(p, gO);
         if (backward_resident<T, 4>(call, p, cells, gA, gB) || backward_resident<T, 2>(call, p, cells, gA, gB) ||
             backward_cells<T, 4>(call, p, cells, gA, gB) || backward_cells<T, 2>(call, p, cells, gA, gB))

@@ -116,6 +116,29 @@ def test_sap_results_at_odd_addresses(oracle, dtype):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("kw,narrow", [
+    (dict(nA=4, nB=4, nO=8, K=100), (True, True, True)), (dict(nA=4, nB=4, nO=8, K=600), (False, False, False)),
+    (dict(nA=1, nB=7, nO=9, K=60), (True, True, True)), (dict(nA=23, nB=10, nO=8, K=250), (False, False, False)),
+    (dict(nA=13, nB=2, nO=3, K=140), (True, True, True)), (dict(nA=20, nB=6, nO=50, K=900), (False, False, False)),
+])
+def test_narrow_sap(oracle, kw, narrow, dtype):
+    """Batches that fill the GPU: narrow operands with few triplets (forward, both gradients, one) stay with the
+    kernels that gather from shared memory."""
+    d = workloads.sap(I=148 * 128 + 1, **kw)
+    d["indices_output"] = np.random.default_rng(7).permutation(d["indices_output"])
+    t = to_dev(d, dtype)
+    args = (t["grad_output"], t["A"], t["B"], t["C"], t["indices_A"], t["indices_B"], t["indices_output"])
+    kernels = list(_sap_kernels(t))
+    want = run_checker(oracle, "sap", d, dtype)
+    for k in ("grad_A", "grad_B"):
+        got = M.sparse_accumulation_of_products_vjp(*args, compute_grad_A=k == "grad_A", compute_grad_B=k == "grad_B")
+        kernels.append(_lib.last_kernels()[0])
+        assert_parity(got[0 if k == "grad_A" else 1].cpu().numpy(), want[k], k)
+    assert tuple("small" in k for k in kernels) == narrow + narrow[-1:], kernels
+    compare("sap", d, dtype, oracle, what=f"sap {kw}")
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("large", [True, False])
 @pytest.mark.parametrize("every", [1, 700])
 @pytest.mark.parametrize("op,kw,kernel", [
