@@ -991,53 +991,38 @@ inline size_t resident_smem(size_t record_bytes, int capacity, int columns) {
     return (record_bytes * capacity + 15) / 16 * 16 + (static_cast<size_t>(columns + 1) * 4 + 15) / 16 * 16;
 }
 
-template <typename T, int NF>
+template <typename T, int NF, int W>
 bool forward_resident(const Call& call, const SapProblem<T>& p, T* O) {
-    const int operand_columns = NF == 1 ? p.nA * p.nB : p.nA + p.nB;
-    const size_t limit = static_cast<size_t>(max_optin_smem(call.device)) - 1024;
-    if (table_smem(p.K, p.nO) > limit || !at_16_bytes(O) || p.K > (1 << 14)) return false;
-    // Most products have to be used (3.5 10^6 rows, 25 x 5 -> 5, 141 triplets, f64: 410 -> 440 us).
-    if (NF == 1 && 2 * p.K < 3 * static_cast<int64_t>(operand_columns)) return false;
-    // f64, products for one row per lane only: 130 000 rows, 14 x 10 -> 8, 254 triplets: 34 -> 38 us.
+    constexpr int rows = kSlabRows * kLaneRows<T, W>;
     const int columns = ones_column(NF, p.nA, p.nB) + 1;
-    if (NF == 1 && sizeof(T) == 8 && columns > kTmemColumns / 4) return false;
+    const size_t limit = static_cast<size_t>(max_optin_smem(call.device)) - 1024;
+    const int64_t tiles = ceil_div(p.I, static_cast<int64_t>(rows));
+    if (table_smem(p.K, p.nO) > limit || !at_16_bytes(O) || p.K > (1 << 14)) return false;
+    if (columns > kTmemColumns / W || tiles < sm_count(call.device)) return false;
     Operands op{};
     op.add(p.A, p.nA);
     op.add(p.B, p.nB);
     const int capacity = static_cast<int>(ceil_div(p.K + static_cast<int64_t>(p.nO) * kLot, kLot) + 3) * kLot;
-    for (int w : {4, 2}) {
-        const int rows = kSlabRows * w / words_of(sizeof(T));
-        const int64_t tiles = ceil_div(p.I, static_cast<int64_t>(rows));
-        if (columns > kTmemColumns / w || tiles < sm_count(call.device)) continue;
-        size_t smem = resident_smem(sizeof(T) + 2 * NF, capacity, p.nO);
-        const ResultStage stage = result_stage<T>(p.nO, rows, smem);
-        smem = (smem + 15) / 16 * 16;
-        const int slabs = static_cast<int>(smem);
-        smem += static_cast<size_t>(w / words_of(sizeof(T))) * op.template slab_bytes<T>();
-        if (smem > limit) continue;
-        note_kernel_f("sap_fwd_resident<%s,NF=%d,W=%d>", scalar_name<T>(), NF, w);
-        const GatherShape shape{w, 1, tiles, smem};
-        auto run = [&](const unsigned char* records, const int32_t* starts) {
-            auto go = [&](auto kernel) {
-                launch_gather(call, kernel, shape, 1, O, op, records, starts, stage, capacity, slabs, p.I, tiles,
-                              call.status);
-            };
-            if (w == 4)
-                go(sap_fwd_resident<T, NF, 4>);
-            else
-                go(sap_fwd_resident<T, NF, 2>);
-        };
-        if constexpr (NF == 1) {
-            with_lots<T, 1>(call, triplet_key(p, -2), ProductSource<T>{p.C, p.PA, p.PB, p.PO, p.nA, p.nB, p.nO}, p.K,
-                            p.nO, w, 1, columns - 1, run);
-        } else {
-            SapSource<T> source{p.C, {p.PA, p.PB, p.PO}, {p.nA, p.nB, p.nO}, static_cast<int>(p.K), {}};
-            source.family[0] = {kO, 0, {kA, kB}, {0, p.nA}};
-            with_lots<T, 2>(call, triplet_key(p, -3), source, p.K, p.nO, w, 1, columns - 1, run);
-        }
-        return true;
+    size_t smem = resident_smem(sizeof(T) + 2 * NF, capacity, p.nO);
+    const ResultStage stage = result_stage<T>(p.nO, rows, smem);
+    smem = (smem + 15) / 16 * 16;
+    const int slabs = static_cast<int>(smem);
+    smem += static_cast<size_t>(kLaneRows<T, W>) * op.template slab_bytes<T>();
+    if (smem > limit) return false;
+    note_kernel_f("sap_fwd_resident<%s,NF=%d,W=%d>", scalar_name<T>(), NF, W);
+    auto run = [&](const unsigned char* records, const int32_t* starts) {
+        launch_gather(call, sap_fwd_resident<T, NF, W>, GatherShape{W, 1, tiles, smem}, 1, O, op, records, starts, stage,
+                      capacity, slabs, p.I, tiles, call.status);
+    };
+    if constexpr (NF == 1) {
+        with_lots<T, 1>(call, triplet_key(p, -2), ProductSource<T>{p.C, p.PA, p.PB, p.PO, p.nA, p.nB, p.nO}, p.K, p.nO,
+                        W, 1, columns - 1, run);
+    } else {
+        SapSource<T> source{p.C, {p.PA, p.PB, p.PO}, {p.nA, p.nB, p.nO}, static_cast<int>(p.K), {}};
+        source.family[0] = {kO, 0, {kA, kB}, {0, p.nA}};
+        with_lots<T, 2>(call, triplet_key(p, -3), source, p.K, p.nO, W, 1, columns - 1, run);
     }
-    return false;
+    return true;
 }
 
 // The VJP's operands, in the kernels' order, and the source of its records.
@@ -1110,9 +1095,22 @@ bool backward_cells(const Call& call, const SapProblem<T>& p, const CellProblem<
 
 template <typename T> bool sap_forward_tmem(const Call& call, const SapProblem<T>& p, T* O) {
     if (fills_gpu(call, p.I) && (few_forward_triplets(p) || narrow_forward(p))) return false;
-    if (forward_resident<T, 1>(call, p, O)) return true;
-    if constexpr (sizeof(T) == 4)
-        if (forward_resident<T, 2>(call, p, O)) return true;
+    // Most products have to be used (3.5 10^6 rows, 25 x 5 -> 5, 141 triplets, f64: 410 -> 440 us). Kernels with
+    // fewer rows per lane, where shared memory or the batch leave no more, come after those by pairs, and behind
+    // gather_sums for many triplets, which it has more rows for: f64 by products with one row 0.87 to 1.06 times
+    // as long as gather_sums up to 1000 triplets, 1.02 to 1.27 mostly beyond; f32 by pairs with two rows 0.58 to
+    // 0.68 up to 268 triplets, 1.14 to 1.42 with 8000 (32 x 8 -> 60, which fits four rows in gather_sums alone).
+    const bool products = 2 * p.K >= 3 * static_cast<int64_t>(p.nA) * p.nB;
+    if (products && forward_resident<T, 1, 4>(call, p, O)) return true;
+    if constexpr (sizeof(T) == 4) {
+        if (forward_resident<T, 2, 4>(call, p, O) || (products && forward_resident<T, 1, 2>(call, p, O)) ||
+            (p.K <= 4000 && forward_resident<T, 2, 2>(call, p, O)))
+            return true;
+    } else {
+        // (more products than fit two rows: 130 000 rows, 14 x 10 -> 8, 254 triplets: 34 -> 38 us)
+        const bool fit_two = ones_column(1, p.nA, p.nB) < kTmemColumns / 4;
+        if (products && fit_two && p.K <= 1000 && forward_resident<T, 1, 2>(call, p, O)) return true;
+    }
     Operands op{};
     op.add(p.A, p.nA);
     op.add(p.B, p.nB);

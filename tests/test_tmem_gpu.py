@@ -43,24 +43,6 @@ def test_sap(oracle, kw, dtype):
     compare("sap", d, dtype, oracle, second_order=True, what=f"sap {kw}")
 
 
-@pytest.mark.parametrize("dtype", DTYPES)
-@pytest.mark.parametrize("kw", [
-    dict(I=148 * 256, nA=20, nB=6, nO=64, K=1000),         # result rows of whole 128-byte lines: one copy each
-    dict(I=148 * 512 + 1, nA=16, nB=4, nO=32, K=600),      # f32: four rows per lane
-    dict(I=2 * 148 * 256 + 255, nA=9, nB=14, nO=3, K=400),  # 126 products, few result columns
-    dict(I=148 * 128 + 1, nA=16, nB=8, nO=9, K=500),       # 128 products: by pairs, two or four rows per lane
-    dict(I=40001, nA=1, nB=1, nO=2, K=50),                 # one cell: three warp groups have nothing to do
-    dict(I=40003, nA=7, nB=11, nO=33, K=511),              # odd rows; the last tile ends inside a 16-byte piece
-    dict(I=20011, nA=32, nB=16, nO=100, K=2000),
-])
-def test_sap_resident(oracle, kw, dtype):
-    """Batches that fill the GPU: records and results in shared memory (sap_fwd_resident, sap_vjp_resident)."""
-    d = workloads.sap(**kw)
-    r = np.random.default_rng(7)
-    d["indices_output"] = r.permutation(d["indices_output"])
-    compare("sap", d, dtype, oracle, what=f"sap {kw}")
-
-
 def _sap_kernels(t):
     """The main kernels of a forward call and of one for both gradients."""
     idx = (t["indices_A"], t["indices_B"], t["indices_output"])
@@ -68,6 +50,71 @@ def _sap_kernels(t):
     forward = _lib.last_kernels()
     M.sparse_accumulation_of_products_vjp(t["grad_output"], t["A"], t["B"], t["C"], *idx)
     return forward[0], _lib.last_kernels()[0]
+
+
+FWD, VJP = "sap_fwd_resident<%s,NF=1,W=4>", "sap_vjp_resident<%s,W=4>"
+BY_PAIRS = "sap_fwd_resident<%s,NF=2,W={}>"
+
+
+@pytest.mark.parametrize("kw,f64,f32", [
+    # (result rows of whole 128-byte lines lie 16 bytes further apart in shared memory)
+    (dict(I=148 * 256, nA=20, nB=6, nO=64, K=1000), (FWD, VJP[:-2] + "2>"),
+     (FWD[:-2] + "2>", VJP[:-2] + "2>")),
+    (dict(I=148 * 512 + 1, nA=16, nB=4, nO=32, K=600), (FWD, VJP), (FWD, VJP)),  # f32: four rows per lane
+    (dict(I=2 * 148 * 256 + 255, nA=9, nB=14, nO=3, K=400), (FWD, VJP), (FWD, VJP)),  # 126 products, few result columns
+    (dict(I=148 * 128 + 1, nA=16, nB=8, nO=9, K=500), ("sap_fwd_tmem", VJP[:-2] + "2>"),  # 128 products
+     ("sap_fwd_tmem", "sap_vjp_tmem")),                                                 # f32: not a tile for every SM
+    (dict(I=148 * 256, nA=32, nB=16, nO=20, K=900), ("sap_fwd_tmem", VJP[:-2] + "2>"),
+     (BY_PAIRS.format(2), VJP[:-2] + "2>")),
+    (dict(I=148 * 512, nA=32, nB=16, nO=20, K=900), ("sap_fwd_tmem", VJP[:-2] + "2>"),
+     (BY_PAIRS.format(4), VJP[:-2] + "2>")),
+    (dict(I=148 * 512 + 9, nA=24, nB=9, nO=7, K=300), ("sap_fwd_tmem", VJP), (BY_PAIRS.format(4), VJP)),  # products hardly used
+    (dict(I=40001, nA=1, nB=1, nO=2, K=900), (FWD, VJP), (FWD[:-2] + "2>", VJP[:-2] + "2>")),  # one cell: three idle groups
+    # odd rows; the last tile ends inside a 16-byte piece
+    (dict(I=40003, nA=7, nB=11, nO=33, K=511), (FWD, VJP), (FWD[:-2] + "2>", VJP[:-2] + "2>")),
+    (dict(I=20003, nA=7, nB=11, nO=33, K=511), (FWD[:-2] + "2>", VJP[:-2] + "2>"), ("sap_fwd_tmem", "sap_vjp_tmem")),
+    (dict(I=20011, nA=32, nB=16, nO=100, K=2000), ("sap_fwd_tmem", "sap_vjp_tmem"), ("sap_fwd_tmem", "sap_vjp_tmem")),
+])
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_sap_resident(oracle, kw, f64, f32, dtype):
+    """Batches that fill the GPU: records and results in shared memory (sap_fwd_resident, sap_vjp_resident), with as
+    many rows per lane as fit, and the shapes next to them that are not taken."""
+    d = workloads.sap(**kw)
+    r = np.random.default_rng(7)
+    d["indices_output"] = r.permutation(d["indices_output"])
+    name = "f64" if dtype == np.float64 else "f32"
+    kernels = _sap_kernels(to_dev(d, dtype))
+    for got, want in zip(kernels, f64 if dtype == np.float64 else f32):
+        assert got.startswith(want % name if "%" in want else want), (kernels, want)
+    compare("sap", d, dtype, oracle, what=f"sap {kw}")
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_sap_resident_in_a_plan_and_with_bad_indices(oracle, dtype):
+    """Tables of a plan serve both kernels of the gradients and the forward again; an index out of range is
+    reported from either, and the call after it works."""
+    d = workloads.sap(I=148 * 512, nA=9, nB=6, nO=17, K=700)
+    t = to_dev(d, dtype)
+    with M.Plan() as plan:
+        first = run_library("sap", t)
+        tables = plan.tables
+        again = run_library("sap", t)
+        assert plan.tables == tables == 2
+    assert all("resident" in k for k in _sap_kernels(t))
+    want = run_checker(oracle, "sap", d, dtype)
+    for k in want:
+        assert_parity(first[k], want[k], k)
+        assert np.array_equal(first[k], again[k]), k
+    for name, size in (("indices_A", 9), ("indices_B", 6), ("indices_output", 17)):
+        bad = dict(t, **{name: t[name].clone()})
+        bad[name][123] = size
+        idx = (bad["indices_A"], bad["indices_B"], bad["indices_output"])
+        with pytest.raises(M.MopsError, match=f"Index array {name} "):
+            M.sparse_accumulation_of_products(t["A"], t["B"], t["C"], *idx, 17)
+        with pytest.raises(M.MopsError, match=f"Index array {name} "):
+            M.sparse_accumulation_of_products_vjp(t["grad_output"], t["A"], t["B"], t["C"], *idx)
+    got = run_library("sap", t)
+    assert all(np.array_equal(first[k], got[k]) for k in first)
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
