@@ -135,8 +135,8 @@ template <typename T, int NF, int W> __device__ __forceinline__ void await(Batch
         for (int k = 0; k < NF; k++) tmem_pin(g.v[b][k]);
 }
 
-// acc[r] += the coefficient times the NF factors of row r, for every record of the batch.
-template <typename T, int NF, int W>
+// acc[r] += the coefficient times the NF factors of row r, for every record of the batch. PRODUCTS: c (a b).
+template <typename T, int NF, int W, bool PRODUCTS = false>
 __device__ __forceinline__ void add_terms(const Batch<T, NF, W>& g, const Records<T, NF, W>& rec,
                                           T (&acc)[Batch<T, NF, W>::R]) {
 #pragma unroll
@@ -148,13 +148,54 @@ __device__ __forceinline__ void add_terms(const Batch<T, NF, W>& g, const Record
             c = __uint_as_float(rec.w[b][0]);
 #pragma unroll
         for (int r = 0; r < Batch<T, NF, W>::R; r++) {
-            // (the coefficient first: a product of operands alone may leave the range where the term does not)
-            T p = c;
+            if constexpr (PRODUCTS) {
+                acc[r] += c * (tmem_value<T>(g.v[b][0], r) * tmem_value<T>(g.v[b][1], r));
+            } else {
+                T p = c;
 #pragma unroll
-            for (int k = 0; k + 1 < NF; k++) p *= tmem_value<T>(g.v[b][k], r);
-            acc[r] += p * tmem_value<T>(g.v[b][NF - 1], r);
+                for (int k = 0; k + 1 < NF; k++) p *= tmem_value<T>(g.v[b][k], r);
+                acc[r] += p * tmem_value<T>(g.v[b][NF - 1], r);
+            }
         }
     }
+}
+
+// ---------------------------------------------------------------- products of operands
+// A product a b may overflow or lose bits to underflow where the term c a b does neither (f32: c = 1e-30,
+// a = b = 1e25), so terms are (c a) b. The f64 forward of SAP takes c (a b) all the same, because large batches
+// form the products once per row (sap_tmem.cu) and a row's sums are to be the same bits in any batch; rows with
+// products out of range are found first, and their terms are (c a) b there, too.
+
+// Exponents of the values of a row that are not zero: whether all products with another row's are normal
+// numbers. (Conservative by one; infinities and NaN come out of c (a b) as they do of (c a) b.)
+template <typename T> struct ExponentRange {
+    static constexpr int kMantissa = sizeof(T) == 8 ? 20 : 23, kBias = sizeof(T) == 8 ? 1023 : 127;
+    uint32_t least = 0xffffffffu, most = 0; // of |v|'s upper word; `least` less one, so that zeros do not count
+    __device__ __forceinline__ void add(T v) {
+        uint32_t word;
+        if constexpr (sizeof(T) == 8) // (a lower word alone makes a value that is not zero)
+            word = (static_cast<uint32_t>(__double2hiint(v)) & 0x7fffffffu) | min(static_cast<uint32_t>(__double2loint(v)), 1u);
+        else
+            word = __float_as_uint(v) & 0x7fffffffu;
+        least = min(least, word - 1);
+        most = max(most, word);
+    }
+    __device__ __forceinline__ bool products_are_normal(const ExponentRange& o) const {
+        if (most == 0 || o.most == 0) return true; // zeros only
+        const int lo = static_cast<int>((least + 1) >> kMantissa), o_lo = static_cast<int>((o.least + 1) >> kMantissa);
+        return lo > 0 && o_lo > 0 && lo + o_lo > kBias + 1 &&
+               static_cast<int>((most >> kMantissa) + (o.most >> kMantissa)) < 3 * kBias;
+    }
+};
+
+// Whether the products of two rows are normal numbers: of every `step`-th value of a from a0 on, all of b.
+template <typename T>
+__device__ __forceinline__ bool products_are_normal(const unsigned char* a, const unsigned char* b, int nA, int nB,
+                                                    int a0 = 0, int step = 1) {
+    ExponentRange<T> range_a, range_b;
+    for (int i = a0; i < nA; i += step) range_a.add(reinterpret_cast<const T*>(a)[i]);
+    for (int i = 0; i < nB; i++) range_b.add(reinterpret_cast<const T*>(b)[i]);
+    return range_a.products_are_normal(range_b);
 }
 
 // f32 sums are taken in pieces of 32 records, which are then added up: one chain over a column's records
@@ -515,10 +556,44 @@ __device__ __forceinline__ int group_column(const int32_t* starts, int columns, 
     return lo;
 }
 
+// PRODUCTS: the columns [n_lo, n_hi) of a tile with a row whose products leave the range (`normal` says which of
+// the lane's do not), straight from the table and to the one result.
+template <typename T, int W>
+__device__ __noinline__ void gather_by_factors(const unsigned char* __restrict__ records, const int32_t* starts, int n_lo,
+                                            int n_hi, uint32_t base, unsigned normal, T* out, int columns,
+                                            int64_t row0, int64_t I) {
+    constexpr int R = W / words_of(sizeof(T)), RB = tmem_record_bytes(sizeof(T), 2);
+    for (int n = n_lo; n < n_hi; n++) {
+        T sum[R];
+#pragma unroll
+        for (int r = 0; r < R; r++) sum[r] = T(0);
+        const int end = uniform(starts[n + 1]);
+        for (int x = uniform(starts[n]); x < end; x++) {
+            const uint4 w = __ldg(reinterpret_cast<const uint4*>(records + static_cast<size_t>(x) * RB));
+            const T c = __hiloint2double(static_cast<int>(w.y), static_cast<int>(w.x));
+            uint32_t a[W], b[W];
+            tmem_load(__byte_perm(w.z, base, 0x7610), a);
+            tmem_load(__byte_perm(w.z, base, 0x7632), b);
+            tmem_wait_load();
+            tmem_pin(a);
+            tmem_pin(b);
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                const T va = tmem_value<T>(a, r), vb = tmem_value<T>(b, r);
+                const bool products = normal >> r & 1;
+                sum[r] = fma(products ? c : c * va, products ? va * vb : vb, sum[r]);
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < R; r++)
+            if (row0 + r * kSlabRows < I) out[(row0 + r * kSlabRows) * columns + n] = sum[r];
+    }
+}
+
 // The result columns are split among parts * 4 warp groups by number of records; a group's four
 // warps (one per quadrant) walk the same records for their own rows, add them up in registers, and
 // store a result when a column ends. `parts` blocks share a tile (they need no reduction).
-template <typename T, int NF, int W>
+template <typename T, int NF, int W, bool PRODUCTS = false>
 __global__ void __launch_bounds__(kTmemThreads, 1)
 gather_sums(const __grid_constant__ Results<T> results, const __grid_constant__ Operands operands,
             const unsigned char* __restrict__ records, const int32_t* __restrict__ n_start, int64_t I,
@@ -560,8 +635,28 @@ gather_sums(const __grid_constant__ Results<T> results, const __grid_constant__ 
     Ring ring(smem + group * 4096, full[group], group, (warp & 3) == 0 && lane == 0,
               records + static_cast<size_t>(x_lo) * RB, batches * B * RB);
     for (int64_t tile = first; tile < tiles; tile += step) {
-        t.load(tile + step < tiles ? tile + step : -1, base, tid, warp, lane);
+        t.load(!PRODUCTS && tile + step < tiles ? tile + step : -1, base, tid, warp, lane);
         const int64_t row0 = tile * (kSlabRows * R) + (warp & 3) * 32 + lane;
+        bool by_factors = false;
+        if constexpr (PRODUCTS) {
+            const int nA = operands.cols[0], nB = operands.cols[1], own = (warp & 3) * 32 + lane;
+            const int a_stride = slab_stride(nA * static_cast<int>(sizeof(T)));
+            const unsigned char* a = slabs + own * a_stride;
+            const unsigned char* b = slabs + kSlabRows * a_stride + own * slab_stride(nB * static_cast<int>(sizeof(T)));
+            int out_of_range = 0; // (rows behind the last one hold anything)
+            for (int r = 0; r < R; r++)
+                out_of_range |= row0 + r * kSlabRows < I &&
+                                !products_are_normal<T>(a + r * t.slab, b + r * t.slab, nA, nB, group, kTmemGroups);
+            by_factors = uniform(__syncthreads_or(out_of_range)) != 0;
+            if (by_factors) {
+                unsigned normal = 0;
+                for (int r = 0; r < R; r++)
+                    normal |= products_are_normal<T>(a + r * t.slab, b + r * t.slab, nA, nB) ? 1u << r : 0u;
+                gather_by_factors<T, W>(records, starts, n_lo, n_hi, base, normal, results.data[0], results.cols[0], row0, I);
+                __syncthreads();
+            }
+            if (tile + step < tiles) t.start(tile + step, tid);
+        }
         T acc[R];
         PieceSum<T, R> sum;
         sum.clear();
@@ -596,7 +691,7 @@ gather_sums(const __grid_constant__ Results<T> results, const __grid_constant__ 
                 at = results.data[which_result] + row0 * cols;
             }
         };
-        if (batches > 0) {
+        if (batches > 0 && !by_factors) {
             ring.start_tile();
             G x, y;
             Records<T, NF, W> rx, ry;
@@ -613,7 +708,7 @@ gather_sums(const __grid_constant__ Results<T> results, const __grid_constant__ 
             for (int i = 0;; i += 2) {
                 await<T, NF, W>(x);
                 issue<T, NF, W>(y, ry, base);
-                add_terms<T, NF, W>(x, rx, acc);
+                add_terms<T, NF, W, PRODUCTS>(x, rx, acc);
                 ahead += 2 * B * RB;
                 if (__builtin_expect(--in_stage == 0, 0)) {
                     if (i + 2 < batches) ring.enter_stage(++stage, lane, st);
@@ -623,7 +718,7 @@ gather_sums(const __grid_constant__ Results<T> results, const __grid_constant__ 
                 fetch<T, NF, W>(rx, ahead);
                 await<T, NF, W>(y);
                 issue<T, NF, W>(x, rx, base);
-                add_terms<T, NF, W>(y, ry, acc);
+                add_terms<T, NF, W, PRODUCTS>(y, ry, acc);
                 sum.template piece<B>(i, acc);
                 if (__builtin_expect(--left == 0, 0)) {
                     close();
@@ -716,7 +811,7 @@ void launch_gather(const Call& call, Kernel kernel, const GatherShape& s, int cl
 // Builds (or takes from the plan) the table of M records over results.total columns and runs the
 // sums. `key` names the table: kind, arrays and sizes; n[8], n[9] are filled in here. Returns
 // false when the problem does not fit (operands too wide for TMEM, too many records to sort).
-template <typename T, int NF, typename Source>
+template <typename T, int NF, bool PRODUCTS = false, typename Source>
 bool run_gather(const Call& call, TableKey key, const Source& source, int64_t M, const Operands& op,
                 const Results<T>& results, int64_t I, const char* name) {
     constexpr int RB = tmem_record_bytes(sizeof(T), NF);
@@ -750,11 +845,11 @@ bool run_gather(const Call& call, TableKey key, const Source& source, int64_t M,
                       static_cast<const int32_t*>(n_start), I, s.parts, s.tiles, call.status);
     };
     if (s.w == 8) {
-        if constexpr (NF * 8 <= 32 && sizeof(T) == 8) go(gather_sums<T, NF, 8>);
+        if constexpr (NF * 8 <= 32 && sizeof(T) == 8) go(gather_sums<T, NF, 8, PRODUCTS>);
     } else if (s.w == 4) {
-        go(gather_sums<T, NF, 4>);
+        go(gather_sums<T, NF, 4, PRODUCTS>);
     } else {
-        go(gather_sums<T, NF, 2>);
+        go(gather_sums<T, NF, 2, PRODUCTS>);
     }
     release_table(call, ref);
     return true;

@@ -80,7 +80,7 @@ template <typename T> bool narrow_backward(const SapProblem<T>& p, bool both) {
     return sizeof(T) == 8 ? p.K + 6 * cells + 8 * columns < 454 : p.K + 8 * cells + 3 * columns < 590;
 }
 
-template <typename T>
+template <typename T, bool PRODUCTS = false>
 bool run(const Call& call, const SapProblem<T>& p, const Family* families, int count, const Operands& op,
          const Results<T>& results, int level, const char* name) {
     SapSource<T> source{p.C, {p.PA, p.PB, p.PO}, {p.nA, p.nB, p.nO}, static_cast<int>(p.K), {}};
@@ -91,7 +91,7 @@ bool run(const Call& call, const SapProblem<T>& p, const Family* families, int c
     key.n[0] = p.K, key.n[1] = p.nA, key.n[2] = p.nB, key.n[3] = p.nO;
     key.n[4] = level, key.n[5] = 1;
     if (p.K * count > (1 << 20)) return false;
-    return run_gather<T, 2>(call, key, source, p.K * count, op, results, p.I, name);
+    return run_gather<T, 2, PRODUCTS>(call, key, source, p.K * count, op, results, p.I, name);
 }
 
 // ---------------------------------------------------------------- large batches
@@ -296,34 +296,14 @@ struct StageGuard {
     }
 };
 
-// Exponents of the values of a row that are not zero: whether all products with another row's are normal
-// numbers. (Conservative by one; infinities and NaN come out of c (a b) as they do of (c a) b.)
-template <typename T> struct ExponentRange {
-    static constexpr int kMantissa = sizeof(T) == 8 ? 20 : 23, kBias = sizeof(T) == 8 ? 1023 : 127;
-    uint32_t least = 0xffffffffu, most = 0; // of |v|'s upper word; `least` less one, so that zeros do not count
-    __device__ __forceinline__ void add(T v) {
-        uint32_t word;
-        if constexpr (sizeof(T) == 8) // (a lower word alone makes a value that is not zero)
-            word = (static_cast<uint32_t>(__double2hiint(v)) & 0x7fffffffu) | min(static_cast<uint32_t>(__double2loint(v)), 1u);
-        else
-            word = __float_as_uint(v) & 0x7fffffffu;
-        least = min(least, word - 1);
-        most = max(most, word);
-    }
-    __device__ __forceinline__ bool products_are_normal(const ExponentRange& o) const {
-        if (most == 0 || o.most == 0) return true; // zeros only
-        const int lo = static_cast<int>((least + 1) >> kMantissa), o_lo = static_cast<int>((o.least + 1) >> kMantissa);
-        return lo > 0 && o_lo > 0 && lo + o_lo > kBias + 1 &&
-               static_cast<int>((most >> kMantissa) + (o.most >> kMantissa)) < 3 * kBias;
-    }
-};
-
 // The columns [n_lo, n_hi) of a tile by factors: the records are those of products (NF = 1), but TMEM holds the
-// operands, A's columns, then B's; the coefficient comes first in every term. (`cell / nB` by multiplication is
-// exact up to 256 cells.) A call of its own, so that the loop over products keeps its registers.
+// operands, A's columns, then B's; the coefficient comes first in the terms of rows that are not `normal`.
+// (`cell / nB` by multiplication is exact up to 256 cells.) A call of its own, so that the loop over products keeps
+// its registers.
 template <typename T, int W>
 __device__ __noinline__ void sum_by_factors(const ResidentRecords<T, 1> records, const int32_t* starts, int n_lo, int n_hi,
-                                            uint32_t base, int nA, int nB, int ones, unsigned char* results, int row_step) {
+                                            uint32_t base, int nA, int nB, int ones, unsigned normal,
+                                            unsigned char* results, int row_step) {
     constexpr int R = kLaneRows<T, W>;
     const uint32_t reciprocal = (65536u + nB - 1) / nB;
     for (int n = n_lo; n < n_hi; n++) {
@@ -346,8 +326,11 @@ __device__ __noinline__ void sum_by_factors(const ResidentRecords<T, 1> records,
 #pragma unroll
             for (int b = 0; b < kLot; b++)
 #pragma unroll
-                for (int r = 0; r < R; r++)
-                    part[r] += rec.c[b] * tmem_value<T>(g.v[b][0], r) * tmem_value<T>(g.v[b][1], r);
+                for (int r = 0; r < R; r++) {
+                    const T va = tmem_value<T>(g.v[b][0], r), vb = tmem_value<T>(g.v[b][1], r);
+                    const bool products = normal >> r & 1;
+                    part[r] = fma(products ? rec.c[b] : rec.c[b] * va, products ? va * vb : vb, part[r]);
+                }
             if (sizeof(T) == 4 && ((i - first) & (kPieceRecords / kLot - 1)) == kPieceRecords / kLot - 1) {
 #pragma unroll
                 for (int r = 0; r < R; r++) {
@@ -357,7 +340,7 @@ __device__ __noinline__ void sum_by_factors(const ResidentRecords<T, 1> records,
             }
         }
 #pragma unroll
-        for (int r = 0; r < R; r++) reinterpret_cast<T*>(results + r * row_step)[n] = sum[r] + part[r];
+        for (int r = 0; r < R; r++) reinterpret_cast<T*>(results + r * row_step)[n] = sizeof(T) == 8 ? part[r] : sum[r] + part[r];
     }
 }
 
@@ -366,10 +349,9 @@ __device__ __noinline__ void sum_by_factors(const ResidentRecords<T, 1> records,
 // (NF = 2; f64 has half the rows per lane here, which gather_sums does not: 10^6 rows, 24 x 11 -> 56, 1321
 // triplets: 520 -> 690 us).
 //
-// A product a b may overflow or lose bits to underflow where the term C a b does neither (f32: C = 1e-30,
-// a = b = 1e25). A tile with a row for which that is possible is done by factors, C a first, as everywhere else.
-// 2^20 rows, 20 x 6 -> 50, 1000 triplets: looking at the operands' exponents makes 305 us 317 (f64) and 198 us
-// 210 (f32); with such a row in every tile it is 640 and 400 (all by gather_sums: 365, 360).
+// A tile with a row whose products may leave the range (ExponentRange) is done by factors.
+// 2^20 rows, 20 x 6 -> 50, 1000 triplets, a call: looking at the operands' exponents makes 318 us 331 (f64) and
+// 210 us 228 (f32); with such a row in every tile it takes 656 and 408 (all by gather_sums: 378, 375).
 template <typename T> struct ProductSource {
     const T* C;
     const int32_t *PA, *PB, *PO;
@@ -502,7 +484,11 @@ sap_fwd_resident(T* __restrict__ O, const __grid_constant__ Operands operands, c
         tmem_fence_before_sync();
         const bool by_factors = uniform(__syncthreads_or(out_of_range)) != 0;
         tmem_fence_after_sync();
+        unsigned normal = 0;
         if (NF == 1 && by_factors) {
+            for (int r = 0; r < R; r++)
+                normal |= products_are_normal<T>(t.slabs + r * t.slab + own * a_stride,
+                                                 t.slabs + r * t.slab + kSlabRows * a_stride + own * b_stride, nA, nB) ? 1u << r : 0u;
             slabs_to_tmem<T, W>(t.slabs, t.slab, a_stride, nA, base, warp, lane);
             slabs_to_tmem<T, W>(t.slabs + kSlabRows * a_stride, t.slab, b_stride, nB, base + nA * W, warp, lane);
             tmem_wait_store();
@@ -546,11 +532,12 @@ sap_fwd_resident(T* __restrict__ O, const __grid_constant__ Operands operands, c
                 left = n < n_hi ? uniform(starts[n + 1] - starts[n]) / kLot : 0;
             }
         };
-        constexpr int kChains = sizeof(T) == 8 ? 1 : 2;
+        constexpr int kChains = sizeof(T) == 8 ? 1 : 2; // (f64: in the order of gather_sums)
         if constexpr (NF == 1) {
             if (by_factors) {
                 guard.pass(warp, lane, st);
-                sum_by_factors<T, W>(records, starts, n_lo, n_hi, base, nA, nB, ones, own_results, kSlabRows * stage.stride);
+                sum_by_factors<T, W>(records, starts, n_lo, n_hi, base, nA, nB, ones, normal, own_results,
+                                     kSlabRows * stage.stride);
             }
         }
         walk_lots<kChains, T, NF, W>(records, first, NF == 1 && by_factors ? 0 : count, base, acc, after);
@@ -646,8 +633,7 @@ sap_vjp_resident(T* __restrict__ gT, T* __restrict__ gS, const __grid_constant__
             const int c = c0 + lane, t = c / nS, s = c - t * nS;
             const int batches = c < c_hi ? (starts[c + 1] - starts[c]) / kLot : 0;
             const unsigned some = __ballot_sync(kFullMask, batches > 0);
-            if (batches > 0)
-            {
+            if (batches > 0) {
                 uint32_t present = 0;
                 for (int s2 = 0; s2 < nS; s2++)
                     present |= starts[t * nS + s2 + 1] > starts[t * nS + s2] ? 1u << s2 : 0u;
@@ -1117,7 +1103,7 @@ template <typename T> bool sap_forward_tmem(const Call& call, const SapProblem<T
     Results<T> results{};
     results.add(O, p.nO);
     const Family f[] = {{kO, 0, {kA, kB}, {0, p.nA}}};
-    return run(call, p, f, 1, op, results, 0, "sap_fwd_tmem");
+    return run<T, sizeof(T) == 8>(call, p, f, 1, op, results, 0, "sap_fwd_tmem");
 }
 
 template <typename T>

@@ -232,6 +232,32 @@ def test_products_of_operands_out_of_range(oracle, op, kw, kernel, every, large,
     assert_parity(got.astype(dtype), want.astype(dtype), f"{op} {kw}")
 
 
+@pytest.mark.parametrize("kw,kernel", [(dict(I=148 * 256 + 31, nA=20, nB=6, nO=50, K=700), "sap_fwd_resident<f64,NF=1,W=4>"),
+                                       (dict(I=148 * 128 + 31, nA=9, nB=11, nO=20, K=500), "sap_fwd_resident<f64,NF=1,W=2>"),
+                                       (dict(I=148 * 256 + 31, nA=16, nB=11, nO=30, K=900), "sap_fwd_tmem")])
+def test_sap_rows_do_not_depend_on_the_batch(kw, kernel):
+    """f64 forward: the same bits for a row in a large batch and in a small one, next to rows whose products of
+    operands overflow or underflow, and for these rows themselves."""
+    import torch
+    d = workloads.sap(**kw)
+    d["C"] = np.ldexp(d["C"], -400)
+    for row, a, b in ((1010, 600, -600), (1077, 660, 660), (1080, -300, -300), (kw["I"] - 3, 700, 400), (kw["I"] - 9, -400, -660)):
+        d["A"][row], d["B"][row] = np.ldexp(d["A"][row], a), np.ldexp(d["B"][row], b)
+    t = to_dev(d, np.float64)
+
+    def forward(rows):
+        return M.sparse_accumulation_of_products(t["A"][rows].contiguous(), t["B"][rows].contiguous(), t["C"],
+                                                 t["indices_A"], t["indices_B"], t["indices_output"], t["output_size"])
+
+    whole = forward(slice(None))
+    assert torch.isfinite(whole).all()
+    assert _lib.last_kernels()[0].startswith(kernel)
+    for rows in (slice(0, 300), slice(1000, 1100), slice(1077, 1078), slice(5000, 9097), slice(kw["I"] - 40, None)):
+        part = forward(rows)
+        assert _lib.last_kernels()[0].startswith("sap_fwd_tmem")
+        assert torch.equal(whole[rows], part), rows
+
+
 @pytest.mark.parametrize("op,kw", [("hpe", dict(I=300, N=13, J=6400, K=4)), ("hpe", dict(I=20000, N=8, J=2000, K=3)),
                                    ("sap", dict(I=100, nA=32, nB=2, nO=3, K=4100)),
                                    ("sap", dict(I=5000, nA=9, nB=15, nO=2, K=2000))])
