@@ -216,3 +216,44 @@ def test_gradients_by_the_lengths_of_rows(oracle, op, K, L, per_row, dtype):
     t = to_dev(d, dtype)
     assert _streamed(op, t)[1] == _long_rows(op, E, n, K, L, dtype)
     compare(op, d, dtype, oracle, what=f"{op} {K}x{L} {per_row}")
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("op", ["opsa", "opsaw"])
+def test_streamed_in_sorted_order_with_skipped_gradients_plans_and_bad_indices(oracle, op, dtype):
+    E, n, K, L = 12007, 150, 13, 32
+    d = workloads.opsa(J=E, K=K, L=L, nO=n) if op == "opsa" else workloads.opsaw(E=E, K=K, L=L, n=n)
+    d["indices_output"] = np.random.default_rng(3).permutation(d["indices_output"])
+    t = to_dev(d, dtype)
+    assert _streamed(op, t) == (True, True)
+    want = run_checker(oracle, op, d, np.float64)
+    with M.Plan():  # (does not keep the table of an unsorted index)
+        for _ in range(2):
+            compare(op, d, dtype, oracle, what=f"{op} in a plan")
+    forward, vjp = ((M.outer_product_scatter_add, M.outer_product_scatter_add_vjp) if op == "opsa" else
+                    (M.outer_product_scatter_add_with_weights, M.outer_product_scatter_add_with_weights_vjp))
+    names = ("A", "B") if op == "opsa" else ("A", "B", "W")
+    index = ("indices_output",) if op == "opsa" else ("indices_W", "indices_output")
+
+    def call(function, tensors, *before, **keep):
+        size = (tensors["output_size"],) if function is forward and op == "opsa" else ()
+        return function(*before, *[tensors[k] for k in names], *[tensors[k] for k in index], *size, **keep)
+
+    for skipped in names:
+        got = call(vjp, t, t["grad_output"], **{f"compute_grad_{k}": k != skipped for k in names})
+        assert any("gathered" in k for k in _lib.last_kernels())
+        for k, g in zip(names, got):
+            assert (g is None) == (k == skipped)
+            if g is not None:
+                scale = np.abs(want[f"grad_{k}"]).max()
+                tolerance = (1e-12 if dtype == np.float64 else 1e-5) * scale
+                assert np.abs(g.cpu().numpy().astype(np.float64) - want[f"grad_{k}"]).max() <= tolerance, (skipped, k)
+    for name in index:
+        for value in (n, -1):
+            bad = dict(t, **{name: t[name].clone()})
+            bad[name][4321] = value
+            with pytest.raises(M.MopsError, match=f"Index array {name} "):
+                call(forward, bad)
+            with pytest.raises(M.MopsError, match=f"Index array {name} "):
+                call(vjp, bad, t["grad_output"])
+    compare(op, d, dtype, oracle, what=f"{op} afterwards")
