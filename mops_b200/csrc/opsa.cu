@@ -744,8 +744,10 @@ void forward(const Call& call, T* O, const T* A, const T* B, const T* W, const i
             wait_stream(call);
             need_fallback = host_saw_unsorted(call);
         }
-        // Few products: atomics per entry are done before the sort is (its six grid barriers are 15 us;
-        // 2700 entries of 6 x 80: 39 against 56 us, 8800 of 4 x 64: 46 against 57).
+        // Few products: atomics per entry are done before the sort is. Time behind a sort / by atomics, at the
+        // line: 0.94 to 1.06 for 9 x 20 and 13 x 32 in calls that wait (at twice as many 0.76 to 0.89), where
+        // the sorted entries are streamed; rows of 4 x 8 cross at 6 10^6, of 6 x 80, which are not streamed, at 10^7,
+        // of 1 x 4 not by 1.2 10^7 (1.9 to 3.5). Asynchronous calls: 1.4 to 2.3, crossing at 8 10^6 to 1.2 10^7.
         if (need_fallback && positions_fit_int(J) && J * KL > kFewProducts) {
             // (Asynchronous calls, which mostly have nothing to do here, make do with one launch.)
             if (!call.wait || !opsa_forward_gathered<T, WEIGHTED>(call, O, A, B, W, PW, P, J, K, L, nO))

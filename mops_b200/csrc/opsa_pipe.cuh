@@ -14,7 +14,7 @@
 // of kilobytes per SM in flight, row boundaries do not interrupt the stream, and the
 // instruction stream is almost only fragment reads and MMAs.
 //
-// Included by opsa.cu (inside its unnamed namespace).
+// Included by opsa.cu and opsa_gathered.cu (inside their unnamed namespaces).
 
 struct PipeLayout {
     int K, L;     // widths of A and B
@@ -302,7 +302,6 @@ __device__ __forceinline__ PipeLayout fixed_layout_or(const PipeLayout& run_time
     }
 }
 
-//
 // GATHERED: an index that is not sorted. The positions are those of a sorted order, `perm`, and the warps
 // split them (`segment` each), not the rows: what a warp has of a row that others share it adds to what is
 // there (zeros: zero_cut_rows).

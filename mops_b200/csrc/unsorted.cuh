@@ -6,7 +6,7 @@
 // row is written once, by one warp, and the entries that share a grad_output row are neighbours.
 // 300 000 entries of 16 x 32, f32: forward 735 us with atomics -> 165 us (23 of them the sort), VJP
 // 209 us in the order of the entries -> 23 + 103 us. (Calls that wait for the result stream the sorted
-// entries instead: opsa_gathered.cu.)
+// entries instead where that is faster: opsa_gathered.cu.)
 #ifndef MOPS_B200_UNSORTED_CUH
 #define MOPS_B200_UNSORTED_CUH
 
