@@ -163,39 +163,22 @@ __device__ __forceinline__ void add_terms(const Batch<T, NF, W>& g, const Record
 // ---------------------------------------------------------------- products of operands
 // A product a b may overflow or lose bits to underflow where the term c a b does neither (f32: c = 1e-30,
 // a = b = 1e25), so terms are (c a) b. The f64 forward of SAP takes c (a b) all the same, because large batches
-// form the products once per row (sap_tmem.cu) and a row's sums are to be the same bits in any batch; rows with
-// products out of range are found first, and their terms are (c a) b there, too.
+// form the products once per row (sap_tmem.cu) and a row's sums are to be the same bits in any batch; rows whose
+// products might be out of range (out_of_band) are found first, and their terms are (c a) b there, too.
 
-// Exponents of the values of a row that are not zero: whether all products with another row's are normal
-// numbers. (Conservative by one; infinities and NaN come out of c (a b) as they do of (c a) b.)
-template <typename T> struct ExponentRange {
-    static constexpr int kMantissa = sizeof(T) == 8 ? 20 : 23, kBias = sizeof(T) == 8 ? 1023 : 127;
-    uint32_t least = 0xffffffffu, most = 0; // of |v|'s upper word; `least` less one, so that zeros do not count
-    __device__ __forceinline__ void add(T v) {
-        uint32_t word;
-        if constexpr (sizeof(T) == 8) // (a lower word alone makes a value that is not zero)
-            word = (static_cast<uint32_t>(__double2hiint(v)) & 0x7fffffffu) | min(static_cast<uint32_t>(__double2loint(v)), 1u);
-        else
-            word = __float_as_uint(v) & 0x7fffffffu;
-        least = min(least, word - 1);
-        most = max(most, word);
+// Which of the lane's rows of `columns` values in TMEM have none out_of_band, a bit each.
+template <typename T, int W> __device__ __forceinline__ unsigned rows_in_band(uint32_t base, int columns) {
+    unsigned rows = ~0u;
+    for (int n = 0; n < columns; n++) {
+        uint32_t v[W];
+        tmem_load(base + n * W, v);
+        tmem_wait_load();
+        tmem_pin(v);
+#pragma unroll
+        for (int r = 0; r < W / words_of(sizeof(T)); r++)
+            rows &= ~(out_of_band(tmem_value<T>(v, r)) << r);
     }
-    __device__ __forceinline__ bool products_are_normal(const ExponentRange& o) const {
-        if (most == 0 || o.most == 0) return true; // zeros only
-        const int lo = static_cast<int>((least + 1) >> kMantissa), o_lo = static_cast<int>((o.least + 1) >> kMantissa);
-        return lo > 0 && o_lo > 0 && lo + o_lo > kBias + 1 &&
-               static_cast<int>((most >> kMantissa) + (o.most >> kMantissa)) < 3 * kBias;
-    }
-};
-
-// Whether the products of two rows are normal numbers: of every `step`-th value of a from a0 on, all of b.
-template <typename T>
-__device__ __forceinline__ bool products_are_normal(const unsigned char* a, const unsigned char* b, int nA, int nB,
-                                                    int a0 = 0, int step = 1) {
-    ExponentRange<T> range_a, range_b;
-    for (int i = a0; i < nA; i += step) range_a.add(reinterpret_cast<const T*>(a)[i]);
-    for (int i = 0; i < nB; i++) range_b.add(reinterpret_cast<const T*>(b)[i]);
-    return range_a.products_are_normal(range_b);
+    return rows;
 }
 
 // f32 sums are taken in pieces of 32 records, which are then added up: one chain over a column's records
@@ -267,8 +250,11 @@ template <typename T, int W> struct Tiles {
         tmem_wait_store();
     }
     // Brings the tile started before into TMEM and starts tile `next` (if >= 0). Ends with the block
-    // synchronised.
-    __device__ void load(int64_t next, uint32_t base, int tid, int warp, int lane) const {
+    // synchronised. CHECK: whether no value of the block's rows of the batch (`live`: the lane's, a bit each) is
+    // out_of_band.
+    template <bool CHECK = false>
+    __device__ bool load(int64_t next, uint32_t base, int tid, int warp, int lane, unsigned live = 0) const {
+        unsigned bad = 0;
         cp_async_wait<0>();
         tmem_fence_before_sync();
         __syncthreads();
@@ -277,15 +263,20 @@ template <typename T, int W> struct Tiles {
         uint32_t column = base;
         for (int q = 0; q < op.count; q++) {
             const int stride = slab_stride(op.cols[q] * static_cast<int>(sizeof(T)));
-            slabs_to_tmem<T, W>(src, slab, stride, op.cols[q], column, warp, lane);
+            bad |= slabs_to_tmem<T, W, CHECK>(src, slab, stride, op.cols[q], column, warp, lane);
             src += kSlabRows * stride;
             column += op.cols[q] * W;
         }
         tmem_wait_store();
         tmem_fence_before_sync();
-        __syncthreads();
+        bool good = true;
+        if constexpr (CHECK)
+            good = uniform(__syncthreads_or(bad & live)) == 0;
+        else
+            __syncthreads();
         tmem_fence_after_sync();
         if (next >= 0) start(next, tid);
+        return good;
     }
 };
 
@@ -556,8 +547,8 @@ __device__ __forceinline__ int group_column(const int32_t* starts, int columns, 
     return lo;
 }
 
-// PRODUCTS: the columns [n_lo, n_hi) of a tile with a row whose products leave the range (`normal` says which of
-// the lane's do not), straight from the table and to the one result.
+// PRODUCTS: the columns [n_lo, n_hi) of a tile with values out_of_band (`normal`: the lane's rows without),
+// straight from the table and to the one result.
 template <typename T, int W>
 __device__ __noinline__ void gather_by_factors(const unsigned char* __restrict__ records, const int32_t* starts, int n_lo,
                                             int n_hi, uint32_t base, unsigned normal, T* out, int columns,
@@ -635,27 +626,19 @@ gather_sums(const __grid_constant__ Results<T> results, const __grid_constant__ 
     Ring ring(smem + group * 4096, full[group], group, (warp & 3) == 0 && lane == 0,
               records + static_cast<size_t>(x_lo) * RB, batches * B * RB);
     for (int64_t tile = first; tile < tiles; tile += step) {
-        t.load(!PRODUCTS && tile + step < tiles ? tile + step : -1, base, tid, warp, lane);
-        const int64_t row0 = tile * (kSlabRows * R) + (warp & 3) * 32 + lane;
+        const int64_t row0 = tile * (kSlabRows * R) + (warp & 3) * 32 + lane, next = tile + step < tiles ? tile + step : -1;
         bool by_factors = false;
         if constexpr (PRODUCTS) {
-            const int nA = operands.cols[0], nB = operands.cols[1], own = (warp & 3) * 32 + lane;
-            const int a_stride = slab_stride(nA * static_cast<int>(sizeof(T)));
-            const unsigned char* a = slabs + own * a_stride;
-            const unsigned char* b = slabs + kSlabRows * a_stride + own * slab_stride(nB * static_cast<int>(sizeof(T)));
-            int out_of_range = 0; // (rows behind the last one hold anything)
-            for (int r = 0; r < R; r++)
-                out_of_range |= row0 + r * kSlabRows < I &&
-                                !products_are_normal<T>(a + r * t.slab, b + r * t.slab, nA, nB, group, kTmemGroups);
-            by_factors = uniform(__syncthreads_or(out_of_range)) != 0;
-            if (by_factors) {
-                unsigned normal = 0;
-                for (int r = 0; r < R; r++)
-                    normal |= products_are_normal<T>(a + r * t.slab, b + r * t.slab, nA, nB) ? 1u << r : 0u;
-                gather_by_factors<T, W>(records, starts, n_lo, n_hi, base, normal, results.data[0], results.cols[0], row0, I);
-                __syncthreads();
-            }
-            if (tile + step < tiles) t.start(tile + step, tid);
+            unsigned in_batch = 0; // (rows behind the last one hold anything)
+#pragma unroll
+            for (int r = 0; r < R; r++) in_batch |= row0 + r * kSlabRows < I ? 1u << r : 0u;
+            by_factors = !t.template load<true>(next, base, tid, warp, lane, in_batch);
+            if (by_factors)
+                gather_by_factors<T, W>(records, starts, n_lo, n_hi, base,
+                                        rows_in_band<T, W>(base, operands.total), results.data[0],
+                                        results.cols[0], row0, I);
+        } else {
+            t.load(next, base, tid, warp, lane);
         }
         T acc[R];
         PieceSum<T, R> sum;
@@ -699,21 +682,32 @@ gather_sums(const __grid_constant__ Results<T> results, const __grid_constant__ 
             // closes it is there once)
             int left = uniform(starts[n_lo + 1] - starts[n_lo]) / (2 * B); // pairs of column n
             constexpr int kPairs = kPerStage / 2;                          // of a stage
+            // Pairs are counted down to the end of a stage, or looked at by their number: which is shorter depends on
+            // what else the compiler keeps in registers. One gradient, 300 000 rows, 20 x 6 -> 50, 12 000 triplets,
+            // f64, four rows' columns: 1157 us counted, 934 not; two more columns per load 234 and 250, f32 598 and
+            // 643, products first 686 and 780; hpe_large (3 factors) 3950 and 4320.
+            constexpr bool kCounted = PRODUCTS || sizeof(T) == 4 || NF != 2 || W != 4;
             int stage = 0, in_stage = kPairs; // pairs until the batches fetched ahead are the next stage's
             ring.enter_stage(0, lane, st);
             const unsigned char* ahead = ring.template at<B * RB>(0);
             fetch<T, NF, W>(rx, ahead);
             issue<T, NF, W>(x, rx, base);
             fetch<T, NF, W>(ry, ahead + B * RB);
-            for (int i = 0;; i += 2) {
+            for (int i = 0; kCounted || i < batches; i += 2) {
                 await<T, NF, W>(x);
                 issue<T, NF, W>(y, ry, base);
                 add_terms<T, NF, W, PRODUCTS>(x, rx, acc);
-                ahead += 2 * B * RB;
-                if (__builtin_expect(--in_stage == 0, 0)) {
-                    if (i + 2 < batches) ring.enter_stage(++stage, lane, st);
+                if constexpr (kCounted) {
+                    ahead += 2 * B * RB;
+                    if (__builtin_expect(--in_stage == 0, 0)) {
+                        if (i + 2 < batches) ring.enter_stage(++stage, lane, st);
+                        ahead = ring.template at<B * RB>(i + 2);
+                        in_stage = kPairs;
+                    }
+                } else {
+                    if ((i & (kPerStage - 1)) == kPerStage - 2 && i + 2 < batches)
+                        ring.enter_stage((i + 2) / kPerStage, lane, st);
                     ahead = ring.template at<B * RB>(i + 2);
-                    in_stage = kPairs;
                 }
                 fetch<T, NF, W>(rx, ahead);
                 await<T, NF, W>(y);
@@ -722,8 +716,8 @@ gather_sums(const __grid_constant__ Results<T> results, const __grid_constant__ 
                 sum.template piece<B>(i, acc);
                 if (__builtin_expect(--left == 0, 0)) {
                     close();
-                    if (n == n_hi) break; // (the last column ends with the last batch)
-                    left = uniform(starts[n + 1] - starts[n]) / (2 * B);
+                    if (kCounted && n == n_hi) break; // (the last column ends with the last batch)
+                    left = kCounted || n < n_hi ? uniform(starts[n + 1] - starts[n]) / (2 * B) : 0;
                 }
                 fetch<T, NF, W>(ry, ahead + B * RB);
             }

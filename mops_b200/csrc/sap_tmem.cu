@@ -349,7 +349,7 @@ __device__ __noinline__ void sum_by_factors(const ResidentRecords<T, 1> records,
 // (NF = 2; f64 has half the rows per lane here, which gather_sums does not: 10^6 rows, 24 x 11 -> 56, 1321
 // triplets: 520 -> 690 us).
 //
-// A tile with a row whose products may leave the range (ExponentRange) is done by factors.
+// A tile with values out_of_band is done by factors.
 // 2^20 rows, 20 x 6 -> 50, 1000 triplets, a call: looking at the operands' exponents makes 318 us 331 (f64) and
 // 210 us 228 (f32); with such a row in every tile it takes 656 and 408 (all by gather_sums: 378, 375).
 template <typename T> struct ProductSource {
@@ -426,12 +426,11 @@ sap_fwd_resident(T* __restrict__ O, const __grid_constant__ Operands operands, c
         before = tile * (kSlabRows * R);
         const int a_stride = slab_stride(nA * static_cast<int>(sizeof(T)));
         const int b_stride = slab_stride(nB * static_cast<int>(sizeof(T)));
-        int out_of_range = 0; // products of this thread's
+        unsigned bad = 0; // rows of the lane's in which this thread sees a value out_of_band
         if constexpr (NF == 1) {
             const unsigned char* a_row = t.slabs + own * a_stride;
             const unsigned char* b_row = t.slabs + kSlabRows * a_stride + own * b_stride;
             constexpr int words = words_of(sizeof(T)), kHeld = 8;
-            ExponentRange<T> range_a[R], range_b[R];
             for (int a0 = group; a0 < nA; a0 += kHeld * kTmemGroups) {
                 T va[kHeld][R];
 #pragma unroll
@@ -443,19 +442,18 @@ sap_fwd_resident(T* __restrict__ O, const __grid_constant__ Operands operands, c
                 for (int b = 0; b < nB; b += 2) { // (behind an odd last column a row is padded)
                     T vb[R][2];
 #pragma unroll
-                    for (int r = 0; r < R; r++) {
-                        load_vec<T, 2>(reinterpret_cast<const T*>(b_row + r * t.slab) + b, vb[r]);
-                        if (b + 1 == nB) vb[r][1] = T(0);
-                    }
+                    for (int r = 0; r < R; r++) load_vec<T, 2>(reinterpret_cast<const T*>(b_row + r * t.slab) + b, vb[r]);
+                    if ((b / 2) % kTmemGroups == group) // (every value is looked at by one thread)
 #pragma unroll
-                    for (int r = 0; r < R; r++) range_b[r].add(vb[r][0]), range_b[r].add(vb[r][1]);
+                        for (int r = 0; r < R; r++)
+                            bad |= (out_of_band(vb[r][0]) | (out_of_band(vb[r][1]) & static_cast<unsigned>(b + 1 < nB))) << r;
 #pragma unroll
                     for (int i = 0; i < kHeld; i++) {
                         const int a = a0 + i * kTmemGroups;
                         if (a >= nA) break;
                         if (b == 0)
 #pragma unroll
-                            for (int r = 0; r < R; r++) range_a[r].add(va[i][r]);
+                            for (int r = 0; r < R; r++) bad |= out_of_band(va[i][r]) << r;
                         uint32_t w[2 * W];
 #pragma unroll
                         for (int c = 0; c < 2; c++)
@@ -475,20 +473,16 @@ sap_fwd_resident(T* __restrict__ O, const __grid_constant__ Operands operands, c
             }
 #pragma unroll
             for (int r = 0; r < R; r++) // (rows behind the last one hold anything)
-                out_of_range |= !range_a[r].products_are_normal(range_b[r]) && before + r * kSlabRows + own < I;
+                if (before + r * kSlabRows + own >= I) bad &= ~(1u << r);
         } else {
             slabs_to_tmem<T, W>(t.slabs, t.slab, a_stride, nA, base, warp, lane);
             slabs_to_tmem<T, W>(t.slabs + kSlabRows * a_stride, t.slab, b_stride, nB, base + nA * W, warp, lane);
         }
         tmem_wait_store();
         tmem_fence_before_sync();
-        const bool by_factors = uniform(__syncthreads_or(out_of_range)) != 0;
+        const bool by_factors = uniform(__syncthreads_or(bad)) != 0;
         tmem_fence_after_sync();
-        unsigned normal = 0;
         if (NF == 1 && by_factors) {
-            for (int r = 0; r < R; r++)
-                normal |= products_are_normal<T>(t.slabs + r * t.slab + own * a_stride,
-                                                 t.slabs + r * t.slab + kSlabRows * a_stride + own * b_stride, nA, nB) ? 1u << r : 0u;
             slabs_to_tmem<T, W>(t.slabs, t.slab, a_stride, nA, base, warp, lane);
             slabs_to_tmem<T, W>(t.slabs + kSlabRows * a_stride, t.slab, b_stride, nB, base + nA * W, warp, lane);
             tmem_wait_store();
@@ -536,7 +530,8 @@ sap_fwd_resident(T* __restrict__ O, const __grid_constant__ Operands operands, c
         if constexpr (NF == 1) {
             if (by_factors) {
                 guard.pass(warp, lane, st);
-                sum_by_factors<T, W>(records, starts, n_lo, n_hi, base, nA, nB, ones, normal, own_results,
+                sum_by_factors<T, W>(records, starts, n_lo, n_hi, base, nA, nB, ones,
+                                     rows_in_band<T, W>(base, nA + nB), own_results,
                                      kSlabRows * stage.stride);
             }
         }

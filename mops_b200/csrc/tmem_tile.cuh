@@ -69,17 +69,30 @@ inline int copy_unit_of(const void* base, size_t row_bytes) {
     return both % 16 == 0 ? 16 : both % 8 == 0 ? 8 : 4;
 }
 
+// 0 if |v| is 0 or in [2^-511, 2^512) (f32: [2^-63, 2^64)), else 1: the product of two such values is 0 or a normal
+// number. (No branches: the loops that look at values also move them.)
+__device__ __forceinline__ unsigned out_of_band(double v) {
+    const uint32_t word = (static_cast<uint32_t>(__double2hiint(v)) & 0x7fffffffu) | min(static_cast<uint32_t>(__double2loint(v)), 1u);
+    return static_cast<unsigned>(word - (512u << 20) >= (1023u << 20)) & static_cast<unsigned>(word != 0);
+}
+__device__ __forceinline__ unsigned out_of_band(float v) {
+    const uint32_t word = __float_as_uint(v) & 0x7fffffffu;
+    return static_cast<unsigned>(word - (64u << 23) >= (127u << 23)) & static_cast<unsigned>(word != 0);
+}
+
 // Moves all R slabs of a tile from shared memory to the TMEM columns of one operand. `column0`: TMEM
 // address of the operand's first column in the warp's quadrant; `slab`: bytes from one slot's rows
 // to the next. The sixteen warps share the columns: warp group g takes 16-byte pieces g, g + 4, ...
 // of the rows; the columns of a piece, with their R slots each, are consecutive in TMEM and go
 // there in one store (one store per scalar took four to eight times as many, and most of the time
-// of a tile with few records).
-template <typename T, int W>
-__device__ __forceinline__ void slabs_to_tmem(const unsigned char* rows, int slab, int stride, int N,
+// of a tile with few records). CHECK: a bit for every slot of which the thread moved a
+// value out_of_band.
+template <typename T, int W, bool CHECK = false>
+__device__ __forceinline__ unsigned slabs_to_tmem(const unsigned char* rows, int slab, int stride, int N,
                                               uint32_t column0, int warp, int lane) {
     constexpr int per16 = 16 / sizeof(T), words = words_of(sizeof(T)), R = W / words;
     const unsigned char* row = rows + ((warp & 3) * 32 + lane) * stride;
+    unsigned bad = 0;
     for (int p = warp >> 2; p * per16 < N; p += kTmemGroups) {
         uint32_t r[per16 * W];
 #pragma unroll
@@ -88,6 +101,19 @@ __device__ __forceinline__ void slabs_to_tmem(const unsigned char* rows, int sla
             const uint32_t word[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
             for (int i = 0; i < 4; i++) r[i / words * W + s * words + i % words] = word[i];
+        }
+        if constexpr (CHECK) {
+#pragma unroll
+            for (int n = 0; n < per16; n++)
+#pragma unroll
+                for (int s = 0; s < R; s++) {
+                    T v;
+                    if constexpr (sizeof(T) == 8)
+                        v = __hiloint2double(static_cast<int>(r[n * W + 2 * s + 1]), static_cast<int>(r[n * W + 2 * s]));
+                    else
+                        v = __uint_as_float(r[n * W + s]);
+                    bad |= (out_of_band(v) & static_cast<unsigned>(p * per16 + n < N)) << s;
+                }
         }
         const uint32_t at = column0 + p * per16 * W;
         if ((p + 1) * per16 <= N) {
@@ -101,6 +127,7 @@ __device__ __forceinline__ void slabs_to_tmem(const unsigned char* rows, int sla
                         tmem_store(at + n * W + i, __uint_as_float(r[n * W + i]));
         }
     }
+    return bad;
 }
 
 } // namespace mops_b200
