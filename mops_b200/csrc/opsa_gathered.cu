@@ -52,15 +52,15 @@ template <typename T, bool WEIGHTED> PipeLayout gathered_layout(int K, int L, bo
 //
 //   f64, K L >= 400          0.50 - 0.95 from 1 on (weighted: 0.71 - 0.94 from 4 on, 0.91 - 1.15 at 2)
 //   f64, 256 <= K L < 400    0.70 - 1.06 from 8 on, 0.85 - 1.12 at 4
-//   f64, 128 <= K L < 256    0.79 - 1.05 from 32 on, 0.81 - 1.11 at 16; fewer products: 0.85 - 1.5 at any length
-//   f32, K L >= 400          0.84 - 0.99 from 32 on, 0.95 - 1.05 at 16
-//   f32, 256 <= K L < 400    0.91 - 1.05 from 64 on, 0.96 - 1.03 at 32; fewer products: 0.9 - 3.2
+//   f64, K L >= 128 or L >= 24   0.77 - 1.05 from 32 on, 0.81 - 1.11 at 16; fewer products 0.88 - 1.5 at any length
+//   f32, K L >= 128 and half of the tiles' 8 or 16 by 16 or 32 in use   0.82 - 1.04 from 32 on, 0.95 - 1.14 at 16;
+//                            others 1.0 - 3.2
 //   f32, weighted            fixed widths 0.91 - 1.03 from 16 on, 1.03 - 1.22 at 8; others 1.01 - 3.4
 template <typename T, bool WEIGHTED> int64_t least_per_row(int K, int L) {
-    const int products = K * L;
+    const int products = K * L, tiles = (K <= 8 ? 8 : 16) * (L <= 16 ? 16 : 32);
     if (sizeof(T) == 4 && WEIGHTED) return fixed_shape(K, L) ? 16 : 0;
-    if (sizeof(T) == 4) return products >= 400 ? 32 : products >= 256 ? 64 : 0;
-    return products >= 400 ? (WEIGHTED ? 4 : 1) : products >= 256 ? 8 : products >= 128 ? 32 : 0;
+    if (sizeof(T) == 4) return products >= 128 && 2 * products >= tiles ? 32 : 0;
+    return products >= 400 ? (WEIGHTED ? 4 : 1) : products >= 256 ? 8 : products >= 128 || L >= 24 ? 32 : 0;
 }
 
 // Calls f with a kernel's widths: fixed ones, or (TILES) tiles that hold K and L.

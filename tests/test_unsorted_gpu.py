@@ -122,9 +122,10 @@ def _long_rows(op, E, n, K, L, dtype):
     if dtype == np.float32 and op == "opsaw":
         least = 16 if L == 32 and K in (9, 13, 16) else None
     elif dtype == np.float32:
-        least = 32 if K * L >= 400 else 64 if K * L >= 256 else None
+        least = 32 if K * L >= 128 and 2 * K * L >= (8 if K <= 8 else 16) * (16 if L <= 16 else 32) else None
     else:
-        least = (4 if op == "opsaw" else 1) if K * L >= 400 else 8 if K * L >= 256 else 32 if K * L >= 128 else None
+        least = ((4 if op == "opsaw" else 1) if K * L >= 400 else 8 if K * L >= 256 else
+                 32 if K * L >= 128 or L >= 24 else None)
     return least is not None and E >= least * n
 
 
@@ -204,7 +205,7 @@ def test_rows_without_entries_take_no_time_of_their_own(op):
 
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
 @pytest.mark.parametrize("op", ["opsa", "opsaw"])
-@pytest.mark.parametrize("K,L", [(13, 32), (16, 20), (8, 16), (5, 8), (12, 32), (1, 4)])
+@pytest.mark.parametrize("K,L", [(13, 32), (16, 20), (8, 16), (5, 8), (12, 32), (1, 4), (9, 20), (1, 24)])
 @pytest.mark.parametrize("per_row", [1, 5, 17, 40, 70])
 def test_gradients_by_the_lengths_of_rows(oracle, op, K, L, per_row, dtype):
     """Both sides of the lines between the two gradient kernels. (All rows streamed: 300 000 entries of 1 x 4 in as
