@@ -7,7 +7,7 @@
 //   gA2[a]  : C gO[PO] ggB[PB]                   (PA = a)     gB2[b] : C gO[PO] ggA[PA] (PB = b)
 //
 // 2^22 rows, 20 x 6 -> 50, 1000 triplets, f64, against the kernels that gather from shared memory:
-// forward 2.99 -> 1.13 ms, VJP 3.04 -> 1.70 ms (the second order by gather_sums). 1000 rows: forward 12 -> 9 us,
+// forward 2.99 -> 1.19 ms, VJP 3.04 -> 1.68 ms (the second order by gather_sums). 1000 rows: forward 12 -> 9 us,
 // VJP 39 -> 13 us, second order 109 -> 19 us.
 #include "gather_tmem.cuh"
 #include "sap_tmem.hpp"
@@ -99,8 +99,8 @@ bool run(const Call& call, const SapProblem<T>& p, const Family* families, int c
 // tiles of a block, and results are collected there, to leave as one bulk copy per tile: the ring, its
 // meetings and the stores of single sectors of the kernels of gather_tmem.cuh cost half of the time of
 // 1000 triplets (2^22 rows, 20 x 6 -> 50, f64: 25 700 clocks per 256 rows in the forward, 11 600 of them
-// whatever the number of triplets; VJP 42 600 and 24 000). Now 19 700 and 10 500, VJP 29 000 and 20 000: forward
-// 1.51 -> 1.13 ms, VJP 2.48 -> 1.70 ms. What bounds them is instruction issue (64 %), then latency with four
+// whatever the number of triplets; VJP 42 600 and 24 000). Now 20 700 and 11 500, VJP 29 000 and 20 000: forward
+// 1.51 -> 1.19 ms, VJP 2.48 -> 1.68 ms. What bounds them is instruction issue (63 %), then latency with four
 // warps per scheduler: a record takes 7.3 instructions (9.5 clocks) for two rows, 4 clocks of them FP64.
 
 // Records in batches of four, coefficients and 16-bit TMEM columns apart.
@@ -350,8 +350,8 @@ __device__ __noinline__ void sum_by_factors(const ResidentRecords<T, 1> records,
 // triplets: 520 -> 690 us).
 //
 // A tile with values out_of_band is done by factors.
-// 2^20 rows, 20 x 6 -> 50, 1000 triplets, a call: looking at the operands' exponents makes 318 us 331 (f64) and
-// 210 us 228 (f32); with such a row in every tile it takes 656 and 408 (all by gather_sums: 378, 375).
+// 2^20 rows, 20 x 6 -> 50, 1000 triplets, a call: looking at the values makes 317 us 328 (f64) and 210 us 216
+// (f32); with such a row in every tile it takes 656 and 408 (all by gather_sums, without a look: 405, 397).
 template <typename T> struct ProductSource {
     const T* C;
     const int32_t *PA, *PB, *PO;
