@@ -133,7 +133,7 @@ template <typename T> struct RowsArgs {
     const T* D;                  // table [pad_out][NA][pad_c]
     int64_t rows;
     int nA, nC, nOut, L;
-    int pad_out, pad_c;
+    int pad_out, pad_a, pad_c;
     int lanes;                   // lanes per edge (a power of two); 32 / lanes edges side by side
     int bit;                     // status bit of `gather`
     const int32_t* longest;      // with a permutation: where its rows are longer than `limit`, they are
@@ -613,10 +613,10 @@ template <typename T, int VEC, int NA> constexpr int kSumBlocks = NA <= 9 ? kEdg
 // (60 000 edges, 1000 rows: 63 -> 45 us against rows dealt out beforehand).
 constexpr int kChunkEdges = 256;
 constexpr int kLeastChunk = 32;
-template <typename Off> __device__ __forceinline__ int chunk_rows(const Off* offsets, int64_t lo, int64_t hi) {
+template <typename Off> __device__ __forceinline__ int chunk_rows(const Off* offsets, int64_t lo, int64_t hi, int warps = kRowWarps) {
     const int64_t edges = offsets[hi] - offsets[lo], rows = hi - lo;
     if (edges <= 0) return 256;
-    const int64_t n = kChunkEdges * rows / edges, fair = rows / (2 * kRowWarps);
+    const int64_t n = kChunkEdges * rows / edges, fair = rows / (2 * warps);
     return static_cast<int>(n < 1 || fair < 1 ? 1 : n < fair ? n : fair);
 }
 //
@@ -692,6 +692,8 @@ sasaw_sum_rows(const __grid_constant__ RowsArgs<T> g, const int64_t* __restrict_
         for_parts<true>(starts, g.rows, g.chunk, sh.counter, lane, [&](const auto& part) { sum(starts, part); });
 }
 
+#include "sasaw_rows_mma.cuh"
+
 // gA and gB. (A kernel of its own: gathering for gW at the same time in half of the warps saves DRAM
 // traffic, but with both loops in one kernel the registers do not suffice.)
 template <typename T, int VEC, int NA, int NC, Mode MODE>
@@ -745,7 +747,7 @@ template <typename T> struct RowsShape {
 template <typename T>
 RowsShape<T> rows_shape(const Call& call, const SasawProblem<T>& p, const T* gathered, bool out_is_m2, int vec) {
     RowsShape<T> s{};
-    s.na = pad_a(p.nA);
+    s.na = s.g.pad_a = pad_a(p.nA);
     s.g.nC = out_is_m2 ? p.nO : p.nW;
     s.g.nOut = out_is_m2 ? p.nW : p.nO;
     s.nc = chunk_c(s.na, s.g.nC);
@@ -856,9 +858,61 @@ template <typename T> void set_chunks(const Call& call, RowsShape<T>& s, const E
         std::max<int64_t>(ceil_div(edges, 2 * warps * kLeastChunk) * kLeastChunk, kLeastChunk), kChunkEdges));
 }
 
+// The sums on the FP64 tensor-core instruction: 16-byte pieces of every operand, and columns that fill at least
+// half of a warp's sixteen; at half only from ten components of A on, whose sums fill the instruction (8 columns:
+// 9 x 16 -> 9 channels 66 -> 82 us, 4 x 9 -> 4 94 -> 103, but 16 x 9 -> 9 435 -> 245).
+template <typename T> bool sums_by_mma(const RowsShape<T>& s, const T* out) {
+    return sizeof(T) == 8 && s.g.L % 2 == 0 && s.g.L >= (s.na == 16 ? 8 : 10) && s.aligned &&
+           reinterpret_cast<uintptr_t>(out) % 16 == 0;
+}
+template <typename F> void for_mma_shape(const RowsShape<double>& s, F&& f) {
+    auto with = [&](auto ma, auto ninth, auto nc) {
+        using Any = std::integral_constant<int, 0>;
+        if (s.g.nC % decltype(nc)::value != 0)
+            f(ma, ninth, nc, std::false_type(), Any());
+        else if (s.g.L != 32)
+            f(ma, ninth, nc, std::true_type(), Any());
+        else
+            f(ma, ninth, nc, std::true_type(), std::integral_constant<int, 32>());
+    };
+    using I1 = std::integral_constant<int, 1>;
+    using I2 = std::integral_constant<int, 2>;
+    using I4 = std::integral_constant<int, 4>;
+    using I5 = std::integral_constant<int, 5>;
+    using I9 = std::integral_constant<int, 9>;
+    if (s.na == 16)
+        s.nc == 4 ? with(I2(), std::false_type(), I4()) : with(I2(), std::false_type(), I5());
+    else if (s.g.nA == 9)
+        s.nc == 4 ? with(I1(), std::true_type(), I4()) : with(I1(), std::true_type(), I9());
+    else
+        s.nc == 4 ? with(I1(), std::false_type(), I4()) : with(I1(), std::false_type(), I9());
+}
+
 template <typename T>
 void launch_sums(const Call& call, const RowsShape<T>& s, const int64_t* offsets, const int32_t* starts,
                  T* out, RowsRun when, int64_t edges) {
+    if constexpr (sizeof(T) == 8) {
+        if (sums_by_mma(s, out)) {
+            for_mma_shape(s, [&](auto ma, auto ninth, auto nc, auto full, auto ll) {
+                constexpr int MA = decltype(ma)::value, NC = decltype(nc)::value, LL = decltype(ll)::value;
+                constexpr bool NINTH = decltype(ninth)::value, FULL = decltype(full)::value;
+                auto kernel = sasaw_sum_rows_mma<MA, NINTH, NC, FULL, LL>;
+                const size_t table = MmaTable<MA, NINTH>::scalars(s.g.nOut, s.g.pad_c) * sizeof(double);
+                const size_t slots = kMmaWarps * MmaSlot<MA, NC>::kBytes;
+                const int depth = table + 3 * slots <= static_cast<size_t>(max_optin_smem(call.device)) - 1024 ? 3 : 2;
+                const size_t smem = table + depth * slots;
+                allow_dynamic_smem(kernel, call.device, smem);
+                const int64_t most = s.g.perm == nullptr ? s.g.rows : std::max(s.g.rows, ceil_div(edges, kLeastChunk));
+                const int64_t blocks = std::min<int64_t>(most, sm_count(call.device));
+                note_kernel_f("sasaw_sum_rows_mma<MA=%d,NINTH=%d,NC=%d,L=%d>", MA, NINTH, NC, LL);
+                kernel<<<static_cast<unsigned>(blocks), kMmaWarps * 32, smem, call.stream>>>(s.g, offsets, starts, out,
+                                                                                            depth, when, call.status);
+            });
+            MOPS_CUDA_OK(cudaGetLastError());
+            return;
+        }
+    }
+    note_kernel_f("sasaw_sum_rows<%s,VEC=%d,NA=%d,NC=%d>", scalar_name<T>(), s.vec, s.na, s.nc);
     for_shape(s, [&](auto vec, auto na, auto nc, auto mode) {
         auto kernel = sasaw_sum_rows<T, decltype(vec)::value, decltype(na)::value, decltype(nc)::value,
                                      decltype(mode)::value>;
@@ -917,7 +971,6 @@ template <typename T> int sasaw_forward_rows(const Call& call, const SasawProble
     s.g.gather = p.J, s.g.perm = nullptr, s.g.D = static_cast<const T*>(table.ptr), s.g.bit = kBitJ;
     bool unsorted = true;
     if (part != ScatterPart::kUnsorted) {
-        note_kernel_f("sasaw_sum_rows<%s,VEC=%d,NA=%d,NC=%d>", scalar_name<T>(), s.vec, s.na, s.nc);
         SegmentTable seg = segment_table(call, p.I, p.E, p.rows);
         launch_sums<T>(call, s, seg.offsets, nullptr, O, kSorted, p.E);
         unsorted = !seg.known_sorted; // asynchronous calls cannot look: always enqueue
@@ -978,7 +1031,6 @@ bool sasaw_backward_rows(const Call& call, const SasawProblem<T>& p, T* gA, T* g
         MOPS_CUDA_OK(cudaMemsetAsync(gW, 0, p.rows * p.nW * p.L * sizeof(T), call.stream));
     }
     if (gW != nullptr) {
-        note_kernel_f("sasaw_sum_rows<%s,VEC=%d,NA=%d,NC=%d>", scalar_name<T>(), s.vec, s.na, s.nc);
         launch_sums<T>(call, s, nullptr, sort.starts, gW, kAlways, p.E);
     }
     release_table(call, order);

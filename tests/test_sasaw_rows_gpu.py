@@ -152,3 +152,32 @@ def test_unsorted_rows(oracle, dtype, kw, rows):
         t["indices_output_1"], t["indices_output_2"], t["output_size"])
     torch.cuda.synchronize()
     assert_parity(out.cpu().numpy(), want["output"].astype(dtype), f"sasaw unsorted {kw} {rows} asynchronous")
+
+
+@pytest.mark.parametrize("channels", [(9, 9, 9), (9, 4, 8), (8, 5, 10), (9, 10, 1), (16, 4, 16), (10, 16, 7), (4, 9, 9)])
+@pytest.mark.parametrize("L", [10, 16, 18, 32, 64, 70])
+def test_sums_by_mma(oracle, channels, L):
+    """The f64 sums on the tensor-core instruction: rows of 0 to 11 edges, so that steps of four are cut everywhere by
+    rows' ends, long ones, passes over more channels than one takes, tiles with one output; an infinity stays in its row."""
+    nA, nW2, nO2 = channels
+    lengths = np.concatenate([np.arange(12), np.arange(12)[::-1], [300, 0, 0, 1, 33], np.full(200, 40)])
+    n = len(lengths)
+    d = workloads.sasaw(E=int(lengths.sum()), n=n, nA=nA, nW2=nW2, nO2=nO2, L=L, N=150)
+    d["indices_output_1"] = np.repeat(np.arange(n), lengths).astype(np.int32)
+    t = to_dev(d, np.float64)
+    idx = [t[k] for k in ("indices_A", "indices_W_1", "indices_W_2", "indices_output_1", "indices_output_2")]
+
+    def forward():
+        return mops_b200.sparse_accumulation_scatter_add_with_weights(
+            t["A"], t["B"], t["C"], t["W"], *idx, t["output_size"])
+
+    got = forward()
+    if nO2 > 1:  # (one output channel and many columns are estimated to be faster by edge)
+        assert any("sasaw_sum_rows_mma" in k for k in _lib.last_kernels()), _lib.last_kernels()
+    want = run_checker(oracle, "sasaw", d, np.float64)
+    assert_parity(got.cpu().numpy(), want["output"], f"sasaw mma {channels} L={L}")
+    row = 16  # (among short rows; its neighbours share steps with it)
+    t["B"][int(lengths[:row].sum())] = float("inf")
+    inf = forward()
+    others = np.arange(n) != row
+    assert np.array_equal(inf.cpu().numpy()[others], got.cpu().numpy()[others])
