@@ -2499,7 +2499,10 @@ constexpr int64_t kShortRows = 24; // edges; from here on the forward by rows is
 template <typename T> double rows_margin(const Problem<T>& p) {
     return p.E >= kShortRows * p.nW0 ? kMargin : 1 / kMargin;
 }
+// On the FP64 tensor-core instruction the sums by rows were the faster ones in all of 207 shapes with a sorted index (5 to
+// 100 edges per row), and in 26 of 30 without, the others (less than 10^4 edges, whose sort counts) by up to a sixth.
 template <typename T> bool sorted_by_rows(const Problem<T>& p) {
+    if (p.E >= p.nW0 && sasaw_rows_by_mma(rows_problem(p), RowsWork::kSorted)) return true;
     const EdgeCost cost = sizeof(T) == 4 ? EdgeCost{33.2, 4.1, 0, 342, 32.1, 2.02, 91.9, 720}
                           : p.L % 2 == 0 ? EdgeCost{46.2, 4.04, 0.0252, 403, 78.6, 4.15, 28, 568}
                                          : EdgeCost{37.7, 7.7, 0, 337, 0, 10.8, 45.7, 998};
@@ -2512,6 +2515,7 @@ template <typename T> bool sorted_by_rows(const Problem<T>& p) {
     return p.E >= p.nW0 && sasaw_rows_cost(rows_problem(p), RowsWork::kSorted) < us * rows_margin(p);
 }
 template <typename T> bool unsorted_by_rows(const Problem<T>& p) {
+    if (p.E >= 10000 && p.E >= p.nW0 && sasaw_rows_by_mma(rows_problem(p), RowsWork::kUnsorted)) return true;
     const EdgeCost cost = sizeof(T) == 4 ? EdgeCost{25.4, 3.54, 0.0224, 413, 18.5, 2.09, 0, 0}
                           : p.L % 2 == 0 ? EdgeCost{39.4, 6.25, 0, 439, 49.2, 2.39, 0, 0}
                                          : EdgeCost{33.7, 1.73, 0, 1110, 23.6, 106, 0, 0};
@@ -2544,6 +2548,8 @@ template <typename T> bool gradients_by_rows(const Problem<T>& p) {
                               : EdgeCost{21.9, 25.6, 0.034, 2510, 12.2, 1.09, 0, 0});
         margin = mma ? 1 / 1.5 : 1 / 1.1;
     }
+    // (on the FP64 tensor-core instruction: of 148 shapes 5 % then take more than 1.1 times the better family's time)
+    if (sasaw_rows_by_mma(rows_problem(p), RowsWork::kGradients)) margin = quad_gradients(p) && p.nW0 < 1184 ? 2 : 1.2;
     return sasaw_rows_cost(rows_problem(p), RowsWork::kGradients) < us * margin;
 }
 

@@ -694,6 +694,17 @@ sasaw_sum_rows(const __grid_constant__ RowsArgs<T> g, const int64_t* __restrict_
 
 #include "sasaw_rows_mma.cuh"
 
+// gW, to which the sums that come next will add.
+template <typename T> __device__ __forceinline__ void clear_for_sums(const RowsArgs<T>& g, T* gW) {
+    if (gW == nullptr) return;
+    const int64_t n = g.rows * g.nOut * g.L;
+    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
+         i += static_cast<int64_t>(gridDim.x) * blockDim.x)
+        gW[i] = T(0);
+}
+
+#include "sasaw_edges_mma.cuh"
+
 // gA and gB. (A kernel of its own: gathering for gW at the same time in half of the warps saves DRAM
 // traffic, but with both loops in one kernel the registers do not suffice.)
 template <typename T, int VEC, int NA, int NC, Mode MODE>
@@ -711,12 +722,7 @@ sasaw_edge_gradients(const __grid_constant__ RowsArgs<T> g, const int32_t* __res
         for_parts<false>(starts, g.rows, 0, sh.counter, lane, gradients);
         return;
     }
-    if (gW != nullptr) { // for the sums, which come next and will add to it
-        const int64_t n = g.rows * g.nOut * g.L;
-        for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-             i += static_cast<int64_t>(gridDim.x) * blockDim.x)
-            gW[i] = T(0);
-    }
+    clear_for_sums(g, gW);
     for_parts<true>(starts, g.rows, g.chunk, sh.counter, lane, gradients);
 }
 
@@ -861,9 +867,20 @@ template <typename T> void set_chunks(const Call& call, RowsShape<T>& s, const E
 // The sums on the FP64 tensor-core instruction: 16-byte pieces of every operand, and columns that fill at least
 // half of a warp's sixteen; at half only from ten components of A on, whose sums fill the instruction (8 columns:
 // 9 x 16 -> 9 channels 66 -> 82 us, 4 x 9 -> 4 94 -> 103, but 16 x 9 -> 9 435 -> 245).
+inline bool sums_shape_by_mma(int nA, int L) { return L % 2 == 0 && L >= (pad_a(nA) == 16 ? 8 : 10); }
 template <typename T> bool sums_by_mma(const RowsShape<T>& s, const T* out) {
-    return sizeof(T) == 8 && s.g.L % 2 == 0 && s.g.L >= (s.na == 16 ? 8 : 10) && s.aligned &&
-           reinterpret_cast<uintptr_t>(out) % 16 == 0;
+    return sizeof(T) == 8 && sums_shape_by_mma(s.g.nA, s.g.L) && s.aligned && reinterpret_cast<uintptr_t>(out) % 16 == 0;
+}
+// The gradients of A and B on the same instruction: up to nine channels, 16-byte pieces of every operand, and a
+// gathered table that L2 holds. (The others take a row's columns eight at a time, 64 bytes, from DRAM: 4.2 10^6
+// edges, 38, 75 and 151 MB: 2.39, 2.59, 3.10 ms against 2.55, 2.70, 2.82.)
+inline bool gradients_shape_by_mma(int nA, int nO, int L, int64_t rows) {
+    constexpr double kCacheBytes = 100e6; // of the 126 MB
+    return nA <= 9 && nO <= 9 && L % 2 == 0 && L >= 8 && static_cast<double>(rows) * nO * L * 8 <= kCacheBytes;
+}
+template <typename T> bool gradients_by_mma(const RowsShape<T>& s, const T* W, const T* gB) {
+    return sizeof(T) == 8 && gradients_shape_by_mma(s.g.nA, s.g.nC, s.g.L, s.g.rows) && s.aligned &&
+           (reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(gB)) % 16 == 0;
 }
 template <typename F> void for_mma_shape(const RowsShape<double>& s, F&& f) {
     auto with = [&](auto ma, auto ninth, auto nc) {
@@ -922,13 +939,75 @@ void launch_sums(const Call& call, const RowsShape<T>& s, const int64_t* offsets
     MOPS_CUDA_OK(cudaGetLastError());
 }
 
+template <typename T>
+void launch_edges_mma(const Call& call, const RowsShape<T>& s, const int32_t* starts, T* gA, T* gB, T* gW, const T* W,
+                      int64_t edges) {
+    if constexpr (sizeof(T) == 8) {
+        auto go = [&](auto ks, auto c9, auto a9, auto ll) {
+            constexpr int KS = decltype(ks)::value, LL = decltype(ll)::value;
+            constexpr bool C9 = decltype(c9)::value, A9 = decltype(a9)::value;
+            auto kernel = sasaw_edge_gradients_mma<KS, C9, A9, LL>;
+            const size_t table = (GradTable<KS>::scalars(s.g.nOut) * sizeof(double) + 127) / 128 * 128;
+            const size_t smem = table + kGradWarps * grad_ring_bytes<KS, C9>();
+            allow_dynamic_smem(kernel, call.device, smem);
+            const int64_t most = std::max(s.g.rows, ceil_div(edges, kLeastChunk));
+            const int64_t blocks = std::min<int64_t>(most, sm_count(call.device));
+            note_kernel_f("sasaw_edge_gradients_mma<KS=%d,C9=%d,A9=%d,L=%d>", KS, C9, A9, LL);
+            kernel<<<static_cast<unsigned>(blocks), kGradWarps * 32, smem, call.stream>>>(s.g, starts, gA, gB, gW, W,
+                                                                                         call.status);
+        };
+        auto with = [&](auto ks, auto c9) {
+            using Any = std::integral_constant<int, 0>;
+            if (s.g.nA == 9 && s.g.L == 32)
+                go(ks, c9, std::true_type(), std::integral_constant<int, 32>());
+            else if (s.g.nA == 9)
+                go(ks, c9, std::true_type(), Any());
+            else
+                go(ks, c9, std::false_type(), Any());
+        };
+        using I1 = std::integral_constant<int, 1>;
+        using I2 = std::integral_constant<int, 2>;
+        if (s.g.nC == 9)
+            with(I2(), std::true_type());
+        else
+            s.g.nC <= 4 ? with(I1(), std::false_type()) : with(I2(), std::false_type());
+        MOPS_CUDA_OK(cudaGetLastError());
+    }
+}
+
 } // namespace
+
+template <typename T> bool sasaw_rows_by_mma(const SasawProblem<T>& p, RowsWork work) {
+    if (sizeof(T) != 8 || !rows_apply(p) || (reinterpret_cast<uintptr_t>(p.B) | reinterpret_cast<uintptr_t>(p.W)) % 16 != 0)
+        return false;
+    return work == RowsWork::kGradients ? gradients_shape_by_mma(p.nA, p.nO, p.L, p.rows) : sums_shape_by_mma(p.nA, p.L);
+}
+
+// The gradients on the FP64 tensor-core instruction, all three of them: microseconds, fitted to 148 shapes up to
+// 2 10^6 edges; eight in ten estimates are within a sixth. Clocks of the instructions of a step, of a row's E, of the sums'
+// steps and coupling, and what the coupling's table takes.
+inline double gradients_mma_cost(int64_t edges, int64_t rows, int nA, int nW, int nO, int L, int64_t N) {
+    const int ks = nO <= 4 ? 1 : 2, c9 = nO == 9 ? 1 : 0, a9 = nA == 9 ? 1 : 0;
+    const int na = pad_a(nA), nc = chunk_c(na, nO);
+    const double E = static_cast<double>(edges), n = static_cast<double>(rows);
+    const double slices = static_cast<double>(ceil_div(L, 8)), columns = static_cast<double>(ceil_div(L, 16));
+    const double step = 8 * (ks * 16 + 4 * c9 + 8 + a9 * (2 * ks + 2 * c9 + 4)), sum_step = nc * 2 * (18 + 2 * a9);
+    const double outs = static_cast<double>(ceil_div(nW, 8)), passes = static_cast<double>(ceil_div(nO, nc));
+    const double table = static_cast<double>(ceil_div(nW, 3)) * 3 * na * passes * nc * static_cast<double>(N);
+    const double few = std::max(0.0, 1 - n / 1184) * E / n; // a row's steps one after the other
+    return 60.2 + 1e-6 * (0.647 * E / 8 * slices * step + 2.59 * n * slices * nW * (ks * 16 + 10) +
+                          1.39 * E / 4 * columns * passes * sum_step + 8.31 * E / 4 * columns * passes * 100 +
+                          3.58 * n * columns * passes * (2 + a9) * nc * 32 * outs + 10.2 * table) +
+           1.64 * few * slices * step / 8e3;
+}
 
 // Microseconds, fitted to 750 shapes up to 2 10^6 edges with 1 to 16 channels, 1 to 100 columns and rows of
 // a fraction of an edge to thousands; nine in ten estimates are within a third where a call takes more
 // than 80 us. A step is an edge (or the edges side by side) in one pass over columns and channels.
 template <typename T> double sasaw_rows_cost(const SasawProblem<T>& p, RowsWork work) {
     if (!rows_apply(p)) return INFINITY;
+    if (work == RowsWork::kGradients && sasaw_rows_by_mma(p, work))
+        return gradients_mma_cost(p.E, p.rows, p.nA, p.nW, p.nO, p.L, p.N);
     struct Cost {
         double call, product, step, exact_product, exact_step; // products and steps in 10^-6
         double contract, contract_once, table, pass, edge, row; // 10^-6, 10^-3, 10^-5, 1, 10^-6, 10^-3
@@ -1018,7 +1097,9 @@ bool sasaw_backward_rows(const Call& call, const SasawProblem<T>& p, T* gA, T* g
     }
     s.g.gather = p.I, s.g.perm = sort.perm, s.g.D = static_cast<const T*>(table.ptr), s.g.bit = kBitI;
     set_chunks(call, s, sort, p.E);
-    if (gA != nullptr || gB != nullptr) {
+    if ((gA != nullptr || gB != nullptr) && gradients_by_mma(s, p.W, gB)) {
+        launch_edges_mma(call, s, sort.starts, gA, gB, gW, p.W, p.E);
+    } else if (gA != nullptr || gB != nullptr) {
         note_kernel_f("sasaw_edge_gradients<%s,VEC=%d,NA=%d,NC=%d>", scalar_name<T>(), s.vec, s.na, s.nc);
         for_shape(s, [&](auto vec, auto na, auto nc, auto mode) {
             auto kernel = sasaw_edge_gradients<T, decltype(vec)::value, decltype(na)::value, decltype(nc)::value,
@@ -1040,6 +1121,7 @@ bool sasaw_backward_rows(const Call& call, const SasawProblem<T>& p, T* gA, T* g
 
 #define INSTANTIATE(T)                                                                             \
     template double sasaw_rows_cost<T>(const SasawProblem<T>&, RowsWork);                          \
+    template bool sasaw_rows_by_mma<T>(const SasawProblem<T>&, RowsWork);                          \
     template int sasaw_forward_rows<T>(const Call&, const SasawProblem<T>&, T*, ScatterPart);      \
     template bool sasaw_backward_rows<T>(const Call&, const SasawProblem<T>&, T*, T*, T*, const T*);
 INSTANTIATE(float)

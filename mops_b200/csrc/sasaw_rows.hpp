@@ -23,6 +23,9 @@ enum : int { kNotApplicable = 0, kComplete = 1, kUnsortedLeft = 2 };
 // Microseconds that the row kernels take, as fitted to measurements; infinite where they do not apply.
 enum class RowsWork { kSorted, kUnsorted, kGradients };
 template <typename T> double sasaw_rows_cost(const SasawProblem<T>& p, RowsWork work);
+// Whether the kernels on the FP64 tensor-core instruction take this work (f64, as far as shapes and the operands
+// known here tell).
+template <typename T> bool sasaw_rows_by_mma(const SasawProblem<T>& p, RowsWork work);
 
 // Enqueue the operation on the call's stream and return true, or return false when its channel
 // counts are too large for these kernels (the forward: as above). Gradients that are nullptr are skipped.

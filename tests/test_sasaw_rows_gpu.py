@@ -181,3 +181,30 @@ def test_sums_by_mma(oracle, channels, L):
     inf = forward()
     others = np.arange(n) != row
     assert np.array_equal(inf.cpu().numpy()[others], got.cpu().numpy()[others])
+
+
+@pytest.mark.parametrize("channels", [(9, 9, 9), (4, 9, 3), (8, 16, 9), (9, 3, 8), (1, 2, 1), (9, 9, 5)])
+@pytest.mark.parametrize("L", [8, 10, 32, 64])
+def test_gradients_by_mma(oracle, channels, L):
+    """The f64 gradients of A and B on the tensor-core instruction: rows of W with 0 to 20 edges, so that steps of eight are cut
+    everywhere, rows of a window of 96 edges and longer ones, the last columns of an incomplete eight; an infinite
+    gradient stays with the edges that read it."""
+    nA, nW2, nO2 = channels
+    lengths = np.concatenate([np.arange(21), np.arange(21)[::-1], [95, 96, 97, 0, 0, 1, 193, 500], np.full(300, 60)])
+    n = len(lengths)
+    d = workloads.sasaw(E=int(lengths.sum()), n=n, nA=nA, nW2=nW2, nO2=nO2, L=L, N=100)
+    r = np.random.default_rng(8)
+    d["indices_W_1"] = r.permutation(np.repeat(np.arange(n), lengths)).astype(np.int32)
+    t = to_dev(d, np.float64)
+    got = run_library("sasaw", t)
+    if channels == (9, 9, 9):
+        assert any("sasaw_edge_gradients_mma" in k for k in _lib.last_kernels()), _lib.last_kernels()
+    want = run_checker(oracle, "sasaw", d, np.float64)
+    for k in want:
+        assert_parity(got[k], want[k], f"sasaw gradients mma {channels} L={L}/{k}")
+    row = 200
+    t["grad_output"][row] = float("inf")
+    inf = run_library("sasaw", t)
+    others = d["indices_output_1"] != row
+    for k in ("grad_A", "grad_B"):
+        assert np.array_equal(inf[k][others], got[k][others]), k
