@@ -138,19 +138,21 @@ template <typename T> struct RowsArgs {
     int bit;                     // status bit of `gather`
     const int32_t* longest;      // with a permutation: where its rows are longer than `limit`, they are
     int limit, chunk;            // taken in chunks of this many edges, whatever rows these belong to
+    int piece_at, piece_room;    // shared memory for the sums of so many pieces (Pieces)
 };
 
-// Some rows. CUT: and of their edges those at positions [p_lo, p_hi); other warps have others, so that sums
-// are added to what is there. (Instantiated for both: with the choice at run time the even case took 3 %
-// longer, f32, 250 000 edges.)
-template <bool CUT> struct Part {
-    static constexpr bool kCut = CUT;
-    int64_t row_lo, row_hi;
-};
-template <> struct Part<true> {
-    static constexpr bool kCut = true;
+// Some rows. kCut: and of their edges those at positions [p_lo, p_hi); other warps have others, so that sums
+// are added to what is there. kPiece: the same, of a block's own rows; the sums of a first row that another warp
+// has begun (`head`) go to shared memory, where the block adds them up. (Instantiated for each: with the choice at run time the even
+// case took 3 % longer, f32, 250 000 edges.)
+enum Cut { kWhole = 0, kCut = 1, kPiece = 2 };
+template <Cut CUT> struct Part {
     int64_t row_lo, row_hi;
     int p_lo, p_hi;
+    unsigned char* head;
+};
+template <> struct Part<kWhole> {
+    int64_t row_lo, row_hi;
 };
 
 // One slot of a warp's ring: NC rows of 32 lanes, B, the A rows of the edges side by side, their numbers.
@@ -192,7 +194,7 @@ enum Mode { kSideBySide = 0, kOneEdge = 1, kExact = 2 };
 // straight-line code (wait, start the copies of the step seven ahead, read, multiply), which the
 // compiler can interleave: at 9 x 9 channels, f64, 337 -> 210 instructions per edge of the sums,
 // 640 -> 450 us at 10^6 edges.
-template <typename T, int VEC, int NA, int NC, Mode MODE, typename Off, bool CUT, typename Begin, typename Step,
+template <typename T, int VEC, int NA, int NC, Mode MODE, typename Off, Cut CUT, typename Begin, typename Step,
           typename End>
 __device__ __forceinline__ void walk_rows(const RowsArgs<T>& g, const Off* __restrict__ offsets,
                                           const Part<CUT>& part, int b0, int c0, unsigned char* ring, int lane,
@@ -217,10 +219,10 @@ __device__ __forceinline__ void walk_rows(const RowsArgs<T>& g, const Off* __res
 
     const int64_t row_lo = part.row_lo, row_hi = part.row_hi;
     int p_lo = static_cast<int>(offsets[row_lo]), p_hi = static_cast<int>(offsets[row_hi]);
-    if constexpr (CUT) p_lo = max(p_lo, part.p_lo), p_hi = min(p_hi, part.p_hi);
+    if constexpr (CUT != kWhole) p_lo = max(p_lo, part.p_lo), p_hi = min(p_hi, part.p_hi);
     auto row_end = [&](int64_t row) {
         const int end = static_cast<int>(offsets[row + 1]);
-        return CUT ? min(end, p_hi) : end;
+        return CUT != kWhole ? min(end, p_hi) : end;
     };
     // Edge numbers and gathered rows, 32 positions per register: the block that the copies have
     // reached (0), the next (1), and of the one after that the edge numbers only (2).
@@ -377,8 +379,8 @@ template <typename T, int NA> __device__ __forceinline__ void load_a(const T* a,
     }
 }
 
-// out[o] (+)= sum_{a,c} D[o][a][c0 + c] acc[a][c] for the lane's column, o = 0 .. nOut - 1. CUT: by atomics.
-template <typename T, int VEC, int NA, int NC, bool CUT>
+// out[o] (+)= sum_{a,c} D[o][a][c0 + c] acc[a][c] for the lane's column, o = 0 .. nOut - 1. ADD: by atomics.
+template <typename T, int VEC, int NA, int NC, bool ADD>
 __device__ __forceinline__ void contract_row(const RowsArgs<T>& g, const T* D, T* out,
                                              typename Pack<T, VEC>::V (&acc)[NA][NC], int c0, bool store,
                                              bool add_to) {
@@ -402,7 +404,7 @@ __device__ __forceinline__ void contract_row(const RowsArgs<T>& g, const T* D, T
             if (store && o + u < g.nOut) {
                 T* at = out + static_cast<int64_t>(o + u) * g.L;
                 V* dst = reinterpret_cast<V*>(at);
-                if constexpr (CUT)
+                if constexpr (ADD)
                     P::add_at(at, v[u]);
                 else
                     *dst = add_to ? P::add(*dst, v[u]) : v[u];
@@ -412,7 +414,7 @@ __device__ __forceinline__ void contract_row(const RowsArgs<T>& g, const T* D, T
 }
 
 // Forward, and the gW part of the gradients: `out` is [rows][nOut][L].
-template <typename T, int VEC, int NA, int NC, Mode MODE, typename Off, bool CUT>
+template <typename T, int VEC, int NA, int NC, Mode MODE, typename Off, Cut CUT>
 __device__ __forceinline__ void outer_rows(const RowsArgs<T>& g, const Off* __restrict__ offsets,
                                            T* __restrict__ out, const Part<CUT>& part, const T* D,
                                            unsigned char* ring, int lane, const Status& st) {
@@ -446,7 +448,7 @@ __device__ __forceinline__ void outer_rows(const RowsArgs<T>& g, const Off* __re
                 },
                 [&](int64_t row, bool any) {
                     T* at = out + row * g.nOut * g.L + b;
-                    if (!CUT || any) contract_row<T, VEC, NA, NC, CUT>(g, D, at, acc, c0, store, c0 > 0);
+                    if (CUT != kCut || any) contract_row<T, VEC, NA, NC, CUT == kCut>(g, D, at, acc, c0, store, c0 > 0);
                 });
         }
     }
@@ -505,7 +507,7 @@ template <int O, int HELD, typename T, int NA> __device__ __forceinline__ void s
 
 // gA and gB. `own` is the matrix of the rows themselves, [rows][nOut][L] (W, where the rows are
 // those of W and g.G is gO).
-template <typename T, int VEC, int NA, int NC, Mode MODE, typename Off, bool CUT>
+template <typename T, int VEC, int NA, int NC, Mode MODE, typename Off, Cut CUT>
 __device__ __forceinline__ void edge_gradients(const RowsArgs<T>& g, const Off* __restrict__ offsets,
                                                T* __restrict__ gA, T* __restrict__ gB,
                                                const T* __restrict__ own, const Part<CUT>& part, const T* D,
@@ -623,33 +625,116 @@ template <typename Off> __device__ __forceinline__ int chunk_rows(const Off* off
 // Rows longer than the limit (or few of them) would leave warps waiting for one another: then the blocks
 // share out chunks of edges instead, and rows are cut where a chunk ends (sums of 60 000 edges, half of
 // them in one of 1000 rows, f32, 9 x 9 x 9 channels: 9.3 ms without).
-template <bool CUT, typename Off, typename F>
-__device__ __forceinline__ void for_parts(const Off* offsets, int64_t rows, int chunk, int* counter, int lane, F&& f) {
-    auto take = [&](int n) {
+template <typename Off, typename F>
+__device__ __forceinline__ void for_rows(const Off* offsets, int64_t lo, int64_t hi, int* counter, int lane, F&& f) {
+    const int n = chunk_rows(offsets, lo, hi);
+    while (true) {
         int at = 0;
         if (lane == 0) at = atomicAdd(counter, n);
-        return __shfl_sync(kFullMask, at, 0);
+        const int64_t r = lo + __shfl_sync(kFullMask, at, 0);
+        if (r >= hi) break;
+        f(Part<kWhole>{r, r + n < hi ? r + n : hi});
+    }
+}
+template <typename Off, typename F>
+__device__ __forceinline__ void for_cuts(const Off* offsets, int64_t rows, int chunk, int* counter, int lane, F&& f) {
+    const int edges = static_cast<int>(offsets[rows]);
+    while (true) {
+        int at = 0;
+        if (lane == 0) at = atomicAdd(counter, 1);
+        const int64_t p = (blockIdx.x + static_cast<int64_t>(__shfl_sync(kFullMask, at, 0)) * gridDim.x) * chunk;
+        if (p >= edges) break;
+        const int end = p + chunk < edges ? static_cast<int>(p) + chunk : edges;
+        // the rows of the first and of the last edge
+        f(Part<kCut>{warp_count_weighted_le(offsets, rows + 1, 0, p, lane) - 1,
+                     warp_count_weighted_le(offsets, rows + 1, 0, end - 1, lane), static_cast<int>(p), end, nullptr});
+    }
+}
+
+// Few rows for a block's warps: dealt out whole, the last ones leave most warps waiting (60 000 edges, 1000 rows: 13.5
+// tasks of a row and sixteen columns for twelve warps). Then the block's edges are cut into equal pieces, as many as
+// warps, whatever rows they belong to. A row belongs to the piece that it begins in; what other pieces add to it, at
+// most one row each, goes to shared memory and is added in their order when all are done: the same bits every time.
+// 60 000 edges, 1000 rows, f64 sums 37 -> 33 us; 250 000 edges, 4099 rows, 64 columns, f32, gradients of A and B, which add
+// up nothing over a row: 195 -> 178 us. (The sums by multiply-adds gain 2 % there, 129 -> 126 us, and lose as much on many
+// rows, 2.07 -> 2.12 ms, to the third way through their loop in the kernel.) From six rows a warp on the last ones matter less than the additional coupling of the cut ones.
+constexpr int kMostPieces = 64; // of all slices of the columns
+constexpr int kFewRowsPerWarp = 6;
+struct Pieces {
+    int64_t lo, hi; // the block's rows
+    int first, edges, count;
+    int64_t* heads; // [slice][piece] (shared memory): the row that the piece goes on with, -1: none
+    unsigned char* sums;
+    int sums_bytes; // of a piece
+};
+// Pieces per slice, 0: the rows are not few, or there is no room.
+template <typename Off>
+__device__ __forceinline__ int piece_count(const Off* offsets, int64_t lo, int64_t hi, int warps, int slices, int room) {
+    if ((hi - lo) * slices >= kFewRowsPerWarp * warps) return 0;
+    if (offsets[hi] - offsets[lo] < 8 * warps) return 0;
+    const int n = slices <= warps && warps % slices == 0 ? warps / slices : (2 * warps + slices - 1) / slices;
+    return n > 1 && n * slices <= room ? n : 0;
+}
+template <typename Off, typename F>
+__device__ __forceinline__ void for_pieces(const Off* offsets, const Pieces& z, int slices, int* counter, int lane, F&& f) {
+    auto at = [&](int t) { return z.first + static_cast<int>(static_cast<int64_t>(z.edges) * t / z.count); };
+    auto row_at = [&](int t) { // the first row that begins at piece t's first edge or behind it
+        if (t <= 0) return z.lo;
+        if (t >= z.count) return z.hi;
+        return z.lo + warp_count_weighted_le(offsets + z.lo, z.hi - z.lo + 1, 0, at(t) - 1, lane);
     };
-    if constexpr (!CUT) {
-        const int64_t lo = balanced_row_split(offsets, rows, blockIdx.x, gridDim.x, lane);
-        const int64_t hi = balanced_row_split(offsets, rows, blockIdx.x + 1, gridDim.x, lane);
-        const int n = chunk_rows(offsets, lo, hi);
-        while (true) {
-            const int64_t r = lo + take(n);
-            if (r >= hi) break;
-            f(Part<false>{r, r + n < hi ? r + n : hi});
-        }
-    } else {
-        const int edges = static_cast<int>(offsets[rows]);
-        while (true) {
-            const int64_t p = (blockIdx.x + static_cast<int64_t>(take(1)) * gridDim.x) * chunk;
-            if (p >= edges) break;
-            const int end = p + chunk < edges ? static_cast<int>(p) + chunk : edges;
-            // the rows of the first and of the last edge
-            f(Part<true>{warp_count_weighted_le(offsets, rows + 1, 0, p, lane) - 1,
-                         warp_count_weighted_le(offsets, rows + 1, 0, end - 1, lane), static_cast<int>(p), end});
+    while (true) {
+        int task = 0;
+        if (lane == 0) task = atomicAdd(counter, 1);
+        task = __shfl_sync(kFullMask, task, 0);
+        if (task >= z.count * slices) break;
+        const int t = task % z.count;
+        const int64_t lo = row_at(t), hi = row_at(t + 1);
+        const bool head = static_cast<int>(offsets[lo]) > at(t);
+        if (lane == 0) z.heads[task] = head ? lo - 1 : -1;
+        f(Part<kPiece>{head ? lo - 1 : lo, hi, at(t), at(t + 1), head ? z.sums + task * z.sums_bytes : nullptr},
+          task / z.count);
+    }
+}
+// Adds the sums of the pieces' heads to their rows, columns [b0, b0 + columns) of slice b0 / columns. All threads of
+// the block, a warp per row.
+template <typename T>
+__device__ __forceinline__ void add_heads(const Pieces& z, int slices, int columns, int n_out, int L, T* out, int warps) {
+    __syncthreads();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int task = warp; task < z.count * slices; task += warps) {
+        const int t = task % z.count, b0 = task / z.count * columns;
+        const int64_t row = z.heads[task];
+        if (row < 0 || (t > 0 && z.heads[task - 1] == row)) continue;
+        const int wide = L - b0 < columns ? L - b0 : columns;
+        for (int x = lane; x < n_out * wide; x += 32) {
+            const int o = x / wide, b = x - o * wide;
+            T* at = out + (row * n_out + o) * L + b0 + b;
+            T sum = *at;
+            for (int i = task; i < task - t + z.count && z.heads[i] == row; i++)
+                sum += reinterpret_cast<const T*>(z.sums + i * z.sums_bytes)[o * columns + b];
+            *at = sum;
         }
     }
+}
+// A block's rows: f(part, slice) for pieces of them where they are few, whole(lo, hi) otherwise. `out`: what f adds
+// up, nullptr where nothing is.
+template <typename T, typename Off, typename F, typename Whole>
+__device__ __forceinline__ void for_few_rows(const RowsArgs<T>& g, const Off* offsets, int warps, int slices, int columns,
+                                             T* out, int64_t* heads, unsigned char* smem, int* counter, int lane, F&& f,
+                                             Whole&& whole) {
+    const int64_t lo = balanced_row_split(offsets, g.rows, blockIdx.x, gridDim.x, lane);
+    const int64_t hi = balanced_row_split(offsets, g.rows, blockIdx.x + 1, gridDim.x, lane);
+    const int count = piece_count(offsets, lo, hi, warps, slices, out != nullptr ? g.piece_room : kMostPieces);
+    if (count == 0) {
+        whole(lo, hi);
+        return;
+    }
+    const int first = static_cast<int>(offsets[lo]);
+    const Pieces z{lo, hi, first, static_cast<int>(offsets[hi]) - first, count, heads, smem + g.piece_at,
+                   (g.nOut * columns * static_cast<int>(sizeof(T)) + 15) / 16 * 16};
+    for_pieces(offsets, z, slices, counter, lane, f);
+    if (out != nullptr) add_heads(z, slices, columns, g.nOut, g.L, out, warps);
 }
 
 // Shared memory of the kernels: the table, the rings, and a counter of rows taken.
@@ -684,12 +769,17 @@ sasaw_sum_rows(const __grid_constant__ RowsArgs<T> g, const int64_t* __restrict_
     auto sum = [&](const auto* at, const auto& part) {
         outer_rows<T, VEC, NA, NC, MODE>(g, at, out, part, sh.D, sh.ring, lane, st);
     };
+    auto rows = [&](const auto* at) {
+        for_rows(at, balanced_row_split(at, g.rows, blockIdx.x, gridDim.x, lane),
+                 balanced_row_split(at, g.rows, blockIdx.x + 1, gridDim.x, lane), sh.counter, lane,
+                 [&](const auto& part) { sum(at, part); });
+    };
     if (run == kSorted)
-        for_parts<false>(offsets, g.rows, 0, sh.counter, lane, [&](const auto& part) { sum(offsets, part); });
+        rows(offsets);
     else if (*g.longest <= g.limit)
-        for_parts<false>(starts, g.rows, 0, sh.counter, lane, [&](const auto& part) { sum(starts, part); });
+        rows(starts);
     else // (`out` has been cleared by a kernel before)
-        for_parts<true>(starts, g.rows, g.chunk, sh.counter, lane, [&](const auto& part) { sum(starts, part); });
+        for_cuts(starts, g.rows, g.chunk, sh.counter, lane, [&](const auto& part) { sum(starts, part); });
 }
 
 #include "sasaw_rows_mma.cuh"
@@ -719,11 +809,14 @@ sasaw_edge_gradients(const __grid_constant__ RowsArgs<T> g, const int32_t* __res
         edge_gradients<T, VEC, NA, NC, MODE>(g, starts, gA, gB, W, part, sh.D, sh.ring, lane, st);
     };
     if (*g.longest <= g.limit) {
-        for_parts<false>(starts, g.rows, 0, sh.counter, lane, gradients);
+        __shared__ int64_t heads[kMostPieces];
+        for_few_rows<T>(g, starts, kRowWarps, 1, g.L, nullptr, heads, smem, sh.counter, lane,
+                        [&](const auto& part, int) { gradients(part); },
+                        [&](int64_t lo, int64_t hi) { for_rows(starts, lo, hi, sh.counter, lane, gradients); });
         return;
     }
     clear_for_sums(g, gW);
-    for_parts<true>(starts, g.rows, g.chunk, sh.counter, lane, gradients);
+    for_cuts(starts, g.rows, g.chunk, sh.counter, lane, gradients);
 }
 
 // ---- the order of the edges by a row index: row starts and permutation (a counting sort)
@@ -916,13 +1009,19 @@ void launch_sums(const Call& call, const RowsShape<T>& s, const int64_t* offsets
                 auto kernel = sasaw_sum_rows_mma<MA, NINTH, NC, FULL, LL>;
                 const size_t table = MmaTable<MA, NINTH>::scalars(s.g.nOut, s.g.pad_c) * sizeof(double);
                 const size_t slots = kMmaWarps * MmaSlot<MA, NC>::kBytes;
-                const int depth = table + 3 * slots <= static_cast<size_t>(max_optin_smem(call.device)) - 1024 ? 3 : 2;
-                const size_t smem = table + depth * slots;
+                const int depth = table + 3 * slots <= static_cast<size_t>(max_optin_smem(call.device)) - 2048 ? 3 : 2;
+                // (behind the rings: what pieces of rows hand on)
+                const size_t head = static_cast<size_t>(s.g.nOut) * kMmaColumns * sizeof(double);
+                const size_t room = (static_cast<size_t>(max_optin_smem(call.device)) - 2048 - table - depth * slots) / head;
+                RowsArgs<T> g = s.g;
+                g.piece_at = static_cast<int>(table + depth * slots);
+                g.piece_room = static_cast<int>(std::min<size_t>(room, 2 * kMmaWarps));
+                const size_t smem = table + depth * slots + g.piece_room * head;
                 allow_dynamic_smem(kernel, call.device, smem);
                 const int64_t most = s.g.perm == nullptr ? s.g.rows : std::max(s.g.rows, ceil_div(edges, kLeastChunk));
                 const int64_t blocks = std::min<int64_t>(most, sm_count(call.device));
                 note_kernel_f("sasaw_sum_rows_mma<MA=%d,NINTH=%d,NC=%d,L=%d>", MA, NINTH, NC, LL);
-                kernel<<<static_cast<unsigned>(blocks), kMmaWarps * 32, smem, call.stream>>>(s.g, offsets, starts, out,
+                kernel<<<static_cast<unsigned>(blocks), kMmaWarps * 32, smem, call.stream>>>(g, offsets, starts, out,
                                                                                             depth, when, call.status);
             });
             MOPS_CUDA_OK(cudaGetLastError());

@@ -57,7 +57,7 @@ template <int MA, bool NINTH> struct MmaTable {
 };
 
 // The columns [b0, b0 + 16) of a part. FULL: the channels fill every pass. LL: L where it is known (0 otherwise).
-template <int MA, bool NINTH, int NC, bool FULL, int LL, typename Off, bool CUT>
+template <int MA, bool NINTH, int NC, bool FULL, int LL, typename Off, Cut CUT>
 __device__ __forceinline__ void mma_sum_rows(const RowsArgs<double>& g, const Off* __restrict__ offsets,
                                              double* __restrict__ out, const Part<CUT>& part, int b0,
                                              const double* table, unsigned char* ring, int depth, int lane,
@@ -68,7 +68,7 @@ __device__ __forceinline__ void mma_sum_rows(const RowsArgs<double>& g, const Of
     const int L = LL > 0 ? LL : g.L;
     const int64_t row_lo = part.row_lo, row_hi = part.row_hi;
     int p_lo = static_cast<int>(offsets[row_lo]), p_hi = static_cast<int>(offsets[row_hi]);
-    if constexpr (CUT) p_lo = max(p_lo, part.p_lo), p_hi = min(p_hi, part.p_hi);
+    if constexpr (CUT != kWhole) p_lo = max(p_lo, part.p_lo), p_hi = min(p_hi, part.p_hi);
     const int last = p_hi - 1, steps = (p_hi - p_lo + kMmaStep - 1) / kMmaStep;
 
     const bool store = b0 + 2 * n < L;
@@ -139,12 +139,19 @@ __device__ __forceinline__ void mma_sum_rows(const RowsArgs<double>& g, const Of
         int lo = p_lo;
         for (int64_t row = row_lo; row < row_hi; row++) {
             int hi = static_cast<int>(offsets[row + 1]);
-            if constexpr (CUT) hi = min(hi, p_hi);
+            if constexpr (CUT != kWhole) hi = min(hi, p_hi);
             double* at = out + row * g.nOut * L + b;
+            int stride = L; // from one output to the next
+            if constexpr (CUT == kPiece) {
+                if (row == row_lo && part.head != nullptr) {
+                    at = reinterpret_cast<double*>(part.head) + 2 * n;
+                    stride = kMmaColumns;
+                }
+            }
             if (lo >= hi) {
-                if (!CUT && c0 == 0 && store)
+                if (CUT != kCut && c0 == 0 && store)
                     for (int o = q; o < g.nOut; o += 4)
-                        *reinterpret_cast<double2*>(at + static_cast<int64_t>(o) * L) = make_double2(0, 0);
+                        *reinterpret_cast<double2*>(at + static_cast<int64_t>(o) * stride) = make_double2(0, 0);
                 continue;
             }
             double acc[NC][2][MA][2], acc9[NC][2];
@@ -257,8 +264,8 @@ __device__ __forceinline__ void mma_sum_rows(const RowsArgs<double>& g, const Of
 #pragma unroll
                     for (int j = 0; j < 2; j++) {
                         if (j >= count) break;
-                        double* to = at + static_cast<int64_t>(first + j) * L;
-                        if constexpr (CUT) {
+                        double* to = at + static_cast<int64_t>(first + j) * stride;
+                        if constexpr (CUT == kCut) {
                             red_add(to, sum[0][j]);
                             red_add(to + 1, sum[1][j]);
                         } else {
@@ -278,44 +285,18 @@ __device__ __forceinline__ void mma_sum_rows(const RowsArgs<double>& g, const Of
     }
 }
 
-// As for_parts: every part of a block's rows once for each slice of sixteen columns, one slice of all parts after the
+// As for_rows and for_cuts: every part once for each slice of sixteen columns, one slice of all parts after the
 // other (so that what they gather is a slice of the table at a time: less to keep in L2).
-template <bool CUT, typename Off, typename F>
-__device__ __forceinline__ void for_slices(const Off* offsets, int64_t rows, int chunk, int slices, int* counter, int lane,
-                                           F&& f) {
-    auto take = [&] {
+template <typename F>
+__device__ __forceinline__ void for_slices(int parts, int slices, int* counter, int lane, F&& f) {
+    int slice = 0, before = 0; // parts of the slices before
+    while (true) {
         int at = 0;
         if (lane == 0) at = atomicAdd(counter, 1);
-        return __shfl_sync(kFullMask, at, 0);
-    };
-    if constexpr (!CUT) {
-        const int64_t lo = balanced_row_split(offsets, rows, blockIdx.x, gridDim.x, lane);
-        const int64_t hi = balanced_row_split(offsets, rows, blockIdx.x + 1, gridDim.x, lane);
-        const int n = chunk_rows(offsets, lo, hi, kMmaWarps), parts = static_cast<int>((hi - lo + n - 1) / n);
-        int slice = 0, before = 0; // parts of the slices before
-        while (true) {
-            const int at = take();
-            while (at - before >= parts && slice < slices) slice++, before += parts;
-            if (slice >= slices) break;
-            const int64_t r = lo + static_cast<int64_t>(at - before) * n;
-            f(Part<false>{r, r + n < hi ? r + n : hi}, slice);
-        }
-    } else {
-        const int edges = static_cast<int>(offsets[rows]);
-        const int chunks = (edges + chunk - 1) / chunk, mine = static_cast<int>(blockIdx.x);
-        const int parts = chunks > mine ? (chunks - mine + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x) : 0;
-        int slice = 0, before = 0;
-        while (true) {
-            const int at = take();
-            while (at - before >= parts && slice < slices) slice++, before += parts;
-            if (slice >= slices) break;
-            const int p = (mine + (at - before) * static_cast<int>(gridDim.x)) * chunk;
-            const int end = edges - p > chunk ? p + chunk : edges;
-            // the rows of the first and of the last edge
-            f(Part<true>{warp_count_weighted_le(offsets, rows + 1, 0, p, lane) - 1,
-                         warp_count_weighted_le(offsets, rows + 1, 0, end - 1, lane), p, end},
-              slice);
-        }
+        at = __shfl_sync(kFullMask, at, 0);
+        while (at - before >= parts && slice < slices) slice++, before += parts;
+        if (slice >= slices) break;
+        f(at - before, slice);
     }
 }
 
@@ -340,15 +321,31 @@ sasaw_sum_rows_mma(const __grid_constant__ RowsArgs<double> g, const int64_t* __
     auto sum = [&](const auto* at, const auto& part, int slice) {
         mma_sum_rows<MA, NINTH, NC, FULL, LL>(g, at, out, part, slice * kMmaColumns, table, ring, depth, lane, st);
     };
-    if (run == kSorted)
-        for_slices<false>(offsets, g.rows, 0, slices, &counter, lane,
-                         [&](const auto& part, int slice) { sum(offsets, part, slice); });
-    else if (*g.longest <= g.limit)
-        for_slices<false>(starts, g.rows, 0, slices, &counter, lane,
-                         [&](const auto& part, int slice) { sum(starts, part, slice); });
-    else // (`out` has been cleared by a kernel before)
-        for_slices<true>(starts, g.rows, g.chunk, slices, &counter, lane,
-                        [&](const auto& part, int slice) { sum(starts, part, slice); });
+    __shared__ int64_t heads[kMostPieces];
+    auto rows = [&](const auto* at) {
+        for_few_rows(g, at, kMmaWarps, slices, kMmaColumns, out, heads, smem, &counter, lane,
+                     [&](const auto& part, int slice) { sum(at, part, slice); }, [&](int64_t lo, int64_t hi) {
+                         const int n = chunk_rows(at, lo, hi, kMmaWarps);
+                         for_slices(static_cast<int>((hi - lo + n - 1) / n), slices, &counter, lane, [&](int i, int slice) {
+                             const int64_t r = lo + static_cast<int64_t>(i) * n;
+                             sum(at, Part<kWhole>{r, r + n < hi ? r + n : hi}, slice);
+                         });
+                     });
+    };
+    if (run == kSorted) {
+        rows(offsets);
+    } else if (*g.longest <= g.limit) {
+        rows(starts);
+    } else { // (`out` has been cleared by a kernel before)
+        const int edges = starts[g.rows], chunks = (edges + g.chunk - 1) / g.chunk;
+        const int mine = static_cast<int>(blockIdx.x), blocks = static_cast<int>(gridDim.x);
+        for_slices(chunks > mine ? (chunks - mine + blocks - 1) / blocks : 0, slices, &counter, lane, [&](int i, int slice) {
+            const int p = (mine + i * blocks) * g.chunk, end = edges - p > g.chunk ? p + g.chunk : edges;
+            // the rows of the first and of the last edge
+            sum(starts, Part<kCut>{warp_count_weighted_le(starts, g.rows + 1, 0, p, lane) - 1,
+                                   warp_count_weighted_le(starts, g.rows + 1, 0, end - 1, lane), p, end, nullptr}, slice);
+        });
+    }
 }
 
 #endif

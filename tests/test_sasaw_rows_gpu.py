@@ -208,3 +208,27 @@ def test_gradients_by_mma(oracle, channels, L):
     others = d["indices_output_1"] != row
     for k in ("grad_A", "grad_B"):
         assert np.array_equal(inf[k][others], got[k][others]), k
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("L", [16, 32, 64, 100])
+@pytest.mark.parametrize("rows", ["even", "long", "gaps", "one"])
+def test_few_rows(oracle, dtype, L, rows):
+    """Fewer rows than six a warp: a block's edges in equal pieces. Rows within one piece, over several, a block's only row,
+    rows without edges at pieces' ends; the same bits in every run."""
+    r = np.random.default_rng(9)
+    lengths = {"even": np.full(300, 61), "long": np.where(np.arange(150) % 50 == 7, 900, 40),
+               "gaps": np.where(r.random(1200) < 0.5, 0, 33), "one": np.r_[np.zeros(40), 9000, np.zeros(3)]}[rows].astype(int)
+    n = len(lengths)
+    d = workloads.sasaw(E=int(lengths.sum()), n=n, nA=9, nW2=9, nO2=10, L=L, N=100)
+    d["indices_output_1"] = np.repeat(np.arange(n), lengths).astype(np.int32)
+    d["indices_W_1"] = r.permutation(d["indices_output_1"])
+    t = to_dev(d, dtype)
+    got = run_library("sasaw", t)
+    rounded = {k: v.astype(dtype).astype(np.float64) if isinstance(v, np.ndarray) and v.dtype == np.float64 else v
+               for k, v in d.items()}
+    want = run_checker(oracle, "sasaw", rounded, np.float64)
+    for k in want:
+        assert_parity(got[k], want[k].astype(dtype), f"sasaw few rows {rows} L={L}/{k}")
+    again = run_library("sasaw", t)
+    assert np.array_equal(again["output"], got["output"])
