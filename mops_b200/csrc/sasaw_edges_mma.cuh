@@ -19,7 +19,7 @@
 //
 // What bounds it: latency at two warps per scheduler (254 registers) and issue slots (34 %), FP64 pipes 35 %. 9 x 9 x 9
 // channels, 32 columns, against the multiply-adds of sasaw_rows.cu: 60 000 edges 66 -> 52 us, 4.2 10^6 edges with
-// tables of 19 MB 2.51 -> 2.24 ms; gathered tables beyond L2 stay there (gradients_shape_by_mma). gA added up in
+// tables of 19 MB 2.53 -> 2.33 ms; gathered tables beyond L2 stay there (gradients_shape_by_mma). gA added up in
 // global memory instead: 3.0 ms; with the hint to bring 256 bytes into L2: slower from 38 MB on.
 #ifndef MOPS_B200_SASAW_EDGES_MMA_CUH
 #define MOPS_B200_SASAW_EDGES_MMA_CUH
@@ -178,7 +178,12 @@ __device__ __forceinline__ void mma_edge_window(const RowsArgs<double>& g, const
             const int hi = min(static_cast<int>(offsets[row + 1]), p_hi);
             if (lo >= hi) continue;
             // E and the ninths' coefficients
-            if (w_row != row || w_slice != slice) fetch_w(row, slice, w_half);
+            if (w_row != row || w_slice != slice) { // (another row's may be on its way to the same place)
+                cp_async_commit();
+                cp_async_wait<0>();
+                __syncwarp();
+                fetch_w(row, slice, w_half);
+            }
             if (w_age < kDepth) {
                 cp_async_commit();
                 cp_async_wait<0>();
@@ -195,7 +200,7 @@ __device__ __forceinline__ void mma_edge_window(const RowsArgs<double>& g, const
                 const double* w = w_rows + w_half * (kWidest * 8);
                 const double* d = table + lane;
                 const double* d9 = table + nW * KS * 32 + q;
-#pragma unroll 1
+#pragma unroll 3
                 for (int m2 = 0; m2 < nW; m2++, w += 8, d += KS * 32, d9 += 20) {
                     double x[kColumns];
 #pragma unroll

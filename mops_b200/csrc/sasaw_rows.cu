@@ -965,10 +965,10 @@ template <typename T> bool sums_by_mma(const RowsShape<T>& s, const T* out) {
     return sizeof(T) == 8 && sums_shape_by_mma(s.g.nA, s.g.L) && s.aligned && reinterpret_cast<uintptr_t>(out) % 16 == 0;
 }
 // The gradients of A and B on the same instruction: up to nine channels, 16-byte pieces of every operand, and a
-// gathered table that L2 holds. (The others take a row's columns eight at a time, 64 bytes, from DRAM: 4.2 10^6
-// edges, 38, 75 and 151 MB: 2.39, 2.59, 3.10 ms against 2.55, 2.70, 2.82.)
+// gathered table that stays in L2 beside what streams through it. (A row's columns are taken eight at a time, 64 bytes: 4.2 10^6
+// edges, tables of 19, 38, 75 and 151 MB: 2.33, 2.39, 2.59 to 2.81, 3.10 ms against 2.53, 2.55, 2.65, 2.82.)
 inline bool gradients_shape_by_mma(int nA, int nO, int L, int64_t rows) {
-    constexpr double kCacheBytes = 100e6; // of the 126 MB
+    constexpr double kCacheBytes = 60e6; // of the 126 MB
     return nA <= 9 && nO <= 9 && L % 2 == 0 && L >= 8 && static_cast<double>(rows) * nO * L * 8 <= kCacheBytes;
 }
 template <typename T> bool gradients_by_mma(const RowsShape<T>& s, const T* W, const T* gB) {
