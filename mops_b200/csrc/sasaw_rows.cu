@@ -907,6 +907,14 @@ template <typename T> bool rows_apply(const SasawProblem<T>& p) {
            p.L >= 1 && p.L <= (1 << 20) && p.E >= 1 && positions_fit_int(p.E) && p.rows >= 1 && p.N <= (1 << 20);
 }
 
+// Shared memory for the table and the rings, beside what the kernels declare themselves (the counter, the pieces' heads).
+// At most 16 channels each, all but these fit: f64, up to 4 columns, 5 to 9 components of A, 10 or more gathered
+// channels and 13 or more outputs, whose table and rings alone take the whole of it.
+constexpr size_t kStaticShared = 1024;
+template <typename T> bool rows_fit(const Call& call, const RowsShape<T>& s) {
+    return s.smem + kStaticShared <= static_cast<size_t>(max_optin_smem(call.device));
+}
+
 // Two columns per lane (f32) from 33 columns on, where every operand allows 8-byte accesses.
 template <typename T> int vector_width(int L, std::initializer_list<const void*> operands) {
     if (sizeof(T) == 8 || L % 2 != 0 || L <= 32) return 1;
@@ -1144,7 +1152,7 @@ template <typename T> double sasaw_rows_cost(const SasawProblem<T>& p, RowsWork 
 template <typename T> int sasaw_forward_rows(const Call& call, const SasawProblem<T>& p, T* O, ScatterPart part) {
     if (!rows_apply(p)) return kNotApplicable;
     RowsShape<T> s = rows_shape(call, p, p.W, false, vector_width<T>(p.L, {p.B, p.W, O}));
-    if (s.smem > static_cast<size_t>(max_optin_smem(call.device))) return kNotApplicable;
+    if (!rows_fit(call, s)) return kNotApplicable;
     TableRef table = dense_table(call, p, s, false);
     s.g.gather = p.J, s.g.perm = nullptr, s.g.D = static_cast<const T*>(table.ptr), s.g.bit = kBitJ;
     bool unsorted = true;
@@ -1179,7 +1187,7 @@ template <typename T>
 bool sasaw_backward_rows(const Call& call, const SasawProblem<T>& p, T* gA, T* gB, T* gW, const T* gO) {
     if (!rows_apply(p)) return false;
     RowsShape<T> s = rows_shape(call, p, gO, true, vector_width<T>(p.L, {p.B, p.W, gO, gB, gW}));
-    if (s.smem > static_cast<size_t>(max_optin_smem(call.device))) return false;
+    if (!rows_fit(call, s)) return false;
     TableRef table = dense_table(call, p, s, true);
     // the edges in the order of J
     const int sorters = sort_blocks(call, p.E, p.rows);

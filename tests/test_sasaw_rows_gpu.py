@@ -232,3 +232,17 @@ def test_few_rows(oracle, dtype, L, rows):
         assert_parity(got[k], want[k].astype(dtype), f"sasaw few rows {rows} L={L}/{k}")
     again = run_library("sasaw", t)
     assert np.array_equal(again["output"], got["output"])
+
+
+@pytest.mark.parametrize("channels", [(9, 10, 13), (9, 13, 10), (9, 16, 13), (9, 16, 16)])
+@pytest.mark.parametrize("E,n", [(2000, 40), (60000, 2500)])
+@pytest.mark.parametrize("order", ["sorted", "unsorted"])
+def test_widest_shared_memory(oracle, channels, E, n, order):
+    """f64, up to four columns: the table and rings of the row kernels take all of the shared memory, or just as much as
+    there is without the kernels' own variables, forward (13 and more outputs) and gradients (13 and more channels
+    of W). Sizes that are estimated to be faster by rows."""
+    nA, nW2, nO2 = channels
+    d = workloads.sasaw(E=E, n=n, nA=nA, nW2=nW2, nO2=nO2, L=4, N=100)
+    if order == "unsorted":
+        d["indices_output_1"] = np.random.default_rng(5).permutation(d["indices_output_1"])
+    compare("sasaw", d, np.float64, oracle, what=f"sasaw {channels} E={E} {order}")
