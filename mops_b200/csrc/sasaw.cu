@@ -2499,19 +2499,42 @@ constexpr int64_t kShortRows = 24; // edges; from here on the forward by rows is
 template <typename T> double rows_margin(const Problem<T>& p) {
     return p.E >= kShortRows * p.nW0 ? kMargin : 1 / kMargin;
 }
-// On the FP64 tensor-core instruction the sums by rows were the faster ones in all of 207 shapes with a sorted index (5 to
-// 100 edges per row), and in 26 of 30 without, the others (less than 10^4 edges, whose sort counts) by up to a sixth.
+// Warps of a block of the quad kernel: wide channels leave it fewer than eight.
+template <typename T> double quad_warps(const Problem<T>& p) {
+    const QuadLayout q = quad_layout(p.nA, p.nW1, p.nO1);
+    const double room = 227.0 * 1024 / sizeof(T) - q.d_scalars;
+    return std::min(8.0, std::max(1.0, std::floor(room / q.warp_scalars)));
+}
+// The quad kernel beside the row sums on the FP64 tensor-core instruction: microseconds, fitted to the same 1400 shapes (sums_mma_cost);
+// nine in ten estimates are within a fifth.
+template <typename T> double quad_cost(const Problem<T>& p) {
+    struct Cost {
+        double call, cell, quad, edge, entry, result, few, row, value; // in 10^-5, -4, -4, -2, -6, -1, -3, -6
+    };
+    constexpr Cost compiled_in{39.4, 0, 0.185, 1.19, 2.92, 1.73, 7.62, 0.494, 0.459};
+    constexpr Cost any{43.1, 0.125, 0.224, 3.59, 3.03, 0.534, 14.5, 1.19, 0.255};
+    const Cost& c = p.nA == p.nW1 && p.nA == p.nO1 && (p.nA == 4 || p.nA == 9 || p.nA == 16) ? compiled_in : any;
+    const double E = static_cast<double>(p.E), n = static_cast<double>(p.nW0), N = static_cast<double>(p.N);
+    const double columns = static_cast<double>(ceil_div(p.L, 32)), warps = quad_warps(p), share = 8 / warps;
+    const double quads = E / 4 + 0.75 * n * (1 - std::exp(-E / n)); // (a row's last one is not full)
+    const double cells = static_cast<double>(ceil_div(p.nW1 * p.nO1, 8) * ceil_div(p.nA, 4));
+    const double quad = p.nW1 * (p.nO1 > 9 ? 8 : 4) * columns;
+    const double few = std::max(0.0, 1 - n / (148 * warps)) * E / n; // a row's edges one after the other
+    return c.call + share * (1e-5 * c.cell * E * cells + 1e-4 * (c.quad * quads * quad + c.edge * E * columns) + 1e-3 * c.row * n * columns) +
+           1e-2 * c.entry * N + 1e-6 * (c.result * n * p.nO1 * p.L + c.value * E * p.nW1 * p.L) +
+           0.1 * c.few * few * (1 + 5e-3 * quad);
+}
+// With short rows the coupling, applied per row, is nearly all of the work of the row sums: of 1400 shapes the quad kernel
+// is the faster one in 221, most of them with 1 to 8 edges per row and wide channels (16 x 9 -> 9, 32 columns, 4 10^5 edges,
+// 2 per row: 0.75 against 1.35 ms by rows). By these estimates 2 % of the shapes take more than 1.1 times the better kernel's time.
 template <typename T> bool sorted_by_rows(const Problem<T>& p) {
-    if (p.E >= p.nW0 && sasaw_rows_by_mma(rows_problem(p), RowsWork::kSorted)) return true;
+    if (p.E >= p.nW0 && sasaw_rows_by_mma(rows_problem(p), RowsWork::kSorted))
+        return sasaw_rows_cost(rows_problem(p), RowsWork::kSorted) < 0.95 * quad_cost(p);
     const EdgeCost cost = sizeof(T) == 4 ? EdgeCost{33.2, 4.1, 0, 342, 32.1, 2.02, 91.9, 720}
                           : p.L % 2 == 0 ? EdgeCost{46.2, 4.04, 0.0252, 403, 78.6, 4.15, 28, 568}
                                          : EdgeCost{37.7, 7.7, 0, 337, 0, 10.8, 45.7, 998};
     double us = edge_cost(p, cost);
-    if (sizeof(T) == 8 && p.L % 2 == 0) { // wide channels leave the quad kernel fewer than eight warps
-        const QuadLayout q = quad_layout(p.nA, p.nW1, p.nO1);
-        const double room = 227.0 * 1024 / sizeof(T) - q.d_scalars, warps = std::max(1.0, std::floor(room / q.warp_scalars));
-        us *= std::max(1.0, 8 / warps);
-    }
+    if (sizeof(T) == 8 && p.L % 2 == 0) us *= 8 / quad_warps(p);
     return p.E >= p.nW0 && sasaw_rows_cost(rows_problem(p), RowsWork::kSorted) < us * rows_margin(p);
 }
 template <typename T> bool unsorted_by_rows(const Problem<T>& p) {

@@ -1090,6 +1090,23 @@ template <typename T> bool sasaw_rows_by_mma(const SasawProblem<T>& p, RowsWork 
     return work == RowsWork::kGradients ? gradients_shape_by_mma(p.nA, p.nO, p.L, p.rows) : sums_shape_by_mma(p.nA, p.L);
 }
 
+// The sums on the FP64 tensor-core instruction, sorted index: microseconds, fitted to 1400 shapes, 1 to 100 edges per row,
+// up to 2 10^6 edges and 1000 coupling entries; nine in ten estimates are within a fifth. Operations of the steps (one more
+// for rows whose ends cut one) and of the coupling (half as much again where the last pass has fewer channels), what each of
+// them costs beside, the coupling's table, a row's steps one after the other where rows are few, results read again by later passes.
+inline double sums_mma_cost(int64_t edges, int64_t rows, int nA, int nW, int nO, int L, int64_t N) {
+    const int na = pad_a(nA), nc = chunk_c(na, nW), ma = na == 16 ? 2 : 1, ninth = nA == 9 ? 1 : 0;
+    const double E = static_cast<double>(edges), n = static_cast<double>(rows);
+    const double passes = static_cast<double>(ceil_div(nW, nc)), columns = static_cast<double>(ceil_div(L, 16));
+    const double steps = (E / 4 + 0.75 * n * (1 - std::exp(-E / n))) * columns * passes, results = n * columns * passes;
+    const double step = nc * 2 * (ma * 16 + 2 * ninth + 2), part = nW % nc != 0 ? 1.5 : 1;
+    const double couple = part * (2 * ma + ninth) * nc * 32 * static_cast<double>(ceil_div(nO, 8));
+    const double table = static_cast<double>(ceil_div(nO, kTableOut)) * kTableOut * na * passes * nc * static_cast<double>(N);
+    const double few = std::max(0.0, 1 - n * columns / 1776) * E / n * passes * nc * ma;
+    return 37.6 + 1e-6 * (steps * (1.32 * step + 84) + results * (0.596 * couple + 117) + 4.4 * table +
+                          1.42 * n * nO * L * (passes - 1)) + 0.0139 * few;
+}
+
 // The gradients on the FP64 tensor-core instruction, all three of them: microseconds, fitted to 148 shapes up to
 // 2 10^6 edges; eight in ten estimates are within a sixth. Clocks of the instructions of a step, of a row's E, of the sums'
 // steps and coupling, and what the coupling's table takes.
@@ -1108,13 +1125,15 @@ inline double gradients_mma_cost(int64_t edges, int64_t rows, int nA, int nW, in
            1.64 * few * slices * step / 8e3;
 }
 
-// Microseconds, fitted to 750 shapes up to 2 10^6 edges with 1 to 16 channels, 1 to 100 columns and rows of
+// By multiply-adds: microseconds, fitted to 750 shapes up to 2 10^6 edges with 1 to 16 channels, 1 to 100 columns and rows of
 // a fraction of an edge to thousands; nine in ten estimates are within a third where a call takes more
 // than 80 us. A step is an edge (or the edges side by side) in one pass over columns and channels.
 template <typename T> double sasaw_rows_cost(const SasawProblem<T>& p, RowsWork work) {
     if (!rows_apply(p)) return INFINITY;
     if (work == RowsWork::kGradients && sasaw_rows_by_mma(p, work))
         return gradients_mma_cost(p.E, p.rows, p.nA, p.nW, p.nO, p.L, p.N);
+    if (work == RowsWork::kSorted && sasaw_rows_by_mma(p, work))
+        return sums_mma_cost(p.E, p.rows, p.nA, p.nW, p.nO, p.L, p.N);
     struct Cost {
         double call, product, step, exact_product, exact_step; // products and steps in 10^-6
         double contract, contract_once, table, pass, edge, row; // 10^-6, 10^-3, 10^-5, 1, 10^-6, 10^-3

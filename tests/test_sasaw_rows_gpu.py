@@ -246,3 +246,26 @@ def test_widest_shared_memory(oracle, channels, E, n, order):
     if order == "unsorted":
         d["indices_output_1"] = np.random.default_rng(5).permutation(d["indices_output_1"])
     compare("sasaw", d, np.float64, oracle, what=f"sasaw {channels} E={E} {order}")
+
+
+def _forward(t):
+    out = mops_b200.sparse_accumulation_scatter_add_with_weights(
+        t["A"], t["B"], t["C"], t["W"], t["indices_A"], t["indices_W_1"], t["indices_W_2"], t["indices_output_1"],
+        t["indices_output_2"], t["output_size"])
+    return out, _lib.last_kernels()
+
+
+# (estimates, by edge and by rows: 0.17 and 0.36, 0.31 and 0.41, 0.125 and 0.158, 0.080 and 0.067, 0.16 and 0.10 ms)
+@pytest.mark.parametrize("channels,L,E,n,by_edge", [
+    ((16, 9, 9), 32, 80000, 40000, True), ((16, 16, 16), 32, 60000, 20000, True), ((9, 9, 9), 32, 90000, 30000, True),
+    ((9, 9, 9), 32, 80000, 2500, False), ((4, 9, 4), 64, 60000, 10000, False)])
+def test_short_rows(oracle, channels, L, E, n, by_edge):
+    """f64, sorted index: rows so short that the coupling per row costs more than the edges go by edge."""
+    nA, nW2, nO2 = channels
+    d = workloads.sasaw(E=E, n=n, nA=nA, nW2=nW2, nO2=nO2, L=L, N=100)
+    got, kernels = _forward(to_dev(d, np.float64))
+    assert any("sasaw_fwd_quad" in k for k in kernels) == by_edge, kernels
+    assert any("sasaw_sum_rows_mma" in k for k in kernels) != by_edge, kernels
+    want = oracle.sasaw(d["A"], d["B"], d["C"], d["W"], d["indices_A"], d["indices_W_1"], d["indices_W_2"],
+                        d["indices_output_1"], d["indices_output_2"], nO2)
+    assert_parity(got.cpu().numpy(), want, f"sasaw short rows {channels}")
