@@ -1090,21 +1090,28 @@ template <typename T> bool sasaw_rows_by_mma(const SasawProblem<T>& p, RowsWork 
     return work == RowsWork::kGradients ? gradients_shape_by_mma(p.nA, p.nO, p.L, p.rows) : sums_shape_by_mma(p.nA, p.L);
 }
 
-// The sums on the FP64 tensor-core instruction, sorted index: microseconds, fitted to 1400 shapes, 1 to 100 edges per row,
-// up to 2 10^6 edges and 1000 coupling entries; nine in ten estimates are within a fifth. Operations of the steps (one more
-// for rows whose ends cut one) and of the coupling (half as much again where the last pass has fewer channels), what each of
-// them costs beside, the coupling's table, a row's steps one after the other where rows are few, results read again by later passes.
-inline double sums_mma_cost(int64_t edges, int64_t rows, int nA, int nW, int nO, int L, int64_t N) {
+// The sums on the FP64 tensor-core instruction: microseconds, fitted to 1400 shapes with a sorted index and 450 without, 1 to 100
+// edges per row, up to 2 10^6 edges and 1000 coupling entries; nine in ten estimates are within a fifth. Operations of the steps
+// (one more for rows whose ends cut one) and of the coupling (half as much again where the last pass has fewer channels), what
+// each of them costs beside, the coupling's table, results read again by later passes, the sort, a row's steps one after the
+// other where rows are few.
+inline double sums_mma_cost(bool sorted, int64_t edges, int64_t rows, int nA, int nW, int nO, int L, int64_t N) {
+    struct Cost {
+        double call, operation, step, couple, result, table, again, edge, few; // in 10^-6 but the first one
+    };
+    constexpr Cost with_order{37.6, 1.32, 84, 0.596, 117, 4.4, 1.42, 0, 13900};
+    constexpr Cost without{62.7, 1.31, 46, 0.771, 52, 4.98, 1.03, 74, 12900};
+    const Cost& c = sorted ? with_order : without;
     const int na = pad_a(nA), nc = chunk_c(na, nW), ma = na == 16 ? 2 : 1, ninth = nA == 9 ? 1 : 0;
     const double E = static_cast<double>(edges), n = static_cast<double>(rows);
     const double passes = static_cast<double>(ceil_div(nW, nc)), columns = static_cast<double>(ceil_div(L, 16));
     const double steps = (E / 4 + 0.75 * n * (1 - std::exp(-E / n))) * columns * passes, results = n * columns * passes;
-    const double step = nc * 2 * (ma * 16 + 2 * ninth + 2), part = nW % nc != 0 ? 1.5 : 1;
+    const double operations = nc * 2 * (ma * 16 + 2 * ninth + 2), part = nW % nc != 0 ? 1.5 : 1;
     const double couple = part * (2 * ma + ninth) * nc * 32 * static_cast<double>(ceil_div(nO, 8));
     const double table = static_cast<double>(ceil_div(nO, kTableOut)) * kTableOut * na * passes * nc * static_cast<double>(N);
     const double few = std::max(0.0, 1 - n * columns / 1776) * E / n * passes * nc * ma;
-    return 37.6 + 1e-6 * (steps * (1.32 * step + 84) + results * (0.596 * couple + 117) + 4.4 * table +
-                          1.42 * n * nO * L * (passes - 1)) + 0.0139 * few;
+    return c.call + 1e-6 * (steps * (c.operation * operations + c.step) + results * (c.couple * couple + c.result) +
+                            c.table * table + c.again * n * nO * L * (passes - 1) + c.edge * E + c.few * few);
 }
 
 // The gradients on the FP64 tensor-core instruction, all three of them: microseconds, fitted to 148 shapes up to
@@ -1132,8 +1139,8 @@ template <typename T> double sasaw_rows_cost(const SasawProblem<T>& p, RowsWork 
     if (!rows_apply(p)) return INFINITY;
     if (work == RowsWork::kGradients && sasaw_rows_by_mma(p, work))
         return gradients_mma_cost(p.E, p.rows, p.nA, p.nW, p.nO, p.L, p.N);
-    if (work == RowsWork::kSorted && sasaw_rows_by_mma(p, work))
-        return sums_mma_cost(p.E, p.rows, p.nA, p.nW, p.nO, p.L, p.N);
+    if (work != RowsWork::kGradients && sasaw_rows_by_mma(p, work))
+        return sums_mma_cost(work == RowsWork::kSorted, p.E, p.rows, p.nA, p.nW, p.nO, p.L, p.N);
     struct Cost {
         double call, product, step, exact_product, exact_step; // products and steps in 10^-6
         double contract, contract_once, table, pass, edge, row; // 10^-6, 10^-3, 10^-5, 1, 10^-6, 10^-3

@@ -269,3 +269,20 @@ def test_short_rows(oracle, channels, L, E, n, by_edge):
     want = oracle.sasaw(d["A"], d["B"], d["C"], d["W"], d["indices_A"], d["indices_W_1"], d["indices_W_2"],
                         d["indices_output_1"], d["indices_output_2"], nO2)
     assert_parity(got.cpu().numpy(), want, f"sasaw short rows {channels}")
+
+
+# (estimates, by edge and by rows: 0.43 and 1.63, 0.19 and 0.30, 0.22 and 0.12, 0.15 and 0.09 ms)
+@pytest.mark.parametrize("channels,L,E,n,by_edge", [
+    ((16, 16, 16), 64, 60000, 45000, True), ((9, 9, 4), 64, 60000, 50000, True), ((9, 9, 9), 32, 120000, 4000, False),
+    ((4, 4, 9), 64, 50000, 5000, False)])
+def test_short_rows_unsorted(oracle, channels, L, E, n, by_edge):
+    """f64, no order in the index: short rows are not sorted but go by edge."""
+    nA, nW2, nO2 = channels
+    d = workloads.sasaw(E=E, n=n, nA=nA, nW2=nW2, nO2=nO2, L=L, N=100)
+    d["indices_output_1"] = np.random.default_rng(7).permutation(d["indices_output_1"])
+    got, kernels = _forward(to_dev(d, np.float64))
+    # (for a sorted index first, and then again, or by edge)
+    assert (sum("sasaw_sum_rows_mma" in k for k in kernels) == 2) != by_edge, kernels
+    want = oracle.sasaw(d["A"], d["B"], d["C"], d["W"], d["indices_A"], d["indices_W_1"], d["indices_W_2"],
+                        d["indices_output_1"], d["indices_output_2"], nO2)
+    assert_parity(got.cpu().numpy(), want, f"sasaw short rows, unsorted {channels}")
