@@ -2558,6 +2558,32 @@ template <typename T> bool unsorted_by_rows(const Problem<T>& p) {
                                          : EdgeCost{33.7, 1.73, 0, 1110, 23.6, 106, 0, 0};
     return sasaw_rows_cost(rows_problem(p), RowsWork::kUnsorted) < edge_cost(p, cost) * rows_margin(p);
 }
+// Whether the kernel by edge on the tensor-core instruction takes the f64 gradients (its tables fit shared memory).
+template <typename T> bool gradients_by_mma(const Problem<T>& p) {
+    switch (fast_width(p.nW1)) {
+    case 4: return vjp_mma_smem<4>(p.nA, p.nW1, p.nO1) <= kVjpMmaSmem;
+    case 8: return vjp_mma_smem<8>(p.nA, p.nW1, p.nO1) <= kVjpMmaSmem;
+    case 12: return vjp_mma_smem<12>(p.nA, p.nW1, p.nO1) <= kVjpMmaSmem;
+    default: return vjp_mma_smem<16>(p.nA, p.nW1, p.nO1) <= kVjpMmaSmem;
+    }
+}
+// The gradients by edge beside the row kernels on the FP64 tensor-core instruction: microseconds, fitted to 652 shapes of rows of 1
+// to 200 edges, 60 to 60 000 of them, nine in ten within a fifth; `us`, as for the other row kernels, of the third family. The kernel
+// with compiled-in widths gives a row of the output to a warp, whose edges come one after the other where there are few rows (66
+// rows of 200 edges: 830 us, 105 by rows); rows of unlike lengths, which the estimate does not know, cost it more: 1.05. By these
+// estimates 4 % of 600 other shapes take more than 1.1 times the better family's time.
+template <typename T> double gradients_cost(const Problem<T>& p, double us) {
+    const double E = static_cast<double>(p.E), n = static_cast<double>(p.nW0), N = static_cast<double>(p.N);
+    const double columns = static_cast<double>(ceil_div(p.L, 32)), cells = static_cast<double>(p.nW1) * p.nO1;
+    if (quad_gradients(p)) {
+        const double few = std::max(0.0, 1 - n / 1184) * E / n; // (eight warps per SM)
+        return 1.05 * (46.6 + columns * (1.235e-3 * E + 1.6e-3 * n + 2.24 * few) + 0.0215 * N + 6.2e-5 * n * p.L);
+    }
+    if (!gradients_by_mma(p)) return 1.2 * us;
+    const double w = static_cast<double>(ceil_div(p.nW1, 4)), o = static_cast<double>(ceil_div(p.nO1, 4));
+    return 0.95 * (43.2 + E * (1e-4 * columns * (0.834 * w * o + 0.925 * w + 5.08) + 1e-6 * p.L * (0.536 * p.nW1 + 0.474 * p.nO1)) +
+                   2.52e-6 * n * p.nW1 * p.L + N * (2.37e-3 * N + 7.2e-7 * E) / cells);
+}
 // The f64 gradients have three kernels by edge. The one with compiled-in widths adds to gW from all over it,
 // which costs more where W and gW are larger than L2 (4.2 10^6 edges, 151 MB each: 5.70 against 4.85 ms),
 // and gives a row of the output to one warp, however long (60 000 edges in one: 45 against 0.16 ms).
@@ -2573,20 +2599,12 @@ template <typename T> bool gradients_by_rows(const Problem<T>& p) {
         us *= 1 + 0.8 * std::max(0.0, 1 - kCacheBytes / tables);
         margin = kMargin;
     } else {
-        size_t smem = 0;
-        switch (fast_width(p.nW1)) {
-        case 4: smem = vjp_mma_smem<4>(p.nA, p.nW1, p.nO1); break;
-        case 8: smem = vjp_mma_smem<8>(p.nA, p.nW1, p.nO1); break;
-        case 12: smem = vjp_mma_smem<12>(p.nA, p.nW1, p.nO1); break;
-        default: smem = vjp_mma_smem<16>(p.nA, p.nW1, p.nO1);
-        }
-        const bool mma = smem <= kVjpMmaSmem;
+        const bool mma = gradients_by_mma(p);
         us = edge_cost(p, mma ? EdgeCost{24.2, 13.6, 0, 541, 45.1, 5.47, 0, 0}
                               : EdgeCost{21.9, 25.6, 0.034, 2510, 12.2, 1.09, 0, 0});
         margin = mma ? 1 / 1.5 : 1 / 1.1;
     }
-    // (on the FP64 tensor-core instruction: of 148 shapes 5 % then take more than 1.1 times the better family's time)
-    if (sasaw_rows_by_mma(rows_problem(p), RowsWork::kGradients)) margin = quad_gradients(p) && p.nW0 < 1184 ? 2 : 1.2;
+    if (sasaw_rows_by_mma(rows_problem(p), RowsWork::kGradients)) us = gradients_cost(p, us), margin = 1;
     return sasaw_rows_cost(rows_problem(p), RowsWork::kGradients) < us * margin;
 }
 

@@ -286,3 +286,15 @@ def test_short_rows_unsorted(oracle, channels, L, E, n, by_edge):
     want = oracle.sasaw(d["A"], d["B"], d["C"], d["W"], d["indices_A"], d["indices_W_1"], d["indices_W_2"],
                         d["indices_output_1"], d["indices_output_2"], nO2)
     assert_parity(got.cpu().numpy(), want, f"sasaw short rows, unsorted {channels}")
+
+
+# (estimates, by edge and by rows: 57 and 71, 82 and 114, 63 and 73; 970 and 162, 147 and 136 us)
+@pytest.mark.parametrize("channels,L,E,n,by_edge", [
+    ((9, 9, 9), 32, 1036, 518, True), ((4, 9, 9), 68, 8220, 137, True), ((9, 8, 9), 10, 17400, 870, True),
+    ((9, 9, 9), 38, 13200, 66, False), ((4, 9, 9), 32, 60000, 2500, False)])
+def test_gradients_by_estimate(oracle, channels, L, E, n, by_edge):
+    """f64, few or short rows: by edge, but not where a warp would have a long row of the output to itself."""
+    nA, nW2, nO2 = channels
+    d = workloads.sasaw(E=E, n=n, nA=nA, nW2=nW2, nO2=nO2, L=L, N=100)
+    compare("sasaw", d, np.float64, oracle, what=f"sasaw gradients {channels} E={E}")
+    assert any("sasaw_vjp_" in k for k in _lib.last_kernels()) == by_edge, _lib.last_kernels()
