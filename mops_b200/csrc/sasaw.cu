@@ -2527,15 +2527,15 @@ template <typename T> double quad_cost(const Problem<T>& p) {
 // With short rows the coupling, applied per row, is nearly all of the work of the row sums: of 1400 shapes the quad kernel
 // is the faster one in 221, most of them with 1 to 8 edges per row and wide channels (16 x 9 -> 9, 32 columns, 4 10^5 edges,
 // 2 per row: 0.75 against 1.35 ms by rows). By these estimates 2 % of the shapes take more than 1.1 times the better kernel's time.
-template <typename T> bool sorted_by_rows(const Problem<T>& p) {
-    if (p.E >= p.nW0 && sasaw_rows_by_mma(rows_problem(p), RowsWork::kSorted))
-        return sasaw_rows_cost(rows_problem(p), RowsWork::kSorted) < 0.95 * quad_cost(p);
+template <typename T> bool sorted_by_rows(const Problem<T>& p, const T* O) {
+    if (p.E >= p.nW0 && sasaw_rows_by_mma(rows_problem(p), RowsWork::kSorted, {O}))
+        return sasaw_rows_cost(rows_problem(p), RowsWork::kSorted, true) < 0.95 * quad_cost(p);
     const EdgeCost cost = sizeof(T) == 4 ? EdgeCost{33.2, 4.1, 0, 342, 32.1, 2.02, 91.9, 720}
                           : p.L % 2 == 0 ? EdgeCost{46.2, 4.04, 0.0252, 403, 78.6, 4.15, 28, 568}
                                          : EdgeCost{37.7, 7.7, 0, 337, 0, 10.8, 45.7, 998};
     double us = edge_cost(p, cost);
     if (sizeof(T) == 8 && p.L % 2 == 0) us *= 8 / quad_warps(p);
-    return p.E >= p.nW0 && sasaw_rows_cost(rows_problem(p), RowsWork::kSorted) < us * rows_margin(p);
+    return p.E >= p.nW0 && sasaw_rows_cost(rows_problem(p), RowsWork::kSorted, false) < us * rows_margin(p);
 }
 // The kernel for an unsorted index beside them: microseconds, fitted to the same 450 shapes. The last term is the order of a
 // cell's coupling entries, made one by one.
@@ -2550,13 +2550,13 @@ template <typename T> double unsorted_cost(const Problem<T>& p) {
 // Rows of an unsorted index are cut where they are long, and the sort counts: of 450 shapes the kernel by edge is the faster
 // one in a third (16 channels each, 64 columns, 7 10^4 edges, 1.3 per row: 0.46 against 1.61 ms by rows). By these estimates 6 %
 // take more than 1.1 times the better kernel's time.
-template <typename T> bool unsorted_by_rows(const Problem<T>& p) {
-    if (sasaw_rows_by_mma(rows_problem(p), RowsWork::kUnsorted))
-        return sasaw_rows_cost(rows_problem(p), RowsWork::kUnsorted) < 0.95 * unsorted_cost(p);
+template <typename T> bool unsorted_by_rows(const Problem<T>& p, const T* O) {
+    if (sasaw_rows_by_mma(rows_problem(p), RowsWork::kUnsorted, {O}))
+        return sasaw_rows_cost(rows_problem(p), RowsWork::kUnsorted, true) < 0.95 * unsorted_cost(p);
     const EdgeCost cost = sizeof(T) == 4 ? EdgeCost{25.4, 3.54, 0.0224, 413, 18.5, 2.09, 0, 0}
                           : p.L % 2 == 0 ? EdgeCost{39.4, 6.25, 0, 439, 49.2, 2.39, 0, 0}
                                          : EdgeCost{33.7, 1.73, 0, 1110, 23.6, 106, 0, 0};
-    return sasaw_rows_cost(rows_problem(p), RowsWork::kUnsorted) < edge_cost(p, cost) * rows_margin(p);
+    return sasaw_rows_cost(rows_problem(p), RowsWork::kUnsorted, false) < edge_cost(p, cost) * rows_margin(p);
 }
 // Whether the kernel by edge on the tensor-core instruction takes the f64 gradients (its tables fit shared memory).
 template <typename T> bool gradients_by_mma(const Problem<T>& p) {
@@ -2587,7 +2587,7 @@ template <typename T> double gradients_cost(const Problem<T>& p, double us) {
 // The f64 gradients have three kernels by edge. The one with compiled-in widths adds to gW from all over it,
 // which costs more where W and gW are larger than L2 (4.2 10^6 edges, 151 MB each: 5.70 against 4.85 ms),
 // and gives a row of the output to one warp, however long (60 000 edges in one: 45 against 0.16 ms).
-template <typename T> bool gradients_by_rows(const Problem<T>& p) {
+template <typename T> bool gradients_by_rows(const Problem<T>& p, const T* gO, const T* gB) {
     constexpr double kCacheBytes = 100e6; // of the 126 MB of L2
     double us, margin;
     if (sizeof(T) == 4) {
@@ -2604,8 +2604,9 @@ template <typename T> bool gradients_by_rows(const Problem<T>& p) {
                               : EdgeCost{21.9, 25.6, 0.034, 2510, 12.2, 1.09, 0, 0});
         margin = mma ? 1 / 1.5 : 1 / 1.1;
     }
-    if (sasaw_rows_by_mma(rows_problem(p), RowsWork::kGradients)) us = gradients_cost(p, us), margin = 1;
-    return sasaw_rows_cost(rows_problem(p), RowsWork::kGradients) < us * margin;
+    const bool by_mma = sasaw_rows_by_mma(rows_problem(p), RowsWork::kGradients, {gO, gB});
+    if (by_mma) us = gradients_cost(p, us), margin = 1;
+    return sasaw_rows_cost(rows_problem(p), RowsWork::kGradients, by_mma) < us * margin;
 }
 
 template <typename T> int forward_by_edge(const Call& call, T* O, const Problem<T>& p, ScatterPart part) {
@@ -2620,7 +2621,7 @@ template <typename T> void forward(const Call& call, T* O, const Problem<T>& p) 
         MOPS_CUDA_OK(cudaMemsetAsync(O, 0, p.nW0 * rowsize * sizeof(T), call.stream));
         return;
     }
-    const bool sorted_rows = sorted_by_rows(p), unsorted_rows = unsorted_by_rows(p);
+    const bool sorted_rows = sorted_by_rows(p, O), unsorted_rows = unsorted_by_rows(p, O);
     // (an asynchronous call enqueues both parts, and would build both families' tables for them)
     const bool mixed = sorted_rows != unsorted_rows && call.wait;
     const ScatterPart first = mixed ? ScatterPart::kSorted : ScatterPart::kBoth;
@@ -2680,7 +2681,7 @@ void backward(const Call& call, T* gA, T* gB, T* gW, const T* gO, const Problem<
     if (gA == nullptr && gB == nullptr && gW == nullptr) return;
     const int64_t wsize = p.nW0 * static_cast<int64_t>(p.nW1) * p.L;
     const bool some = p.E > 0 && p.N > 0 && p.L > 0;
-    if (some && gradients_by_rows(p) && sasaw_backward_rows<T>(call, rows_problem(p), gA, gB, gW, gO)) return;
+    if (some && gradients_by_rows(p, gO, gB) && sasaw_backward_rows<T>(call, rows_problem(p), gA, gB, gW, gO)) return;
     if (gW != nullptr && wsize > 0)
         MOPS_CUDA_OK(cudaMemsetAsync(gW, 0, wsize * sizeof(T), call.stream));
     if (p.E == 0) return;

@@ -1084,9 +1084,11 @@ void launch_edges_mma(const Call& call, const RowsShape<T>& s, const int32_t* st
 
 } // namespace
 
-template <typename T> bool sasaw_rows_by_mma(const SasawProblem<T>& p, RowsWork work) {
-    if (sizeof(T) != 8 || !rows_apply(p) || (reinterpret_cast<uintptr_t>(p.B) | reinterpret_cast<uintptr_t>(p.W)) % 16 != 0)
-        return false;
+template <typename T>
+bool sasaw_rows_by_mma(const SasawProblem<T>& p, RowsWork work, std::initializer_list<const void*> others) {
+    uintptr_t all = reinterpret_cast<uintptr_t>(p.B) | reinterpret_cast<uintptr_t>(p.W);
+    for (const void* x : others) all |= reinterpret_cast<uintptr_t>(x);
+    if (sizeof(T) != 8 || !rows_apply(p) || all % 16 != 0) return false;
     return work == RowsWork::kGradients ? gradients_shape_by_mma(p.nA, p.nO, p.L, p.rows) : sums_shape_by_mma(p.nA, p.L);
 }
 
@@ -1135,12 +1137,10 @@ inline double gradients_mma_cost(int64_t edges, int64_t rows, int nA, int nW, in
 // By multiply-adds: microseconds, fitted to 750 shapes up to 2 10^6 edges with 1 to 16 channels, 1 to 100 columns and rows of
 // a fraction of an edge to thousands; nine in ten estimates are within a third where a call takes more
 // than 80 us. A step is an edge (or the edges side by side) in one pass over columns and channels.
-template <typename T> double sasaw_rows_cost(const SasawProblem<T>& p, RowsWork work) {
+template <typename T> double sasaw_rows_cost(const SasawProblem<T>& p, RowsWork work, bool mma) {
     if (!rows_apply(p)) return INFINITY;
-    if (work == RowsWork::kGradients && sasaw_rows_by_mma(p, work))
-        return gradients_mma_cost(p.E, p.rows, p.nA, p.nW, p.nO, p.L, p.N);
-    if (work != RowsWork::kGradients && sasaw_rows_by_mma(p, work))
-        return sums_mma_cost(work == RowsWork::kSorted, p.E, p.rows, p.nA, p.nW, p.nO, p.L, p.N);
+    if (mma && work == RowsWork::kGradients) return gradients_mma_cost(p.E, p.rows, p.nA, p.nW, p.nO, p.L, p.N);
+    if (mma) return sums_mma_cost(work == RowsWork::kSorted, p.E, p.rows, p.nA, p.nW, p.nO, p.L, p.N);
     struct Cost {
         double call, product, step, exact_product, exact_step; // products and steps in 10^-6
         double contract, contract_once, table, pass, edge, row; // 10^-6, 10^-3, 10^-5, 1, 10^-6, 10^-3
@@ -1253,8 +1253,8 @@ bool sasaw_backward_rows(const Call& call, const SasawProblem<T>& p, T* gA, T* g
 }
 
 #define INSTANTIATE(T)                                                                             \
-    template double sasaw_rows_cost<T>(const SasawProblem<T>&, RowsWork);                          \
-    template bool sasaw_rows_by_mma<T>(const SasawProblem<T>&, RowsWork);                          \
+    template bool sasaw_rows_by_mma<T>(const SasawProblem<T>&, RowsWork, std::initializer_list<const void*>); \
+    template double sasaw_rows_cost<T>(const SasawProblem<T>&, RowsWork, bool);                    \
     template int sasaw_forward_rows<T>(const Call&, const SasawProblem<T>&, T*, ScatterPart);      \
     template bool sasaw_backward_rows<T>(const Call&, const SasawProblem<T>&, T*, T*, T*, const T*);
 INSTANTIATE(float)

@@ -2,6 +2,8 @@
 #ifndef MOPS_B200_SASAW_ROWS_HPP
 #define MOPS_B200_SASAW_ROWS_HPP
 
+#include <initializer_list>
+
 #include "runtime.hpp"
 
 namespace mops_b200 {
@@ -20,12 +22,14 @@ enum class ScatterPart { kBoth, kSorted, kUnsorted };
 // enqueued, and the one for an unsorted index is still to come.
 enum : int { kNotApplicable = 0, kComplete = 1, kUnsortedLeft = 2 };
 
-// Microseconds that the row kernels take, as fitted to measurements; infinite where they do not apply.
+// Whether the kernels on the FP64 tensor-core instruction take this work (f64, 16-byte aligned operands), with `others`
+// beside the operands of `p`: the result of a forward, gO and gB of the gradients.
 enum class RowsWork { kSorted, kUnsorted, kGradients };
-template <typename T> double sasaw_rows_cost(const SasawProblem<T>& p, RowsWork work);
-// Whether the kernels on the FP64 tensor-core instruction take this work (f64, as far as shapes and the operands
-// known here tell).
-template <typename T> bool sasaw_rows_by_mma(const SasawProblem<T>& p, RowsWork work);
+template <typename T>
+bool sasaw_rows_by_mma(const SasawProblem<T>& p, RowsWork work, std::initializer_list<const void*> others);
+// Microseconds that the row kernels take, by that instruction (mma) or by multiply-adds, as fitted to measurements; infinite
+// where they do not apply.
+template <typename T> double sasaw_rows_cost(const SasawProblem<T>& p, RowsWork work, bool mma);
 
 // Enqueue the operation on the call's stream and return true, or return false when its channel
 // counts are too large for these kernels (the forward: as above). Gradients that are nullptr are skipped.

@@ -298,3 +298,31 @@ def test_gradients_by_estimate(oracle, channels, L, E, n, by_edge):
     d = workloads.sasaw(E=E, n=n, nA=nA, nW2=nW2, nO2=nO2, L=L, N=100)
     compare("sasaw", d, np.float64, oracle, what=f"sasaw gradients {channels} E={E}")
     assert any("sasaw_vjp_" in k for k in _lib.last_kernels()) == by_edge, _lib.last_kernels()
+
+
+@pytest.mark.parametrize("which", ["output", "grad_B", "grad_output"])
+def test_results_off_sixteen_bytes(oracle, which):
+    """f64 results or gradients an element past a 16-byte boundary, which the tensor-core row kernels do not take: sizes that
+    go by rows on their account go by edge then."""
+    import torch
+    # (estimates, by rows on tensor cores and with multiply-adds, by edge: 107, 154, 131; 157, 233, 186 us)
+    nA, nW2, nO2 = (16, 4, 9) if which == "output" else (9, 9, 4)
+    n = 10000 if which == "output" else 1500
+    d = workloads.sasaw(E=60000, n=n, nA=nA, nW2=nW2, nO2=nO2, L=64, N=100)
+    t = to_dev(d, np.float64)
+    idx = ("indices_A", "indices_W_1", "indices_W_2", "indices_output_1", "indices_output_2")
+    t.update(output=t["grad_output"].new_empty(n, nO2, 64), grad_A=t["A"].new_empty(t["A"].shape),
+             grad_B=t["B"].new_empty(t["B"].shape), grad_W=t["W"].new_empty(t["W"].shape))
+    forward = which == "output"
+    first = ("output",) if forward else ("grad_A", "grad_B", "grad_W", "grad_output")
+    name = "mops_cuda_sparse_accumulation_scatter_add_with_weights_" + ("f64" if forward else "vjp_f64")
+    want = run_checker(oracle, "sasaw", d, np.float64)
+    for off in (0, 1):
+        if off:
+            flat = t[which].new_empty(t[which].numel() + 1)
+            t[which] = flat[1:].view(t[which].shape).copy_(t[which])
+        torch.cuda.synchronize()
+        _lib.call(name, [_lib.make_struct(t[k].data_ptr(), t[k].shape) for k in first + ("A", "B", "C", "W") + idx])
+        assert any("sasaw_sum_rows" in k for k in _lib.last_kernels()) == (off == 0), _lib.last_kernels()
+        for k in first[:3]:
+            assert_parity(t[k].cpu().numpy(), want[k], f"sasaw {which} off by {off}/{k}")
