@@ -326,3 +326,29 @@ def test_results_off_sixteen_bytes(oracle, which):
         assert any("sasaw_sum_rows" in k for k in _lib.last_kernels()) == (off == 0), _lib.last_kernels()
         for k in first[:3]:
             assert_parity(t[k].cpu().numpy(), want[k], f"sasaw {which} off by {off}/{k}")
+
+
+# (nA, nW, nO) by what they have compiled in: groups of four m3, a ninth m3, a ninth m1
+@pytest.mark.parametrize("channels,instance", [
+    ((8, 9, 3), (1, 0, 0)), ((1, 16, 2), (1, 0, 0)), ((9, 9, 4), (1, 0, 1)), ((9, 16, 3), (1, 0, 1)),
+    ((4, 9, 8), (2, 0, 0)), ((3, 16, 7), (2, 0, 0)), ((9, 9, 5), (2, 0, 1)), ((9, 12, 8), (2, 0, 1)),
+    ((8, 16, 9), (2, 1, 0)), ((9, 9, 9), (2, 1, 1))])
+@pytest.mark.parametrize("L", [8, 32, 34])
+@pytest.mark.parametrize("rows", ["whole", "cut"])
+def test_every_gradient_kernel(oracle, channels, instance, L, rows):
+    """Every instantiation of the f64 gradients of A and B on the tensor-core instruction, at sizes that are estimated to be
+    faster by it (1.1 times or more). Rows of W without edges and of one to nine between rows longer than a window of 96 edges, which follow one
+    another whole; with one of 300, all are cut into chunks of edges."""
+    nA, nW2, nO2 = channels
+    lengths = np.tile([0, 0, 1, 3, 8, 9, 25, 95, 96, 97, 128, 128, 0, 60, 100], 160)
+    n = len(lengths)  # (2400 rows: whole up to 128 edges)
+    if rows == "cut":
+        lengths[1200] += 300
+    d = workloads.sasaw(E=int(lengths.sum()), n=n, nA=nA, nW2=nW2, nO2=nO2, L=L, N=100)
+    d["indices_W_1"] = np.random.default_rng(10).permutation(np.repeat(np.arange(n), lengths)).astype(np.int32)
+    got = run_library("sasaw", to_dev(d, np.float64))
+    ran = "sasaw_edge_gradients_mma<KS=%d,C9=%d,A9=%d,L=%d>" % (*instance, 32 if nA == 9 and L == 32 else 0)
+    assert ran in _lib.last_kernels(), _lib.last_kernels()
+    want = run_checker(oracle, "sasaw", d, np.float64)
+    for k in want:
+        assert_parity(got[k], want[k], f"sasaw gradients {channels} L={L} {rows}/{k}")
