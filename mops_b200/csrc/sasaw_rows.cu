@@ -658,6 +658,9 @@ __device__ __forceinline__ void for_cuts(const Off* offsets, int64_t rows, int c
 // 60 000 edges, 1000 rows, f64 sums 37 -> 33 us; 250 000 edges, 4099 rows, 64 columns, f32, gradients of A and B, which add
 // up nothing over a row: 195 -> 178 us. (The sums by multiply-adds gain 2 % there, 129 -> 126 us, and lose as much on many
 // rows, 2.07 -> 2.12 ms, to the third way through their loop in the kernel.) From six rows a warp on the last ones matter less than the additional coupling of the cut ones.
+// (Rows are dealt out whole all the same where the sums have no room for what the pieces hand on: with nine components of A
+// 9 x 9 -> 9 channels have room for twelve pieces, 10 gathered channels and 9 outputs for none; and for 5, 7 and 9 to 11 slices of
+// columns, for which two pieces a warp, rounded up, are more than there is ever room for.)
 constexpr int kMostPieces = 64; // of all slices of the columns
 constexpr int kFewRowsPerWarp = 6;
 struct Pieces {
@@ -1028,7 +1031,7 @@ void launch_sums(const Call& call, const RowsShape<T>& s, const int64_t* offsets
                 allow_dynamic_smem(kernel, call.device, smem);
                 const int64_t most = s.g.perm == nullptr ? s.g.rows : std::max(s.g.rows, ceil_div(edges, kLeastChunk));
                 const int64_t blocks = std::min<int64_t>(most, sm_count(call.device));
-                note_kernel_f("sasaw_sum_rows_mma<MA=%d,NINTH=%d,NC=%d,L=%d>", MA, NINTH, NC, LL);
+                note_kernel_f("sasaw_sum_rows_mma<MA=%d,NINTH=%d,NC=%d,L=%d>,PIECES=%d", MA, NINTH, NC, LL, g.piece_room);
                 kernel<<<static_cast<unsigned>(blocks), kMmaWarps * 32, smem, call.stream>>>(g, offsets, starts, out,
                                                                                             depth, when, call.status);
             });

@@ -352,3 +352,38 @@ def test_every_gradient_kernel(oracle, channels, instance, L, rows):
     want = run_checker(oracle, "sasaw", d, np.float64)
     for k in want:
         assert_parity(got[k], want[k], f"sasaw gradients {channels} L={L} {rows}/{k}")
+
+
+@pytest.mark.parametrize("channels", [(9, 9, 9), (4, 4, 5), (16, 4, 9), (9, 4, 1)])
+@pytest.mark.parametrize("L", [16, 34, 64, 96])
+@pytest.mark.parametrize("rows", ["even", "aligned", "long", "gaps", "one"])
+def test_sums_in_pieces(oracle, channels, L, rows):
+    """The f64 sums on the tensor-core instruction where a block has fewer than 72 rows and slices of sixteen columns: its edges in 12, 4, 3
+    or 2 pieces per slice, for which there is room beside the table and the rings. Rows of several pieces, a row as long as a piece or
+    two of them, a block's only row, rows without edges; the same bits in every run. nO = 1: a tile of one output."""
+    nA, nW2, nO2 = channels
+    r = np.random.default_rng(9)
+    lengths = {"even": np.full(300, 61), "aligned": np.full(592, 24), "long": np.where(np.arange(150) % 50 == 7, 900, 40),
+               "gaps": np.where(r.random(1200) < 0.5, 0, 33), "one": np.r_[np.zeros(40), 9000, np.zeros(3)]}[rows].astype(int)
+    n = len(lengths)
+    d = workloads.sasaw(E=int(lengths.sum()), n=n, nA=nA, nW2=nW2, nO2=nO2, L=L, N=100)
+    d["indices_output_1"] = np.repeat(np.arange(n), lengths).astype(np.int32)
+    t = to_dev(d, np.float64)
+
+    def room(kernels):
+        return [int(k.split("PIECES=")[1]) for k in kernels if "sasaw_sum_rows_mma" in k]
+
+    got, kernels = _forward(t)
+    slices = (L + 15) // 16
+    assert room(kernels) and room(kernels)[0] >= 12 // slices * slices, kernels
+    want = run_checker(oracle, "sasaw", d, np.float64)
+    assert_parity(got.cpu().numpy(), want["output"], f"sasaw pieces {channels} {rows} L={L}")
+    for _ in range(3):
+        assert np.array_equal(_forward(t)[0].cpu().numpy(), got.cpu().numpy())
+    if channels == (9, 9, 9) and rows == "even":  # gW, behind a sort
+        d["indices_W_1"] = r.permutation(d["indices_output_1"])
+        gradients = run_library("sasaw", to_dev(d, np.float64))
+        assert room(_lib.last_kernels())[0] >= 12 // slices * slices, _lib.last_kernels()
+        want = run_checker(oracle, "sasaw", d, np.float64)
+        for k in want:
+            assert_parity(gradients[k], want[k], f"sasaw pieces {channels} {rows} L={L}/{k}")
