@@ -1019,21 +1019,23 @@ void launch_sums(const Call& call, const RowsShape<T>& s, const int64_t* offsets
                 constexpr bool NINTH = decltype(ninth)::value, FULL = decltype(full)::value;
                 auto kernel = sasaw_sum_rows_mma<MA, NINTH, NC, FULL, LL>;
                 const size_t table = MmaTable<MA, NINTH>::scalars(s.g.nOut, s.g.pad_c) * sizeof(double);
-                const size_t slots = kMmaWarps * MmaSlot<MA, NC>::kBytes;
-                const int depth = table + 3 * slots <= static_cast<size_t>(max_optin_smem(call.device)) - 2048 ? 3 : 2;
+                constexpr size_t rings = kMmaWarps * kMmaRing<MA, NC>;
+                // (fits with the most channels there are, of every instantiation, on any GPU with 227 KB a block)
+                static_assert(MmaTable<MA, NINTH>::scalars(kWidest, (kWidest + NC - 1) / NC * NC) * sizeof(double) + kMmaWarps * kMmaRing<MA, NC> <=
+                              227 * 1024 - 2048);
                 // (behind the rings: what pieces of rows hand on)
                 const size_t head = static_cast<size_t>(s.g.nOut) * kMmaColumns * sizeof(double);
-                const size_t room = (static_cast<size_t>(max_optin_smem(call.device)) - 2048 - table - depth * slots) / head;
+                const size_t room = (static_cast<size_t>(max_optin_smem(call.device)) - 2048 - table - rings) / head;
                 RowsArgs<T> g = s.g;
-                g.piece_at = static_cast<int>(table + depth * slots);
+                g.piece_at = static_cast<int>(table + rings);
                 g.piece_room = static_cast<int>(std::min<size_t>(room, 2 * kMmaWarps));
-                const size_t smem = table + depth * slots + g.piece_room * head;
+                const size_t smem = table + rings + g.piece_room * head;
                 allow_dynamic_smem(kernel, call.device, smem);
                 const int64_t most = s.g.perm == nullptr ? s.g.rows : std::max(s.g.rows, ceil_div(edges, kLeastChunk));
                 const int64_t blocks = std::min<int64_t>(most, sm_count(call.device));
                 note_kernel_f("sasaw_sum_rows_mma<MA=%d,NINTH=%d,NC=%d,L=%d>,PIECES=%d", MA, NINTH, NC, LL, g.piece_room);
                 kernel<<<static_cast<unsigned>(blocks), kMmaWarps * 32, smem, call.stream>>>(g, offsets, starts, out,
-                                                                                            depth, when, call.status);
+                                                                                            when, call.status);
             });
             MOPS_CUDA_OK(cudaGetLastError());
             return;

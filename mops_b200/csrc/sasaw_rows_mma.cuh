@@ -26,6 +26,7 @@
 constexpr int kMmaWarps = 12;
 constexpr int kMmaColumns = 16; // of a warp
 constexpr int kMmaStep = 4;     // edges
+constexpr int kMmaDepth = 3;    // steps of a warp's ring
 
 // One step's operands: for every edge NC rows of sixteen columns and B's (an odd multiple of 32 bytes apart, so that
 // the 16-byte loads of eight lanes, two pieces of four edges, meet no bank twice), then the A rows.
@@ -36,12 +37,13 @@ template <int MA, int NC> struct MmaSlot {
     static constexpr int kARow = MA == 1 ? 96 : 160; // (four lanes' edges at 8-byte loads: other banks)
     static constexpr int kBytes = kA + kMmaStep * kARow;
 };
+template <int MA, int NC> constexpr int kMmaRing = kMmaDepth * MmaSlot<MA, NC>::kBytes;
 
 // Fragments of the coupling: [tile of eight outputs][c][s][lane], s = 2 m + j the components 8 m + 2 q + j of A and
 // behind them the ninth. A last tile of one output holds it for all n.
 template <int MA, bool NINTH> struct MmaTable {
     static constexpr int S = 2 * MA + (NINTH ? 1 : 0);
-    static __host__ __device__ size_t scalars(int n_out, int pad_c) {
+    static constexpr __host__ __device__ size_t scalars(int n_out, int pad_c) {
         return static_cast<size_t>((n_out + 7) / 8) * pad_c * S * 32;
     }
     static __device__ void fill(double* table, const double* __restrict__ D, int n_out, int pad_c, int na) {
@@ -60,7 +62,7 @@ template <int MA, bool NINTH> struct MmaTable {
 template <int MA, bool NINTH, int NC, bool FULL, int LL, typename Off, Cut CUT>
 __device__ __forceinline__ void mma_sum_rows(const RowsArgs<double>& g, const Off* __restrict__ offsets,
                                              double* __restrict__ out, const Part<CUT>& part, int b0,
-                                             const double* table, unsigned char* ring, int depth, int lane,
+                                             const double* table, unsigned char* ring, int lane,
                                              const Status& st) {
     constexpr int S = MmaTable<MA, NINTH>::S;
     using Slot = MmaSlot<MA, NC>;
@@ -127,14 +129,13 @@ __device__ __forceinline__ void mma_sum_rows(const RowsArgs<double>& g, const Of
             cp_async_commit();
             ahead++;
         };
-        const int ring_bytes = depth * Slot::kBytes;
         if (steps > 0) {
             __syncwarp(); // (the ring's last readers)
 #pragma unroll 1
-            for (int i = 0; i < depth - 1; i++) start(i * Slot::kBytes);
+            for (int i = 0; i < kMmaDepth - 1; i++) start(i * Slot::kBytes);
         }
         // `slot`: of step `now`, whose copies have arrived; before the first one the last of the ring
-        int now = -1, slot = (depth - 1) * Slot::kBytes;
+        int now = -1, slot = (kMmaDepth - 1) * Slot::kBytes;
 
         int lo = p_lo;
         for (int64_t row = row_lo; row < row_hi; row++) {
@@ -164,14 +165,11 @@ __device__ __forceinline__ void mma_sum_rows(const RowsArgs<double>& g, const Of
                     acc9[c][t] = 0;
                 }
             auto advance = [&] {
-                if (depth == 3)
-                    cp_async_wait<1>();
-                else
-                    cp_async_wait<0>();
+                cp_async_wait<kMmaDepth - 2>();
                 __syncwarp();
                 start(slot);
                 slot += Slot::kBytes;
-                if (slot == ring_bytes) slot = 0;
+                if (slot == kMmaRing<MA, NC>) slot = 0;
                 now++;
             };
             // The row's edges of step `now`: all four, or (SOME) those for which `live`.
@@ -304,22 +302,22 @@ __device__ __forceinline__ void for_slices(int parts, int slices, int* counter, 
 template <int MA, bool NINTH, int NC, bool FULL, int LL>
 __global__ void __launch_bounds__(kMmaWarps * 32, 1)
 sasaw_sum_rows_mma(const __grid_constant__ RowsArgs<double> g, const int64_t* __restrict__ offsets,
-                   const int32_t* __restrict__ starts, double* __restrict__ out, int depth, RowsRun run, Status st) {
+                   const int32_t* __restrict__ starts, double* __restrict__ out, RowsRun run, Status st) {
     if (run != kAlways && saw_unsorted(st) != (run == kIfUnsorted)) return;
     __shared__ int counter;
     extern __shared__ __align__(128) unsigned char smem[];
     const int warp = __shfl_sync(kFullMask, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     double* table = reinterpret_cast<double*>(smem);
-    const int ring_bytes = depth * MmaSlot<MA, NC>::kBytes;
-    unsigned char* ring = smem + MmaTable<MA, NINTH>::scalars(g.nOut, g.pad_c) * sizeof(double) + warp * ring_bytes;
+    constexpr int kRing = kMmaRing<MA, NC>;
+    unsigned char* ring = smem + MmaTable<MA, NINTH>::scalars(g.nOut, g.pad_c) * sizeof(double) + warp * kRing;
     if (threadIdx.x == 0) counter = 0;
     MmaTable<MA, NINTH>::fill(table, g.D, g.nOut, g.pad_c, g.pad_a);
-    for (int x = lane * 16; x < ring_bytes; x += 512) // (components of A beyond nA stay zero)
+    for (int x = lane * 16; x < kRing; x += 512) // (components of A beyond nA stay zero)
         *reinterpret_cast<uint4*>(ring + x) = make_uint4(0, 0, 0, 0);
     __syncthreads();
     const int slices = (g.L + kMmaColumns - 1) / kMmaColumns;
     auto sum = [&](const auto* at, const auto& part, int slice) {
-        mma_sum_rows<MA, NINTH, NC, FULL, LL>(g, at, out, part, slice * kMmaColumns, table, ring, depth, lane, st);
+        mma_sum_rows<MA, NINTH, NC, FULL, LL>(g, at, out, part, slice * kMmaColumns, table, ring, lane, st);
     };
     __shared__ int64_t heads[kMostPieces];
     auto rows = [&](const auto* at) {
