@@ -2478,7 +2478,8 @@ template <typename T> SasawProblem<T> rows_problem(const Problem<T>& p) {
     return {p.A, p.B, p.C, p.W, p.M1, p.Jw, p.M2, p.Io, p.M3, p.E, p.N, p.nW0, p.nA, p.nW1, p.nO1, p.L};
 }
 
-// The row kernels (sasaw_rows.cu) or the ones here, by estimates of their time, fitted to the same 750 shapes
+// The row kernels (sasaw_rows.cu) or the ones here, by estimates of their time; where the former use the FP64 tensor-core
+// instruction by quad_cost, unsorted_cost and gradients_cost below, otherwise by formulas fitted to the same 750 shapes
 // (sasaw_rows_cost) in every direction. The estimates miss by a third in one of ten, so the family that is
 // usually the faster one gives way only where the other is estimated to be so by kMargin. Of 3000 calls (those
 // shapes, forward and gradients, waiting and not) 16 % then take more than 1.07 and 5 % more than 1.25 times

@@ -17,7 +17,7 @@
 // done once for each of its rows, and every edge's results are stored by its own. Windows of 96 edges bound the
 // shared memory of gA; the columns of a window come one slice after the other without a gap in the copies.
 //
-// What bounds it: latency at two warps per scheduler (254 registers) and issue slots (34 %), FP64 pipes 35 %. 9 x 9 x 9
+// What bounds it: latency at two warps per scheduler (255 registers; 228 instructions per edge, issue slots 33 %, FP64 pipes 33 %). 9 x 9 x 9
 // channels, 32 columns, against the multiply-adds of sasaw_rows.cu: 60 000 edges 66 -> 52 us, 4.2 10^6 edges with
 // tables of 19 MB 2.53 -> 2.33 ms; gathered tables beyond L2 stay there (gradients_shape_by_mma). gA added up in
 // global memory instead: 3.0 ms; with the hint to bring 256 bytes into L2: slower from 38 MB on.

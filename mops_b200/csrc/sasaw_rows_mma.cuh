@@ -11,15 +11,15 @@
 // DMMA, with m1 = 2q and m1 = 2q + 1 as two contracted groups of four.
 //
 // A warp has sixteen columns of a row: 108 registers of sums for 9 x 9 channels, so that twelve warps
-// fit an SM. Its operands come through a ring of asynchronous copies, three steps deep, laid out without bank
+// fit an SM (168 registers, of which 9 x 9 channels spill 36 to 140 bytes and no other channels any). Its operands come through a ring of asynchronous copies, three steps deep, laid out without bank
 // conflicts. (Loaded straight into registers, which needs no ring, the same loads touch four lines per eight
-// lanes, and the L1 pipe was 83 % busy: 1.60 against 1.04 ms.) The steps run along the positions whatever rows they belong to: one that a row's end cuts is
+// lanes, and the L1 pipe was 83 % busy: 1.60 against 1.04 ms in the same run.) The steps run along the positions whatever rows they belong to: one that a row's end cuts is
 // multiplied once for each of its rows, the other edges as zeros.
 //
-// What bounds it: the FP64 pipe (36 DMMA, 36 DFMA and 36 DMUL for four edges and 32 columns, 60 % busy), latency
-// at three warps per scheduler. 9 x 9 x 9 channels, 32 columns, against the multiply-adds of sasaw_rows.cu:
-// 4.2 10^6 edges forward 1.65 -> 1.27 ms (tables that fit L2: 1.47 -> 1.04), 1.2 10^6 609 -> 432 us; 16 x 9 -> 9
-// channels, 16 columns, 3.9 10^5 edges 320 -> 151 us.
+// What bounds it: the FP64 pipe (36 DMMA, 36 DFMA and 36 DMUL for four edges and 32 columns, 64 % busy), latency
+// at three warps per scheduler; 107 instructions per edge. 9 x 9 x 9 channels, 32 columns, against the multiply-adds of
+// sasaw_rows.cu: 4.2 10^6 edges forward 1.65 -> 1.16 to 1.27 ms (tables that fit L2: 1.47 -> 0.99), 1.2 10^6, 60 per row,
+// 609 -> 377 us; 16 x 9 -> 9 channels, 16 columns, 3.9 10^5 edges 320 -> 144 to 160 us.
 #ifndef MOPS_B200_SASAW_ROWS_MMA_CUH
 #define MOPS_B200_SASAW_ROWS_MMA_CUH
 
