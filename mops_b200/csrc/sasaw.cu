@@ -2525,12 +2525,13 @@ template <typename T> double quad_cost(const Problem<T>& p) {
            1e-2 * c.entry * N + 1e-6 * (c.result * n * p.nO1 * p.L + c.value * E * p.nW1 * p.L) +
            0.1 * c.few * few * (1 + 5e-3 * quad);
 }
-// With short rows the coupling, applied per row, is nearly all of the work of the row sums: of 1400 shapes the quad kernel
-// is the faster one in 221, most of them with 1 to 8 edges per row and wide channels (16 x 9 -> 9, 32 columns, 4 10^5 edges,
-// 2 per row: 0.75 against 1.35 ms by rows). By these estimates 2 % of the shapes take more than 1.1 times the better kernel's time.
+// With short rows the coupling, applied per row, is nearly all of the work of the row sums: of 2281 shapes the quad kernel
+// is the faster one in 200, most of them with 1 to 8 edges per row and wide channels (16 x 9 -> 9, 32 columns, 4 10^5 edges,
+// 2 per row: 0.75 against 1.35 ms by rows). By these estimates 1.5 % of the shapes take more than 1.1 times the better kernel's
+// time; 4 shapes go by edge that are more than 1.1 times as fast by rows.
 template <typename T> bool sorted_by_rows(const Problem<T>& p, const T* O) {
     if (p.E >= p.nW0 && sasaw_rows_by_mma(rows_problem(p), RowsWork::kSorted, {O}))
-        return sasaw_rows_cost(rows_problem(p), RowsWork::kSorted, true) < 0.95 * quad_cost(p);
+        return sasaw_rows_cost(rows_problem(p), RowsWork::kSorted, true) < quad_cost(p);
     const EdgeCost cost = sizeof(T) == 4 ? EdgeCost{33.2, 4.1, 0, 342, 32.1, 2.02, 91.9, 720}
                           : p.L % 2 == 0 ? EdgeCost{46.2, 4.04, 0.0252, 403, 78.6, 4.15, 28, 568}
                                          : EdgeCost{37.7, 7.7, 0, 337, 0, 10.8, 45.7, 998};

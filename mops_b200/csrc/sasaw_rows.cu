@@ -1097,27 +1097,29 @@ bool sasaw_rows_by_mma(const SasawProblem<T>& p, RowsWork work, std::initializer
     return work == RowsWork::kGradients ? gradients_shape_by_mma(p.nA, p.nO, p.L, p.rows) : sums_shape_by_mma(p.nA, p.L);
 }
 
-// The sums on the FP64 tensor-core instruction: microseconds, fitted to 1400 shapes with a sorted index and 450 without, 1 to 100
-// edges per row, up to 2 10^6 edges and 1000 coupling entries; nine in ten estimates are within a fifth. Operations of the steps
-// (one more for rows whose ends cut one) and of the coupling (half as much again where the last pass has fewer channels), what
-// each of them costs beside, the coupling's table, results read again by later passes, the sort, a row's steps one after the
+// The sums on the FP64 tensor-core instruction: microseconds, fitted to 1400 shapes with a sorted index and 450 without, and where the
+// last were off to 3700 others, 1 to 200 edges per row, up to 2 10^6 edges and 1000 coupling entries. Operations of the steps (one
+// more for rows whose ends cut one; those of channels that the last pass does not have apart) and of the coupling, each by whether A
+// has one tile, one and a ninth component, or two; what a step and a result cost beside; what the coupling costs more where the
+// last pass has fewer channels; the coupling's table; results read again by later passes; the sort; a row's steps one after the
 // other where rows are few.
 inline double sums_mma_cost(bool sorted, int64_t edges, int64_t rows, int nA, int nW, int nO, int L, int64_t N) {
     struct Cost {
-        double call, operation, step, couple, result, table, again, edge, few; // in 10^-6 but the first one
+        double call, operation[3], missing, step, couple[3], part, result, table, again, edge, few; // in 10^-6 but the first one
     };
-    constexpr Cost with_order{37.6, 1.32, 84, 0.596, 117, 4.4, 1.42, 0, 13900};
-    constexpr Cost without{62.7, 1.31, 46, 0.771, 52, 4.98, 1.03, 74, 12900};
+    constexpr Cost with_order{37.6, {1.32, 1.32, 1.12}, 1.2, 84, {0.596, 0.596, 0.507}, 0.28, 117, 4.4, 1.42, 0, 13900};
+    constexpr Cost without{62.7, {1.31, 1.31, 1.31}, 1.31, 46, {0.771, 0.771, 0.771}, 0.386, 52, 4.98, 1.03, 74, 12900};
     const Cost& c = sorted ? with_order : without;
-    const int na = pad_a(nA), nc = chunk_c(na, nW), ma = na == 16 ? 2 : 1, ninth = nA == 9 ? 1 : 0;
+    const int na = pad_a(nA), nc = chunk_c(na, nW), ma = na == 16 ? 2 : 1, ninth = nA == 9 ? 1 : 0, kind = ma == 2 ? 2 : ninth;
     const double E = static_cast<double>(edges), n = static_cast<double>(rows);
     const double passes = static_cast<double>(ceil_div(nW, nc)), columns = static_cast<double>(ceil_div(L, 16));
     const double steps = (E / 4 + 0.75 * n * (1 - std::exp(-E / n))) * columns * passes, results = n * columns * passes;
-    const double operations = nc * 2 * (ma * 16 + 2 * ninth + 2), part = nW % nc != 0 ? 1.5 : 1;
-    const double couple = part * (2 * ma + ninth) * nc * 32 * static_cast<double>(ceil_div(nO, 8));
+    const double channel = 2 * (ma * 16 + 2 * ninth + 2), channels = nW / passes;
+    const double couple = (2 * ma + ninth) * nc * 32 * static_cast<double>(ceil_div(nO, 8));
     const double table = static_cast<double>(ceil_div(nO, kTableOut)) * kTableOut * na * passes * nc * static_cast<double>(N);
     const double few = std::max(0.0, 1 - n * columns / 1776) * E / n * passes * nc * ma;
-    return c.call + 1e-6 * (steps * (c.operation * operations + c.step) + results * (c.couple * couple + c.result) +
+    return c.call + 1e-6 * (steps * (channel * (c.operation[kind] * channels + c.missing * (nc - channels)) + c.step) +
+                            results * (couple * (c.couple[kind] + (nW % nc != 0 ? c.part : 0)) + c.result) +
                             c.table * table + c.again * n * nO * L * (passes - 1) + c.edge * E + c.few * few);
 }
 

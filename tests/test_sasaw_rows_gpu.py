@@ -387,3 +387,19 @@ def test_sums_in_pieces(oracle, channels, L, rows):
         want = run_checker(oracle, "sasaw", d, np.float64)
         for k in want:
             assert_parity(gradients[k], want[k], f"sasaw pieces {channels} {rows} L={L}/{k}")
+
+
+# (by rows and by edge: 212 and 324, 100 and 146, 164 and 238 us; 755 and 458 us)
+@pytest.mark.parametrize("channels,L,E,n,N,by_edge", [
+    ((13, 9, 9), 64, 157122, 4155, 33, False), ((14, 9, 9), 66, 21257, 2103, 282, False),
+    ((16, 16, 9), 64, 33079, 2610, 461, False), ((16, 9, 9), 52, 158976, 45932, 47, True)])
+def test_wide_rows(oracle, channels, L, E, n, N, by_edge):
+    """f64, sorted index, ten and more components of A: by rows unless these are short."""
+    nA, nW2, nO2 = channels
+    d = workloads.sasaw(E=E, n=n, nA=nA, nW2=nW2, nO2=nO2, L=L, N=N)
+    got, kernels = _forward(to_dev(d, np.float64))
+    assert any("sasaw_fwd_quad" in k for k in kernels) == by_edge, kernels
+    assert any("sasaw_sum_rows_mma" in k for k in kernels) != by_edge, kernels
+    want = oracle.sasaw(d["A"], d["B"], d["C"], d["W"], d["indices_A"], d["indices_W_1"], d["indices_W_2"],
+                        d["indices_output_1"], d["indices_output_2"], nO2)
+    assert_parity(got.cpu().numpy(), want, f"sasaw wide rows {channels}")
