@@ -2539,22 +2539,22 @@ template <typename T> bool sorted_by_rows(const Problem<T>& p, const T* O) {
     if (sizeof(T) == 8 && p.L % 2 == 0) us *= 8 / quad_warps(p);
     return p.E >= p.nW0 && sasaw_rows_cost(rows_problem(p), RowsWork::kSorted, false) < us * rows_margin(p);
 }
-// The kernel for an unsorted index beside them: microseconds, fitted to the same 450 shapes. The last term is the order of a
+// The kernel for an unsorted index beside them: microseconds, fitted to the same 929 shapes. The last term is the order of a
 // cell's coupling entries, made one by one.
 template <typename T> double unsorted_cost(const Problem<T>& p) {
     const double E = static_cast<double>(p.E), n = static_cast<double>(p.nW0), N = static_cast<double>(p.N);
     const double columns = static_cast<double>(ceil_div(p.L, 32)), tiles = static_cast<double>(ceil_div(p.nW1, 4));
-    return 59 + E * (3.44e-6 * p.nO1 * tiles * static_cast<double>(ceil_div(p.nA, 4)) +
-                     columns * (5.01e-5 * tiles * static_cast<double>(ceil_div(p.nO1, 8)) + 2.9e-4) +
-                     1e-6 * p.L * (1.06 * p.nO1 + 0.546 * p.nW1)) +
-           6.71e-3 * N + 2.88e-6 * n * p.nO1 * p.L + 2.14e-3 * N * N / (p.nW1 * p.nO1);
+    return 60 + E * (1.51e-6 * p.nO1 * tiles * static_cast<double>(ceil_div(p.nA, 4)) +
+                     columns * (1.33e-4 * tiles + 2.26e-4) + 1.55e-6 * p.nO1 * p.L) +
+           5.5e-3 * N + 2.39e-6 * n * p.nO1 * p.L + 2.33e-3 * N * N / (p.nW1 * p.nO1);
 }
-// Rows of an unsorted index are cut where they are long, and the sort counts: of 450 shapes the kernel by edge is the faster
-// one in a third (16 channels each, 64 columns, 7 10^4 edges, 1.3 per row: 0.46 against 1.61 ms by rows). By these estimates 6 %
-// take more than 1.1 times the better kernel's time.
+// Rows of an unsorted index are cut where they are long, and the sort counts: of 929 shapes the kernel by edge is the faster
+// one in a third (16 channels each, 64 columns, 7 10^4 edges, 1.3 per row: 0.46 against 1.61 ms by rows). By these estimates 9 %
+// take more than 1.1 times the better kernel's time, nearly all of them calls of 50 to 100 us; 4 shapes go by edge that are
+// more than 1.1 times as fast by rows.
 template <typename T> bool unsorted_by_rows(const Problem<T>& p, const T* O) {
     if (sasaw_rows_by_mma(rows_problem(p), RowsWork::kUnsorted, {O}))
-        return sasaw_rows_cost(rows_problem(p), RowsWork::kUnsorted, true) < 0.95 * unsorted_cost(p);
+        return sasaw_rows_cost(rows_problem(p), RowsWork::kUnsorted, true) < 1.03 * unsorted_cost(p);
     const EdgeCost cost = sizeof(T) == 4 ? EdgeCost{25.4, 3.54, 0.0224, 413, 18.5, 2.09, 0, 0}
                           : p.L % 2 == 0 ? EdgeCost{39.4, 6.25, 0, 439, 49.2, 2.39, 0, 0}
                                          : EdgeCost{33.7, 1.73, 0, 1110, 23.6, 106, 0, 0};

@@ -1097,8 +1097,8 @@ bool sasaw_rows_by_mma(const SasawProblem<T>& p, RowsWork work, std::initializer
     return work == RowsWork::kGradients ? gradients_shape_by_mma(p.nA, p.nO, p.L, p.rows) : sums_shape_by_mma(p.nA, p.L);
 }
 
-// The sums on the FP64 tensor-core instruction: microseconds, fitted to 1400 shapes with a sorted index and 450 without, and where the
-// last were off to 3700 others, 1 to 200 edges per row, up to 2 10^6 edges and 1000 coupling entries. Operations of the steps (one
+// The sums on the FP64 tensor-core instruction: microseconds, fitted to 1400 shapes with a sorted index (and where they
+// were off to 2281 others) and to 929 without, 1 to 200 edges per row, up to 2 10^6 edges and 1000 coupling entries. Operations of the steps (one
 // more for rows whose ends cut one; those of channels that the last pass does not have apart) and of the coupling, each by whether A
 // has one tile, one and a ninth component, or two; what a step and a result cost beside; what the coupling costs more where the
 // last pass has fewer channels; the coupling's table; results read again by later passes; the sort; a row's steps one after the
@@ -1108,7 +1108,7 @@ inline double sums_mma_cost(bool sorted, int64_t edges, int64_t rows, int nA, in
         double call, operation[3], missing, step, couple[3], part, result, table, again, edge, few; // in 10^-6 but the first one
     };
     constexpr Cost with_order{37.6, {1.32, 1.32, 1.12}, 1.2, 84, {0.596, 0.596, 0.507}, 0.28, 117, 4.4, 1.42, 0, 13900};
-    constexpr Cost without{62.7, {1.31, 1.31, 1.31}, 1.31, 46, {0.771, 0.771, 0.771}, 0.386, 52, 4.98, 1.03, 74, 12900};
+    constexpr Cost without{60.2, {1.82, 2.23, 1.4}, 1.1, 39, {0.53, 0.52, 0.46}, 0.29, 152, 4.86, 2.6, 21.5, 1100};
     const Cost& c = sorted ? with_order : without;
     const int na = pad_a(nA), nc = chunk_c(na, nW), ma = na == 16 ? 2 : 1, ninth = nA == 9 ? 1 : 0, kind = ma == 2 ? 2 : ninth;
     const double E = static_cast<double>(edges), n = static_cast<double>(rows);

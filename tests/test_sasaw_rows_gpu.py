@@ -403,3 +403,18 @@ def test_wide_rows(oracle, channels, L, E, n, N, by_edge):
     want = oracle.sasaw(d["A"], d["B"], d["C"], d["W"], d["indices_A"], d["indices_W_1"], d["indices_W_2"],
                         d["indices_output_1"], d["indices_output_2"], nO2)
     assert_parity(got.cpu().numpy(), want, f"sasaw wide rows {channels}")
+
+
+# (by rows and by edge: 63 and 101, 62 and 93, 63 and 95 us)
+@pytest.mark.parametrize("channels,L,E,n,N", [((9, 9, 4), 32, 9595, 50, 470), ((16, 4, 16), 32, 11901, 74, 438),
+                                              ((16, 4, 9), 16, 1441, 9, 528)])
+def test_few_edges_unsorted(oracle, channels, L, E, n, N):
+    """f64, no order in the index, few long rows: sorted, and then by rows."""
+    nA, nW2, nO2 = channels
+    d = workloads.sasaw(E=E, n=n, nA=nA, nW2=nW2, nO2=nO2, L=L, N=N)
+    d["indices_output_1"] = np.random.default_rng(7).permutation(d["indices_output_1"])
+    got, kernels = _forward(to_dev(d, np.float64))
+    assert "sasaw_sum_rows_mma" in kernels[-1] and (len(kernels) == 2 or "quad" in kernels[0]), kernels
+    want = oracle.sasaw(d["A"], d["B"], d["C"], d["W"], d["indices_A"], d["indices_W_1"], d["indices_W_2"],
+                        d["indices_output_1"], d["indices_output_2"], nO2)
+    assert_parity(got.cpu().numpy(), want, f"sasaw few edges, unsorted {channels}")
