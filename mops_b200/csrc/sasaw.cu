@@ -2572,19 +2572,21 @@ template <typename T> bool gradients_by_mma(const Problem<T>& p) {
 // The gradients by edge beside the row kernels on the FP64 tensor-core instruction: microseconds, fitted to 652 shapes of rows of 1
 // to 200 edges, 60 to 60 000 of them, nine in ten within a fifth; `us`, as for the other row kernels, of the third family. The kernel
 // with compiled-in widths gives a row of the output to a warp, whose edges come one after the other where there are few rows (66
-// rows of 200 edges: 830 us, 105 by rows); rows of unlike lengths, which the estimate does not know, cost it more: 1.05. By these
-// estimates 4 % of 600 other shapes take more than 1.1 times the better family's time.
+// rows of 200 edges: 830 us, 105 by rows); rows of unlike lengths, which the estimate does not know, cost it more, and an index without
+// order sends its edges to a third kernel behind it: 1.1. By these estimates, each with its factor, 5 % of 1677
+// shapes take more than 1.1 times the better family's time, most of them calls of less than 100 us. The order of a cell's coupling entries
+// counts as seven tenths of what it costs a call without a plan, which keeps it.
 template <typename T> double gradients_cost(const Problem<T>& p, double us) {
     const double E = static_cast<double>(p.E), n = static_cast<double>(p.nW0), N = static_cast<double>(p.N);
     const double columns = static_cast<double>(ceil_div(p.L, 32)), cells = static_cast<double>(p.nW1) * p.nO1;
     if (quad_gradients(p)) {
         const double few = std::max(0.0, 1 - n / 1184) * E / n; // (eight warps per SM)
-        return 1.05 * (46.6 + columns * (1.235e-3 * E + 1.6e-3 * n + 2.24 * few) + 0.0215 * N + 6.2e-5 * n * p.L);
+        return 1.1 * (46.6 + columns * (1.235e-3 * E + 1.6e-3 * n + 2.24 * few) + 0.0215 * N + 6.2e-5 * n * p.L);
     }
-    if (!gradients_by_mma(p)) return 1.2 * us;
+    if (!gradients_by_mma(p)) return 1.4 * us;
     const double w = static_cast<double>(ceil_div(p.nW1, 4)), o = static_cast<double>(ceil_div(p.nO1, 4));
-    return 0.95 * (43.2 + E * (1e-4 * columns * (0.834 * w * o + 0.925 * w + 5.08) + 1e-6 * p.L * (0.536 * p.nW1 + 0.474 * p.nO1)) +
-                   2.52e-6 * n * p.nW1 * p.L + N * (2.37e-3 * N + 7.2e-7 * E) / cells);
+    return 1.04 * (43.2 + E * (1e-4 * columns * (0.834 * w * o + 0.925 * w + 5.08) + 1e-6 * p.L * (0.536 * p.nW1 + 0.474 * p.nO1)) +
+                   2.52e-6 * n * p.nW1 * p.L + N * (1.66e-3 * N + 5.0e-7 * E) / cells);
 }
 // The f64 gradients have three kernels by edge. The one with compiled-in widths adds to gW from all over it,
 // which costs more where W and gW are larger than L2 (4.2 10^6 edges, 151 MB each: 5.70 against 4.85 ms),

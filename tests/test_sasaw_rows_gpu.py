@@ -418,3 +418,14 @@ def test_few_edges_unsorted(oracle, channels, L, E, n, N):
     want = oracle.sasaw(d["A"], d["B"], d["C"], d["W"], d["indices_A"], d["indices_W_1"], d["indices_W_2"],
                         d["indices_output_1"], d["indices_output_2"], nO2)
     assert_parity(got.cpu().numpy(), want, f"sasaw few edges, unsorted {channels}")
+
+
+# (by rows and by edge: 245 and 367, 130 and 152, 105 and 124 us)
+@pytest.mark.parametrize("channels,L,E,n,N", [((9, 13, 9), 16, 35378, 29742, 232), ((9, 16, 4), 32, 65925, 5626, 147),
+                                              ((4, 9, 9), 44, 17856, 399, 113)])
+def test_gradients_near_the_line(oracle, channels, L, E, n, N):
+    """f64 gradients that are a little faster by rows, beside each of the kernels by edge that are not compiled for the widths."""
+    nA, nW2, nO2 = channels
+    d = workloads.sasaw(E=E, n=n, nA=nA, nW2=nW2, nO2=nO2, L=L, N=N)
+    compare("sasaw", d, np.float64, oracle, what=f"sasaw gradients {channels} E={E}")
+    assert any("sasaw_edge_gradients_mma" in k for k in _lib.last_kernels()), _lib.last_kernels()
